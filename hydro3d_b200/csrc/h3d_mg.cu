@@ -1164,23 +1164,21 @@ int check_block_host_dims(h3d_mg* h, const h3d_block_desc& d) {
 // staging and the padded layout.  stage_out writes back whole host planes, so
 // it is only used in calls that staged the same host array in (the planes'
 // other cells then round-trip unchanged).
-int ensure_stage(h3d_mg* h) {
-  if (h->stage[0]) return H3D_OK;
+int ensure_stage(h3d_mg* h, int f) {
+  if (h->stage[f]) return H3D_OK;
   size_t n = 0;
   h->stage_off.clear();
   for (const auto& d : h->blocks) {
     h->stage_off.push_back(n);
     n += (size_t)d.ttc[0] * d.ttc[1] * d.ttc[2];
   }
-  TRY(dalloc(h, &h->stage[0], n));
-  TRY(dalloc(h, &h->stage[1], n));
-  return H3D_OK;
+  return dalloc(h, &h->stage[f], n);
 }
 
 int stage_in(h3d_mg* h, int f, int ib, const double* host, double* dev_level, bool with_ghosts) {
   const h3d_block_desc& d = h->blocks[ib];
   TRY(check_block_host_dims(h, d));
-  TRY(ensure_stage(h));
+  TRY(ensure_stage(h, f));
   const BlkLev& B = h->lev[1].geom.bl[ib];
   double* stg = h->stage[f] + h->stage_off[ib];
   CU(cudaMemcpyAsync(stg, host, (size_t)d.ttc[0] * d.ttc[1] * d.ttc[2] * sizeof(double), cudaMemcpyHostToDevice,
@@ -1203,6 +1201,32 @@ int stage_out(h3d_mg* h, int f, int ib, double* host, double* dev_level, bool wi
   CU(cudaMemcpyAsync(host + z0 * plane, stg + z0 * plane, nzp * plane * sizeof(double), cudaMemcpyDeviceToHost,
                      h->st));
   return H3D_OK;
+}
+
+// One host block array into a resident level-1 field.  The rows of a strided
+// copy are a few hundred bytes, which reach the device at 6 GB/s from pinned
+// host memory (96^3 blocks; 12.4 ms for a solve with its 58 MB initial guess
+// up and its pressure down) where a contiguous copy has the PCIe rate (4.6
+// ms), so the host array moves whole through the staging buffer, unless it is
+// mostly cells the call does not read or no staging memory is left.
+// Downwards the strided copy runs at 40-50 GB/s and stays: through the
+// staging buffer 32 blocks of 80x64x64 took 0.27 ms longer.
+int field_in(h3d_mg* h, const double* host, int ib, double* dev_level, bool with_ghosts) {
+  const h3d_block_desc& d = h->blocks[ib];
+  const BlkLev& B = h->lev[1].geom.bl[ib];
+  const size_t whole = (size_t)d.ttc[0] * d.ttc[1] * d.ttc[2];
+  const size_t need = (size_t)(B.nx + 2) * (B.ny + 2) * (B.nz + 2);
+  if (whole <= 2 * need) {
+    const int rc = ensure_stage(h, 0);
+    if (rc == H3D_OK) return stage_in(h, 0, ib, host, dev_level, with_ghosts);
+    if (rc != H3D_ERR_OOM) return rc;
+    cudaGetLastError();
+  }
+  return copy_field_3d(h, true, dev_level, B, const_cast<double*>(host), d, with_ghosts);
+}
+
+int field_out(h3d_mg* h, double* host, int ib, double* dev_level, bool with_ghosts) {
+  return copy_field_3d(h, false, dev_level, h->lev[1].geom.bl[ib], host, h->blocks[ib], with_ghosts);
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
@@ -2736,7 +2760,7 @@ int h3d_mg_set_density(h3d_mg* h, int32_t ib, const double* dens) {
   if (!h->var) return fail(h, H3D_ERR_ARG, "handle was created with var_coef = 0");
   TRY(check_block_host_dims(h, h->blocks[ib]));
   CU(cudaSetDevice(h->device));
-  TRY(copy_field_3d(h, true, h->lev[1].dens, h->lev[1].geom.bl[ib], const_cast<double*>(dens), h->blocks[ib], true));
+  TRY(field_in(h, dens, ib, h->lev[1].dens, true));
   CU(cudaStreamSynchronize(h->st));
   h->coeffs_ready = false;
   return H3D_OK;
@@ -2788,15 +2812,14 @@ int h3d_mg_upload(h3d_mg* h, int32_t field, int32_t ib, const double* host) {
   if (!h || !host || ib < 0 || ib >= (int)h->blocks.size()) return H3D_ERR_ARG;
   TRY(check_block_host_dims(h, h->blocks[ib]));
   CU(cudaSetDevice(h->device));
-  const BlkLev& B = h->lev[1].geom.bl[ib];
-  if (field == H3D_FIELD_P) TRY(copy_field_3d(h, true, h->p64[h->pc], B, const_cast<double*>(host), h->blocks[ib], true));
-  else if (field == H3D_FIELD_B) TRY(copy_field_3d(h, true, h->b64, B, const_cast<double*>(host), h->blocks[ib], false));
+  if (field == H3D_FIELD_P) TRY(field_in(h, host, ib, h->p64[h->pc], true));
+  else if (field == H3D_FIELD_B) TRY(field_in(h, host, ib, h->b64, false));
   else if (field >= H3D_FIELD_U && field <= H3D_FIELD_WSTAR) {
     TRY(ensure_velocity(h));
-    TRY(copy_field_3d(h, true, velocity_field(h, field), B, const_cast<double*>(host), h->blocks[ib], true));
+    TRY(field_in(h, host, ib, velocity_field(h, field), true));
   } else if (field == H3D_FIELD_PP) {
     TRY(ensure_sip(h));
-    TRY(copy_field_3d(h, true, h->sip_pp, B, const_cast<double*>(host), h->blocks[ib], true));
+    TRY(field_in(h, host, ib, h->sip_pp, true));
   } else
     return H3D_ERR_ARG;
   return H3D_OK;
@@ -2806,15 +2829,14 @@ int h3d_mg_download(h3d_mg* h, int32_t field, int32_t ib, double* host) {
   if (!h || !host || ib < 0 || ib >= (int)h->blocks.size()) return H3D_ERR_ARG;
   TRY(check_block_host_dims(h, h->blocks[ib]));
   CU(cudaSetDevice(h->device));
-  const BlkLev& B = h->lev[1].geom.bl[ib];
-  if (field == H3D_FIELD_P) TRY(copy_field_3d(h, false, h->p64[h->pc], B, host, h->blocks[ib], true));
-  else if (field == H3D_FIELD_B) TRY(copy_field_3d(h, false, h->b64, B, host, h->blocks[ib], false));
+  if (field == H3D_FIELD_P) TRY(field_out(h, host, ib, h->p64[h->pc], true));
+  else if (field == H3D_FIELD_B) TRY(field_out(h, host, ib, h->b64, false));
   else if (field >= H3D_FIELD_U && field <= H3D_FIELD_WSTAR) {
     TRY(ensure_velocity(h));
-    TRY(copy_field_3d(h, false, velocity_field(h, field), B, host, h->blocks[ib], true));
+    TRY(field_out(h, host, ib, velocity_field(h, field), true));
   } else if (field == H3D_FIELD_PP) {
     TRY(ensure_sip(h));
-    TRY(copy_field_3d(h, false, h->sip_pp, B, host, h->blocks[ib], true));
+    TRY(field_out(h, host, ib, h->sip_pp, true));
   } else
     return H3D_ERR_ARG;
   CU(cudaStreamSynchronize(h->st));
@@ -3316,24 +3338,22 @@ int h3d_mg_project(h3d_mg* h, double* const* p, double* const* u, double* const*
   for (int ib = 0; ib < nb; ++ib) {
     const h3d_block_desc& d = h->blocks[ib];
     TRY(check_block_host_dims(h, d));
-    const BlkLev& B = h->lev[1].geom.bl[ib];
-    TRY(copy_field_3d(h, true, h->p64[h->pc], B, p[ib], d, true));
-    TRY(copy_field_3d(h, true, h->vel[0], B, u[ib], d, true));
-    TRY(copy_field_3d(h, true, h->vel[1], B, v[ib], d, true));
-    TRY(copy_field_3d(h, true, h->vel[2], B, w[ib], d, true));
-    TRY(copy_field_3d(h, true, h->vstar[0], B, const_cast<double*>(ustar[ib]), d, true));
-    TRY(copy_field_3d(h, true, h->vstar[1], B, const_cast<double*>(vstar[ib]), d, true));
-    TRY(copy_field_3d(h, true, h->vstar[2], B, const_cast<double*>(wstar[ib]), d, true));
+    TRY(field_in(h, p[ib], ib, h->p64[h->pc], true));
+    TRY(field_in(h, u[ib], ib, h->vel[0], true));
+    TRY(field_in(h, v[ib], ib, h->vel[1], true));
+    TRY(field_in(h, w[ib], ib, h->vel[2], true));
+    TRY(field_in(h, ustar[ib], ib, h->vstar[0], true));
+    TRY(field_in(h, vstar[ib], ib, h->vstar[1], true));
+    TRY(field_in(h, wstar[ib], ib, h->vstar[2], true));
   }
   int rc = h3d_mg_project_resident(h, dt, alfapr, opts, info);
   if (rc != H3D_OK && rc != H3D_ERR_NOT_CONVERGED) return rc;
   for (int ib = 0; ib < nb; ++ib) {
     const h3d_block_desc& d = h->blocks[ib];
-    const BlkLev& B = h->lev[1].geom.bl[ib];
-    TRY(copy_field_3d(h, false, h->p64[h->pc], B, p[ib], d, true));
-    TRY(copy_field_3d(h, false, h->vel[0], B, u[ib], d, true));
-    TRY(copy_field_3d(h, false, h->vel[1], B, v[ib], d, true));
-    TRY(copy_field_3d(h, false, h->vel[2], B, w[ib], d, true));
+    TRY(field_out(h, p[ib], ib, h->p64[h->pc], true));
+    TRY(field_out(h, u[ib], ib, h->vel[0], true));
+    TRY(field_out(h, v[ib], ib, h->vel[1], true));
+    TRY(field_out(h, w[ib], ib, h->vel[2], true));
   }
   CU(cudaStreamSynchronize(h->st));
   return rc;
