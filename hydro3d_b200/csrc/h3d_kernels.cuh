@@ -279,6 +279,20 @@ cudaError_t launch_sip_factor(const BlkLev* bl, int nb, SipArrays a, cudaStream_
 // One sweep of every block on fi with rhs su; partials[4b] = sum |res| of block b.
 cudaError_t launch_sip_sweep(const BlkLev* bl, int nb, SipArrays a, double* fi, const double* su, double* partials,
                              cudaStream_t st);
+// The same by clusters of CTAs, factors and residual in a skewed layout of
+// nz*(nx+ny-1)*ny words a block from offs[block] (h3d_seq.cu).  The sweep's
+// partials: one quadruple per CTA of `interior` (256 cells each).
+struct SipPlan {
+  int ctas = 1;
+  bool one = false, fits = false;
+  int smem_factor = 0, smem_subst = 0;
+};
+SipPlan sip_plan(const std::vector<BlkLev>& bl);
+cudaError_t init_seq_attributes();
+cudaError_t launch_sip_factor_c(const SipPlan& P, const BlkLev* bl, const long long* offs, int nb, SipArrays a,
+                                cudaStream_t st);
+cudaError_t launch_sip_sweep_c(const SipPlan& P, const BlkLev* bl, const long long* offs, CellTab interior,
+                               SipArrays a, double* fi, const double* su, double* partials, cudaStream_t st);
 // a[dst[e]] = a[src[e]].
 cudaError_t launch_gather1(const uint32_t* dst, const uint32_t* src, int64_t n, double* a, cudaStream_t st);
 

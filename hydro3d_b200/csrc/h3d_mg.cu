@@ -202,6 +202,8 @@ struct h3d_mg {
   uint32_t* d_vsrc = nullptr;
   int64_t nvfill = 0;
   double* sip[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};  // SIP factors, res
+  SipPlan sip_plan;                  // sip: in the skewed layout of the cluster kernels where d_sip_off is set
+  long long* d_sip_off = nullptr;    // first word of each block there
   double* sip_pp = nullptr;  // the SIP pressure correction (level-1 layout)
   bool proj = false;        // outer iterations end with p += pp, calvel, calmas
   double proj_dtal = 0.0;   // dt*alfapr
@@ -2408,6 +2410,7 @@ int h3d_mg_destroy(h3d_mg* h) {
   dfree(h->d_vdst);
   dfree(h->d_vsrc);
   for (int q = 0; q < 8; ++q) dfree(h->sip[q]);
+  dfree(h->d_sip_off);
   dfree(h->sip_pp);
   if (h->h_res) cudaFreeHost(h->h_res);
   if (h->st) cudaStreamDestroy(h->st);
@@ -2511,7 +2514,8 @@ int h3d_mg_create(h3d_mg** out, const h3d_mg_desc* desc) {
   if (cudaSetDevice(h->device) != cudaSuccess) return bail(fail(h, H3D_ERR_NO_DEVICE, "cudaSetDevice failed"));
   if (cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking) != cudaSuccess)
     return bail(fail(h, H3D_ERR_CUDA, "stream create failed"));
-  if (init_kernel_attributes() != cudaSuccess || init_kernel_attributes_2() != cudaSuccess)
+  if (init_kernel_attributes() != cudaSuccess || init_kernel_attributes_2() != cudaSuccess ||
+      init_seq_attributes() != cudaSuccess)
     return bail(fail(h, H3D_ERR_CUDA, "kernel attributes"));
   h->lev.resize(h->L + 1);
   for (int g = 1; g <= h->L; ++g) {
@@ -3084,8 +3088,39 @@ static int ensure_sip(h3d_mg* h) {
   if ((int)h->blocks.size() > h->npartials) return fail(h, H3D_ERR_BAD_CONFIG, "SIP: too many blocks");
   if (h->sip_pp) return H3D_OK;
   TRY(ensure_face_table(h));
-  const size_t n = (size_t)h->lev[1].geom.n_elems;
-  for (int q = 0; q < 8; ++q) TRY(dalloc(h, &h->sip[q], n));
+  const LevelGeom& G = h->lev[1].geom;
+  const size_t n = (size_t)G.n_elems;
+  auto alloc_factors = [&](size_t words) -> int {
+    for (int q = 0; q < 8; ++q) {
+      dfree(h->sip[q]);
+      h->sip[q] = nullptr;
+    }
+    for (int q = 0; q < 8; ++q) TRY(dalloc(h, &h->sip[q], words));
+    return H3D_OK;
+  };
+  // the skewed layout of the cluster kernels, up to twice a level, where the
+  // blocks' cross-sections and the device's memory allow it
+  h->sip_plan = sip_plan(G.bl);
+  int rc = H3D_ERR_OOM;
+  if (h->sip_plan.fits) {
+    std::vector<long long> off;
+    long long words = 0;
+    for (const auto& B : G.bl) {
+      off.push_back(words);
+      words += ((long long)B.nz * (B.nx + B.ny - 1) * B.ny + 15) / 16 * 16;
+    }
+    rc = alloc_factors((size_t)words);
+    if (rc == H3D_OK && !h->d_sip_off) {
+      TRY(dalloc(h, &h->d_sip_off, off.size()));
+      CU(cudaMemcpy(h->d_sip_off, off.data(), off.size() * sizeof(long long), cudaMemcpyHostToDevice));
+    }
+  }
+  if (rc == H3D_ERR_OOM) {
+    cudaGetLastError();
+    h->sip_plan.fits = false;
+    rc = alloc_factors(n);
+  }
+  if (rc != H3D_OK) return rc;
   TRY(dalloc(h, &h->sip_pp, n));
   return H3D_OK;
 }
@@ -3099,18 +3134,23 @@ static int sip_run(h3d_mg* h, int nswp, int* nsweep, double* resab_last) {
   Level& V = h->lev[1];
   const int nb = (int)V.geom.bl.size();
   SipArrays a{h->sip[0], h->sip[1], h->sip[2], h->sip[3], h->sip[4], h->sip[5], h->sip[6], h->sip[7]};
-  CU(launch_sip_factor(V.d_bl, nb, a, h->st));
+  const bool clusters = h->sip_plan.fits;
+  const CellTab interior{V.d_cta_int, nb, V.ncta_int};
+  if (clusters) CU(launch_sip_factor_c(h->sip_plan, V.d_bl, h->d_sip_off, nb, a, h->st));
+  else CU(launch_sip_factor(V.d_bl, nb, a, h->st));
   h->kernels += 1;
   const double small = 1e-20;
   double relast = 0.0, res1 = 0.0, resab = 0.0;
   int ns;
   for (ns = 1; ns <= nswp; ++ns) {
-    CU(launch_sip_sweep(V.d_bl, nb, a, h->sip_pp, h->b64, h->partials, h->st));
+    if (clusters)
+      CU(launch_sip_sweep_c(h->sip_plan, V.d_bl, h->d_sip_off, interior, a, h->sip_pp, h->b64, h->partials, h->st));
+    else CU(launch_sip_sweep(V.d_bl, nb, a, h->sip_pp, h->b64, h->partials, h->st));
     CU(launch_gather1(h->d_vdst, h->d_vsrc, h->nvfill, h->sip_pp, h->st));
-    CU(launch_reduce4(h->partials, nb, h->d_res, h->st));
+    CU(launch_reduce4(h->partials, clusters ? V.ncta_int : nb, h->d_res, h->st));
     CU(cudaMemcpyAsync(h->h_res, h->d_res, 4 * sizeof(double), cudaMemcpyDeviceToHost, h->st));
     CU(cudaStreamSynchronize(h->st));
-    h->kernels += 3;
+    h->kernels += clusters ? 5 : 3;
     resab = h->h_res[0];
     if (!std::isfinite(resab)) return fail(h, H3D_ERR_DIVERGED, "SIP residual is not finite");
     if (ns == 1) res1 = resab;
