@@ -27,7 +27,9 @@ namespace {
 // x = d-y-z; the three predecessors are the values that it and the threads
 // (y-1, z), (y, z-1) computed one step earlier, exchanged through shared
 // memory (two buffers, one barrier a step); the factors of the next steps are
-// loaded kAhead steps ahead into registers.  The factor and residual arrays are
+// copied kAhead steps ahead into shared memory (cp.async;
+// register prefetches of several steps share scoreboards and wait for the
+// newest).  The factor and residual arrays are
 // laid out for those loads: cell (x, y, z) of a block at (z*(nx+ny-1) + x+y)*ny
 // + y, so that the threads of one z read consecutive addresses.
 //
@@ -39,7 +41,8 @@ namespace {
 // 48x32x40 blocks (118 steps a pass): one CTA per block with a barrier a step,
 // reading everything from global memory at the point of use, took 859 us a
 // sweep (3.6 us a step); four such blocks, 100 sweeps with their residuals, stop
-// tests and projection steps: 76.5 ms then, 20.9 ms now.
+// tests and projection steps: 76.5 ms then, 14.8 ms now (20.9 ms with register
+// prefetches).
 constexpr int kPhase = 8, kRing = 4 * kPhase, kAhead = 4;
 constexpr int kSipThreads = 512, kSipMaxCtas = 8, kSipMaxSmem = 200 * 1024;
 
@@ -57,32 +60,44 @@ struct SipSkew {
   }
 };
 
+template <typename T>
+__device__ __forceinline__ void cp_async_word(T* s, const T* g) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(s);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(a), "l"(g), "n"(sizeof(T)) : "memory");
+}
+
 // One CTA's share of a march over `steps` hyperplanes: step(d, k) for its
 // active ones, in ascending (FWD) or descending order, a CTA barrier after
-// each, a cluster barrier after every phase.
+// each, a cluster barrier after every phase.  prefetch(d, k) starts a thread's
+// copies for step d into its slot k, kAhead steps before they are read.
 template <bool FWD, typename Prefetch, typename Step>
 __device__ __forceinline__ void sip_march(int steps, int rank, int nranks, Prefetch&& prefetch, Step&& step) {
   const int nblk = (steps + kPhase - 1) / kPhase;
   const int lag = FWD ? rank : nranks - 1 - rank;
 #pragma unroll
-  for (int k = 0; k < kAhead; ++k) prefetch(FWD ? k : steps - 1 - k, k);
+  for (int k = 0; k < kAhead; ++k) {
+    prefetch(FWD ? k : steps - 1 - k, k);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  }
   for (int p = 0; p < nblk + nranks - 1; ++p) {
     const int blk = p - lag;
     if (blk >= 0 && blk < nblk) {
 #pragma unroll
       for (int k = 0; k < kPhase; ++k) {
         const int t = blk * kPhase + k;
-        const int d = FWD ? t : steps - 1 - t;
         if (t < steps) {
-          step(d, k % kAhead);
+          asm volatile("cp.async.wait_group %0;\n" ::"n"(kAhead - 1) : "memory");
+          step(FWD ? t : steps - 1 - t, k % kAhead);
           const int tn = t + kAhead;
-          if (tn < steps) prefetch(FWD ? tn : steps - 1 - tn, k % kAhead);
+          prefetch(FWD ? tn : steps - 1 - tn, k % kAhead);
+          asm volatile("cp.async.commit_group;\n" ::: "memory");
           __syncthreads();
         }
       }
     }
     if (nranks > 1) cg::this_cluster().sync();
   }
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
 }
 
 // Shared memory of a march of NV values a cell: the two step buffers
@@ -204,7 +219,9 @@ __global__ void __launch_bounds__(kSipThreads) k_sip_subst(const BlkLev* __restr
   const int tz = has ? (int)threadIdx.x / ny : 0, ty = has ? (int)threadIdx.x - tz * ny : 0;
   const long long row = S.at(0, ty, z0 + tz);
   const int to = tz * v.pitch + ty + 1, tx = ty + z0 + tz;  // x = d - tx
-  double f0[kAhead], f1[kAhead], f2[kAhead], f3[kAhead], f4[kAhead];
+  // its operands of the next kAhead steps: word j of slot k at pf[(5k + j) * kSipThreads]
+  double* pf = sm + part + threadIdx.x;
+  auto F = [&](int k, int j) -> double& { return pf[(5 * k + j) * kSipThreads]; };
   pdl_wait();
 
   // forward: res = (res - lb*res(z-1) - lw*res(x-1) - ls*res(y-1)) * lpr
@@ -219,11 +236,11 @@ __global__ void __launch_bounds__(kSipThreads) k_sip_subst(const BlkLev* __restr
           const int x = d - tx;
           if (ONE && has && x >= 0 && x < nx) {
             const long long i = row + (long long)x * ny;
-            f0[k] = lu.res[i];
-            f1[k] = lu.lb[i];
-            f2[k] = lu.lw[i];
-            f3[k] = lu.ls[i];
-            f4[k] = lu.lpr[i];
+            cp_async_word(&F(k, 0), lu.res + i);
+            cp_async_word(&F(k, 1), lu.lb + i);
+            cp_async_word(&F(k, 2), lu.lw + i);
+            cp_async_word(&F(k, 3), lu.ls + i);
+            cp_async_word(&F(k, 4), lu.lpr + i);
           }
         },
         [&](int d, int k) {
@@ -232,7 +249,8 @@ __global__ void __launch_bounds__(kSipThreads) k_sip_subst(const BlkLev* __restr
             const int x = d - tx;
             if (has && x >= 0 && x < nx) {
               const double b = tz > 0 ? v.cur[r + to - v.pitch] : v.ring[((d - 1) & (kRing - 1)) * ny + ty];
-              const double n = (f0[k] - f1[k] * b - f2[k] * v.cur[r + to] - f3[k] * v.cur[r + to - 1]) * f4[k];
+              const double n =
+                  (F(k, 0) - F(k, 1) * b - F(k, 2) * v.cur[r + to] - F(k, 3) * v.cur[r + to - 1]) * F(k, 4);
               v.cur[w + to] = n;
               lu.res[row + (long long)x * ny] = n;
               if (next && z0 + tz == z1 - 1) next[ring + (long long)(d & (kRing - 1)) * ny + ty] = n;
@@ -266,10 +284,10 @@ __global__ void __launch_bounds__(kSipThreads) k_sip_subst(const BlkLev* __restr
           const int x = d - tx;
           if (ONE && has && x >= 0 && x < nx) {
             const long long i = row + (long long)x * ny;
-            f0[k] = lu.res[i];
-            f1[k] = lu.un[i];
-            f2[k] = lu.ue[i];
-            f3[k] = lu.ut[i];
+            cp_async_word(&F(k, 0), lu.res + i);
+            cp_async_word(&F(k, 1), lu.un + i);
+            cp_async_word(&F(k, 2), lu.ue + i);
+            cp_async_word(&F(k, 3), lu.ut + i);
           }
         },
         [&](int d, int k) {
@@ -278,7 +296,7 @@ __global__ void __launch_bounds__(kSipThreads) k_sip_subst(const BlkLev* __restr
             const int x = d - tx;
             if (has && x >= 0 && x < nx) {
               const double t = z0 + tz < z1 - 1 ? v.cur[r + to + v.pitch] : v.ring[((d + 1) & (kRing - 1)) * ny + ty];
-              const double n = f0[k] - f1[k] * v.cur[r + to + 1] - f2[k] * v.cur[r + to] - f3[k] * t;
+              const double n = F(k, 0) - F(k, 1) * v.cur[r + to + 1] - F(k, 2) * v.cur[r + to] - F(k, 3) * t;
               v.cur[w + to] = n;
               lu.res[row + (long long)x * ny] = n;
               if (next && tz == 0) next[ring + (long long)(d & (kRing - 1)) * ny + ty] = n;
@@ -315,7 +333,8 @@ __device__ __forceinline__ bool sip_cell(const BlkLev* __restrict__ bls, const i
 
 // Residual of every block (sipsol.for:146-157) into the skewed res, and the
 // CTA's sum |res| in a fixed order into partials[4 * cta].
-__global__ void __launch_bounds__(256) k_sip_residual(const BlkLev* __restrict__ bls, const long long* __restrict__ offs,
+__global__ void __launch_bounds__(256) k_sip_residual(const BlkLev* __restrict__ bls,
+                                                      const long long* __restrict__ offs,
                                                       const int* __restrict__ cta_start, int nb,
                                                       const double* __restrict__ fi_all,
                                                       const double* __restrict__ su_all, double* __restrict__ res,
@@ -403,7 +422,7 @@ SipPlan sip_plan(const std::vector<BlkLev>& bl) {
   const long long words = 2LL * hz * (ny + 2) + (long long)kRing * ny;
   P.fits = 3 * 8 * words <= kSipMaxSmem;
   P.smem_factor = P.fits ? (int)(3 * 8 * words) : 0;
-  P.smem_subst = P.fits ? (int)(8 * words) : 0;
+  P.smem_subst = P.fits ? (int)(8 * words) + (P.one ? 5 * kAhead * kSipThreads * 8 : 0) : 0;
   return P;
 }
 
@@ -429,8 +448,9 @@ cudaError_t launch_sip_sweep_c(const SipPlan& P, const BlkLev* bl, const long lo
   SipLU lu{a.lb, a.lw, a.ls, a.lpr, a.un, a.ue, a.ut, a.res};
   pdl_launch(k_sip_residual, interior.ncta, 256, 0, st, bl, offs, interior.cta_start, interior.nb, fi, su, a.res,
              partials);
-  cudaError_t e = P.one ? cluster_launch(k_sip_subst<true>, interior.nb, P.ctas, kSipThreads, P.smem_subst, st, bl, offs, lu)
-                        : cluster_launch(k_sip_subst<false>, interior.nb, P.ctas, kSipThreads, P.smem_subst, st, bl, offs, lu);
+  const int nb = interior.nb;
+  cudaError_t e = P.one ? cluster_launch(k_sip_subst<true>, nb, P.ctas, kSipThreads, P.smem_subst, st, bl, offs, lu)
+                        : cluster_launch(k_sip_subst<false>, nb, P.ctas, kSipThreads, P.smem_subst, st, bl, offs, lu);
   if (e != cudaSuccess) return e;
   pdl_launch(k_sip_correct, interior.ncta, 256, 0, st, bl, offs, interior.cta_start, interior.nb, fi, a.res);
   return cudaGetLastError();

@@ -88,3 +88,14 @@ def test_sip_rejects_variable_coefficients(h3d):
         s.sipsol(3)
     assert e.value.code == h3d._lib.H3D_ERR_BAD_CONFIG
     s.close()
+
+
+@pytest.mark.parametrize("layout", [
+    ((1, 1, 1), (2, 2, 2), [W] * 6),             # fewer rows of z than CTAs, a march of a few steps
+    ((1, 2, 1), (6, 34, 18), [P, P, W, W, W, W]),   # three CTAs a block, the last slab of z shorter
+    ((1, 1, 2), (4, 50, 44), [W] * 6),           # eight CTAs a block (2200 rows)
+    ((1, 1, 1), (4, 80, 66), [W, W, P, P, W, W]),   # more rows of a CTA than threads
+    ((1, 1, 1), (2, 162, 160), [W] * 6),         # step buffers beyond shared memory: one CTA, global memory
+])
+def test_sipsol_cluster_edges_bitexact(oracle_mod, h3d, layout):
+    test_sipsol_bitexact(oracle_mod, h3d, layout, 3)
