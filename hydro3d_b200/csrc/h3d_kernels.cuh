@@ -166,6 +166,17 @@ cudaError_t launch_rbgs_zero32(const BlkLev* bl, const Tile* tiles, int ntiles, 
 template <typename T>
 cudaError_t launch_seq_smoother(int itrsch, bool var, bool zero, const BlkLev* bl, int nb, const T* src, T* dst,
                                 const T* rhs, T* acoef, const T* fx, const T* fy, const T* fz, cudaStream_t st);
+// The TDMA sweep with the chains' operands in shared memory (h3d_seq.cu).
+// scratch: 3 * words * nb words (kDiagonals only).
+struct TdmaPlan {
+  enum Mode { kGlobal = 0, kWhole = 1, kDiagonals = 2 };
+  int mode = kGlobal, smem = 0, nbuf = 0;
+  long long words = 0;
+};
+TdmaPlan tdma_plan(const std::vector<BlkLev>& bl, bool var, int word);
+template <typename T>
+cudaError_t launch_tdma(const TdmaPlan& P, bool zero, const BlkLev* bl, CellTab all, const T* src, T* dst,
+                        const T* rhs, T* scratch, cudaStream_t st);
 template <typename T>
 cudaError_t launch_relax_small(bool var, const BlkLev* bl, const int* start, int nb, T* phi, const T* rhs,
                                const T* fx, const T* fy, const T* fz, const uint32_t* fdst, const uint32_t* fsrc,

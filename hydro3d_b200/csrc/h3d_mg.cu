@@ -113,7 +113,8 @@ struct Level {
   Tile* d_ztiles = nullptr;     // FP32 zero-source sweep tiles (launch_rbgs_zero32), or none
   bool use_z32 = true;          // the zero-source kernel beat the tuned sweep's zero mode (autotuner)
   int nztiles = 0, zzc = 1;
-  double* seq64 = nullptr;      // line-TDMA scratch a(s) of every cell (mg_itrsch 2)
+  TdmaPlan tdma;                // the line-TDMA kernel of the level (mg_itrsch 2) and its scratch
+  double* seq64 = nullptr;
   float* seq32 = nullptr;
   // local mesh refinement
   bool expr = false;            // the level's fills are expression tables (neighbours of different rdv)
@@ -590,11 +591,16 @@ struct Exec {
     }
     if (h->desc.mg_itrsch != 3) {  // lexicographic GS or line TDMA: one CTA per block
       const int nb = (int)V.geom.bl.size();
+      const CellTab all{V.d_cta_all, nb, V.ncta_all};
+      if (h->desc.mg_itrsch == 2 && V.tdma.mode == TdmaPlan::kDiagonals) h->kernels += 6;
       if (mixed_level(g)) {
         float* src = V.phi32[V.cur32];
         float* dst = V.phi32[1 - V.cur32];
-        CU(launch_seq_smoother<float>(h->desc.mg_itrsch, h->var, V.zero32, V.d_bl, nb, src, dst, V.rhs32, V.seq32,
-                                      V.fx32, V.fy32, V.fz32, st));
+        if (h->desc.mg_itrsch == 2 && V.tdma.mode != TdmaPlan::kGlobal)
+          CU(launch_tdma<float>(V.tdma, V.zero32, V.d_bl, all, src, dst, V.rhs32, V.seq32, st));
+        else
+          CU(launch_seq_smoother<float>(h->desc.mg_itrsch, h->var, V.zero32, V.d_bl, nb, src, dst, V.rhs32, V.seq32,
+                                        V.fx32, V.fy32, V.fz32, st));
         TRY(chk("sequential sweep fp32", g));
         if (e1) CU(record(e1));
         TRY(sweep_fill<float>(V, V.sweep, dst, src, V.zero32, &h->kernels));
@@ -604,8 +610,11 @@ struct Exec {
       } else {
         double* src = V.phi64[V.cur64];
         double* dst = V.phi64[1 - V.cur64];
-        CU(launch_seq_smoother<double>(h->desc.mg_itrsch, h->var, V.zero64, V.d_bl, nb, src, dst, V.rhs64, V.seq64,
-                                       V.fx64, V.fy64, V.fz64, st));
+        if (h->desc.mg_itrsch == 2 && V.tdma.mode != TdmaPlan::kGlobal)
+          CU(launch_tdma<double>(V.tdma, V.zero64, V.d_bl, all, src, dst, V.rhs64, V.seq64, st));
+        else
+          CU(launch_seq_smoother<double>(h->desc.mg_itrsch, h->var, V.zero64, V.d_bl, nb, src, dst, V.rhs64,
+                                         V.seq64, V.fx64, V.fy64, V.fz64, st));
         TRY(chk("sequential sweep fp64", g));
         if (e1) CU(record(e1));
         TRY(sweep_fill<double>(V, V.sweep, dst, src, V.zero64, &h->kernels));
@@ -2540,8 +2549,20 @@ int h3d_mg_create(h3d_mg** out, const h3d_mg_desc* desc) {
         return bail(rc);
     }
     if (D.mg_itrsch == 2) {
-      if (need64 && (rc = dalloc(h, &V.seq64, n))) return bail(rc);
-      if (need32 && (rc = dalloc(h, &V.seq32, n))) return bail(rc);
+      // (a level sweeps in one precision; out of memory: the kernel that needs one word a cell)
+      const bool f32 = f32_level(h, g);
+      V.tdma = tdma_plan(V.geom.bl, h->var, f32 ? 4 : 8);
+      auto scratch = [&](size_t words) { return f32 ? dalloc(h, &V.seq32, words) : dalloc(h, &V.seq64, words); };
+      rc = H3D_OK;
+      if (V.tdma.mode == TdmaPlan::kDiagonals) {
+        rc = scratch(3 * (size_t)V.tdma.words * V.geom.bl.size());
+        if (rc == H3D_ERR_OOM) {
+          cudaGetLastError();
+          V.tdma.mode = TdmaPlan::kGlobal;
+        }
+      }
+      if (V.tdma.mode == TdmaPlan::kGlobal) rc = scratch(n);
+      if (rc != H3D_OK) return bail(rc);
     }
     if (h->var) {
       if ((rc = dalloc(h, &V.dens, n)) || (rc = dalloc(h, &V.fx64, n)) || (rc = dalloc(h, &V.fy64, n)) ||

@@ -1,5 +1,6 @@
-// Sequentially ordered solvers on the device: Stone's SIP (sipsol.for).  Their
-// recurrences run as wavefronts; a block is one thread-block cluster.
+// Sequentially ordered solvers on the device: Stone's SIP (sipsol.for) and the
+// line-TDMA sweep (mgsolver.for:434-549).  Their recurrences run as wavefronts,
+// a block by one CTA or one thread-block cluster.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -404,6 +405,411 @@ cudaError_t cluster_launch(K k, int nb, int ctas, int threads, int smem, cudaStr
 
 }  // namespace
 
+namespace {
+
+// ---------------------------------------------------------------------------
+// Line-TDMA sweep of a level (mgrelax, mg_itrsch = 2, mgsolver.for:434-549),
+// constant coefficients: j-lines, then i-lines, then k-lines of every block,
+// every value the reference's, in its operand order.  A line (u, v) (u, v the
+// two indices across it) follows (u-1, v) and (u, v-1), so the lines of an
+// anti-diagonal u + v are independent: one thread a line forms the right-hand
+// sides t(s) from the four cross neighbours and runs the recurrences c(s) =
+// (t(s) - lo c(s-1)) apr(s) and phi(s) = c(s) - a(s) phi(s+1).  apr(s) = 1/(ap - lo a(s-1)) and a(s) =
+// hi apr(s) depend on the line only through the walls beside it: they are
+// tabulated per axis for the 16 combinations of "first / last u" and "first /
+// last v", which takes the division out of the chain.
+//
+// The chain of (diagonals) x (5 FP64 operations a cell of a line) bounds the
+// sweep, so its operands are in shared memory: whole small blocks (k_tdma_s), or the
+// diagonals around the current one, copied by the other warps while the chains
+// run (k_tdma_g).  For the latter every pass is preceded by a rearrangement of
+// the level, by the whole chip, into rows d = u + v of (s, u), where the data
+// of a diagonal are contiguous.
+//
+// Four 32x32x48 blocks, FP64 solve of 21 cycles: 327-345 ms with one thread a line
+// reading global memory at the point of use and the division in the chain
+// (k_tdma), 43 ms now (150 us a pass of 79 diagonals of 32-cell lines).
+constexpr int kTdmaThreads = 256, kTdmaMaxSmem = 227 * 1024;
+
+template <int AXIS>
+struct LineAxes {  // (u, v, s) of AXIS: 0 lines along x, 1 along y, 2 along z
+  static constexpr int US = AXIS == 0 ? 1 : 0, VS = AXIS == 2 ? 1 : 2, SS = AXIS;
+};
+
+template <int AXIS>
+__device__ __forceinline__ int ext_of(const BlkLev& B, int a) {
+  return a == 0 ? B.nx : a == 1 ? B.ny : B.nz;
+}
+
+// Wall-aware face coefficients along the three axes of a line cell.
+template <typename T, int AXIS>
+struct LineCoef {
+  T au, av, as;
+  bool ulo, uhi, vlo, vhi, slo, shi;
+  __device__ __forceinline__ explicit LineCoef(const BlkLev& B) {
+    const T a[3] = {(T)B.ax, (T)B.ay, (T)B.az};
+    using L = LineAxes<AXIS>;
+    au = a[L::US];
+    av = a[L::VS];
+    as = a[L::SS];
+    ulo = B.phys >> (2 * L::US) & 1;
+    uhi = B.phys >> (2 * L::US + 1) & 1;
+    vlo = B.phys >> (2 * L::VS) & 1;
+    vhi = B.phys >> (2 * L::VS + 1) & 1;
+    slo = B.phys >> (2 * L::SS) & 1;
+    shi = B.phys >> (2 * L::SS + 1) & 1;
+  }
+};
+
+// Class of a line: bit 0 / 1 first / last u, bit 2 / 3 first / last v.
+__device__ __forceinline__ int line_class(int u, int nu, int v, int nv) {
+  return (u == 1 ? 1 : 0) | (u == nu ? 2 : 0) | (v == 1 ? 4 : 0) | (v == nv ? 8 : 0);
+}
+
+// tab[(s * 16 + class) * 2] = apr(s), a(s), s = 1..n, by threads 0..15.
+template <typename T, int AXIS>
+__device__ __forceinline__ void line_table(const LineCoef<T, AXIS>& C, int n, T* tab) {
+  const int cl = threadIdx.x;
+  if (cl >= 16) return;
+  const T lu = (cl & 1) && C.ulo ? T(0) : C.au, hu = (cl & 2) && C.uhi ? T(0) : C.au;
+  const T lv = (cl & 4) && C.vlo ? T(0) : C.av, hv = (cl & 8) && C.vhi ? T(0) : C.av;
+  T aprev = T(0);
+  for (int s = 1; s <= n; ++s) {
+    const T lo = s == 1 && C.slo ? T(0) : C.as, hi = s == n && C.shi ? T(0) : C.as;
+    Coef<T> c;
+    c.aw = AXIS == 0 ? lo : lu;
+    c.ae = AXIS == 0 ? hi : hu;
+    c.as = AXIS == 1 ? lo : AXIS == 0 ? lu : lv;
+    c.an = AXIS == 1 ? hi : AXIS == 0 ? hu : hv;
+    c.ab = AXIS == 2 ? lo : lv;
+    c.at = AXIS == 2 ? hi : hv;
+    const T apr = gs_div(T(1), coef_ap(c) - lo * aprev);
+    aprev = hi * apr;
+    tab[(s * 16 + cl) * 2] = apr;
+    tab[(s * 16 + cl) * 2 + 1] = aprev;
+  }
+}
+
+// t = rhs - the four cross terms in the reference's order (j- and i-lines: the u
+// pair first; k-lines: the v pair first).
+template <typename T, int AXIS>
+__device__ __forceinline__ T line_rhs(T r, T hu, T lu, T hv, T lv, T e, T w, T t, T b) {
+  if (AXIS == 2) return r - hv * t - lv * b - hu * e - lu * w;
+  return r - hu * e - lu * w - hv * t - lv * b;
+}
+
+__device__ __forceinline__ double lds_word(unsigned a, double) {
+  double v;
+  asm volatile("ld.shared.f64 %0, [%1];\n" : "=d"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ float lds_word(unsigned a, float) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];\n" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void sts_word(unsigned a, double v) {
+  asm volatile("st.shared.f64 [%0], %1;\n" ::"r"(a), "d"(v) : "memory");
+}
+__device__ __forceinline__ void sts_word(unsigned a, float v) {
+  asm volatile("st.shared.f32 [%0], %1;\n" ::"r"(a), "f"(v) : "memory");
+}
+
+// Shared-memory addresses of position 0 of a line: right-hand side, cross
+// neighbours u+1, u-1, v+1, v-1 and the line's own values; st: bytes a position.
+struct LineAddr {
+  unsigned r, e, w, t, b, c, st;
+};
+
+// One line: the right-hand sides t(s) and c(s) = (t(s) - lo c(s-1)) apr(s)
+// upwards, c(s) into the line's own places (no other line of the diagonal reads
+// them), then out(s, phi(s)) for s = n down to 1.  tab: the line's class in the
+// table; c0 and after: the ghosts at both ends.
+//
+// Groups of eight positions in two sets of registers: the operands of the next
+// group are loaded, and its t(s) formed, in the shadow of the current group's
+// chain, never past the line.  FP64 operations complete 8 cycles after issue: the
+// chain's floor is 24 cycles a position upwards and 16 downwards; with the loads in
+// the chain's way (a loop unrolled by the compiler) it takes 52 upwards.
+template <typename T, int AXIS, typename Out>
+__device__ __forceinline__ void line_solve(const LineAddr& A, unsigned tab, int n, T hu, T lu, T hv, T lv, T lo1,
+                                           T lo, T c0, T after, Out&& out) {
+  constexpr int G = 8;
+  constexpr unsigned TP = 32 * sizeof(T);  // table bytes a position
+  const T z = T(0);
+  T t[2][G], a[2][G];
+  // operands of position s, t(s) in t and apr(s) in ap
+  auto rhs_at = [&](unsigned s, T& tt, T& ap) {
+    const unsigned o = s * A.st;
+    const T r = lds_word(A.r + o, z), e = lds_word(A.e + o, z), w = lds_word(A.w + o, z), q = lds_word(A.t + o, z),
+            b = lds_word(A.b + o, z);
+    ap = lds_word(tab + s * TP, z);
+    tt = line_rhs<T, AXIS>(r, hu, lu, hv, lv, e, w, q, b);
+  };
+  const int groups = n / G, head = n % G;
+  T c = c0, l = lo1;
+  for (int s = 1; s <= head; ++s) {  // the remainder first
+    rhs_at(s, t[0][0], a[0][0]);
+    c = (t[0][0] - l * c) * a[0][0];
+    l = lo;
+    sts_word(A.c + s * A.st, c);
+  }
+  auto load = [&](int h, int s) {
+#pragma unroll
+    for (int k = 0; k < G; ++k) rhs_at(s + k, t[h][k], a[h][k]);
+  };
+  auto chain = [&](int h, int s) {
+#pragma unroll
+    for (int k = 0; k < G; ++k) {
+      c = (t[h][k] - l * c) * a[h][k];
+      l = lo;
+      sts_word(A.c + (s + k) * A.st, c);
+    }
+  };
+  if (groups > 0) {
+    int s = head + 1;
+    load(0, s);
+    for (int left = groups - 1;; s += 2 * G) {
+      if (left > 0) load(1, s + G);
+      chain(0, s);
+      if (left-- == 0) break;
+      if (left > 0) load(0, s + 2 * G);
+      chain(1, s + G);
+      if (left-- == 0) break;
+    }
+  }
+  T x = after;
+  auto loadb = [&](int h, int s) {
+#pragma unroll
+    for (int k = 0; k < G; ++k) {
+      t[h][k] = lds_word(A.c + (s - k) * A.st, z);
+      a[h][k] = lds_word(tab + (s - k) * TP + (unsigned)sizeof(T), z);
+    }
+  };
+  auto back = [&](int h, int s) {
+#pragma unroll
+    for (int k = 0; k < G; ++k) {
+      x = t[h][k] - a[h][k] * x;
+      out(s - k, x);
+    }
+  };
+  if (groups > 0) {
+    int s = n;
+    loadb(0, s);
+    for (int left = groups - 1;; s -= 2 * G) {
+      if (left > 0) loadb(1, s - G);
+      back(0, s);
+      if (left-- == 0) break;
+      if (left > 0) loadb(0, s - 2 * G);
+      back(1, s - G);
+      if (left-- == 0) break;
+    }
+  }
+  for (int s = head; s >= 1; --s) {
+    x = lds_word(A.c + s * A.st, z) - lds_word(tab + s * TP + (unsigned)sizeof(T), z) * x;
+    out(s, x);
+  }
+}
+
+// ---- whole block in shared memory -----------------------------------------
+// Pitches of the block there: rows 3 mod 4 and planes even, so that lanes on a
+// diagonal fall into different banks (two-way conflicts for k-lines).
+__host__ __device__ inline int tdma_s_sx(int nx) { return ((nx + 2 + 4) / 4) * 4 - 1; }
+__host__ __device__ inline int tdma_s_sxy(int nx, int ny) { return (tdma_s_sx(nx) * (ny + 2) + 1) / 2 * 2; }
+
+template <typename T, int AXIS>
+__device__ __forceinline__ void tdma_s_pass(const BlkLev& B, T* D, const T* R, T* tab) {
+  using L = LineAxes<AXIS>;
+  const int sx = tdma_s_sx(B.nx), sxy = tdma_s_sxy(B.nx, B.ny);
+  const int ex[3] = {B.nx, B.ny, B.nz}, pt[3] = {1, sx, sxy};
+  const int nu = ex[L::US], nv = ex[L::VS], n = ex[L::SS];
+  const int pu = pt[L::US], pv = pt[L::VS], ps = pt[L::SS];
+  const LineCoef<T, AXIS> C(B);
+  line_table<T, AXIS>(C, n, tab);
+  const unsigned W = sizeof(T);
+  const unsigned aD = (unsigned)__cvta_generic_to_shared(D), aR = (unsigned)__cvta_generic_to_shared(R);
+  const unsigned aA = (unsigned)__cvta_generic_to_shared(tab);
+  const T z = T(0);
+  __syncthreads();
+  for (int d = 2; d <= nu + nv; ++d) {
+    const int u = max(1, d - nv) + (int)threadIdx.x, v = d - u;
+    if (u <= min(nu, d - 1)) {
+      const T hu = u == nu && C.uhi ? z : C.au, lu = u == 1 && C.ulo ? z : C.au;
+      const T hv = v == nv && C.vhi ? z : C.av, lv = v == 1 && C.vlo ? z : C.av;
+      const unsigned o = (u * pu + v * pv) * W, c = aD + o, st = ps * W;
+      const LineAddr A{aR + o, c + pu * W, c - pu * W, c + pv * W, c - pv * W, c, st};
+      line_solve<T, AXIS>(A, aA + 2 * W * line_class(u, nu, v, nv), n, hu, lu, hv, lv, C.slo ? z : C.as, C.as,
+                          lds_word(c, z), lds_word(c + (n + 1) * st, z), [&](int s, T x) { sts_word(c + s * st, x); });
+    }
+    __syncthreads();
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kTdmaThreads) k_tdma_s(const BlkLev* __restrict__ bls, const T* __restrict__ src,
+                                                         T* __restrict__ dst, const T* __restrict__ rhs, bool zero) {
+  extern __shared__ __align__(16) unsigned char tdma_smem[];
+  pdl_trigger();
+  const BlkLev B = bls[blockIdx.x];
+  const int sx = tdma_s_sx(B.nx), sxy = tdma_s_sxy(B.nx, B.ny);
+  T* D = reinterpret_cast<T*>(tdma_smem);
+  T* R = D + (size_t)sxy * (B.nz + 2);
+  T* tab = R + (size_t)sxy * (B.nz + 2);
+  pdl_wait();
+  const int ex = B.nx + 2, ey = B.ny + 2, ncell = ex * ey * (B.nz + 2);
+  for (int q = threadIdx.x; q < ncell; q += blockDim.x) {
+    const int x = q % ex, y = (q / ex) % ey, z = q / (ex * ey);
+    const long long i = B.off + (long long)z * B.sxy + (long long)y * B.sx + x;
+    const int o = z * sxy + y * sx + x;
+    D[o] = zero ? T(0) : src[i];
+    R[o] = rhs[i];
+  }
+  __syncthreads();
+  tdma_s_pass<T, 1>(B, D, R, tab);
+  tdma_s_pass<T, 0>(B, D, R, tab);
+  tdma_s_pass<T, 2>(B, D, R, tab);
+  for (int q = threadIdx.x; q < ncell; q += blockDim.x) {
+    const int x = q % ex, y = (q / ex) % ey, z = q / (ex * ey);
+    dst[B.off + (long long)z * B.sxy + (long long)y * B.sx + x] = D[z * sxy + y * sx + x];
+  }
+}
+
+// ---- larger blocks: diagonal rows in global scratch --------------------------
+// Words of a block rearranged for AXIS: rows d = u + v (ghosts included: 0 ..
+// nu+nv+2) of (s = 0 .. n+1, u = 0 .. nu+1).
+__host__ __device__ inline long long tdma_rows(int nu, int nv, int n) {
+  return (long long)(nu + nv + 3) * (n + 2) * (nu + 2);
+}
+
+template <int AXIS>
+__device__ __forceinline__ long long tdma_at(const BlkLev& B, int x, int y, int z) {
+  const int u = AXIS == 0 ? y : x, v = AXIS == 2 ? y : z, s = AXIS == 0 ? x : AXIS == 1 ? y : z;
+  const int nu = AXIS == 0 ? B.ny : B.nx, n = AXIS == 0 ? B.nx : AXIS == 1 ? B.ny : B.nz;
+  return ((long long)(u + v) * (n + 2) + s) * (nu + 2) + u;
+}
+
+// Rearranges the iterate and the right-hand side of every block for the pass
+// along AXIS: from the level (FROM < 0; zero: the zero iterate) or from the rows of
+// the pass along FROM.  256 cells a CTA, ghosts included.
+template <typename T, int FROM, int AXIS>
+__global__ void __launch_bounds__(256) k_tdma_rows(const BlkLev* __restrict__ bls, const int* __restrict__ cta_start,
+                                                   int nb, const T* __restrict__ src, const T* __restrict__ rhs,
+                                                   const T* __restrict__ from, T* __restrict__ to,
+                                                   T* __restrict__ rows, long long words, bool zero) {
+  pdl_trigger();
+  pdl_wait();
+  const int b = find_block(cta_start, nb, blockIdx.x);
+  const BlkLev& B = bls[b];
+  const int ex = B.nx + 2, ey = B.ny + 2, q = (blockIdx.x - cta_start[b]) * blockDim.x + threadIdx.x;
+  if (q >= ex * ey * (B.nz + 2)) return;
+  const int x = q % ex, y = (q / ex) % ey, z = q / (ex * ey);
+  const long long i = B.off + (long long)z * B.sxy + (long long)y * B.sx + x;
+  const long long o = b * words + tdma_at<AXIS>(B, x, y, z);
+  if (FROM < 0) to[o] = zero ? T(0) : src[i];
+  else to[o] = from[b * words + tdma_at<FROM < 0 ? 0 : FROM>(B, x, y, z)];
+  rows[o] = rhs[i];
+}
+
+// The rows of the last pass (along z) back into the level.
+template <typename T>
+__global__ void __launch_bounds__(256) k_tdma_level(const BlkLev* __restrict__ bls, const int* __restrict__ cta_start,
+                                                    int nb, const T* __restrict__ from, T* __restrict__ dst,
+                                                    long long words) {
+  pdl_trigger();
+  pdl_wait();
+  const int b = find_block(cta_start, nb, blockIdx.x);
+  const BlkLev& B = bls[b];
+  const int ex = B.nx + 2, ey = B.ny + 2, q = (blockIdx.x - cta_start[b]) * blockDim.x + threadIdx.x;
+  if (q >= ex * ey * (B.nz + 2)) return;
+  const int x = q % ex, y = (q / ex) % ey, z = q / (ex * ey);
+  dst[B.off + (long long)z * B.sxy + (long long)y * B.sx + x] = from[b * words + tdma_at<2>(B, x, y, z)];
+}
+
+// One pass, a CTA per block, on the rearranged iterate (in place) and rhs.
+template <typename T, int AXIS>
+__global__ void __launch_bounds__(kTdmaThreads) k_tdma_g(const BlkLev* __restrict__ bls, T* __restrict__ iter,
+                                                         const T* __restrict__ rows, long long words, int nbuf) {
+  extern __shared__ __align__(16) unsigned char tdma_smem[];
+  using L = LineAxes<AXIS>;
+  pdl_trigger();
+  const BlkLev B = bls[blockIdx.x];
+  T* Dk = iter + blockIdx.x * words;
+  const T* Rk = rows + blockIdx.x * words;
+  const int ex[3] = {B.nx, B.ny, B.nz};
+  const int nu = ex[L::US], nv = ex[L::VS], n = ex[L::SS], pitch = nu + 2, row = (n + 2) * pitch;
+  T* P = reinterpret_cast<T*>(tdma_smem);  // [2][n + 2][pitch]: c and phi of the current and the previous diagonal
+  // nbuf (two: copied while the previous diagonal's chains run) times: the rhs of
+  // a diagonal's lines, the old values of the next diagonal's, (u+1, v) and
+  // (u, v+1), and the ghosts before and after its lines
+  T* ops = P + 2 * row;
+  const int opw = 2 * row + 2 * pitch;
+  T* tab = ops + nbuf * opw;  // [n + 1][16][2]
+  const LineCoef<T, AXIS> C(B);
+  const int tid = threadIdx.x;
+  line_table<T, AXIS>(C, n, tab);
+  // copies the operands of diagonal d, by threads t0, t0 + nt, ...; the ghost
+  // lines u = 0 and v = 0 that its lines read go to the places of the previous
+  // diagonal's buffer that no line of that diagonal uses
+  auto stage = [&](int d, int t0, int nt) {
+    const T* r = Rk + (long long)d * row;
+    const T* o = Dk + (long long)(d + 1) * row;
+    const T* b = Dk + (long long)(d - 1) * row;
+    const T* e = Dk + (long long)d * row;
+    T* prev = P + ((d - 1) & 1) * row;
+    T* SR = ops + (d & (nbuf - 1)) * opw;
+    T *ST = SR + row, *E0 = ST + row, *E1 = E0 + pitch;
+    for (int q = pitch + t0; q < (n + 1) * pitch; q += nt) {
+      cp_async_word(SR + q, r + q);
+      cp_async_word(ST + q, o + q);
+    }
+    for (int s = 1 + t0; s <= n; s += nt) {
+      cp_async_word(prev + s * pitch, b + s * pitch);
+      if (d - 1 <= nu) cp_async_word(prev + s * pitch + d - 1, b + s * pitch + d - 1);
+    }
+    for (int u = t0; u < pitch; u += nt) {
+      cp_async_word(E0 + u, e + u);
+      cp_async_word(E1 + u, e + (n + 1) * pitch + u);
+    }
+  };
+  pdl_wait();
+  stage(2, tid, blockDim.x);
+  const unsigned W = sizeof(T), rowb = row * W, aP = (unsigned)__cvta_generic_to_shared(P);
+  const unsigned aA = (unsigned)__cvta_generic_to_shared(tab);
+  const T z = T(0);
+  const int chain = 32 * ((min(nu, nv) + 31) / 32);  // threads of the warps that have lines
+  for (int d = 2; d <= nu + nv; ++d) {
+    const unsigned cur = aP + (d & 1) * rowb, prv = aP + ((d + 1) & 1) * rowb;
+    const int u = max(1, d - nv) + tid, v = d - u;
+    const bool mine = u <= min(nu, d - 1);
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads();
+    if (nbuf == 2 && d < nu + nv) {
+      if (chain >= kTdmaThreads) stage(d + 1, tid, kTdmaThreads);
+      else if (tid >= chain) stage(d + 1, tid - chain, kTdmaThreads - chain);
+    }
+    if (mine) {
+      const T hu = u == nu && C.uhi ? z : C.au, lu = u == 1 && C.ulo ? z : C.au;
+      const T hv = v == nv && C.vhi ? z : C.av, lv = v == 1 && C.vlo ? z : C.av;
+      const T* E0 = ops + (d & (nbuf - 1)) * opw + 2 * row;
+      const unsigned c = u * W, aSR = aP + 2 * rowb + (d & (nbuf - 1)) * (unsigned)(opw * W), aST = aSR + rowb;
+      const LineAddr A{aSR + c, aST + c + W, prv + c - W, aST + c, prv + c, cur + c, pitch * W};
+      T* o = Dk + (long long)d * row + n * pitch + u;  // out() runs from s = n down
+      line_solve<T, AXIS>(A, aA + 2 * W * line_class(u, nu, v, nv), n, hu, lu, hv, lv, C.slo ? z : C.as, C.as, E0[u],
+                          E0[pitch + u], [&](int s, T x) {
+                            sts_word(A.c + s * A.st, x);
+                            *o = x;
+                            o -= pitch;
+                          });
+    }
+    if (nbuf == 1 && d < nu + nv) {
+      __syncthreads();
+      stage(d + 1, tid, kTdmaThreads);
+    }
+  }
+}
+
+}  // namespace
+
 // CTAs of a block's cluster: 256 rows (y, z) each, up to the portable eight.
 // fits: the step buffers of the factors, the largest, fit shared memory (blocks
 // of 128x128 rows do, 160x160 do not: those keep one CTA per block and global
@@ -432,6 +838,14 @@ cudaError_t init_seq_attributes() {
   cudaError_t e = cudaFuncSetAttribute(k_sip_factor_c, a, kSipMaxSmem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sip_subst<true>, a, kSipMaxSmem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sip_subst<false>, a, kSipMaxSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_tdma_s<double>, a, kTdmaMaxSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_tdma_s<float>, a, kTdmaMaxSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_tdma_g<double, 0>, a, kTdmaMaxSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_tdma_g<double, 1>, a, kTdmaMaxSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_tdma_g<double, 2>, a, kTdmaMaxSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_tdma_g<float, 0>, a, kTdmaMaxSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_tdma_g<float, 1>, a, kTdmaMaxSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_tdma_g<float, 2>, a, kTdmaMaxSmem);
   return e;
 }
 
@@ -455,5 +869,63 @@ cudaError_t launch_sip_sweep_c(const SipPlan& P, const BlkLev* bl, const long lo
   pdl_launch(k_sip_correct, interior.ncta, 256, 0, st, bl, offs, interior.cta_start, interior.nb, fi, a.res);
   return cudaGetLastError();
 }
+
+// Which TDMA kernel a level takes: whole blocks in shared memory where they fit
+// (16x16x24 cells in FP64), else clusters with the diagonals around the current
+// one there (80^3 in FP64), else, and with variable coefficients, one thread a
+// line in global memory (k_tdma).
+TdmaPlan tdma_plan(const std::vector<BlkLev>& bl, bool var, int word) {
+  TdmaPlan P;
+  if (var) return P;
+  long long whole = 0, diag[2] = {0, 0}, lines = 0;  // words; diag: one and two operand buffers
+  for (const auto& B : bl) {
+    const long long ex[3] = {B.nx, B.ny, B.nz}, mx = std::max(B.nx, std::max(B.ny, B.nz)) + 2;
+    whole = std::max(whole, 2LL * tdma_s_sxy(B.nx, B.ny) * (B.nz + 2) + mx * 32);
+    for (int axis = 0; axis < 3; ++axis) {
+      const long long nu = axis == 0 ? ex[1] : ex[0], nv = axis == 2 ? ex[1] : ex[2], n = ex[axis];
+      for (int k = 0; k < 2; ++k)
+        diag[k] = std::max(diag[k], 2 * (n + 2) * (nu + 2) + (k + 1) * (2 * (n + 2) + 2) * (nu + 2) + (n + 1) * 32);
+      lines = std::max(lines, std::min(nu, nv));
+      P.words = std::max(P.words, (tdma_rows((int)nu, (int)nv, (int)n) + 15) / 16 * 16);
+    }
+  }
+  if (lines > kTdmaThreads) return P;
+  if (whole * word <= kTdmaMaxSmem) {
+    P.mode = TdmaPlan::kWhole;
+    P.smem = (int)(whole * word);
+  } else if (diag[0] * word <= kTdmaMaxSmem) {
+    P.mode = TdmaPlan::kDiagonals;
+    P.nbuf = diag[1] * word <= kTdmaMaxSmem ? 2 : 1;
+    P.smem = (int)(diag[P.nbuf - 1] * word);
+  }
+  return P;
+}
+
+template <typename T>
+cudaError_t launch_tdma(const TdmaPlan& P, bool zero, const BlkLev* bl, CellTab all, const T* src, T* dst,
+                        const T* rhs, T* scratch, cudaStream_t st) {
+  const int nb = all.nb;
+  if (nb <= 0) return cudaSuccess;
+  if (P.mode == TdmaPlan::kWhole) {
+    pdl_launch(k_tdma_s<T>, nb, kTdmaThreads, (size_t)P.smem, st, bl, src, dst, rhs, zero);
+    return cudaGetLastError();
+  }
+  if (P.mode != TdmaPlan::kDiagonals) return cudaErrorInvalidValue;
+  const long long w = P.words;
+  const size_t sm = (size_t)P.smem;
+  T *a = scratch, *b = a + nb * w, *rows = b + nb * w;
+  pdl_launch(k_tdma_rows<T, -1, 1>, all.ncta, 256, 0, st, bl, all.cta_start, nb, src, rhs, b, a, rows, w, zero);
+  pdl_launch(k_tdma_g<T, 1>, nb, kTdmaThreads, sm, st, bl, a, rows, w, P.nbuf);
+  pdl_launch(k_tdma_rows<T, 1, 0>, all.ncta, 256, 0, st, bl, all.cta_start, nb, src, rhs, a, b, rows, w, zero);
+  pdl_launch(k_tdma_g<T, 0>, nb, kTdmaThreads, sm, st, bl, b, rows, w, P.nbuf);
+  pdl_launch(k_tdma_rows<T, 0, 2>, all.ncta, 256, 0, st, bl, all.cta_start, nb, src, rhs, b, a, rows, w, zero);
+  pdl_launch(k_tdma_g<T, 2>, nb, kTdmaThreads, sm, st, bl, a, rows, w, P.nbuf);
+  pdl_launch(k_tdma_level<T>, all.ncta, 256, 0, st, bl, all.cta_start, nb, a, dst, w);
+  return cudaGetLastError();
+}
+template cudaError_t launch_tdma<double>(const TdmaPlan&, bool, const BlkLev*, CellTab, const double*, double*,
+                                         const double*, double*, cudaStream_t);
+template cudaError_t launch_tdma<float>(const TdmaPlan&, bool, const BlkLev*, CellTab, const float*, float*, const float*,
+                                        float*, cudaStream_t);
 
 }  // namespace h3d
