@@ -1,0 +1,666 @@
+// Coarse levels of the V-cycle: relaxation visits of small levels in one launch
+// and the fused coarse end (one CTA, or one thread-block cluster).
+#include <cooperative_groups.h>
+
+#include <cstdint>
+#include <type_traits>
+
+#include "h3d_device.cuh"
+#include "h3d_kernels.cuh"
+
+namespace h3d {
+
+// ---------------------------------------------------------------------------
+// Several sweeps of a small level (mgrelax with `sweeps` iterations) in one
+// CTA, in place: per sweep the red cells (x+y+z odd), a barrier, the black
+// cells, a barrier, then the ghost fill from the level's sweep table (every
+// entry reads an interior cell, so the gather is order-free in place), a
+// barrier.  Same cell values as the out-of-place sweep + fill kernels: the
+// FP64 update keeps the reference's operand order and IEEE division.
+// zero: the iterate is known zero; it is cleared (ghosts included) first.
+// start[b]: first flat interior index of block b (start[nb] = all cells).
+// sb / ss: the block table and those starts, in shared memory.
+template <typename T, bool VAR>
+__device__ void small_relax(const BlkLev* sb, const int* ss, int nb, T* __restrict__ phi, const T* __restrict__ rhs,
+                            const T* __restrict__ fx, const T* __restrict__ fy, const T* __restrict__ fz,
+                            const uint32_t* __restrict__ fdst, const uint32_t* __restrict__ fsrc, int nfill,
+                            int sweeps, int zero, long long nelems, float om, int rb) {
+  const int ncell = ss[nb];
+  if (zero) {
+    for (long long q = threadIdx.x; q < nelems; q += blockDim.x) phi[q] = T(0);
+    __syncthreads();
+  }
+  for (int it = 0; it < sweeps; ++it) {
+    for (int colour = 1; colour >= 0; --colour) {  // red (x+y+z odd) first
+      for (int c = threadIdx.x; c < ncell; c += blockDim.x) {
+        int b = 0;
+        while (b + 1 < nb && ss[b + 1] <= c) ++b;
+        const BlkLev& B = sb[b];
+        const int local = c - ss[b];
+        const int x = 1 + local % B.nx, y = 1 + (local / B.nx) % B.ny, z = 1 + local / (B.nx * B.ny);
+        if (((x + y + z) & 1) != colour) continue;
+        const long long i = B.off + (long long)z * B.sxy + (long long)y * B.sx + x;
+        const Coef<T> cf = cell_coef<T, VAR>(B, x, y, z, i - B.off, VAR ? fx + B.off : nullptr,
+                                             VAR ? fy + B.off : nullptr, VAR ? fz + B.off : nullptr);
+        const T ap = coef_ap(cf);
+        T v = gs_div(rhs[i] - (cf.aw * phi[i - 1] + cf.ae * phi[i + 1] + cf.as * phi[i - B.sx] +
+                               cf.an * phi[i + B.sx] + cf.ab * phi[i - B.sxy] + cf.at * phi[i + B.sxy]),
+                     ap);
+        if constexpr (sizeof(T) == 4) v = sorf(phi[i], v, om);
+        phi[i] = v;
+      }
+      __syncthreads();
+      if (rb && colour == 1) {  // red-black order across block faces: the new red cells into the ghosts
+        for (int q = threadIdx.x; q < nfill; q += blockDim.x) phi[fdst[q]] = phi[fsrc[q] & kIdxMask];
+        __syncthreads();
+      }
+    }
+    for (int q = threadIdx.x; q < nfill; q += blockDim.x) phi[fdst[q]] = phi[fsrc[q] & kIdxMask];
+    __syncthreads();
+  }
+}
+
+// All sweeps of one relaxation visit of a level whose ghost fill stays inside
+// every block (independent blocks, a single block, periodic wraps onto
+// itself): one CTA per block, in place, the cell arithmetic of small_relax;
+// fill entries of block b are fstart[b] .. fstart[b+1]-1 (sources in block b).
+template <typename T, bool VAR>
+__global__ void __launch_bounds__(1024) k_relax_blocks(const BlkLev* __restrict__ bls, const int* __restrict__ fstart,
+                                                       T* __restrict__ phi, const T* __restrict__ rhs,
+                                                       const T* __restrict__ fx, const T* __restrict__ fy,
+                                                       const T* __restrict__ fz, const uint32_t* __restrict__ fdst,
+                                                       const uint32_t* __restrict__ fsrc, int sweeps, int zero,
+                                                       float om) {
+  pdl_trigger();
+  const BlkLev B = bls[blockIdx.x];
+  const int f0 = fstart[blockIdx.x], f1 = fstart[blockIdx.x + 1];
+  pdl_wait();
+  if (zero) {
+    const long long n = (long long)(B.nz + 2) * B.sxy;
+    for (long long q = threadIdx.x; q < n; q += blockDim.x) phi[B.off + q] = T(0);
+    __syncthreads();
+  }
+  const int ncell = B.nx * B.ny * B.nz;
+  for (int it = 0; it < sweeps; ++it) {
+    for (int colour = 1; colour >= 0; --colour) {  // red (x+y+z odd) first
+      for (int c = threadIdx.x; c < ncell; c += blockDim.x) {
+        const int x = 1 + c % B.nx, y = 1 + (c / B.nx) % B.ny, z = 1 + c / (B.nx * B.ny);
+        if (((x + y + z) & 1) != colour) continue;
+        const long long i = B.off + (long long)z * B.sxy + (long long)y * B.sx + x;
+        const Coef<T> cf = cell_coef<T, VAR>(B, x, y, z, i - B.off, VAR ? fx + B.off : nullptr,
+                                             VAR ? fy + B.off : nullptr, VAR ? fz + B.off : nullptr);
+        const T ap = coef_ap(cf);
+        T v = gs_div(rhs[i] - (cf.aw * phi[i - 1] + cf.ae * phi[i + 1] + cf.as * phi[i - B.sx] +
+                               cf.an * phi[i + B.sx] + cf.ab * phi[i - B.sxy] + cf.at * phi[i + B.sxy]),
+                     ap);
+        if constexpr (sizeof(T) == 4) v = sorf(phi[i], v, om);
+        phi[i] = v;
+      }
+      __syncthreads();
+    }
+    for (int q = f0 + threadIdx.x; q < f1; q += blockDim.x) phi[fdst[q]] = phi[fsrc[q] & kIdxMask];
+    __syncthreads();
+  }
+}
+
+template <typename T, bool VAR>
+__global__ void __launch_bounds__(1024) k_relax_small(const BlkLev* __restrict__ bls, const int* __restrict__ start,
+                                                      int nb, T* __restrict__ phi, const T* __restrict__ rhs,
+                                                      const T* __restrict__ fx, const T* __restrict__ fy,
+                                                      const T* __restrict__ fz, const uint32_t* __restrict__ fdst,
+                                                      const uint32_t* __restrict__ fsrc, int nfill, int sweeps,
+                                                      int zero, long long nelems, float om, int rb) {
+  pdl_trigger();
+  __shared__ BlkLev sb[kSmallLevelBlocks];
+  __shared__ int ss[kSmallLevelBlocks + 1];
+  // the block table and cell starts are written once at setup: read them
+  // while the predecessor finishes
+  for (int b = threadIdx.x; b < nb; b += blockDim.x) sb[b] = bls[b];
+  for (int b = threadIdx.x; b <= nb; b += blockDim.x) ss[b] = start[b];
+  pdl_wait();
+  __syncthreads();
+  small_relax<T, VAR>(sb, ss, nb, phi, rhs, fx, fy, fz, fdst, fsrc, nfill, sweeps, zero, nelems, om, rb);
+}
+
+// The fused coarse tail keeps every tail level in shared memory, in a
+// compact layout: the iterate as the padded blocks back to back (block b at
+// cbl[b].off, pitches nx+2 and (nx+2)(ny+2)), the rhs as the interior cells
+// in natural order (block b from cbl[b].pad).  Cells come from per-level
+// tables built at setup, one 64-bit entry a cell: compact index (bits 0-23),
+// x, y, z (bits 24-31, 32-39, 40-47) and block (bits 48-53); interior
+// tables list the red cells (x+y+z odd) first.
+struct CellRef {
+  int i, x, y, z, b;
+};
+__device__ __forceinline__ CellRef cell_ref(unsigned long long e) {
+  CellRef c;
+  c.i = (int)(e & 0xffffffull);
+  c.x = (int)((e >> 24) & 0xff);
+  c.y = (int)((e >> 32) & 0xff);
+  c.z = (int)((e >> 40) & 0xff);
+  c.b = (int)((e >> 48) & 0x3f);
+  return c;
+}
+__device__ __forceinline__ int rhs_index(const BlkLev& B, int x, int y, int z) {
+  return B.pad + ((z - 1) * B.ny + (y - 1)) * B.nx + (x - 1);
+}
+__device__ __forceinline__ long long global_index(const BlkLev& G, int x, int y, int z) {
+  return G.off + (long long)z * G.sxy + (long long)y * G.sx + x;
+}
+
+// The red then the black cells of one in-place sweep of a tail level; same
+// cell arithmetic as small_relax.
+template <typename T>
+__device__ void tail_colours(const BlkLev* cb, const TailLevel& L, T* phi, const T* rhs, int only = -1) {
+  for (int colour = 0; colour < 2; ++colour) {  // red (x+y+z odd) first
+    if (only >= 0 && colour != only) continue;
+    const int k0 = colour ? L.nred : 0, k1 = colour ? L.nint : L.nred;
+    for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
+      const CellRef c = cell_ref(L.cells[k]);
+      const BlkLev& B = cb[c.b];
+      const int i = c.i;
+      const Coef<T> cf = cell_coef<T, false>(B, c.x, c.y, c.z, i - B.off, nullptr, nullptr, nullptr);
+      const T ap = coef_ap(cf);
+      T v = gs_div(rhs[rhs_index(B, c.x, c.y, c.z)] -
+                       (cf.aw * phi[i - 1] + cf.ae * phi[i + 1] + cf.as * phi[i - B.sx] +
+                        cf.an * phi[i + B.sx] + cf.ab * phi[i - B.sxy] + cf.at * phi[i + B.sxy]),
+                   ap);
+      if constexpr (sizeof(T) == 4) v = sorf(phi[i], v, L.om);
+      phi[i] = v;
+    }
+    __syncthreads();
+  }
+}
+
+// `sweeps` in-place red-black sweeps of a tail level, each followed by its
+// ghost fill.
+template <typename T>
+__device__ void tail_relax(const BlkLev* cb, const TailLevel& L, T* phi, const T* rhs, int sweeps) {
+  for (int it = 0; it < sweeps; ++it) {
+    if (L.rb_global) {  // a fill after each colour: the red-black order across block faces
+      for (int colour = 0; colour < 2; ++colour) {
+        tail_colours<T>(cb, L, phi, rhs, colour);
+        for (int q = threadIdx.x; q < L.nfill; q += blockDim.x) phi[L.fdst[q]] = phi[L.fsrc[q]];
+        __syncthreads();
+      }
+      continue;
+    }
+    tail_colours<T>(cb, L, phi, rhs);
+    for (int q = threadIdx.x; q < L.nfill; q += blockDim.x) phi[L.fdst[q]] = phi[L.fsrc[q]];
+    __syncthreads();
+  }
+}
+
+// mgrestr into a tail level: the same residual sum over the eight children,
+// in the same order, as k_restrict; one thread a coarse cell.
+template <typename T>
+__device__ void tail_restrict(const BlkLev* fb, const BlkLev* cb, const TailLevel& Cl, const T* phi, const T* rhs,
+                              T* rhs_c, int zero_fine) {
+  for (int k = threadIdx.x; k < Cl.nint; k += blockDim.x) {
+    const CellRef cc = cell_ref(Cl.cells[k]);
+    const BlkLev& F = fb[cc.b];
+    const int X = cc.x, Y = cc.y, Z = cc.z;
+    const T* P = phi + F.off;
+    T sum = T(0);
+#pragma unroll
+    for (int dk = 0; dk < 2; ++dk)
+#pragma unroll
+      for (int dj = 0; dj < 2; ++dj)
+#pragma unroll
+        for (int di = 0; di < 2; ++di) {
+          const int x = 2 * X - 1 + di, y = 2 * Y - 1 + dj, z = 2 * Z - 1 + dk;
+          const int i = z * (int)F.sxy + y * F.sx + x;
+          const T rv = rhs[rhs_index(F, x, y, z)];
+          T r;
+          if (zero_fine) {
+            r = rv - T(0);
+          } else {
+            Coef<T> cf = cell_coef<T, false>(F, x, y, z, i, nullptr, nullptr, nullptr);
+            const T ap = coef_ap(cf);
+            r = rv - (cf.aw * P[i - 1] + cf.ae * P[i + 1] + cf.as * P[i - F.sx] + cf.an * P[i + F.sx] +
+                      cf.ab * P[i - F.sxy] + cf.at * P[i + F.sxy] + ap * P[i]);
+          }
+          sum = (di | dj | dk) ? sum + r : r;
+        }
+    rhs_c[rhs_index(cb[cc.b], X, Y, Z)] = T(0.125) * sum;
+  }
+  __syncthreads();
+}
+
+// mgcorr + mgbound of cell (x, y, z) (ghosts included) of block F: the value
+// k_prolong writes there, reading the old iterate from `old`.
+template <typename T>
+__device__ __forceinline__ T tail_prolong_value(const BlkLev& F, const BlkLev& C, const T* phi_c, const T* old, int x,
+                                                int y, int z, int zero_old) {
+  const int ph = F.phys;
+  int sx = x, sy = y, sz = z;
+  if (x == 0 && (ph & 1)) sx = 1;
+  if (x == F.nx + 1 && (ph & 2)) sx = F.nx;
+  if (y == 0 && (ph & 4)) sy = 1;
+  if (y == F.ny + 1 && (ph & 8)) sy = F.ny;
+  if (z == 0 && (ph & 16)) sz = 1;
+  if (z == F.nz + 1 && (ph & 32)) sz = F.nz;
+  const T wx0 = (sx & 1) ? T(1) : T(3), wx1 = (sx & 1) ? T(3) : T(1);
+  const T wy0 = (sy & 1) ? T(1) : T(3), wy1 = (sy & 1) ? T(3) : T(1);
+  const T wz0 = (sz & 1) ? T(1) : T(3), wz1 = (sz & 1) ? T(3) : T(1);
+  const int cy = C.sx, cz = (int)C.sxy;
+  const T* Q = phi_c + C.off + (sz >> 1) * cz + (sy >> 1) * cy + (sx >> 1);
+  // term order (di,dj,dk): 000, 010, 001, 011, 100, 110, 101, 111
+  T s = (wx0 * wy0 * wz0) * Q[0];
+  s = s + (wx0 * wy1 * wz0) * Q[cy];
+  s = s + (wx0 * wy0 * wz1) * Q[cz];
+  s = s + (wx0 * wy1 * wz1) * Q[cy + cz];
+  s = s + (wx1 * wy0 * wz0) * Q[1];
+  s = s + (wx1 * wy1 * wz0) * Q[1 + cy];
+  s = s + (wx1 * wy0 * wz1) * Q[1 + cz];
+  s = s + (wx1 * wy1 * wz1) * Q[1 + cy + cz];
+  const T o = zero_old ? T(0) : old[F.off + sz * (int)F.sxy + sy * F.sx + sx];
+  return o + s / T(64);
+}
+
+// mgcorr + mgbound into a tail level in place: the ghost cells read interior
+// and ghost cells of the old iterate, so their new values go to `scratch`
+// (one value a ghost-table entry) first; then the interior cells (each reads
+// only itself) update in place, then the ghosts are copied back.
+template <typename T>
+__device__ void tail_prolong(const BlkLev* fb, const BlkLev* cb, const TailLevel& F, const T* phi_c, T* phi,
+                             T* scratch, int zero_old) {
+  for (int k = threadIdx.x; k < F.nghost; k += blockDim.x) {
+    const CellRef c = cell_ref(F.ghosts[k]);
+    scratch[k] = tail_prolong_value(fb[c.b], cb[c.b], phi_c, phi, c.x, c.y, c.z, zero_old);
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < F.nint; k += blockDim.x) {
+    const CellRef c = cell_ref(F.cells[k]);
+    phi[c.i] = tail_prolong_value(fb[c.b], cb[c.b], phi_c, phi, c.x, c.y, c.z, zero_old);
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < F.nghost; k += blockDim.x) phi[(int)(F.ghosts[k] & 0xffffffull)] = scratch[k];
+  __syncthreads();
+}
+
+// The rhs of a tail level from global memory (the restriction into the
+// first tail level ran outside); eight loads in flight a thread.
+template <typename T>
+__device__ void tail_load_rhs(const BlkLev* gb, const BlkLev* cb, const TailLevel& L, const T* __restrict__ g, T* rhs) {
+  constexpr int U = 8;
+  for (int k0 = threadIdx.x; k0 < L.nint; k0 += U * blockDim.x) {
+    T v[U];
+    int ri[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = k0 + u * blockDim.x;
+      ri[u] = -1;
+      if (k < L.nint) {
+        const CellRef c = cell_ref(L.cells[k]);
+        v[u] = g[global_index(gb[c.b], c.x, c.y, c.z)];
+        ri[u] = rhs_index(cb[c.b], c.x, c.y, c.z);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (ri[u] >= 0) rhs[ri[u]] = v[u];
+  }
+  __syncthreads();
+}
+
+// A tail level back to global memory: iterate (interior and ghost cells) and rhs.
+template <typename T>
+__device__ void tail_store(const BlkLev* gb, const BlkLev* cb, const TailLevel& L, const T* phi, const T* rhs,
+                           T* __restrict__ gphi, T* __restrict__ grhs) {
+  for (int k = threadIdx.x; k < L.nint + L.nghost; k += blockDim.x) {
+    const CellRef c = cell_ref(k < L.nint ? L.cells[k] : L.ghosts[k - L.nint]);
+    const long long gi = global_index(gb[c.b], c.x, c.y, c.z);
+    gphi[gi] = phi[c.i];
+    if (k < L.nint) grhs[gi] = rhs[rhs_index(cb[c.b], c.x, c.y, c.z)];
+  }
+  __syncthreads();
+}
+
+// The coarse end of a V-cycle in one CTA, every level in shared memory: the
+// relaxations, restrictions, precision conversions and corrections of the
+// tail levels run as the ops of a program built on the host, in order, with
+// the CTA's barriers between them instead of kernel boundaries; one op loads
+// the first tail level's rhs, the last ones store every tail level.
+// curmask bit 2l (2l+1) selects the global FP32 (FP64) iterate buffer of
+// tail level l.
+__global__ void __launch_bounds__(1024) k_coarse_tail(const TailLevel* __restrict__ lv, const TailOp* __restrict__ ops,
+                                                      int nops, unsigned curmask) {
+  pdl_trigger();
+  __shared__ BlkLev fb[kSmallLevelBlocks], cb[kSmallLevelBlocks], gb[kSmallLevelBlocks];
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* arena = smem_base128(smem_raw);
+  pdl_wait();
+  for (int o = 0; o < nops; ++o) {
+    const TailOp op = ops[o];
+    const TailLevel& F = lv[op.fine];
+    const TailLevel& C = lv[op.coarse];
+    const int nb = F.nb;
+    __syncthreads();  // the previous op is done with the tables
+    for (int b = threadIdx.x; b < nb; b += blockDim.x) {
+      fb[b] = F.cbl[b];
+      cb[b] = C.cbl[b];
+      gb[b] = F.gbl[b];
+    }
+    __syncthreads();
+    auto at32 = [&](int off) { return reinterpret_cast<float*>(arena + off); };
+    auto at64 = [&](int off) { return reinterpret_cast<double*>(arena + off); };
+    switch (op.kind) {
+      case kTailLoadRhs:
+        if (op.f64) tail_load_rhs<double>(gb, fb, F, F.rhs64, at64(F.s_rhs64));
+        else tail_load_rhs<float>(gb, fb, F, F.rhs32, at32(F.s_rhs32));
+        break;
+      case kTailRelax:
+        if (op.f64) {
+          double* phi = at64(F.s_phi64);
+          if (op.zero) {
+            for (int q = threadIdx.x; q < F.npad; q += blockDim.x) phi[q] = 0.0;
+            __syncthreads();
+          }
+          tail_relax<double>(fb, F, phi, at64(F.s_rhs64), op.sweeps);
+        } else {
+          float* phi = at32(F.s_phi32);
+          if (op.zero) {
+            for (int q = threadIdx.x; q < F.npad; q += blockDim.x) phi[q] = 0.f;
+            __syncthreads();
+          }
+          tail_relax<float>(fb, F, phi, at32(F.s_rhs32), op.sweeps);
+        }
+        break;
+      case kTailRestrict:  // into the coarse rhs of the fine level's precision
+        if (op.f64) tail_restrict<double>(fb, cb, C, at64(F.s_phi64), at64(F.s_rhs64), at64(C.s_rhs64), op.zero);
+        else tail_restrict<float>(fb, cb, C, at32(F.s_phi32), at32(F.s_rhs32), at32(C.s_rhs32), op.zero);
+        break;
+      case kTailProlong:
+        if (op.f64)
+          tail_prolong<double>(fb, cb, F, at64(C.s_phi64), at64(F.s_phi64), at64(op.sweeps), op.zero);
+        else
+          tail_prolong<float>(fb, cb, F, at32(C.s_phi32), at32(F.s_phi32), at32(op.sweeps), op.zero);
+        break;
+      case kTailRhsF2D: {  // the coarsest rhs of a mixed solve to FP64
+        const float* a = at32(F.s_rhs32);
+        double* b = at64(F.s_rhs64);
+        for (int q = threadIdx.x; q < F.nint; q += blockDim.x) b[q] = (double)a[q];
+        __syncthreads();
+        break;
+      }
+      case kTailPhiD2F: {  // the coarsest iterate of a mixed solve to FP32
+        const double* a = at64(F.s_phi64);
+        float* b = at32(F.s_phi32);
+        for (int q = threadIdx.x; q < F.npad; q += blockDim.x) b[q] = (float)a[q];
+        __syncthreads();
+        break;
+      }
+      case kTailStore: {
+        const int c32 = (curmask >> (2 * op.fine)) & 1, c64 = (curmask >> (2 * op.fine + 1)) & 1;
+        if (F.s_phi32 >= 0) tail_store<float>(gb, fb, F, at32(F.s_phi32), at32(F.s_rhs32), F.phi32[c32], F.rhs32);
+        if (F.s_phi64 >= 0) tail_store<double>(gb, fb, F, at64(F.s_phi64), at64(F.s_rhs64), F.phi64[c64], F.rhs64);
+        break;
+      }
+      default:
+        break;
+    }
+  }
+}
+
+// The coarse end of a V-cycle as one thread-block cluster: CTA b holds block
+// b of every tail level in its shared memory (compact layout, every block of
+// a level the same size) and runs the same op program as k_coarse_tail on
+// it.  Restrictions, corrections and conversions only touch the CTA's own
+// block; after the colours of a sweep the cluster synchronises, every CTA
+// gathers its ghost cells from the other CTAs' shared memory (fdst: own
+// compact index; fsrc: source rank << 24 | its compact index), and the
+// cluster synchronises again before any interior changes.
+__global__ void __launch_bounds__(kClusterTailThreads) k_coarse_cluster(const TailLevel* __restrict__ lvg,
+                                                                        const TailOp* __restrict__ opsg, int nops,
+                                                                        int nlev, unsigned curmask) {
+  pdl_trigger();
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  const int b = (int)cl.block_rank();
+  __shared__ TailLevel lv[kTailMaxLevels];
+  __shared__ BlkLev gtab[kTailMaxLevels], ctab[kTailMaxLevels];  // this block per level: global / compact layout
+  __shared__ TailOp ops[kClusterTailMaxOps];
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* arena = smem_base128(smem_raw);
+  // the program, the level records and this block's tables are setup data:
+  // stage them in shared memory (cell and ghost tables, this block's fill
+  // entries) while the predecessor finishes
+  for (int q = threadIdx.x; q < nops; q += blockDim.x) ops[q] = opsg[q];
+  if (threadIdx.x < nlev) lv[threadIdx.x] = lvg[threadIdx.x];
+  __syncthreads();
+  for (int l = 0; l < nlev; ++l) {
+    const TailLevel& G = lvg[l];
+    unsigned long long* cs = reinterpret_cast<unsigned long long*>(arena + lv[l].s_cells);
+    for (int k = threadIdx.x; k < G.nint + G.nghost; k += blockDim.x)
+      cs[k] = k < G.nint ? __ldg(G.cells + k) : __ldg(G.ghosts + (k - G.nint));
+    const int f0 = __ldg(G.fstart + b), f1 = __ldg(G.fstart + b + 1);
+    uint32_t* fd = reinterpret_cast<uint32_t*>(arena + lv[l].s_fill);
+    for (int k = threadIdx.x; k < f1 - f0; k += blockDim.x) {
+      fd[2 * k] = __ldg(G.fdst + f0 + k);
+      fd[2 * k + 1] = __ldg(G.fsrc + f0 + k);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      lv[l].cells = cs;
+      lv[l].ghosts = cs + G.nint;
+      lv[l].fdst = fd;
+      lv[l].nfill = f1 - f0;
+    }
+  }
+  __syncthreads();
+  pdl_wait();
+  auto compact = [](BlkLev B) {
+    B.off = 0;
+    B.sx = B.nx + 2;
+    B.sxy = (long long)(B.nx + 2) * (B.ny + 2);
+    B.pad = 0;
+    return B;
+  };
+  if (threadIdx.x < nlev) {
+    const BlkLev G = lvg[threadIdx.x].gbl[b];
+    gtab[threadIdx.x] = G;
+    ctab[threadIdx.x] = compact(G);
+  }
+  __syncthreads();
+  for (int o = 0; o < nops; ++o) {
+    const TailOp op = ops[o];
+    const TailLevel& F = lv[op.fine];
+    const TailLevel& C = lv[op.coarse];
+    // this block's tables at the op's levels (staged once; every op ends with
+    // a barrier of the CTA or the cluster)
+    const BlkLev* gb = gtab + op.fine;
+    const BlkLev* fb = ctab + op.fine;
+    const BlkLev* cb = ctab + op.coarse;
+    auto at32 = [&](int off) { return reinterpret_cast<float*>(arena + off); };
+    auto at64 = [&](int off) { return reinterpret_cast<double*>(arena + off); };
+    switch (op.kind) {
+      case kTailLoadRhs:
+        if (op.f64) tail_load_rhs<double>(gb, fb, F, F.rhs64, at64(F.s_rhs64));
+        else tail_load_rhs<float>(gb, fb, F, F.rhs32, at32(F.s_rhs32));
+        break;
+      case kTailRelax: {
+        auto relax = [&](auto* phi, const auto* rhs) {
+          using T = typename std::remove_pointer<decltype(phi)>::type;
+          if (op.zero) {
+            for (int q = threadIdx.x; q < F.npad; q += blockDim.x) phi[q] = T(0);
+            __syncthreads();
+          }
+          const int ncol = F.rb_global ? 2 : 1;  // 2: a fill after each colour (order across blocks)
+          for (int it = 0; it < op.sweeps; ++it) {
+            for (int pass = 0; pass < ncol; ++pass) {
+              tail_colours<T>(fb, F, phi, rhs, ncol == 2 ? pass : -1);
+              cl.sync();  // every block's sweep done
+              for (int q = threadIdx.x; q < F.nfill; q += blockDim.x) {  // (dst, src) pairs of this block
+                const uint32_t dsti = F.fdst[2 * q], src = F.fdst[2 * q + 1];
+                const T* remote = cl.map_shared_rank(phi, (int)(src >> 24));
+                phi[dsti] = remote[src & 0xffffffu];
+              }
+              cl.sync();  // every ghost gathered before any interior changes
+            }
+          }
+        };
+        if (op.f64) relax(at64(F.s_phi64), (const double*)at64(F.s_rhs64));
+        else relax(at32(F.s_phi32), (const float*)at32(F.s_rhs32));
+        break;
+      }
+      case kTailDense: {  // x = P b over the cells of every block (FP64), then the sweep fill
+        double* phi = at64(F.s_phi64);
+        const double* rhs = at64(F.s_rhs64);
+        if (op.zero) {
+          for (int q = threadIdx.x; q < F.npad; q += blockDim.x) phi[q] = 0.0;
+        }
+        cl.sync();  // every block's rhs is complete
+        const int nper = F.nint, n = F.dense_n;
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+        const BlkLev& B = fb[0];
+        for (int i = warp; i < nper; i += nwarp) {  // a warp per row of this block; lanes split the columns
+          const double* Pr = F.dense + (long long)(b * nper + i) * n;
+          double s = 0.0;
+          for (int j = lane; j < n; j += 32) {
+            const double* r = cl.map_shared_rank(rhs, j / nper);
+            s += __ldg(Pr + j) * r[j % nper];
+          }
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+          if (lane == 0) {
+            const int x = i % B.nx + 1, y = (i / B.nx) % B.ny + 1, z = i / (B.nx * B.ny) + 1;
+            phi[(long long)z * B.sxy + (long long)y * B.sx + x] = s;
+          }
+        }
+        cl.sync();  // every block's interior is written
+        for (int q = threadIdx.x; q < F.nfill; q += blockDim.x) {
+          const uint32_t dsti = F.fdst[2 * q], src = F.fdst[2 * q + 1];
+          const double* remote = cl.map_shared_rank(phi, (int)(src >> 24));
+          phi[dsti] = remote[src & 0xffffffu];
+        }
+        cl.sync();  // every ghost gathered before any interior changes
+        break;
+      }
+      case kTailRestrict:
+        if (op.f64) tail_restrict<double>(fb, cb, C, at64(F.s_phi64), at64(F.s_rhs64), at64(C.s_rhs64), op.zero);
+        else tail_restrict<float>(fb, cb, C, at32(F.s_phi32), at32(F.s_rhs32), at32(C.s_rhs32), op.zero);
+        break;
+      case kTailProlong:
+        if (op.f64) tail_prolong<double>(fb, cb, F, at64(C.s_phi64), at64(F.s_phi64), at64(op.sweeps), op.zero);
+        else tail_prolong<float>(fb, cb, F, at32(C.s_phi32), at32(F.s_phi32), at32(op.sweeps), op.zero);
+        break;
+      case kTailRhsF2D: {
+        const float* x = at32(F.s_rhs32);
+        double* y = at64(F.s_rhs64);
+        for (int q = threadIdx.x; q < F.nint; q += blockDim.x) y[q] = (double)x[q];
+        __syncthreads();
+        break;
+      }
+      case kTailPhiD2F: {
+        const double* x = at64(F.s_phi64);
+        float* y = at32(F.s_phi32);
+        for (int q = threadIdx.x; q < F.npad; q += blockDim.x) y[q] = (float)x[q];
+        __syncthreads();
+        break;
+      }
+      case kTailStore: {
+        const int c32 = (curmask >> (2 * op.fine)) & 1, c64 = (curmask >> (2 * op.fine + 1)) & 1;
+        if (F.s_phi32 >= 0) tail_store<float>(gb, fb, F, at32(F.s_phi32), at32(F.s_rhs32), F.phi32[c32], F.rhs32);
+        if (F.s_phi64 >= 0) tail_store<double>(gb, fb, F, at64(F.s_phi64), at64(F.s_rhs64), F.phi64[c64], F.rhs64);
+        break;
+      }
+      default:
+        break;
+    }
+  }
+  cl.sync();  // no CTA leaves while another may still read its shared memory
+}
+
+cudaError_t coarse_tail_attributes() {
+  cudaError_t e = cudaFuncSetAttribute(k_coarse_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmemBytes);
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(k_coarse_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmemBytes);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(k_coarse_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+}
+
+static cudaError_t cluster_config(int nb, int smem_bytes, cudaStream_t st, cudaLaunchConfig_t* cfg,
+                                  cudaLaunchAttribute* at) {
+  *cfg = cudaLaunchConfig_t{};
+  cfg->gridDim = dim3(nb);
+  cfg->blockDim = dim3(kClusterTailThreads);
+  cfg->dynamicSmemBytes = (size_t)smem_bytes;
+  cfg->stream = st;
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = nb;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg->attrs = at;
+  cfg->numAttrs = 1;
+  return cudaSuccess;
+}
+
+int coarse_cluster_fits(int nb, int smem_bytes) {
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at[1];
+  cluster_config(nb, smem_bytes, nullptr, &cfg, at);
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, k_coarse_cluster, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return n;
+}
+
+cudaError_t launch_coarse_cluster(int nb, const TailLevel* lv, int nlev, const TailOp* ops, int nops,
+                                  unsigned curmask, int smem_bytes, cudaStream_t st) {
+  if (nops <= 0 || nops > kClusterTailMaxOps || nlev > kTailMaxLevels) return cudaErrorInvalidValue;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at[1];
+  cluster_config(nb, smem_bytes, st, &cfg, at);
+  return cudaLaunchKernelEx(&cfg, k_coarse_cluster, lv, ops, nops, nlev, curmask);
+}
+
+cudaError_t launch_coarse_tail(const TailLevel* lv, const TailOp* ops, int nops, unsigned curmask, int smem_bytes,
+                               cudaStream_t st) {
+  if (nops <= 0) return cudaSuccess;
+  pdl_launch(k_coarse_tail, 1, 1024, (size_t)smem_bytes, st, lv, ops, nops, curmask);
+  return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t launch_relax_small(bool var, const BlkLev* bl, const int* start, int nb, T* phi, const T* rhs,
+                               const T* fx, const T* fy, const T* fz, const uint32_t* fdst, const uint32_t* fsrc,
+                               int nfill, int sweeps, bool zero, long long nelems, float om, bool rb,
+                               cudaStream_t st) {
+  if (var)
+    pdl_launch(k_relax_small<T, true>, 1, 1024, 0, st, bl, start, nb, phi, rhs, fx, fy, fz, fdst, fsrc, nfill, sweeps,
+               (int)zero, nelems, om, (int)rb);
+  else
+    pdl_launch(k_relax_small<T, false>, 1, 1024, 0, st, bl, start, nb, phi, rhs, fx, fy, fz, fdst, fsrc, nfill,
+               sweeps, (int)zero, nelems, om, (int)rb);
+  return cudaGetLastError();
+}
+template <typename T>
+cudaError_t launch_relax_blocks(bool var, const BlkLev* bl, int nb, const int* fstart, T* phi, const T* rhs,
+                                const T* fx, const T* fy, const T* fz, const uint32_t* fdst, const uint32_t* fsrc,
+                                int sweeps, bool zero, float om, cudaStream_t st) {
+  if (nb <= 0) return cudaSuccess;
+  if (var)
+    pdl_launch(k_relax_blocks<T, true>, nb, 1024, 0, st, bl, fstart, phi, rhs, fx, fy, fz, fdst, fsrc, sweeps,
+               (int)zero, om);
+  else
+    pdl_launch(k_relax_blocks<T, false>, nb, 1024, 0, st, bl, fstart, phi, rhs, fx, fy, fz, fdst, fsrc, sweeps,
+               (int)zero, om);
+  return cudaGetLastError();
+}
+template cudaError_t launch_relax_blocks<double>(bool, const BlkLev*, int, const int*, double*, const double*,
+                                                 const double*, const double*, const double*, const uint32_t*,
+                                                 const uint32_t*, int, bool, float, cudaStream_t);
+template cudaError_t launch_relax_blocks<float>(bool, const BlkLev*, int, const int*, float*, const float*,
+                                                const float*, const float*, const float*, const uint32_t*,
+                                                const uint32_t*, int, bool, float, cudaStream_t);
+template cudaError_t launch_relax_small<double>(bool, const BlkLev*, const int*, int, double*, const double*,
+                                                const double*, const double*, const double*, const uint32_t*,
+                                                const uint32_t*, int, int, bool, long long, float, bool, cudaStream_t);
+template cudaError_t launch_relax_small<float>(bool, const BlkLev*, const int*, int, float*, const float*,
+                                               const float*, const float*, const float*, const uint32_t*,
+                                               const uint32_t*, int, int, bool, long long, float, bool, cudaStream_t);
+
+}  // namespace h3d

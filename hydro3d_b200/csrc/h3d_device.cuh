@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <cstdint>
 #include <cstdlib>
 
 #include "h3d_internal.h"
@@ -104,5 +105,21 @@ __device__ __forceinline__ T coef_ap(const Coef<T>& c) {
 // arithmetic); the FP32 inner solve uses the 2-ulp reciprocal division.
 __device__ __forceinline__ double gs_div(double a, double b) { return a / b; }
 __device__ __forceinline__ float gs_div(float a, float b) { return __fdividef(a, b); }
+
+// Over-relaxed red-black update of the FP32 inner solve: x + om (gs - x), om
+// the handle's over-relaxation factor (1: Gauss-Seidel up to rounding).  The
+// FP64 sweeps keep the reference's update.
+__device__ __forceinline__ float sorf(float old, float gs, float om) { return fmaf(om, gs - old, old); }
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+
+// First 128-byte boundary of the dynamic shared memory, by pointer arithmetic
+// on the shared array itself so that accesses through it stay shared-memory
+// instructions (a round trip through an integer would make them generic).
+__device__ __forceinline__ unsigned char* smem_base128(unsigned char* raw) {
+  return raw + ((128u - (smem_u32(raw) & 127u)) & 127u);
+}
 
 }  // namespace h3d
