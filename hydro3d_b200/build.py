@@ -12,6 +12,7 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
@@ -61,7 +62,7 @@ def build(verbose: bool = False, ptxas_info: bool = False) -> str:
     if debug:
         base += ["-DH3D_BOUNDS_CHECK"]
     hdrs = [os.path.join(CSRC, h) for h in HEADERS] + [os.path.join(ROOT, "include", "h3d_mg.h")]
-    objs = []
+    objs, cmds = [], []
     for src in SOURCES:
         s = os.path.join(CSRC, src)
         o = os.path.join(BUILD, src + (".dbg.o" if debug else ".o"))
@@ -70,7 +71,10 @@ def build(verbose: bool = False, ptxas_info: bool = False) -> str:
             cmd = base + ["-c", s, "-o", o]
             if verbose:
                 print(" ".join(cmd))
-            subprocess.run(cmd, check=True)
+            cmds.append(cmd)
+    with ThreadPoolExecutor() as pool:  # one compiler a file
+        for _ in pool.map(lambda c: subprocess.run(c, check=True), cmds):
+            pass
     stamp = os.path.join(BUILD, "flavor")
     flavor = "debug" if debug else "release"
     last = open(stamp).read() if os.path.exists(stamp) else ""

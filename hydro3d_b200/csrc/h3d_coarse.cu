@@ -2,8 +2,10 @@
 // and the fused coarse end (one CTA, or one thread-block cluster).
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <type_traits>
+#include <vector>
 
 #include "h3d_device.cuh"
 #include "h3d_kernels.cuh"
@@ -60,6 +62,124 @@ __device__ void small_relax(const BlkLev* sb, const int* ss, int nb, T* __restri
   }
 }
 
+// ---------------------------------------------------------------------------
+// Exact division by a known divisor: a / b correctly rounded, as the IEEE
+// division the reference's update uses, from y = RN(1/b): q = RN(a y) is at most two
+// units off, one residual step q + (a - b q) y makes it faithful, a second one
+// correctly rounded (P. Markstein, Computation of elementary functions on the IBM
+// RISC System/6000 processor, 1990).  The residuals are exact while nothing
+// under- or overflows: other operands take the division itself.  Five
+// multiply-adds where the division is a subroutine.
+__device__ __forceinline__ bool div_range(double v) {
+  return ((unsigned)(__double2hiint(v) >> 20) & 0x7ffu) - 523u < 1000u;  // 2^-500 <= |v| < 2^500
+}
+__device__ __forceinline__ double div_known(double a, double b, double y) {
+  double q = a * y;
+  q = fma(fma(-b, q, a), y, q);
+  q = fma(fma(-b, q, a), y, q);
+  return __builtin_expect(div_range(a) && div_range(b), 1) ? q : a / b;
+}
+
+// One update of a cell of a constant-coefficient level: sum of the neighbours in
+// the reference's order (FP64), fused in FP32.
+__device__ __forceinline__ double cell_update(const double* p, int sx, int sxy, double ax, double ay, double az,
+                                              double r, double ap, double inv, float) {
+  return div_known(r - (ax * p[-1] + ax * p[1] + ay * p[-sx] + ay * p[sx] + az * p[-sxy] + az * p[sxy]), ap, inv);
+}
+__device__ __forceinline__ float cell_update(const float* p, int sx, int sxy, float ax, float ay, float az, float r,
+                                             float, float inv, float om) {
+  const float s = fmaf(az, p[sxy], fmaf(az, p[-sxy], fmaf(ay, p[sx], fmaf(ay, p[-sx], fmaf(ax, p[1], ax * p[-1])))));
+  return sorf(p[0], (r - s) * inv, om);
+}
+
+// Relaxation of one block in shared memory (compact layout, constant
+// coefficients) with its cells resident in registers: a thread owns K pairs of
+// x-neighbours, one red and one black cell each, and keeps their places and
+// right-hand sides for all sweeps, so that a colour is six loads, the sum, five
+// multiply-adds and a store.  (The table-driven form decoded a cell entry,
+// selected six coefficients and divided for every update: 1.2 us a colour of 512
+// cells in FP64, 0.25 us here.)  The caller has zeroed the ghosts of physical walls, whose
+// faces have a zero coefficient, so all cells use the interior ones.
+// rhs_at(x, y, z): right-hand side.  fill(last): after the black cells (ncol 2:
+// after each colour), a barrier, the ghosts the next sweep reads, or all of them
+// after the last sweep, and a barrier.
+// diag: 128 words of shared memory (diagonal and reciprocal by wall faces).
+template <typename T, int K, typename Rhs, typename Fill>
+__device__ __forceinline__ void relax_resident(const BlkLev& B, T* phi, T* diag, Rhs&& rhs_at, int sweeps, float om,
+                                               int ncol, Fill&& fill) {
+  const int nx = B.nx, ny = B.ny, nz = B.nz, hx = (nx + 1) / 2, np = hx * ny * nz;
+  const int sx = nx + 2, sxy = sx * (ny + 2);
+  const T ax = (T)B.ax, ay = (T)B.ay, az = (T)B.az;
+  if (threadIdx.x < 64) {
+    const int m = threadIdx.x;
+    Coef<T> c;
+    c.aw = m & 1 ? T(0) : ax;
+    c.ae = m & 2 ? T(0) : ax;
+    c.as = m & 4 ? T(0) : ay;
+    c.an = m & 8 ? T(0) : ay;
+    c.ab = m & 16 ? T(0) : az;
+    c.at = m & 32 ? T(0) : az;
+    diag[2 * m] = coef_ap(c);
+    diag[2 * m + 1] = T(1) / coef_ap(c);
+  }
+  int at[2][K];  // place in phi (24 bits), wall faces above
+  T r[2][K];
+#pragma unroll
+  for (int j = 0; j < K; ++j) {
+    const int p = threadIdx.x + j * blockDim.x;
+    const int xp = p % hx, y = (p / hx) % ny + 1, z = p / (hx * ny) + 1;
+    const int odd = (1 + y + z) & 1;  // the first cell of the pair is red (x+y+z odd)
+    const int m = (y == 1 ? 4 : 0) | (y == ny ? 8 : 0) | (z == 1 ? 16 : 0) | (z == nz ? 32 : 0);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const int x = 2 * xp + (c == 0 ? 2 - odd : 1 + odd);
+      const bool in = p < np && x <= nx;
+      const int w = (m | (x == 1 ? 1 : 0) | (x == nx ? 2 : 0)) & B.phys;
+      at[c][j] = in ? (z * sxy + y * sx + x) | w << 24 : -1;
+      r[c][j] = in ? rhs_at(x, y, z) : T(0);
+    }
+  }
+  __syncthreads();
+  for (int it = 0; it < sweeps; ++it) {
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      T v[K];
+#pragma unroll
+      for (int j = 0; j < K; ++j)
+        if (at[c][j] >= 0) {
+          const int w = at[c][j] >> 24;
+          v[j] = cell_update(phi + (at[c][j] & 0xffffff), sx, sxy, ax, ay, az, r[c][j], diag[2 * w], diag[2 * w + 1],
+                             om);
+        }
+#pragma unroll
+      for (int j = 0; j < K; ++j)
+        if (at[c][j] >= 0) phi[at[c][j] & 0xffffff] = v[j];
+      if (c == 1) fill(it + 1 == sweeps);
+      else if (ncol == 2) fill(false);
+      else __syncthreads();
+    }
+  }
+}
+
+// Sweeps of a visit from which relax_resident pays in the fused coarse end: its
+// code and set-up, cold in every launch, cost about 10 us there (2 to 3 sweeps a level: 39.7
+// us with the tables, 52 us resident; 32 sweeps of 512 cells: a solve of
+// eight such launches 1.18 against 0.98 ms).
+constexpr int kResidentSweeps = 8;
+
+// Pairs a thread needs for a block (relax_resident), or 0: more than four.
+__device__ __forceinline__ int resident_pairs(const BlkLev& B) {
+  const int np = (B.nx + 1) / 2 * B.ny * B.nz, k = (np + (int)blockDim.x - 1) / (int)blockDim.x;
+  return k <= 1 ? 1 : k <= 2 ? 2 : k <= 4 ? 4 : 0;
+}
+
+// True for the ghost cell (x, y, z) of a physical wall.
+__device__ __forceinline__ bool wall_ghost(const BlkLev& B, int x, int y, int z) {
+  const int ph = B.phys;
+  return (x == 0 && (ph & 1)) || (x == B.nx + 1 && (ph & 2)) || (y == 0 && (ph & 4)) || (y == B.ny + 1 && (ph & 8)) ||
+         (z == 0 && (ph & 16)) || (z == B.nz + 1 && (ph & 32));
+}
+
 // All sweeps of one relaxation visit of a level whose ghost fill stays inside
 // every block (independent blocks, a single block, periodic wraps onto
 // itself): one CTA per block, in place, the cell arithmetic of small_relax;
@@ -100,6 +220,48 @@ __global__ void __launch_bounds__(1024) k_relax_blocks(const BlkLev* __restrict_
     }
     for (int q = f0 + threadIdx.x; q < f1; q += blockDim.x) phi[fdst[q]] = phi[fsrc[q] & kIdxMask];
     __syncthreads();
+  }
+}
+
+// The same visit with the block in shared memory and its cells in registers
+// (constant coefficients, at most 4 x 512 cell pairs a block).  cdst / csrc:
+// the block's fill entries in the compact layout, those that a sweep reads first
+// (live[b] of them).  27 uneven blocks of up to 16^3 cells, 32 FP64 sweeps: 245
+// us from global memory, 67 us here.
+constexpr int kResidentThreads = 512;
+template <typename T>
+__global__ void __launch_bounds__(kResidentThreads) k_relax_resident(
+    const BlkLev* __restrict__ bls, const int* __restrict__ fstart, const int* __restrict__ live, T* __restrict__ phi,
+    const T* __restrict__ rhs, const uint32_t* __restrict__ cdst, const uint32_t* __restrict__ csrc, int sweeps,
+    int zero, float om) {
+  extern __shared__ __align__(16) unsigned char block_smem[];
+  __shared__ T diag[128];
+  pdl_trigger();
+  const BlkLev B = bls[blockIdx.x];
+  const int f0 = fstart[blockIdx.x], f1 = fstart[blockIdx.x + 1], fl = f0 + live[blockIdx.x];
+  T* P = reinterpret_cast<T*>(block_smem);
+  const int ex = B.nx + 2, ey = B.ny + 2, n = ex * ey * (B.nz + 2);
+  pdl_wait();
+  for (int q = threadIdx.x; q < n; q += blockDim.x) {
+    const int x = q % ex, y = (q / ex) % ey, z = q / (ex * ey);
+    P[q] = zero || wall_ghost(B, x, y, z) ? T(0) : phi[B.off + (long long)z * B.sxy + (long long)y * B.sx + x];
+  }
+  auto rhs_at = [&](int x, int y, int z) { return rhs[B.off + (long long)z * B.sxy + (long long)y * B.sx + x]; };
+  auto fill = [&](bool last) {
+    __syncthreads();
+    const int e = last ? f1 : fl;
+    if (e > f0) {
+      for (int q = f0 + threadIdx.x; q < e; q += blockDim.x) P[cdst[q]] = P[csrc[q]];
+      __syncthreads();
+    }
+  };
+  const int k = resident_pairs(B);
+  if (k == 1) relax_resident<T, 1>(B, P, diag, rhs_at, sweeps, om, 1, fill);
+  else if (k == 2) relax_resident<T, 2>(B, P, diag, rhs_at, sweeps, om, 1, fill);
+  else relax_resident<T, 4>(B, P, diag, rhs_at, sweeps, om, 1, fill);
+  for (int q = threadIdx.x; q < n; q += blockDim.x) {
+    const int x = q % ex, y = (q / ex) % ey, z = q / (ex * ey);
+    phi[B.off + (long long)z * B.sxy + (long long)y * B.sx + x] = P[q];
   }
 }
 
@@ -421,6 +583,7 @@ __global__ void __launch_bounds__(kClusterTailThreads) k_coarse_cluster(const Ta
   __shared__ TailLevel lv[kTailMaxLevels];
   __shared__ BlkLev gtab[kTailMaxLevels], ctab[kTailMaxLevels];  // this block per level: global / compact layout
   __shared__ TailOp ops[kClusterTailMaxOps];
+  __shared__ double diag64[128];
   extern __shared__ unsigned char smem_raw[];
   unsigned char* arena = smem_base128(smem_raw);
   // the program, the level records and this block's tables are setup data:
@@ -446,6 +609,7 @@ __global__ void __launch_bounds__(kClusterTailThreads) k_coarse_cluster(const Ta
       lv[l].ghosts = cs + G.nint;
       lv[l].fdst = fd;
       lv[l].nfill = f1 - f0;
+      lv[l].nlive = __ldg(G.flive + b);
     }
   }
   __syncthreads();
@@ -487,18 +651,48 @@ __global__ void __launch_bounds__(kClusterTailThreads) k_coarse_cluster(const Ta
             __syncthreads();
           }
           const int ncol = F.rb_global ? 2 : 1;  // 2: a fill after each colour (order across blocks)
-          for (int it = 0; it < op.sweeps; ++it) {
-            for (int pass = 0; pass < ncol; ++pass) {
-              tail_colours<T>(fb, F, phi, rhs, ncol == 2 ? pass : -1);
-              cl.sync();  // every block's sweep done
-              for (int q = threadIdx.x; q < F.nfill; q += blockDim.x) {  // (dst, src) pairs of this block
-                const uint32_t dsti = F.fdst[2 * q], src = F.fdst[2 * q + 1];
-                const T* remote = cl.map_shared_rank(phi, (int)(src >> 24));
-                phi[dsti] = remote[src & 0xffffffu];
-              }
-              cl.sync();  // every ghost gathered before any interior changes
+          const bool alone = F.nb == 1;
+          auto barrier = [&] {
+            if (alone) __syncthreads();
+            else cl.sync();
+          };
+          // ghosts from every block's interior: all of them after the last sweep, before
+          // that the ones that a sweep reads
+          auto fill = [&](bool last) {
+            if (!last && !F.any_live) {
+              __syncthreads();
+              return;
+            }
+            barrier();  // every block's sweep done
+            const int n = last ? F.nfill : F.nlive;
+            for (int q = threadIdx.x; q < n; q += blockDim.x) {  // (dst, src) pairs of this block
+              const uint32_t dsti = F.fdst[2 * q], src = F.fdst[2 * q + 1];
+              const T* remote = cl.map_shared_rank(phi, (int)(src >> 24));
+              phi[dsti] = remote[src & 0xffffffu];
+            }
+            barrier();  // every ghost gathered before any interior changes
+          };
+          if constexpr (sizeof(T) == 8) {
+            // many sweeps (the converged coarsest level): cells resident in registers
+            const int k = op.sweeps >= kResidentSweeps ? resident_pairs(*fb) : 0;
+            if (k) {
+              if (!op.zero)
+                for (int q = threadIdx.x; q < F.nghost; q += blockDim.x) {
+                  const CellRef c = cell_ref(F.ghosts[q]);
+                  if (wall_ghost(*fb, c.x, c.y, c.z)) phi[c.i] = T(0);
+                }
+              auto rhs_at = [&](int x, int y, int z) { return rhs[rhs_index(*fb, x, y, z)]; };
+              if (k == 1) relax_resident<T, 1>(*fb, phi, diag64, rhs_at, op.sweeps, F.om, ncol, fill);
+              else if (k == 2) relax_resident<T, 2>(*fb, phi, diag64, rhs_at, op.sweeps, F.om, ncol, fill);
+              else relax_resident<T, 4>(*fb, phi, diag64, rhs_at, op.sweeps, F.om, ncol, fill);
+              return;
             }
           }
+          for (int it = 0; it < op.sweeps; ++it)
+            for (int pass = 0; pass < ncol; ++pass) {
+              tail_colours<T>(fb, F, phi, rhs, ncol == 2 ? pass : -1);
+              fill(it + 1 == op.sweeps && pass + 1 == ncol);
+            }
         };
         if (op.f64) relax(at64(F.s_phi64), (const double*)at64(F.s_rhs64));
         else relax(at32(F.s_phi32), (const float*)at32(F.s_rhs32));
@@ -575,6 +769,10 @@ __global__ void __launch_bounds__(kClusterTailThreads) k_coarse_cluster(const Ta
 cudaError_t coarse_tail_attributes() {
   cudaError_t e = cudaFuncSetAttribute(k_coarse_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmemBytes);
   if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(k_relax_resident<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmemBytes);
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(k_relax_resident<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmemBytes);
+  if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(k_coarse_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmemBytes);
   if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(k_coarse_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -591,6 +789,8 @@ static cudaError_t cluster_config(int nb, int smem_bytes, cudaStream_t st, cudaL
   at[0].val.clusterDim.x = nb;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg->attrs = at;
   cfg->numAttrs = 1;
   return cudaSuccess;
@@ -598,7 +798,7 @@ static cudaError_t cluster_config(int nb, int smem_bytes, cudaStream_t st, cudaL
 
 int coarse_cluster_fits(int nb, int smem_bytes) {
   cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   cluster_config(nb, smem_bytes, nullptr, &cfg, at);
   int n = 0;
   if (cudaOccupancyMaxActiveClusters(&n, k_coarse_cluster, &cfg) != cudaSuccess) {
@@ -612,8 +812,10 @@ cudaError_t launch_coarse_cluster(int nb, const TailLevel* lv, int nlev, const T
                                   unsigned curmask, int smem_bytes, cudaStream_t st) {
   if (nops <= 0 || nops > kClusterTailMaxOps || nlev > kTailMaxLevels) return cudaErrorInvalidValue;
   cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   cluster_config(nb, smem_bytes, st, &cfg, at);
+  cfg.numAttrs = 2;  // (its tables are staged while the predecessor finishes)
+  g_prev_grid = nb;
   return cudaLaunchKernelEx(&cfg, k_coarse_cluster, lv, ops, nops, nlev, curmask);
 }
 
@@ -650,6 +852,30 @@ cudaError_t launch_relax_blocks(bool var, const BlkLev* bl, int nb, const int* f
                (int)zero, om);
   return cudaGetLastError();
 }
+template <typename T>
+cudaError_t launch_relax_resident(const BlkLev* bl, int nb, const int* fstart, const int* live, T* phi, const T* rhs,
+                                  const uint32_t* cdst, const uint32_t* csrc, int smem, int sweeps, bool zero,
+                                  float om, cudaStream_t st) {
+  if (nb <= 0) return cudaSuccess;
+  pdl_launch(k_relax_resident<T>, nb, kResidentThreads, (size_t)smem, st, bl, fstart, live, phi, rhs, cdst, csrc,
+             sweeps, (int)zero, om);
+  return cudaGetLastError();
+}
+// Shared memory of launch_relax_resident for these blocks, or 0 where one does not fit it.
+int resident_smem(const std::vector<BlkLev>& bl, int word) {
+  long long n = 0;
+  for (const auto& B : bl) {
+    if ((long long)(B.nx + 1) / 2 * B.ny * B.nz > 4 * kResidentThreads) return 0;
+    n = std::max(n, (long long)(B.nx + 2) * (B.ny + 2) * (B.nz + 2) * word);
+  }
+  return n <= kTailSmemBytes ? (int)n : 0;
+}
+template cudaError_t launch_relax_resident<double>(const BlkLev*, int, const int*, const int*, double*, const double*,
+                                                   const uint32_t*, const uint32_t*, int, int, bool, float,
+                                                   cudaStream_t);
+template cudaError_t launch_relax_resident<float>(const BlkLev*, int, const int*, const int*, float*, const float*,
+                                                  const uint32_t*, const uint32_t*, int, int, bool, float,
+                                                  cudaStream_t);
 template cudaError_t launch_relax_blocks<double>(bool, const BlkLev*, int, const int*, double*, const double*,
                                                  const double*, const double*, const double*, const uint32_t*,
                                                  const uint32_t*, int, bool, float, cudaStream_t);

@@ -105,7 +105,9 @@ struct TailLevel {
   const unsigned long long* ghosts;  // ghost cells of the padded blocks
   const uint32_t* fdst;              // sweep fill table, compact indices (cluster tail: own block)
   const uint32_t* fsrc;              // (cluster tail: source rank << 24 | compact index in its block)
-  const int* fstart;                 // cluster tail: fill entries of block b are fstart[b] .. fstart[b+1]-1
+  const int* fstart;                 // cluster tail: fill entries of block b are fstart[b] .. fstart[b+1]-1,
+  const int* flive;                  // the flive[b] first of them are ghosts that a sweep reads
+  int nlive, any_live;               // cluster tail: this block's flive; some block has one
   int nb, nint, nred, nghost, npad, nfill;
   float* phi32[2];
   float* rhs32;
@@ -280,6 +282,15 @@ template <typename T>
 cudaError_t launch_relax_blocks(bool var, const BlkLev* bl, int nb, const int* fstart, T* phi, const T* rhs,
                                 const T* fx, const T* fy, const T* fz, const uint32_t* fdst, const uint32_t* fsrc,
                                 int sweeps, bool zero, float om, cudaStream_t st);
+
+// The same with constant coefficients, the blocks in shared memory (`smem` from
+// resident_smem): fill entries in the compact layout (pitches nx+2 and
+// (nx+2)(ny+2)), the live[b] that a sweep reads first.
+int resident_smem(const std::vector<BlkLev>& bl, int word);
+template <typename T>
+cudaError_t launch_relax_resident(const BlkLev* bl, int nb, const int* fstart, const int* live, T* phi, const T* rhs,
+                                  const uint32_t* cdst, const uint32_t* csrc, int smem, int sweeps, bool zero,
+                                  float om, cudaStream_t st);
 
 // Stone's SIP (sipsol.for) on level 1: factor arrays and the residual
 // (level-1 layout, zero outside the interior).

@@ -107,6 +107,9 @@ struct Level {
   bool blocal = false;      // the sweep fill stays inside every block: a visit is one launch, a CTA per block
   Halo lfill;               // that fill, sorted by block
   int* d_lfstart = nullptr; // its per-block entry ranges (nb + 1)
+  int resident_smem = 0;    // blocal with constant coefficients: shared memory of the resident kernel (0: not taken)
+  Halo cfill;               // lfill in the compact layout, the entries that a sweep reads first
+  int* d_clive = nullptr;   // ... and their number, per block
   bool tailable = false;    // small enough for the fused coarse tail (has d_cstart)
   int cur64 = 0, cur32 = 0;
   bool zero64 = false, zero32 = false;
@@ -696,12 +699,21 @@ struct Exec {
     if (it > 0 && V.blocal && g > 1 && h->desc.mg_itrsch == 3) {  // a visit in one launch, a CTA per block
       const int nb = (int)V.geom.bl.size();
       if (mixed_level(g)) {
-        CU(launch_relax_blocks<float>(h->var, V.d_bl, nb, V.d_lfstart, V.phi32[V.cur32], V.rhs32, V.fx32, V.fy32,
-                                      V.fz32, V.lfill.d_dst, V.lfill.d_src, it, V.zero32, h->omega, h->st));
+        if (V.resident_smem)
+          CU(launch_relax_resident<float>(V.d_bl, nb, V.d_lfstart, V.d_clive, V.phi32[V.cur32], V.rhs32,
+                                          V.cfill.d_dst, V.cfill.d_src, V.resident_smem, it, V.zero32, h->omega,
+                                          h->st));
+        else
+          CU(launch_relax_blocks<float>(h->var, V.d_bl, nb, V.d_lfstart, V.phi32[V.cur32], V.rhs32, V.fx32, V.fy32,
+                                        V.fz32, V.lfill.d_dst, V.lfill.d_src, it, V.zero32, h->omega, h->st));
         V.zero32 = false;
       } else {
-        CU(launch_relax_blocks<double>(h->var, V.d_bl, nb, V.d_lfstart, V.phi64[V.cur64], V.rhs64, V.fx64, V.fy64,
-                                       V.fz64, V.lfill.d_dst, V.lfill.d_src, it, V.zero64, 1.f, h->st));
+        if (V.resident_smem)
+          CU(launch_relax_resident<double>(V.d_bl, nb, V.d_lfstart, V.d_clive, V.phi64[V.cur64], V.rhs64,
+                                           V.cfill.d_dst, V.cfill.d_src, V.resident_smem, it, V.zero64, 1.f, h->st));
+        else
+          CU(launch_relax_blocks<double>(h->var, V.d_bl, nb, V.d_lfstart, V.phi64[V.cur64], V.rhs64, V.fx64, V.fy64,
+                                         V.fz64, V.lfill.d_dst, V.lfill.d_src, it, V.zero64, 1.f, h->st));
         V.zero64 = false;
       }
       TRY(chk("relax blocks", g));
@@ -2178,6 +2190,28 @@ int build_dense_coarse(h3d_mg* h) {
   return H3D_OK;
 }
 
+// Compact index (pitches nx+2 and (nx+2)(ny+2)) of level cell gi of block B, and its coordinates.
+uint32_t compact_cell(const BlkLev& B, uint32_t gi, int* x, int* y, int* z) {
+  const long long l = (long long)gi - B.off;
+  *z = (int)(l / B.sxy);
+  *y = (int)((l % B.sxy) / B.sx);
+  *x = (int)(l % B.sx);
+  return (uint32_t)((*z * (B.ny + 2) + *y) * (B.nx + 2) + *x);
+}
+
+// A ghost cell that a sweep reads with a non-zero coefficient: on a face of the
+// block that is not a physical wall (edges and corners are not read).
+bool sweep_reads(const BlkLev& B, int x, int y, int z) {
+  const int out[6] = {x == 0, x == B.nx + 1, y == 0, y == B.ny + 1, z == 0, z == B.nz + 1};
+  int n = 0, f = -1;
+  for (int q = 0; q < 6; ++q)
+    if (out[q]) {
+      n += 1;
+      f = q;
+    }
+  return n == 1 && !(B.phys & (1 << f));
+}
+
 int build_cluster_tail(h3d_mg* h) {
   const int Lv = h->L;
   const int nb = (int)h->blocks.size();
@@ -2236,7 +2270,7 @@ int build_cluster_tail(h3d_mg* h) {
   std::vector<unsigned long long> cells;
   std::vector<uint32_t> fills;
   std::vector<int> starts;
-  struct At { size_t cells, ghosts, fdst, fsrc, fstart; int nred, nint, nghost; };
+  struct At { size_t cells, ghosts, fdst, fsrc, fstart, flive; int nred, nint, nghost, any_live; };
   std::vector<At> at;
   for (int q = g0; q <= Lv; ++q) {
     const Level& V = h->lev[q];
@@ -2290,12 +2324,22 @@ int build_cluster_tail(h3d_mg* h) {
     a.fdst = fills.size();
     std::vector<uint32_t> fd, fs;
     int acc = 0;
+    std::vector<int> live;  // entries that a sweep reads come first
     for (int b = 0; b < nb; ++b) {
+      const BlkLev& Bb = V.geom.bl[b];
+      auto read = [&](const std::pair<uint32_t, uint32_t>& pr) {
+        return sweep_reads(Bb, (int)(pr.first % sx), (int)(pr.first / sx % (Bb.ny + 2)), (int)(pr.first / sxy));
+      };
+      const auto mid = std::stable_partition(per[b].begin(), per[b].end(), read);
+      live.push_back((int)(mid - per[b].begin()));
+      a.any_live |= live.back() > 0;
       starts.push_back(acc);
       for (auto& pr : per[b]) { fd.push_back(pr.first); fs.push_back(pr.second); }
       acc += (int)per[b].size();
     }
     starts.push_back(acc);
+    a.flive = starts.size();
+    starts.insert(starts.end(), live.begin(), live.end());
     fills.insert(fills.end(), fd.begin(), fd.end());
     a.fsrc = fills.size();
     fills.insert(fills.end(), fs.begin(), fs.end());
@@ -2327,6 +2371,8 @@ int build_cluster_tail(h3d_mg* h) {
     t.fdst = d_fills + a.fdst;
     t.fsrc = d_fills + a.fsrc;
     t.fstart = d_starts + a.fstart;
+    t.flive = d_starts + a.flive;
+    t.any_live = a.any_live;
     t.nb = nb;
     t.nint = a.nint;
     t.nred = a.nred;
@@ -2390,6 +2436,7 @@ int h3d_mg_destroy(h3d_mg* h) {
                   V.phi32[1], V.rhs32, V.fx64, V.fy64, V.fz64, V.fx32, V.fy32, V.fz32, V.dens,
                   V.sweep.d_dst, V.sweep.d_src, V.faces.d_dst, V.faces.d_src, V.exch.d_dst, V.exch.d_src,
                   V.bound.d_dst, V.bound.d_src, V.sweep_push.d_dst, V.sweep_push.d_src, V.live.d_dst, V.live.d_src, V.live_push.d_dst, V.live_push.d_src, V.red.d_dst, V.red.d_src, V.d_red_info, V.d_push, V.d_maps, V.d_rmaps, V.d_rtiles, V.d_ptiles, V.d_qtiles, V.d_dtiles, V.d_cstart, V.d_dstart, V.d_pstart, V.seq64, V.seq32, V.d_ztiles, V.lfill.d_dst, V.lfill.d_src, V.d_lfstart,
+                  V.cfill.d_dst, V.cfill.d_src, V.d_clive,
                   V.xs.d_nodes, V.xs.d_dst, V.xs.d_src, V.xe.d_nodes, V.xe.d_dst, V.xe.d_src, V.xscratch, V.d_rsame,
                   V.d_psame, V.d_prows};
     for (void* p : ps) dfree(p);
@@ -2653,6 +2700,29 @@ int h3d_mg_create(h3d_mg** out, const h3d_mg_desc* desc) {
         if (cudaMemcpy(V.d_lfstart, st.data(), st.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
           return bail(fail(h, H3D_ERR_CUDA, "block-local fill table"));
         V.blocal = true;
+        const int sm = h->var ? 0 : resident_smem(V.geom.bl, f32_level(h, g) ? 4 : 8);
+        if (sm) {
+          std::vector<uint32_t> cd, cs;
+          std::vector<int> live;
+          for (size_t b = 0; b < per.size(); ++b) {
+            const BlkLev& B = V.geom.bl[b];
+            live.push_back(0);
+            for (int pass = 0; pass < 2; ++pass)
+              for (const auto& pr : per[b]) {
+                int x, y, z;
+                const uint32_t d0 = compact_cell(B, pr.first, &x, &y, &z);
+                if (sweep_reads(B, x, y, z) != (pass == 0)) continue;
+                cd.push_back(d0);
+                cs.push_back(compact_cell(B, pr.second, &x, &y, &z));
+                live.back() += pass == 0;
+              }
+          }
+          if ((rc = upload_halo(h, V.cfill, cd, cs)) != H3D_OK || (rc = dalloc(h, &V.d_clive, live.size())) != H3D_OK)
+            return bail(rc);
+          if (cudaMemcpy(V.d_clive, live.data(), live.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
+            return bail(fail(h, H3D_ERR_CUDA, "block-local fill table"));
+          V.resident_smem = sm;
+        }
       }
     }
     if (g == 1 && !V.expr) {  // (with refinement the pressure halo is the sweep's expression fill)
