@@ -122,4 +122,25 @@ __device__ __forceinline__ unsigned char* smem_base128(unsigned char* raw) {
   return raw + ((128u - (smem_u32(raw) & 127u)) & 127u);
 }
 
+// ---------------------------------------------------------------------------
+template <int NT>
+__device__ __forceinline__ void block_reduce4(double a0, double a1, double a2, double a3, double* out) {
+  __shared__ double sh[4][NT / 32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a0 += __shfl_xor_sync(0xffffffffu, a0, o);
+    a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+    a2 = fmax(a2, __shfl_xor_sync(0xffffffffu, a2, o));
+    a3 += __shfl_xor_sync(0xffffffffu, a3, o);
+  }
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  if (l == 0) { sh[0][w] = a0; sh[1][w] = a1; sh[2][w] = a2; sh[3][w] = a3; }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
+    for (int q = 0; q < NT / 32; ++q) { s0 += sh[0][q]; s1 += sh[1][q]; s2 = fmax(s2, sh[2][q]); s3 += sh[3][q]; }
+    out[0] = s0; out[1] = s1; out[2] = s2; out[3] = s3;
+  }
+}
+
 }  // namespace h3d

@@ -1209,34 +1209,30 @@ __global__ void __launch_bounds__(256) k_prolong(const BlkLev* __restrict__ fine
   }
 }
 
-// ---------------------------------------------------------------------------
-template <int NT>
-__device__ __forceinline__ void block_reduce4(double a0, double a1, double a2, double a3, double* out) {
-  __shared__ double sh[4][NT / 32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    a0 += __shfl_xor_sync(0xffffffffu, a0, o);
-    a1 += __shfl_xor_sync(0xffffffffu, a1, o);
-    a2 = fmax(a2, __shfl_xor_sync(0xffffffffu, a2, o));
-    a3 += __shfl_xor_sync(0xffffffffu, a3, o);
-  }
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) { sh[0][w] = a0; sh[1][w] = a1; sh[2][w] = a2; sh[3][w] = a3; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
-    for (int q = 0; q < NT / 32; ++q) { s0 += sh[0][q]; s1 += sh[1][q]; s2 = fmax(s2, sh[2][q]); s3 += sh[3][q]; }
-    out[0] = s0; out[1] = s1; out[2] = s2; out[3] = s3;
+
+// p_next = p + e over whole level arrays (ghosts included, newsolv_mg.for:39-48).
+template <typename TE>
+__global__ void __launch_bounds__(256) k_apply(const double* __restrict__ p, const TE* __restrict__ e,
+                                               double* __restrict__ p_next, int64_t n) {
+  pdl_trigger();
+  pdl_wait();
+  using E2 = typename std::conditional<sizeof(TE) == 4, float2, double2>::type;
+  for (int64_t i = 2 * (blockIdx.x * (int64_t)blockDim.x + threadIdx.x); i < n;
+       i += 2 * (int64_t)gridDim.x * blockDim.x) {
+    const double2 a = *reinterpret_cast<const double2*>(p + i);
+    const E2 d = *reinterpret_cast<const E2*>(e + i);
+    *reinterpret_cast<double2*>(p_next + i) = make_double2(a.x + (double)d.x, a.y + (double)d.y);
   }
 }
 
-// newsolv_mg.for:39-55 as defect correction: p += pp over the whole block
-// (ghosts included, :40-48), then r = b - A p (mgrestr's residual form).
-// One warp per level-1 row (all rows incl. ghosts); per-CTA partial sums.
-template <typename TE, typename TR, bool HAS_E, bool VAR>
+// r = b - A p (mgrestr's residual form) as the right-hand side of the next
+// correction.  One warp per interior level-1 row; per-CTA partial sums.  (The correction
+// p + e is a pass of its own before it: added at each of the seven points of
+// the stencil it took 505 us on 256^3 cells with variable coefficients, against
+// 206 us for this kernel and 50 us for the pass.)
+template <typename TR, bool VAR>
 __global__ void __launch_bounds__(256) k_defect(const BlkLev* __restrict__ bls, const int* __restrict__ row_start,
                                                 int nb, int nrows, const double* __restrict__ p,
-                                                const TE* __restrict__ e, double* __restrict__ p_next,
                                                 const double* __restrict__ bvec, TR* __restrict__ rhs_out,
                                                 double mean_b, double rscale, const double* __restrict__ fx,
                                                 const double* __restrict__ fy, const double* __restrict__ fz,
@@ -1247,31 +1243,23 @@ __global__ void __launch_bounds__(256) k_defect(const BlkLev* __restrict__ bls, 
   double rr = 0, bb = 0, rm = 0, rs = 0;
   for (int rid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; rid < nrows; rid += (gridDim.x * blockDim.x) >> 5) {
     const RowRef ref = row_of(bls, row_start, nb, rid, false);
+    if (ref.y < 1 || ref.z < 1 || ref.y > bls[ref.b].ny || ref.z > bls[ref.b].nz) continue;
     const BlkLev B = bls[ref.b];
     const int y = ref.y, z = ref.z;
-    const bool row_in = y >= 1 && y <= B.ny && z >= 1 && z <= B.nz;
     const long long rowg = B.off + (long long)z * B.sxy + (long long)y * B.sx;
-    auto pv = [&](long long j) -> double {
-      if (HAS_E) return p[j] + (double)e[j];
-      return p[j];
-    };
-    for (int x = lane; x <= B.nx + 1; x += 32) {
+    for (int x = 1 + lane; x <= B.nx; x += 32) {
       const long long i = rowg + x;
-      const double pc = pv(i);
-      if (HAS_E) p_next[i] = pc;
-      if (row_in && x >= 1 && x <= B.nx) {
-        Coef<double> c = cell_coef<double, VAR>(B, x, y, z, i - B.off, VAR ? fx + B.off : nullptr,
-                                                VAR ? fy + B.off : nullptr, VAR ? fz + B.off : nullptr);
-        const double ap = coef_ap(c);
-        const double bv = bvec[i];
-        const double r = bv - (c.aw * pv(i - 1) + c.ae * pv(i + 1) + c.as * pv(i - B.sx) + c.an * pv(i + B.sx) +
-                               c.ab * pv(i - B.sxy) + c.at * pv(i + B.sxy) + ap * pc);
-        rhs_out[i] = (TR)(r - mean_b);
-        rr += r * r;
-        bb += bv * bv;
-        rm = fmax(rm, fabs(r) * (rscale < 0.0 ? B.dv : rscale));
-        rs += r;
-      }
+      Coef<double> c = cell_coef<double, VAR>(B, x, y, z, i - B.off, VAR ? fx + B.off : nullptr,
+                                              VAR ? fy + B.off : nullptr, VAR ? fz + B.off : nullptr);
+      const double ap = coef_ap(c);
+      const double bv = bvec[i];
+      const double r = bv - (c.aw * p[i - 1] + c.ae * p[i + 1] + c.as * p[i - B.sx] + c.an * p[i + B.sx] +
+                             c.ab * p[i - B.sxy] + c.at * p[i + B.sxy] + ap * p[i]);
+      rhs_out[i] = (TR)(r - mean_b);
+      rr += r * r;
+      bb += bv * bv;
+      rm = fmax(rm, fabs(r) * (rscale < 0.0 ? B.dv : rscale));
+      rs += r;
     }
   }
   block_reduce4<256>(rr, bb, rm, rs, partials + 4 * (size_t)blockIdx.x);
@@ -2842,22 +2830,26 @@ template cudaError_t launch_defect_vec<float, float>(const BlkLev*, const Tile*,
                                                      double*, const double*, float*, double, double, double*, int,
                                                      cudaStream_t);
 
-template <typename TE, typename TR>
-cudaError_t launch_defect(bool var, const BlkLev* bl, RowTab rt, const double* p, const TE* e, double* p_next,
-                          const double* b, TR* rhs_out, double mean_b, double rscale, const double* fx,
-                          const double* fy, const double* fz, double* partials, cudaStream_t st) {
-  if (rt.nrows <= 0) return cudaSuccess;
-  const int g = defect_grid(rt.nrows);
-  if (e) {
-    if (var) pdl_launch(k_defect<TE, TR, true, true>, g, 256, 0, st, bl, rt.start, rt.nb, rt.nrows, p, e, p_next, b, rhs_out, mean_b, rscale, fx, fy, fz, partials);
-    else pdl_launch(k_defect<TE, TR, true, false>, g, 256, 0, st, bl, rt.start, rt.nb, rt.nrows, p, e, p_next, b, rhs_out, mean_b, rscale, fx, fy, fz, partials);
-  } else {
-    if (var) pdl_launch(k_defect<TE, TR, false, true>, g, 256, 0, st, bl, rt.start, rt.nb, rt.nrows, p, e, p_next, b, rhs_out, mean_b, rscale, fx, fy, fz, partials);
-    else pdl_launch(k_defect<TE, TR, false, false>, g, 256, 0, st, bl, rt.start, rt.nb, rt.nrows, p, e, p_next, b, rhs_out, mean_b, rscale, fx, fy, fz, partials);
-  }
+template <typename TE>
+cudaError_t launch_apply(const double* p, const TE* e, double* p_next, int64_t n, cudaStream_t st) {
+  pdl_launch(k_apply<TE>, (int)std::min<int64_t>((n / 2 + 255) / 256, 148 * 16), 256, 0, st, p, e, p_next, n);
   return cudaGetLastError();
 }
 
+template <typename TR>
+cudaError_t launch_defect(bool var, const BlkLev* bl, RowTab rt, const double* p, const double* b, TR* rhs_out,
+                          double mean_b, double rscale, const double* fx, const double* fy, const double* fz,
+                          double* partials, cudaStream_t st) {
+  if (rt.nrows <= 0) return cudaSuccess;
+  const int g = defect_grid(rt.nrows);
+  if (var)
+    pdl_launch(k_defect<TR, true>, g, 256, 0, st, bl, rt.start, rt.nb, rt.nrows, p, b, rhs_out, mean_b, rscale, fx,
+               fy, fz, partials);
+  else
+    pdl_launch(k_defect<TR, false>, g, 256, 0, st, bl, rt.start, rt.nb, rt.nrows, p, b, rhs_out, mean_b, rscale, fx,
+               fy, fz, partials);
+  return cudaGetLastError();
+}
 
 // ---------------------------------------------------------------------------
 // TMA-staged restriction (mgrestr, mgsolver.for:623-766): fine residuals
@@ -3636,12 +3628,13 @@ template cudaError_t launch_prolong<double>(bool, const BlkLev*, const BlkLev*, 
                                             double*, cudaStream_t);
 template cudaError_t launch_prolong<float>(bool, const BlkLev*, const BlkLev*, RowTab, const float*, const float*,
                                            float*, cudaStream_t);
-template cudaError_t launch_defect<double, double>(bool, const BlkLev*, RowTab, const double*, const double*, double*,
-                                                   const double*, double*, double, double, const double*,
-                                                   const double*, const double*, double*, cudaStream_t);
-template cudaError_t launch_defect<float, float>(bool, const BlkLev*, RowTab, const double*, const float*, double*,
-                                                 const double*, float*, double, double, const double*, const double*,
-                                                 const double*, double*, cudaStream_t);
+template cudaError_t launch_apply<float>(const double*, const float*, double*, int64_t, cudaStream_t);
+template cudaError_t launch_apply<double>(const double*, const double*, double*, int64_t, cudaStream_t);
+template cudaError_t launch_defect<double>(bool, const BlkLev*, RowTab, const double*, const double*, double*, double,
+                                           double, const double*, const double*, const double*, double*,
+                                           cudaStream_t);
+template cudaError_t launch_defect<float>(bool, const BlkLev*, RowTab, const double*, const double*, float*, double,
+                                          double, const double*, const double*, const double*, double*, cudaStream_t);
 
 // ---------------------------------------------------------------------------
 // Local mesh refinement (LMR).

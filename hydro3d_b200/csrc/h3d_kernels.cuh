@@ -232,15 +232,24 @@ cudaError_t launch_defect_march(int gp, const BlkLev* bl, const Tile* tiles, int
                                 double rscale, double* partials, cudaStream_t st);
 int defect_march_rows();
 
-// Level-1 FP64 defect: pn = p + e (all cells, when e != null), r = b - A pn on
-// the interior, rhs_out = r - mean_b (as TR), per-CTA partial sums
-// {sum r^2, sum b^2, max |r|*rscale, sum r} into partials[4*cta]; rscale < 0
-// stands for each block's own cell volume dv.
-template <typename TE, typename TR>
-cudaError_t launch_defect(bool var, const BlkLev* bl, RowTab rt, const double* p, const TE* e,
-                          double* p_next, const double* b, TR* rhs_out, double mean_b, double rscale,
-                          const double* fx, const double* fy, const double* fz, double* partials,
-                          cudaStream_t st);
+// pn = p + e on n words (level arrays: a multiple of two).
+template <typename TE>
+cudaError_t launch_apply(const double* p, const TE* e, double* p_next, int64_t n, cudaStream_t st);
+// Level-1 FP64 defect: r = b - A p on the interior, rhs_out = r - mean_b (as
+// TR), per-CTA partial sums {sum r^2, sum b^2, max |r|*rscale, sum r} into
+// partials[4*cta]; rscale < 0 stands for each block's own cell volume dv.
+template <typename TR>
+cudaError_t launch_defect(bool var, const BlkLev* bl, RowTab rt, const double* p, const double* b, TR* rhs_out,
+                          double mean_b, double rscale, const double* fx, const double* fy, const double* fz,
+                          double* partials, cudaStream_t st);
+// The same with variable coefficients as a z march (every nx even, at most
+// 512): tiles of defect_var_rows(nx) rows of a block over zc planes, one CTA and
+// partial sum each (h3d_var.cu).
+int defect_var_rows(int nx);
+template <typename TR>
+cudaError_t launch_defect_var(const BlkLev* bl, const Tile* tiles, int ntiles, int zc, const double* p,
+                              const double* b, TR* rhs_out, double mean_b, double rscale, const double* fx,
+                              const double* fy, const double* fz, double* partials, cudaStream_t st);
 // Deterministic reduction of n partial quadruples into out[4].
 cudaError_t launch_reduce4(const double* partials, int n, double* out, cudaStream_t st);
 // Per-block sums: out[4b..4b+3] from partials start[b] .. start[b+1]-1.

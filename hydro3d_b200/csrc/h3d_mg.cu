@@ -914,41 +914,43 @@ struct Exec {
     const double* fz = h->var ? V.fz64 : nullptr;
     double* pin = h->p64[h->pc];
     double* pout = h->p64[1 - h->pc];
-    // the z-march and tiled kernels need constant coefficients and nx even
+    // the z-march and tiled kernels that take p + e themselves need constant
+    // coefficients and nx even; the others follow a pass p + e
     const bool march = V.dgp > 0 && !h->var;
     const bool tiled = !march && V.d_ptiles && V.pvec64 && !h->var;
-    const int ngrid = march ? V.ndtiles : tiled ? V.nptiles : defect_grid(ct.nrows);
-    if (h->mixed) {
-      const float* e = nullptr;
+    const bool vmarch = h->var && V.ndtiles > 0;
+    const int ngrid = march || vmarch ? V.ndtiles : tiled ? V.nptiles : defect_grid(ct.nrows);
+    auto run = [&](auto* it, bool* zero, auto* rhs, auto&& materialize) -> int {
+      using T = typename std::remove_pointer<decltype(rhs)>::type;
+      const T* e = nullptr;
       if (with_e) {
-        if (V.zero32) TRY(materialize_zero32(1));
-        e = V.phi32[V.cur32];
+        if (*zero) TRY(materialize());
+        e = it;
       }
-      if (march)
-        CU(launch_defect_march<float, float>(V.dgp, V.d_bl, V.d_dtiles, V.ndtiles, V.dzc, pin, e, pout, h->b64,
-                                             V.rhs32, h->mean_b, rscale, h->partials, h->st));
-      else if (tiled)
-        CU(launch_defect_vec<float, float>(V.d_bl, V.d_ptiles, V.nptiles, pin, e, pout, h->b64, V.rhs32, h->mean_b,
-                                           rscale, h->partials, ngrid, h->st));
-      else
-        CU(launch_defect<float, float>(h->var, V.d_bl, ct, pin, e, pout, h->b64, V.rhs32, h->mean_b, rscale, fx, fy,
-                                       fz, h->partials, h->st));
-    } else {
-      const double* e = nullptr;
-      if (with_e) {
-        if (V.zero64) TRY(materialize_zero64(1));
-        e = V.phi64[V.cur64];
+      if (march) {
+        CU(launch_defect_march<T, T>(V.dgp, V.d_bl, V.d_dtiles, V.ndtiles, V.dzc, pin, e, pout, h->b64, rhs,
+                                     h->mean_b, rscale, h->partials, h->st));
+        return H3D_OK;
       }
-      if (march)
-        CU(launch_defect_march<double, double>(V.dgp, V.d_bl, V.d_dtiles, V.ndtiles, V.dzc, pin, e, pout, h->b64,
-                                               V.rhs64, h->mean_b, rscale, h->partials, h->st));
-      else if (tiled)
-        CU(launch_defect_vec<double, double>(V.d_bl, V.d_ptiles, V.nptiles, pin, e, pout, h->b64, V.rhs64,
-                                             h->mean_b, rscale, h->partials, ngrid, h->st));
+      if (tiled) {
+        CU(launch_defect_vec<T, T>(V.d_bl, V.d_ptiles, V.nptiles, pin, e, pout, h->b64, rhs, h->mean_b, rscale,
+                                   h->partials, ngrid, h->st));
+        return H3D_OK;
+      }
+      if (e) {
+        CU(launch_apply<T>(pin, e, pout, V.geom.n_elems, h->st));
+        h->kernels += 1;
+      }
+      const double* q = e ? pout : pin;
+      if (vmarch)
+        CU(launch_defect_var<T>(V.d_bl, V.d_dtiles, V.ndtiles, V.dzc, q, h->b64, rhs, h->mean_b, rscale, fx, fy, fz,
+                                h->partials, h->st));
       else
-        CU(launch_defect<double, double>(h->var, V.d_bl, ct, pin, e, pout, h->b64, V.rhs64, h->mean_b, rscale, fx,
-                                         fy, fz, h->partials, h->st));
-    }
+        CU(launch_defect<T>(h->var, V.d_bl, ct, q, h->b64, rhs, h->mean_b, rscale, fx, fy, fz, h->partials, h->st));
+      return H3D_OK;
+    };
+    if (h->mixed) TRY(run(V.phi32[V.cur32], &V.zero32, V.rhs32, [&] { return materialize_zero32(1); }));
+    else TRY(run(V.phi64[V.cur64], &V.zero64, V.rhs64, [&] { return materialize_zero64(1); }));
     TRY(chk("defect", 1));
     if (with_e) h->pc = 1 - h->pc;
     CU(launch_reduce4(h->partials, ngrid, h->d_res, h->st));
@@ -2788,17 +2790,21 @@ int h3d_mg_create(h3d_mg** out, const h3d_mg_desc* desc) {
         V.nztiles = (int)zt.size();
       }
     }
-    if (g == 1 && !h->var) {  // z-march defect tiles: 8 rows of a block over a chunk of planes
+    if (g == 1) {  // z-march defect tiles: some rows of a block over a chunk of planes
       int maxnx = 0, maxnz = 0, nyt = 0;
       bool even = true;
+      auto tile_rows = [&](const BlkLev& B) {
+        return !h->var ? defect_march_rows() : std::max(1, B.nx > 1 ? defect_var_rows(B.nx) : 1);
+      };
       for (const auto& B : V.geom.bl) {
         maxnx = std::max(maxnx, B.nx);
         maxnz = std::max(maxnz, B.nz);
         even = even && B.nx % 2 == 0;
-        nyt += (B.ny + defect_march_rows() - 1) / defect_march_rows();
+        const int r = tile_rows(B);
+        nyt += (B.ny + r - 1) / r;
       }
-      V.dgp = !even ? 0 : maxnx <= 64 ? 1 : maxnx <= 128 ? 2 : maxnx <= 256 ? 4 : 0;
-      if (V.dgp) {
+      if (!h->var) V.dgp = !even ? 0 : maxnx <= 64 ? 1 : maxnx <= 128 ? 2 : maxnx <= 256 ? 4 : 0;
+      if (h->var ? even && maxnx <= 512 : V.dgp > 0) {
         // about six CTAs per SM in all, chunks of at least four planes
         const int chunks = std::max(1, std::min((148 * 6 + nyt - 1) / nyt, maxnz / 4));
         V.dzc = std::max(1, (maxnz + chunks - 1) / chunks);
@@ -2806,7 +2812,7 @@ int h3d_mg_create(h3d_mg** out, const h3d_mg_desc* desc) {
         for (size_t b = 0; b < V.geom.bl.size(); ++b) {
           const BlkLev& B = V.geom.bl[b];
           for (int z0 = 1; z0 <= B.nz; z0 += V.dzc)
-            for (int y0 = 1; y0 <= B.ny; y0 += defect_march_rows()) dt.push_back(Tile{(int)b, 0, y0, z0});
+            for (int y0 = 1; y0 <= B.ny; y0 += tile_rows(B)) dt.push_back(Tile{(int)b, 0, y0, z0});
         }
         if ((rc = dalloc(h, &V.d_dtiles, dt.size())) != H3D_OK) return bail(rc);
         if (cudaMemcpy(V.d_dtiles, dt.data(), dt.size() * sizeof(Tile), cudaMemcpyHostToDevice) != cudaSuccess)
