@@ -63,23 +63,6 @@ __device__ void small_relax(const BlkLev* sb, const int* ss, int nb, T* __restri
 }
 
 // ---------------------------------------------------------------------------
-// Exact division by a known divisor: a / b correctly rounded, as the IEEE
-// division the reference's update uses, from y = RN(1/b): q = RN(a y) is at most two
-// units off, one residual step q + (a - b q) y makes it faithful, a second one
-// correctly rounded (P. Markstein, Computation of elementary functions on the IBM
-// RISC System/6000 processor, 1990).  The residuals are exact while nothing
-// under- or overflows: other operands take the division itself.  Five
-// multiply-adds where the division is a subroutine.
-__device__ __forceinline__ bool div_range(double v) {
-  return ((unsigned)(__double2hiint(v) >> 20) & 0x7ffu) - 523u < 1000u;  // 2^-500 <= |v| < 2^500
-}
-__device__ __forceinline__ double div_known(double a, double b, double y) {
-  double q = a * y;
-  q = fma(fma(-b, q, a), y, q);
-  q = fma(fma(-b, q, a), y, q);
-  return __builtin_expect(div_range(a) && div_range(b), 1) ? q : a / b;
-}
-
 // One update of a cell of a constant-coefficient level: sum of the neighbours in
 // the reference's order (FP64), fused in FP32.
 __device__ __forceinline__ double cell_update(const double* p, int sx, int sxy, double ax, double ay, double az,

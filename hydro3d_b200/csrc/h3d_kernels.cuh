@@ -232,7 +232,7 @@ cudaError_t launch_defect_march(int gp, const BlkLev* bl, const Tile* tiles, int
                                 double rscale, double* partials, cudaStream_t st);
 int defect_march_rows();
 
-// pn = p + e on n words (level arrays: a multiple of two).
+// p_next = p + e on n words (level arrays: a multiple of two); p_next may be p.
 template <typename TE>
 cudaError_t launch_apply(const double* p, const TE* e, double* p_next, int64_t n, cudaStream_t st);
 // Level-1 FP64 defect: r = b - A p on the interior, rhs_out = r - mean_b (as
@@ -330,7 +330,7 @@ cudaError_t launch_gather1(const uint32_t* dst, const uint32_t* src, int64_t n, 
 // The projection on level 1 (press.for:2-144, newsolv_mg.for:39-49).
 // calvel: u, v, w from ustar, vstar, wstar and p (dtal = dt*alfapr; dens read
 // for L_LSM only).
-cudaError_t launch_calvel(bool lsm, const BlkLev* bl, RowTab interior_rows, const double* h3, const double* p,
+cudaError_t launch_calvel(bool lsm, const BlkLev* bl, CellTab interior, const double* h3, const double* p,
                           const double* dens, const double* us, const double* vs, const double* ws, double* u,
                           double* v, double* w, double dtal, cudaStream_t st);
 // a_c[dst[e]] = a_c[src[e]] for the three arrays (velocity face ghosts).
@@ -339,13 +339,9 @@ cudaError_t launch_gather3(const uint32_t* dst, const uint32_t* src, int64_t n, 
 // calmas: su into bout (FP64) and rhs_out (TR); partials {sum su^2, 0, rmax,
 // sum su} per CTA (*nparts of them, reduce with launch_reduce4).
 template <typename TR>
-cudaError_t launch_calmas(bool lsm, const BlkLev* bl, RowTab interior_rows, const double* h3, const double* u,
+cudaError_t launch_calmas(bool lsm, const BlkLev* bl, CellTab interior, const double* h3, const double* u,
                           const double* v, const double* w, double dt, double* bout, TR* rhs_out, double* partials,
                           int* nparts, cudaStream_t st);
-// p += e on every cell of every row (ghost layer included).
-template <typename TE>
-cudaError_t launch_padd(const BlkLev* bl, RowTab all_rows, double* p, const TE* e, cudaStream_t st);
-
 // Local mesh refinement.  Expression fill of a level (see ExprTable): one
 // launch per node depth (depth_start: host array of ndepth + 1 offsets), then
 // the ghost writes out[dst[e]] = ref(src[e]).  cur: current values (may be

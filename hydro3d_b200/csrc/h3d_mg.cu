@@ -162,7 +162,7 @@ struct h3d_mg {
   bool per_block = false;    // the defect also reduces its partial sums per block (stop_rule 2)
   double* d_resb = nullptr;  // per block {sum r^2, sum b^2, max|r| dV, sum r}
   double* h_resb = nullptr;  // pinned copy of d_resb
-  double* d_h3 = nullptr;   // per-block dx,dy,dz
+  double* d_h3 = nullptr;   // per-block dx,dy,dz, then their reciprocals
   int* d_err = nullptr;     // set by a device wait that gave up
   double mean_b = 0.0;
   bool coeffs_ready = false;
@@ -986,14 +986,13 @@ struct Exec {
       // p += e, then the pressure halo of p itself (exchange(4) + pbound,
       // newsolv_mg.for:39-52): with refinement the ghosts are averages and
       // extrapolations, so the ghosts of p + e are not those of p plus e's
-      RowTab ra{V.d_rows_all, (int)V.geom.bl.size(), V.nrows_all};
       double* p = h->p64[h->pc];
       if (h->mixed) {
         if (V.zero32) TRY(materialize_zero32(1));
-        CU(launch_padd<float>(V.d_bl, ra, p, V.phi32[V.cur32], h->st));
+        CU(launch_apply<float>(p, V.phi32[V.cur32], p, V.geom.n_elems, h->st));
       } else {
         if (V.zero64) TRY(materialize_zero64(1));
-        CU(launch_padd<double>(V.d_bl, ra, p, V.phi64[V.cur64], h->st));
+        CU(launch_apply<double>(p, V.phi64[V.cur64], p, V.geom.n_elems, h->st));
       }
       TRY(chk("p update", 1));
       TRY(pressure_halo(h));
@@ -1008,14 +1007,13 @@ struct Exec {
   // layer, then exchange(4) + pbound (the face ghosts of the interior rows).
   int proj_update() {
     Level& V = L(1);
-    RowTab ra{V.d_rows_all, (int)V.geom.bl.size(), V.nrows_all};
     double* p = h->p64[h->pc];
     if (h->mixed) {
       if (V.zero32) TRY(materialize_zero32(1));
-      CU(launch_padd<float>(V.d_bl, ra, p, V.phi32[V.cur32], h->st));
+      CU(launch_apply<float>(p, V.phi32[V.cur32], p, V.geom.n_elems, h->st));
     } else {
       if (V.zero64) TRY(materialize_zero64(1));
-      CU(launch_padd<double>(V.d_bl, ra, p, V.phi64[V.cur64], h->st));
+      CU(launch_apply<double>(p, V.phi64[V.cur64], p, V.geom.n_elems, h->st));
     }
     TRY(chk("p update", 1));
     CU(launch_fill<double>(V.faces.d_dst, V.faces.d_src, V.faces.n, p, p, p, false, h->st));
@@ -1028,7 +1026,7 @@ struct Exec {
   // side and the FP64 su (newsolv_mg.for:54-55); the sums reach h_res.
   int vel_defect() {
     Level& V = L(1);
-    RowTab ri{V.d_rows_int, (int)V.geom.bl.size(), V.nrows_int};
+    CellTab ri{V.d_cta_int, (int)V.geom.bl.size(), V.ncta_int};
     CU(launch_calvel(h->var, V.d_bl, ri, h->d_h3, h->p64[h->pc], V.dens, h->vstar[0], h->vstar[1], h->vstar[2],
                      h->vel[0], h->vel[1], h->vel[2], h->proj_dtal, h->st));
     TRY(chk("calvel", 1));
@@ -2991,6 +2989,8 @@ int h3d_mg_solve_resident(h3d_mg* h, const h3d_solve_opts* opts, h3d_solve_info*
   CU(cudaEventCreate(&t1));
   int64_t k0 = h->kernels;
   CU(cudaEventRecord(t0, h->st));
+  for (const auto& d : h->blocks)
+    for (double v : d.h) h3.push_back(1.0 / v);
   Level& V = h->lev[1];
   // pressure halo (exchange(4) + pbound, newsolv_mg.for:51-52)
   TRY(pressure_halo(h));
@@ -3281,7 +3281,6 @@ int h3d_mg_pressure_1sweep(h3d_mg* h, double dt, double alfapr, double eps, int3
   TRY(ensure_sip(h));
   TRY(ensure_velocity(h));
   Level& V = h->lev[1];
-  RowTab ra{V.d_rows_all, (int)V.geom.bl.size(), V.nrows_all};
   h3d_solve_info I{};
   h->history.clear();
   cudaEvent_t t0, t1;
@@ -3304,7 +3303,7 @@ int h3d_mg_pressure_1sweep(h3d_mg* h, double dt, double alfapr, double eps, int3
     TRY(sip_run(h, nswp, &ns, nullptr));
     total += ns;
     double* p = h->p64[h->pc];
-    CU(launch_padd<double>(V.d_bl, ra, p, h->sip_pp, h->st));  // p = p + (pp - ppref), ppref = 0
+    CU(launch_apply<double>(p, h->sip_pp, p, V.geom.n_elems, h->st));  // p = p + (pp - ppref), ppref = 0
     CU(cudaMemsetAsync(h->sip_pp, 0, bytes, h->st));
     CU(launch_fill<double>(V.faces.d_dst, V.faces.d_src, V.faces.n, p, p, p, false, h->st));  // exchange(4), pbound
     h->kernels += 2;
@@ -3354,7 +3353,7 @@ int h3d_mg_calvel(h3d_mg* h, double dt, double alfapr) {
   TRY(ensure_velocity(h));
   set_projection_scalars(h, dt, alfapr);
   Level& V = h->lev[1];
-  RowTab ri{V.d_rows_int, (int)V.geom.bl.size(), V.nrows_int};
+  CellTab ri{V.d_cta_int, (int)V.geom.bl.size(), V.ncta_int};
   CU(launch_calvel(h->var, V.d_bl, ri, h->d_h3, h->p64[h->pc], V.dens, h->vstar[0], h->vstar[1], h->vstar[2],
                    h->vel[0], h->vel[1], h->vel[2], h->proj_dtal, h->st));
   CU(launch_gather3(h->d_vdst, h->d_vsrc, h->nvfill, h->vel[0], h->vel[1], h->vel[2], h->st));
@@ -3368,7 +3367,7 @@ int h3d_mg_calmas(h3d_mg* h, double dt, double* rmax, double* su2) {
   CU(cudaSetDevice(h->device));
   TRY(ensure_velocity(h));
   Level& V = h->lev[1];
-  RowTab ri{V.d_rows_int, (int)V.geom.bl.size(), V.nrows_int};
+  CellTab ri{V.d_cta_int, (int)V.geom.bl.size(), V.ncta_int};
   int np = 0;
   if (h->mixed)
     CU(launch_calmas<float>(h->var, V.d_bl, ri, h->d_h3, h->vel[0], h->vel[1], h->vel[2], dt, h->b64, V.rhs32,
