@@ -514,6 +514,14 @@ struct RowGs {
       }
   }
 
+  // FP64, constant coefficients: the update from a zero iterate, rhs / diagonal.
+  __device__ __forceinline__ T from_zero(int k, int m, int z, T rv) const {
+    if (z > 1 && z < nz)
+      return div_known(rv, -((m ? cxy[k][1] : cxy[k][0]) + az + az), m ? cinv[k][1] : cinv[k][0]);
+    const T ab = (z == 1 && (ph & 16)) ? T(0) : az, at = (z == nz && (ph & 32)) ? T(0) : az;
+    return gs_div(rv, -((m ? cxy[k][1] : cxy[k][0]) + ab + at));
+  }
+
   // New value of the cell at smem index s (row pitch sp) of plane z, pair k,
   // member m; rv = its right-hand side; i = its offset in the block (VAR).
   __device__ __forceinline__ T update(const T* P, const T* Pm, const T* Pp, int s, int sp, int k, int m, int z,
@@ -743,7 +751,7 @@ struct Tma2Cfg {
   static constexpr size_t SMEM = (size_t)NS * SLOT + 128 + NS * 8;
 };
 
-template <typename T, int TPR, int CP, int TY, int D, bool VAR>
+template <typename T, int TPR, int CP, int TY, int D, bool VAR, bool ZERO = false>
 __global__ void __launch_bounds__(TPR*(TY + 2)) k_rbgs_tma2(const BlkLev* __restrict__ bls,
                                                            const Tile* __restrict__ tiles, int zc,
                                                            const CUtensorMap* __restrict__ maps,
@@ -774,7 +782,7 @@ __global__ void __launch_bounds__(TPR*(TY + 2)) k_rbgs_tma2(const BlkLev* __rest
   const int ze = min(zs + zc - 1, nz);
   const int zlo = max(zs - 1, 1), zhi = min(ze + 1, nz);
   const int BX = ((nx + 2 + kXOff + C::VEC - 1) / C::VEC) * C::VEC;  // smem row pitch == TMA box width
-  const uint32_t tx_bytes = (uint32_t)(BX * (2 * TY + 6) * (int)sizeof(T));
+  const uint32_t tx_bytes = (uint32_t)(BX * (ZERO ? TY + 2 : 2 * TY + 6) * (int)sizeof(T));
   const int tr = threadIdx.x / TPR, tc = threadIdx.x - (threadIdx.x / TPR) * TPR;
   const int y = y0 - 1 + tr;
   const int prow = (tr + 1) * BX + kXOff;  // cell (x, y) of an iterate slot (slot row 0 = y0-2)
@@ -789,6 +797,10 @@ __global__ void __launch_bounds__(TPR*(TY + 2)) k_rbgs_tma2(const BlkLev* __rest
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(bars + q)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
+  if (ZERO)  // the iterate's slots: zero but for the red cells this kernel writes
+    for (int q = threadIdx.x; q < NS * (C::PSLOT / 16); q += TPR * (TY + 2))
+      *reinterpret_cast<float4*>(base + (q / (C::PSLOT / 16)) * C::SLOT + q % (C::PSLOT / 16) * 16) =
+          make_float4(0.f, 0.f, 0.f, 0.f);
   __syncthreads();
 
   auto pslot = [&](int z) -> T* { return reinterpret_cast<T*>(base + (z % NS) * C::SLOT); };
@@ -799,8 +811,9 @@ __global__ void __launch_bounds__(TPR*(TY + 2)) k_rbgs_tma2(const BlkLev* __rest
     const uint32_t bar = smem_u32(bars + (z % NS));
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(tx_bytes) : "memory");
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n" ::
+    if (!ZERO)
+      asm volatile(
+          "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n" ::
             "r"(smem_u32(pslot(z))),
         "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(y0 - 2), "r"(z), "r"(bar)
         : "memory");
@@ -828,7 +841,9 @@ __global__ void __launch_bounds__(TPR*(TY + 2)) k_rbgs_tma2(const BlkLev* __rest
 #pragma unroll
     for (int k = 0; k < CP; ++k) {
       const int x = 2 * (tc + k * TPR) + 1 + j;
-      if (x <= nx && H3D_IN(44, t.b, prow + x - BX, C::PSLOT / (int)sizeof(T) - 2 * BX))
+      if (ZERO) {
+        if (x <= nx) P[prow + x] = gs.from_zero(k, j, z, Rr[x]);
+      } else if (x <= nx && H3D_IN(44, t.b, prow + x - BX, C::PSLOT / (int)sizeof(T) - 2 * BX))
         P[prow + x] = gs.update(P, Pm, Pp, prow + x, BX, k, j, z, Rr[x], FX, FY, FZ, zo + x, sx, sxy);
     }
   };
@@ -863,6 +878,13 @@ __global__ void __launch_bounds__(TPR*(TY + 2)) k_rbgs_tma2(const BlkLev* __rest
     if (z <= zhi) {
       wait_plane(z + 1);
       red(z);
+    } else if (ZERO && z == nz + 1 && row_in) {  // the ghost plane above, in a slot that held red cells
+      T* P = pslot(z) + prow;
+#pragma unroll
+      for (int k = 0; k < CP; ++k) {
+        const int x = 2 * (tc + k * TPR) + 1;
+        if (x <= nx) P[x] = P[x + 1] = T(0);
+      }
     }
     if (z - 2 >= zs && z - 2 <= ze) black_store(z - 2);
     // this phase's shared-memory writes are ordered before the TMA that reuses their slot
@@ -1684,10 +1706,14 @@ static cudaError_t tma2_attr() {
   cudaError_t e;
   if ((e = cudaFuncSetAttribute(k_rbgs_tma2<T, TPR, CP, TY, D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))) return e;
   return cudaFuncSetAttribute(k_rbgs_tma2<T, TPR, CP, TY, D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+  if constexpr (sizeof(T) == 8) {
+    e = cudaFuncSetAttribute(k_rbgs_tma2<T, TPR, CP, TY, D, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    if (e != cudaSuccess) return e;
+  }
 }
 
 template <typename T, int TPR, int CP, int TY, int D0>
-static cudaError_t tma2_dispatch(bool var, const BlkLev* bl, const Tile* tiles, int ntiles, int zc,
+static cudaError_t tma2_dispatch(bool var, bool zero, const BlkLev* bl, const Tile* tiles, int ntiles, int zc,
                                  const CUtensorMap* maps, const CUtensorMap* rmaps, int* err, T* dst, const T* fx,
                                  const T* fy, const T* fz, float om, cudaStream_t st) {
   if (ntiles <= 0) return cudaSuccess;
@@ -1695,6 +1721,11 @@ static cudaError_t tma2_dispatch(bool var, const BlkLev* bl, const Tile* tiles, 
   constexpr int NT = TPR * (TY + 2);
   constexpr size_t SM = Tma2Cfg<T, TPR, CP, TY, D>::SMEM;
   if (var) pdl_launch(k_rbgs_tma2<T, TPR, CP, TY, D, true>, ntiles, NT, SM, st, bl, tiles, zc, maps, rmaps, dst, fx, fy, fz, err, om);
+  if constexpr (sizeof(T) == 8)
+    if (zero && !var) {
+      pdl_launch(k_rbgs_tma2<T, TPR, CP, TY, D, false, true>, ntiles, NT, SM, st, bl, tiles, zc, maps, rmaps, dst, fx, fy, fz, err, om);
+      return cudaGetLastError();
+    }
   else pdl_launch(k_rbgs_tma2<T, TPR, CP, TY, D, false>, ntiles, NT, SM, st, bl, tiles, zc, maps, rmaps, dst, fx, fy, fz, err, om);
   return cudaGetLastError();
 }
@@ -2167,11 +2198,14 @@ cudaError_t launch_rbgs(int variant, bool var, bool zero_src, const BlkLev* bl, 
   // ghost pushes need the register-window sweep to run as asked
   if (push && (!rbgs_pushes(variant, var, sizeof(T) == 4) || !maps || !rmaps)) return cudaErrorInvalidValue;
   if (variant >= 0 && variant < num_tile_shapes() && kShapes[variant].tma) {
-    // nothing to stage from a zero source: the equivalent plain-load kernel zero-fills;
-    // the vectorised sweep is FP32 with constant coefficients only
+    // a zero source is not staged: the register-window and the FP64 sweeps with constant
+    // coefficients have a form without it (FP64, eight 96^3 blocks: 103
+    // us by the plain-load kernel, 64 us), the others take the equivalent plain-load
+    // kernel; the vectorised sweep is FP32 with constant coefficients only
     const int tk = kShapes[variant].tma;
     const bool win = variant >= kFirstWinShape;  // register-window sweeps handle a zero source themselves
-    if ((zero_src && !(win && sizeof(T) == 4 && !var)) || !maps || (tk >= 2 && !rmaps) ||
+    const bool zero_form = !var && (sizeof(T) == 4 ? win : tk == 2);
+    if ((zero_src && !zero_form) || !maps || (tk >= 2 && !rmaps) ||
         (tk == 3 && (var || sizeof(T) != 4)))
       variant = kShapes[variant].alt;
   }
@@ -2202,7 +2236,7 @@ cudaError_t launch_rbgs(int variant, bool var, bool zero_src, const BlkLev* bl, 
     H3D_ROW_SHAPES(X)
 #undef X
 #define X(v, tpr, cp, ty, d) \
-    case v: return tma2_dispatch<T, tpr, cp, ty, d>(var, bl, tiles, ntiles, zc, maps, rmaps, err, dst, fx, fy, fz, om, st);
+    case v: return tma2_dispatch<T, tpr, cp, ty, d>(var, zero_src, bl, tiles, ntiles, zc, maps, rmaps, err, dst, fx, fy, fz, om, st);
     H3D_TMA2_SHAPES(X)
 #undef X
     default: return cudaErrorInvalidValue;

@@ -80,7 +80,7 @@ struct Level {
   Halo sweep, faces, exch, bound;
   Halo sweep_push;              // the sweep fill without the faces the register-window sweeps push
   Halo live, live_push;         // the parts of sweep / sweep_push that the next sweep or restriction reads
-  bool live_ok = false;         // live fills may stand in for the full fill (FP32 RBGS levels)
+  bool live_ok = false;         // live fills may stand in for the full fill (RBGS levels)
   Halo red;                     // red cells next to block faces and the ghosts that show them (k_red_ahead)
   int* d_red_info = nullptr;    // their blocks and wall faces (k_red_ahead)
   bool red_ok = false;          // FP32 sweeps of this level take the red-black order across block faces
@@ -180,6 +180,8 @@ struct h3d_mg {
   double* stage[2] = {nullptr, nullptr};
   std::vector<size_t> stage_off;
   // fused coarse tail: levels tail_g..L in one single-CTA launch (tail_g = 0: none)
+  bool solving = false;     // inside a solve (its FP64 sweeps fill the live ghosts only)
+  bool unclean = true;      // some level array may hold a NaN or infinity, which a ghost left unfilled would keep
   int tail_g = 0;
   bool lmr = false;  // blocks of different refinement ratio or level count (LMR = 2)
   TailLevel* d_tail_lv = nullptr;
@@ -666,7 +668,8 @@ struct Exec {
                              V.fx64, V.fy64, V.fz64, nullptr, 1.f, st));
       TRY(chk("sweep fp64", g));
       if (e1) CU(record(e1));
-      TRY(sweep_fill<double>(V, V.sweep, dst, src, V.zero64, &h->kernels));
+      // (live fills in solves only: the level entry points show every ghost)
+      TRY(sweep_fill<double>(V, partial && V.live_ok && h->solving ? V.live : V.sweep, dst, src, V.zero64, &h->kernels));
       TRY(chk("fill fp64", g));
       V.cur64 = 1 - V.cur64;
       V.zero64 = false;
@@ -1188,6 +1191,29 @@ int check_block_host_dims(h3d_mg* h, const h3d_block_desc& d) {
 // it is only used in calls that staged the same host array in (the planes'
 // other cells then round-trip unchanged).
 int ensure_stage(h3d_mg* h, int f) {
+// A solve leaves the ghosts of physical walls unfilled between its sweeps (live
+// fills): they must be finite.  Clears the level iterates after calls that may
+// have put anything there; a solve that ends with a finite residual leaves them
+// finite.
+struct SolveScope {
+  h3d_mg* h;
+  explicit SolveScope(h3d_mg* h_) : h(h_) { h->solving = true; }
+  ~SolveScope() { h->solving = false; }
+  int begin() {
+    if (!h->unclean) return H3D_OK;
+    for (int g = 1; g <= h->L; ++g) {
+      Level& V = h->lev[g];
+      for (int q = 0; q < 2; ++q) {
+        const size_t n = (size_t)V.geom.n_elems;
+        if (V.phi64[q]) CU(cudaMemsetAsync(V.phi64[q], 0, n * sizeof(double), h->st));
+        if (V.phi32[q]) CU(cudaMemsetAsync(V.phi32[q], 0, n * sizeof(float), h->st));
+      }
+    }
+    h->unclean = false;
+    return H3D_OK;
+  }
+};
+
   if (h->stage[f]) return H3D_OK;
   size_t n = 0;
   h->stage_off.clear();
@@ -1678,7 +1704,7 @@ int build_live(h3d_mg* h, Level& V, const std::vector<uint32_t>& d, const std::v
   std::vector<uint32_t> ld, ls;
   V.live_ok = live_entries(V.geom, d, s, &ld, &ls);
   if (V.live_ok) TRY(upload_halo(h, V.live, ld, ls));
-  if (V.live_ok && h->mixed && h->desc.mg_itrsch == 3 && h->rb_global) TRY(build_red_ahead(h, V, ld, ls));
+  if (V.live_ok && V.f32 && h->desc.mg_itrsch == 3 && h->rb_global) TRY(build_red_ahead(h, V, ld, ls));
   return H3D_OK;
 }
 
@@ -2632,7 +2658,7 @@ int h3d_mg_create(h3d_mg** out, const h3d_mg_desc* desc) {
         return bail(fail(h, rc, err));
       if ((rc = upload_halo(h, V.sweep, d, s)) != H3D_OK) return bail(rc);
     }
-    if (!V.expr && f32_level(h, g) && (rc = build_live(h, V, d, s)) != H3D_OK) return bail(rc);
+    if (!V.expr && h->desc.mg_itrsch == 3 && (rc = build_live(h, V, d, s)) != H3D_OK) return bail(rc);
     if (!V.expr && f32_level(h, g) && !h->var && (rc = build_push(h, V, d, s)) != H3D_OK) return bail(rc);
     if (h->lmr) {  // blocks past their last level restrict by a copy and correct by an add
       if (g >= 2 && (rc = upload_block_list(h, V.geom, V.geom.clamped, false, &V.d_rsame, &V.nrsame,
@@ -2696,6 +2722,8 @@ int h3d_mg_create(h3d_mg** out, const h3d_mg_desc* desc) {
           st.push_back((int)ld.size());
         }
         if ((rc = upload_halo(h, V.lfill, ld, ls)) != H3D_OK) return bail(rc);
+    V.f32 = f32_level(h, g);
+    V.var = h->var;
         if ((rc = dalloc(h, &V.d_lfstart, st.size())) != H3D_OK) return bail(rc);
         if (cudaMemcpy(V.d_lfstart, st.data(), st.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
           return bail(fail(h, H3D_ERR_CUDA, "block-local fill table"));
@@ -2729,8 +2757,6 @@ int h3d_mg_create(h3d_mg** out, const h3d_mg_desc* desc) {
       if ((rc = build_halo_table(h->blocks, g, kHaloFaces, true, d, s, &err)) != H3D_OK) return bail(fail(h, rc, err));
       if ((rc = upload_halo(h, V.faces, d, s)) != H3D_OK) return bail(rc);
     }
-    V.f32 = f32_level(h, g);
-    V.var = h->var;
     if (g < h->L) {
       // prolongation tiles: plane pairs (2m, 2m+1) of a block, ghost planes included;
       // level 1 also: row tiles of the tiled defect (kProlongRows rows of one plane)
@@ -2989,6 +3015,7 @@ int h3d_mg_solve_resident(h3d_mg* h, const h3d_solve_opts* opts, h3d_solve_info*
   CU(cudaEventCreate(&t1));
   int64_t k0 = h->kernels;
   CU(cudaEventRecord(t0, h->st));
+  h->unclean = true;
   for (const auto& d : h->blocks)
     for (double v : d.h) h3.push_back(1.0 / v);
   Level& V = h->lev[1];
@@ -3046,7 +3073,7 @@ int h3d_mg_solve_resident(h3d_mg* h, const h3d_solve_opts* opts, h3d_solve_info*
     rinf = h->h_res[2];
     relb = block_max();
     if (opts->record_history) h->history.push_back(opts->stop_rule == 2 ? relb : rel);
-    if (!std::isfinite(rel) || rel > 1e8 || !std::isfinite(relb)) { status = 2; break; }
+    if (!std::isfinite(rel) || rel > 1e8 || !std::isfinite(relb)) { status = 2; h->unclean = true; break; }
     if (opts->stop_rule == 0 && rel <= opts->tol) status = 0;
     if (opts->stop_rule == 1 && rinf < opts->tol && iter > 1) status = 0;  // newsolv_mg.for:57
     if (opts->stop_rule == 2 && relb <= opts->tol) status = 0;
@@ -3101,6 +3128,8 @@ int h3d_mg_history(h3d_mg* h, double* out, int32_t cap, int32_t* n) {
   int k = (int)std::min<size_t>(h->history.size(), (size_t)std::max(cap, 0));
   if (out)
     for (int q = 0; q < k; ++q) out[q] = h->history[q];
+  SolveScope scope(h);
+  TRY(scope.begin());
   *n = (int)h->history.size();
   return H3D_OK;
 }
@@ -3437,7 +3466,7 @@ int h3d_mg_project_resident(h3d_mg* h, double dt, double alfapr, const h3d_solve
     rel = std::sqrt(h->h_res[0]) / bn;
     rmax = h->h_res[2];
     if (opts->record_history) h->history.push_back(opts->stop_rule == 1 ? rmax : rel);
-    if (!std::isfinite(rel) || !std::isfinite(rmax) || rel > 1e8) { status = 2; break; }
+    if (!std::isfinite(rel) || !std::isfinite(rmax) || rel > 1e8) { status = 2; h->unclean = true; break; }
     if (opts->stop_rule == 0 && rel <= opts->tol) status = 0;
     if (opts->stop_rule == 1 && rmax < opts->tol && iter > 1) status = 0;  // newsolv_mg.for:57
   }
@@ -3529,6 +3558,8 @@ int h3d_mg_put_level(h3d_mg* h, int32_t g, int32_t field, int32_t ib, const doub
     std::memcpy(buf.data(), a, nb * 8);
   } else {
     for (int z = 1; z <= B.nz; ++z)
+  SolveScope scope(h);
+  TRY(scope.begin());
       for (int y = 1; y <= B.ny; ++y)
         for (int x = 1; x <= B.nx; ++x)
           buf[((size_t)z * (B.ny + 2) + y) * (B.nx + 2) + x] = a[((size_t)(z - 1) * B.ny + (y - 1)) * B.nx + (x - 1)];
@@ -3639,6 +3670,7 @@ static int apply_table_hook(h3d_mg* h, int g, int kind) {
     std::vector<uint32_t> d, s;
     std::string err;
     int rc = build_halo_table(h->blocks, g, kind, true, d, s, &err);
+  h->unclean = true;
     if (rc != H3D_OK) return fail(h, rc, err);
     TRY(upload_halo(h, *H, d, s));
     H->built = true;
@@ -3697,6 +3729,7 @@ int h3d_mg_mgkcyc(h3d_mg* h, double* const* pp, const double* const* su) {
     } else {
       TRY(stage_in(h, 0, ib, pp[ib], V.phi64[V.cur64], true));
       TRY(stage_in(h, 1, ib, su[ib], V.rhs64, false));
+  h->unclean = true;
     }
   }
   if (h->mixed) {
@@ -3707,6 +3740,7 @@ int h3d_mg_mgkcyc(h3d_mg* h, double* const* pp, const double* const* su) {
     V.zero64 = false;
   }
   Exec ex{h};
+  h->unclean = true;
   TRY(ex.vcycle());
   if (h->mixed) CU(launch_convert_f2d(V.phi32[V.cur32], h->p64[1 - h->pc], V.geom.n_elems, h->st));
   for (int ib = 0; ib < (int)h->blocks.size(); ++ib)
@@ -3721,6 +3755,7 @@ int h3d_mg_sync(h3d_mg* h) {
   CU(cudaStreamSynchronize(h->st));
   return H3D_OK;
 }
+  h->unclean = true;
 
 int h3d_mg_set_wait_limit(h3d_mg* h, int64_t clocks) {
   if (!h) return H3D_ERR_ARG;
@@ -3730,6 +3765,7 @@ int h3d_mg_set_wait_limit(h3d_mg* h, int64_t clocks) {
   return H3D_OK;
 }
 
+  h->unclean = true;
 int h3d_mg_wait_probe(h3d_mg* h) {
   if (!h) return H3D_ERR_ARG;
   CU(cudaSetDevice(h->device));
@@ -3796,4 +3832,6 @@ int h3d_mg_smoother_bytes(h3d_mg* h, double* bytes) {
   return H3D_OK;
 }
 
+  h->unclean = true;
 }  // extern "C"
+  h->unclean = true;
