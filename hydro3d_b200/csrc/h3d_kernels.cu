@@ -1232,10 +1232,11 @@ __global__ void __launch_bounds__(256) k_prolong(const BlkLev* __restrict__ fine
 }
 
 
-// p_next = p + e over whole level arrays (ghosts included, newsolv_mg.for:39-48).
+// p_next = p + e over whole level arrays (ghosts included, newsolv_mg.for:39-48);
+// p_next may be p.
 template <typename TE>
-__global__ void __launch_bounds__(256) k_apply(const double* __restrict__ p, const TE* __restrict__ e,
-                                               double* __restrict__ p_next, int64_t n) {
+__global__ void __launch_bounds__(256) k_apply(const double* p, const TE* __restrict__ e, double* p_next,
+                                               int64_t n) {
   pdl_trigger();
   pdl_wait();
   using E2 = typename std::conditional<sizeof(TE) == 4, float2, double2>::type;
@@ -1705,11 +1706,11 @@ static cudaError_t tma2_attr() {
   const int sm = (int)Tma2Cfg<T, TPR, CP, TY, D>::SMEM;
   cudaError_t e;
   if ((e = cudaFuncSetAttribute(k_rbgs_tma2<T, TPR, CP, TY, D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))) return e;
-  return cudaFuncSetAttribute(k_rbgs_tma2<T, TPR, CP, TY, D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
   if constexpr (sizeof(T) == 8) {
     e = cudaFuncSetAttribute(k_rbgs_tma2<T, TPR, CP, TY, D, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     if (e != cudaSuccess) return e;
   }
+  return cudaFuncSetAttribute(k_rbgs_tma2<T, TPR, CP, TY, D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
 }
 
 template <typename T, int TPR, int CP, int TY, int D0>
@@ -1720,12 +1721,12 @@ static cudaError_t tma2_dispatch(bool var, bool zero, const BlkLev* bl, const Ti
   constexpr int D = tma2_depth<T, TPR, CP, TY, D0>();
   constexpr int NT = TPR * (TY + 2);
   constexpr size_t SM = Tma2Cfg<T, TPR, CP, TY, D>::SMEM;
-  if (var) pdl_launch(k_rbgs_tma2<T, TPR, CP, TY, D, true>, ntiles, NT, SM, st, bl, tiles, zc, maps, rmaps, dst, fx, fy, fz, err, om);
   if constexpr (sizeof(T) == 8)
     if (zero && !var) {
       pdl_launch(k_rbgs_tma2<T, TPR, CP, TY, D, false, true>, ntiles, NT, SM, st, bl, tiles, zc, maps, rmaps, dst, fx, fy, fz, err, om);
       return cudaGetLastError();
     }
+  if (var) pdl_launch(k_rbgs_tma2<T, TPR, CP, TY, D, true>, ntiles, NT, SM, st, bl, tiles, zc, maps, rmaps, dst, fx, fy, fz, err, om);
   else pdl_launch(k_rbgs_tma2<T, TPR, CP, TY, D, false>, ntiles, NT, SM, st, bl, tiles, zc, maps, rmaps, dst, fx, fy, fz, err, om);
   return cudaGetLastError();
 }
@@ -3279,6 +3280,18 @@ __global__ void __launch_bounds__(256) k_face_coef_sum(const BlkLev* __restrict_
     cfz[ic] = (((ffz[fi(X, Y, Z)] + ffz[fi(X + 1, Y, Z)]) + ffz[fi(X, Y + 1, Z)]) + ffz[fi(X + 1, Y + 1, Z)]) * 0.0625;
   }
 }
+// Interior cell (from 1) of this thread in cell tile c (256 cells of a block).
+__device__ __forceinline__ bool interior_cell(const BlkLev* __restrict__ bls, const int* __restrict__ cta_start,
+                                              int nb, int c, int* b, int* x, int* y, int* z) {
+  *b = find_block(cta_start, nb, c);
+  const int nx = bls[*b].nx, ny = bls[*b].ny;
+  const int q = (c - cta_start[*b]) * 256 + threadIdx.x;
+  *x = q % nx + 1;
+  *y = q / nx % ny + 1;
+  *z = q / (nx * ny) + 1;
+  return *z <= bls[*b].nz;
+}
+
 
 // ---------------------------------------------------------------------------
 // The projection (press.for:2-144).  Face velocities live in the level-1
@@ -3291,44 +3304,38 @@ __global__ void __launch_bounds__(256) k_face_coef_sum(const BlkLev* __restrict_
 // physical wall: ieu = iep - 1, localparameters.for:186-192; v and w alike),
 // divided by the face density 0.5*(dens(i)+dens(i+1)) for L_LSM.  Operand
 // order as written there (dtal = dt*alfapr, then *(dp), /dx, /face density).
-// One warp per interior row.
+// h3: spacings of every block, then their reciprocals.
 template <bool LSM>
-__global__ void __launch_bounds__(256) k_calvel(const BlkLev* __restrict__ bls, const int* __restrict__ row_start,
-                                                int nb, int nrows, const double* __restrict__ h3,
+__global__ void __launch_bounds__(256) k_calvel(const BlkLev* __restrict__ bls, const int* __restrict__ cta_start,
+                                                int nb, int ncta, const double* __restrict__ h3,
                                                 const double* __restrict__ p, const double* __restrict__ dens,
                                                 const double* __restrict__ us, const double* __restrict__ vs,
                                                 const double* __restrict__ ws, double* __restrict__ u,
                                                 double* __restrict__ v, double* __restrict__ w, double dtal) {
   pdl_trigger();
   pdl_wait();
-  const int lane = threadIdx.x & 31;
-  for (int rid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; rid < nrows; rid += (gridDim.x * blockDim.x) >> 5) {
-    const RowRef ref = row_of(bls, row_start, nb, rid, true);
-    const BlkLev B = bls[ref.b];
-    const int y = ref.y, z = ref.z;
-    const double dx = h3[3 * ref.b], dy = h3[3 * ref.b + 1], dz = h3[3 * ref.b + 2];
-    const int nxu = B.nx - ((B.phys & 2) ? 1 : 0);
-    const bool vrow = y <= B.ny - ((B.phys & 8) ? 1 : 0);
-    const bool wrow = z <= B.nz - ((B.phys & 32) ? 1 : 0);
-    const long long rowg = B.off + (long long)z * B.sxy + (long long)y * B.sx;
-    for (int x = 1 + lane; x <= B.nx; x += 32) {
-      const long long i = rowg + x;
-      const double pc = p[i];
-      if (x <= nxu) {
-        double t = dtal * (p[i + 1] - pc) / dx;
-        if (LSM) t = t / (0.5 * (dens[i] + dens[i + 1]));
-        u[i] = us[i] - t;
-      }
-      if (vrow) {
-        double t = dtal * (p[i + B.sx] - pc) / dy;
-        if (LSM) t = t / (0.5 * (dens[i] + dens[i + B.sx]));
-        v[i] = vs[i] - t;
-      }
-      if (wrow) {
-        double t = dtal * (p[i + B.sxy] - pc) / dz;
-        if (LSM) t = t / (0.5 * (dens[i] + dens[i + B.sxy]));
-        w[i] = ws[i] - t;
-      }
+  for (int c = blockIdx.x; c < ncta; c += gridDim.x) {
+    int b, x, y, z;
+    if (!interior_cell(bls, cta_start, nb, c, &b, &x, &y, &z)) continue;
+    const BlkLev& B = bls[b];
+    const double dx = h3[3 * b], dy = h3[3 * b + 1], dz = h3[3 * b + 2];
+    const double* ih = h3 + 3 * (nb + b);  // their reciprocals
+    const long long sy = B.sx, sz = B.sxy, i = B.off + z * sz + y * sy + x;
+    const double pc = p[i];
+    if (x <= B.nx - ((B.phys & 2) ? 1 : 0)) {
+      double t = div_known(dtal * (p[i + 1] - pc), dx, ih[0]);
+      if (LSM) t = t / (0.5 * (dens[i] + dens[i + 1]));
+      u[i] = us[i] - t;
+    }
+    if (y <= B.ny - ((B.phys & 8) ? 1 : 0)) {
+      double t = div_known(dtal * (p[i + sy] - pc), dy, ih[1]);
+      if (LSM) t = t / (0.5 * (dens[i] + dens[i + sy]));
+      v[i] = vs[i] - t;
+    }
+    if (z <= B.nz - ((B.phys & 32) ? 1 : 0)) {
+      double t = div_known(dtal * (p[i + sz] - pc), dz, ih[2]);
+      if (LSM) t = t / (0.5 * (dens[i] + dens[i + sz]));
+      w[i] = ws[i] - t;
     }
   }
 }
@@ -3353,53 +3360,37 @@ __global__ void __launch_bounds__(256) k_gather3(const uint32_t* __restrict__ ds
 // rmax = max |fact*dx*dy*dz|.  su goes to bout (FP64) and to the level-1
 // right-hand side rhs_out (as TR); per-CTA partials {sum su^2, 0, rmax,
 // sum su}.
+// One thread a cell, eight CTAs an SM: a warp a row kept too few loads in
+// flight (2.6M cells: 75 us, 46 us here), and the divisions by the spacings and
+// dt are exact multiply-adds (div_known).
 template <bool LSM, typename TR>
-__global__ void __launch_bounds__(256) k_calmas(const BlkLev* __restrict__ bls, const int* __restrict__ row_start,
-                                                int nb, int nrows, const double* __restrict__ h3,
+__global__ void __launch_bounds__(256) k_calmas(const BlkLev* __restrict__ bls, const int* __restrict__ cta_start,
+                                                int nb, int ncta, const double* __restrict__ h3,
                                                 const double* __restrict__ u, const double* __restrict__ v,
                                                 const double* __restrict__ w, double dt, double* __restrict__ bout,
                                                 TR* __restrict__ rhs_out, double* __restrict__ partials) {
   pdl_trigger();
   pdl_wait();
-  const int lane = threadIdx.x & 31;
   double ss = 0, rm = 0, rs = 0;
-  for (int rid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; rid < nrows; rid += (gridDim.x * blockDim.x) >> 5) {
-    const RowRef ref = row_of(bls, row_start, nb, rid, true);
-    const BlkLev B = bls[ref.b];
-    const double dx = h3[3 * ref.b], dy = h3[3 * ref.b + 1], dz = h3[3 * ref.b + 2];
-    const long long rowg = B.off + (long long)ref.z * B.sxy + (long long)ref.y * B.sx;
-    for (int x = 1 + lane; x <= B.nx; x += 32) {
-      const long long i = rowg + x;
-      const double fact = (u[i] - u[i - 1]) / dx + (v[i] - v[i - B.sx]) / dy + (w[i] - w[i - B.sxy]) / dz;
-      const double s = LSM ? fact * dx * dy * dz / dt : fact / dt;
-      bout[i] = s;
-      rhs_out[i] = (TR)s;
-      ss += s * s;
-      rs += s;
-      const double a = fabs(fact * dx * dy * dz);
-      if (!(a <= rm)) rm = a;  // keeps a NaN
-    }
+  const double idt = 1.0 / dt;
+  for (int c = blockIdx.x; c < ncta; c += gridDim.x) {
+    int b, x, y, z;
+    if (!interior_cell(bls, cta_start, nb, c, &b, &x, &y, &z)) continue;
+    const BlkLev& B = bls[b];
+    const double dx = h3[3 * b], dy = h3[3 * b + 1], dz = h3[3 * b + 2];
+    const double* ih = h3 + 3 * (nb + b);  // their reciprocals
+    const long long sy = B.sx, sz = B.sxy, i = B.off + z * sz + y * sy + x;
+    const double fact = div_known(u[i] - u[i - 1], dx, ih[0]) + div_known(v[i] - v[i - sy], dy, ih[1]) +
+                        div_known(w[i] - w[i - sz], dz, ih[2]);
+    const double s = div_known(LSM ? fact * dx * dy * dz : fact, dt, idt);
+    bout[i] = s;
+    rhs_out[i] = (TR)s;
+    ss += s * s;
+    rs += s;
+    const double a = fabs(fact * dx * dy * dz);
+    if (!(a <= rm)) rm = a;  // keeps a NaN
   }
   block_reduce4<256>(ss, 0.0, rm, rs, partials + 4 * (size_t)blockIdx.x);
-}
-
-// p = p + (pp - ppref) over the block and its ghost layer (newsolv_mg.for:
-// 39-49, ppref = 0): one warp per row of every row.
-template <typename TE>
-__global__ void __launch_bounds__(256) k_padd(const BlkLev* __restrict__ bls, const int* __restrict__ row_start,
-                                              int nb, int nrows, double* __restrict__ p, const TE* __restrict__ e) {
-  pdl_trigger();
-  pdl_wait();
-  const int lane = threadIdx.x & 31;
-  for (int rid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; rid < nrows; rid += (gridDim.x * blockDim.x) >> 5) {
-    const RowRef ref = row_of(bls, row_start, nb, rid, false);
-    const BlkLev B = bls[ref.b];
-    const long long rowg = B.off + (long long)ref.z * B.sxy + (long long)ref.y * B.sx;
-    for (int x = lane; x <= B.nx + 1; x += 32) {
-      const long long i = rowg + x;
-      p[i] = p[i] + ((double)e[i] - 0.0);
-    }
-  }
 }
 
 }  // namespace
@@ -3583,13 +3574,19 @@ cudaError_t launch_face_coef_sum(const BlkLev* fine, const BlkLev* coarse, CellT
   return cudaGetLastError();
 }
 
-cudaError_t launch_calvel(bool lsm, const BlkLev* bl, RowTab rt, const double* h3, const double* p,
+constexpr int kCellCtas = 148 * 8;  // CTAs of the cell kernels of the projection
+
+cudaError_t launch_calvel(bool lsm, const BlkLev* bl, CellTab ct, const double* h3, const double* p,
                           const double* dens, const double* us, const double* vs, const double* ws, double* u,
                           double* v, double* w, double dtal, cudaStream_t st) {
-  if (rt.nrows <= 0) return cudaSuccess;
-  const int g = defect_grid(rt.nrows);
-  if (lsm) pdl_launch(k_calvel<true>, g, 256, 0, st, bl, rt.start, rt.nb, rt.nrows, h3, p, dens, us, vs, ws, u, v, w, dtal);
-  else pdl_launch(k_calvel<false>, g, 256, 0, st, bl, rt.start, rt.nb, rt.nrows, h3, p, dens, us, vs, ws, u, v, w, dtal);
+  if (ct.ncta <= 0) return cudaSuccess;
+  const int g = ct.ncta;
+  if (lsm)
+    pdl_launch(k_calvel<true>, g, 256, 0, st, bl, ct.cta_start, ct.nb, ct.ncta, h3, p, dens, us, vs, ws, u, v, w,
+               dtal);
+  else
+    pdl_launch(k_calvel<false>, g, 256, 0, st, bl, ct.cta_start, ct.nb, ct.ncta, h3, p, dens, us, vs, ws, u, v, w,
+               dtal);
   return cudaGetLastError();
 }
 
@@ -3601,31 +3598,25 @@ cudaError_t launch_gather3(const uint32_t* dst, const uint32_t* src, int64_t n, 
 }
 
 template <typename TR>
-cudaError_t launch_calmas(bool lsm, const BlkLev* bl, RowTab rt, const double* h3, const double* u, const double* v,
+cudaError_t launch_calmas(bool lsm, const BlkLev* bl, CellTab ct, const double* h3, const double* u, const double* v,
                           const double* w, double dt, double* bout, TR* rhs_out, double* partials, int* nparts,
                           cudaStream_t st) {
   *nparts = 0;
-  if (rt.nrows <= 0) return cudaSuccess;
-  const int g = defect_grid(rt.nrows);
-  if (lsm) pdl_launch(k_calmas<true, TR>, g, 256, 0, st, bl, rt.start, rt.nb, rt.nrows, h3, u, v, w, dt, bout, rhs_out, partials);
-  else pdl_launch(k_calmas<false, TR>, g, 256, 0, st, bl, rt.start, rt.nb, rt.nrows, h3, u, v, w, dt, bout, rhs_out, partials);
+  if (ct.ncta <= 0) return cudaSuccess;
+  const int g = std::min(ct.ncta, kCellCtas);
+  if (lsm)
+    pdl_launch(k_calmas<true, TR>, g, 256, 0, st, bl, ct.cta_start, ct.nb, ct.ncta, h3, u, v, w, dt, bout, rhs_out,
+               partials);
+  else
+    pdl_launch(k_calmas<false, TR>, g, 256, 0, st, bl, ct.cta_start, ct.nb, ct.ncta, h3, u, v, w, dt, bout, rhs_out,
+               partials);
   *nparts = g;
   return cudaGetLastError();
 }
-template cudaError_t launch_calmas<double>(bool, const BlkLev*, RowTab, const double*, const double*, const double*,
+template cudaError_t launch_calmas<double>(bool, const BlkLev*, CellTab, const double*, const double*, const double*,
                                            const double*, double, double*, double*, double*, int*, cudaStream_t);
-template cudaError_t launch_calmas<float>(bool, const BlkLev*, RowTab, const double*, const double*, const double*,
+template cudaError_t launch_calmas<float>(bool, const BlkLev*, CellTab, const double*, const double*, const double*,
                                           const double*, double, double*, float*, double*, int*, cudaStream_t);
-
-template <typename TE>
-cudaError_t launch_padd(const BlkLev* bl, RowTab rt, double* p, const TE* e, cudaStream_t st) {
-  if (rt.nrows <= 0) return cudaSuccess;
-  pdl_launch(k_padd<TE>, defect_grid(rt.nrows), 256, 0, st, bl, rt.start, rt.nb, rt.nrows, p, e);
-  return cudaGetLastError();
-}
-template cudaError_t launch_padd<double>(const BlkLev*, RowTab, double*, const double*, cudaStream_t);
-template cudaError_t launch_padd<float>(const BlkLev*, RowTab, double*, const float*, cudaStream_t);
-
 
 cudaError_t launch_dens_restrict(const BlkLev* fine, const BlkLev* coarse, CellTab ct, const double* df, double* dc,
                                  cudaStream_t st) {

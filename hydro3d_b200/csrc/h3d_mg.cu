@@ -173,6 +173,8 @@ struct h3d_mg {
   int64_t kernels = 0;
   std::map<std::vector<int>, CachedGraph> graphs;
   bool capturing = false;
+  bool solving = false;     // inside a solve (its FP64 sweeps fill the live ghosts only)
+  bool unclean = true;      // some level array may hold a NaN or infinity, which a ghost left unfilled would keep
   bool debug_sync = false;  // H3D_DEBUG_SYNC=1: synchronize and check after every launch
   std::vector<double> history;
   // whole host block arrays staged on the device (0: pressure, 1: rhs) for
@@ -180,8 +182,6 @@ struct h3d_mg {
   double* stage[2] = {nullptr, nullptr};
   std::vector<size_t> stage_off;
   // fused coarse tail: levels tail_g..L in one single-CTA launch (tail_g = 0: none)
-  bool solving = false;     // inside a solve (its FP64 sweeps fill the live ghosts only)
-  bool unclean = true;      // some level array may hold a NaN or infinity, which a ghost left unfilled would keep
   int tail_g = 0;
   bool lmr = false;  // blocks of different refinement ratio or level count (LMR = 2)
   TailLevel* d_tail_lv = nullptr;
@@ -1151,6 +1151,29 @@ int run_iteration(h3d_mg* h, int inner, double* prof_ms, int64_t* prof_n, double
   return accumulate_events(h, it->second.events, it->second.bytes, prof_ms, prof_n, prof_bytes);
 }
 
+// A solve leaves the ghosts of physical walls unfilled between its sweeps (live
+// fills): they must be finite.  Clears the level iterates after calls that may
+// have put anything there; a solve that ends with a finite residual leaves them
+// finite.
+struct SolveScope {
+  h3d_mg* h;
+  explicit SolveScope(h3d_mg* h_) : h(h_) { h->solving = true; }
+  ~SolveScope() { h->solving = false; }
+  int begin() {
+    if (!h->unclean) return H3D_OK;
+    for (int g = 1; g <= h->L; ++g) {
+      Level& V = h->lev[g];
+      for (int q = 0; q < 2; ++q) {
+        const size_t n = (size_t)V.geom.n_elems;
+        if (V.phi64[q]) CU(cudaMemsetAsync(V.phi64[q], 0, n * sizeof(double), h->st));
+        if (V.phi32[q]) CU(cudaMemsetAsync(V.phi32[q], 0, n * sizeof(float), h->st));
+      }
+    }
+    h->unclean = false;
+    return H3D_OK;
+  }
+};
+
 bool is_all_neumann(const h3d_mg* h) {
   for (const auto& d : h->blocks)
     for (int f = 0; f < 6; ++f)
@@ -1191,29 +1214,6 @@ int check_block_host_dims(h3d_mg* h, const h3d_block_desc& d) {
 // it is only used in calls that staged the same host array in (the planes'
 // other cells then round-trip unchanged).
 int ensure_stage(h3d_mg* h, int f) {
-// A solve leaves the ghosts of physical walls unfilled between its sweeps (live
-// fills): they must be finite.  Clears the level iterates after calls that may
-// have put anything there; a solve that ends with a finite residual leaves them
-// finite.
-struct SolveScope {
-  h3d_mg* h;
-  explicit SolveScope(h3d_mg* h_) : h(h_) { h->solving = true; }
-  ~SolveScope() { h->solving = false; }
-  int begin() {
-    if (!h->unclean) return H3D_OK;
-    for (int g = 1; g <= h->L; ++g) {
-      Level& V = h->lev[g];
-      for (int q = 0; q < 2; ++q) {
-        const size_t n = (size_t)V.geom.n_elems;
-        if (V.phi64[q]) CU(cudaMemsetAsync(V.phi64[q], 0, n * sizeof(double), h->st));
-        if (V.phi32[q]) CU(cudaMemsetAsync(V.phi32[q], 0, n * sizeof(float), h->st));
-      }
-    }
-    h->unclean = false;
-    return H3D_OK;
-  }
-};
-
   if (h->stage[f]) return H3D_OK;
   size_t n = 0;
   h->stage_off.clear();
@@ -2603,6 +2603,8 @@ int h3d_mg_create(h3d_mg** out, const h3d_mg_desc* desc) {
   for (int g = 1; g <= h->L; ++g) {
     Level& V = h->lev[g];
     V.geom = make_level_geom(h->blocks, g, true);
+    V.f32 = f32_level(h, g);
+    V.var = h->var;
     if ((rc = dalloc(h, &V.d_bl, V.geom.bl.size())) != H3D_OK) return bail(rc);
     if (cudaMemcpy(V.d_bl, V.geom.bl.data(), V.geom.bl.size() * sizeof(BlkLev), cudaMemcpyHostToDevice) != cudaSuccess)
       return bail(fail(h, H3D_ERR_CUDA, "copy level geometry"));
@@ -2722,8 +2724,6 @@ int h3d_mg_create(h3d_mg** out, const h3d_mg_desc* desc) {
           st.push_back((int)ld.size());
         }
         if ((rc = upload_halo(h, V.lfill, ld, ls)) != H3D_OK) return bail(rc);
-    V.f32 = f32_level(h, g);
-    V.var = h->var;
         if ((rc = dalloc(h, &V.d_lfstart, st.size())) != H3D_OK) return bail(rc);
         if (cudaMemcpy(V.d_lfstart, st.data(), st.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
           return bail(fail(h, H3D_ERR_CUDA, "block-local fill table"));
@@ -2870,6 +2870,8 @@ int h3d_mg_create(h3d_mg** out, const h3d_mg_desc* desc) {
     return bail(fail(h, H3D_ERR_OOM, "pinned result buffer"));
   std::vector<double> h3;
   for (const auto& d : h->blocks) { h3.push_back(d.h[0]); h3.push_back(d.h[1]); h3.push_back(d.h[2]); }
+  for (const auto& d : h->blocks)
+    for (double v : d.h) h3.push_back(1.0 / v);
   if ((rc = dalloc(h, &h->d_h3, h3.size())) != H3D_OK) return bail(rc);
   if ((rc = dalloc(h, &h->d_err, 1)) != H3D_OK) return bail(rc);
   if (cudaMemcpy(h->d_h3, h3.data(), h3.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess)
@@ -2894,6 +2896,7 @@ int h3d_mg_set_density(h3d_mg* h, int32_t ib, const double* dens) {
 int h3d_mg_coeff(h3d_mg* h) {
   if (!h) return H3D_ERR_ARG;
   CU(cudaSetDevice(h->device));
+  h->unclean = true;
   if (h->var) {
     for (int g = 1; g <= h->L; ++g) {
       Level& V = h->lev[g];
@@ -3006,6 +3009,8 @@ int h3d_mg_solve_resident(h3d_mg* h, const h3d_solve_opts* opts, h3d_solve_info*
     ~PerBlock() { h->per_block = false; }
   } pb_guard{h};
   h->per_block = opts->stop_rule == 2 && nb > 1;
+  SolveScope scope(h);
+  TRY(scope.begin());
   h3d_solve_info I{};
   const int maxcy = opts->maxcy > 0 ? opts->maxcy : h->desc.maxcy;
   const int inner = h->mixed ? h->desc.inner_cycles : 1;
@@ -3015,9 +3020,6 @@ int h3d_mg_solve_resident(h3d_mg* h, const h3d_solve_opts* opts, h3d_solve_info*
   CU(cudaEventCreate(&t1));
   int64_t k0 = h->kernels;
   CU(cudaEventRecord(t0, h->st));
-  h->unclean = true;
-  for (const auto& d : h->blocks)
-    for (double v : d.h) h3.push_back(1.0 / v);
   Level& V = h->lev[1];
   // pressure halo (exchange(4) + pbound, newsolv_mg.for:51-52)
   TRY(pressure_halo(h));
@@ -3128,8 +3130,6 @@ int h3d_mg_history(h3d_mg* h, double* out, int32_t cap, int32_t* n) {
   int k = (int)std::min<size_t>(h->history.size(), (size_t)std::max(cap, 0));
   if (out)
     for (int q = 0; q < k; ++q) out[q] = h->history[q];
-  SolveScope scope(h);
-  TRY(scope.begin());
   *n = (int)h->history.size();
   return H3D_OK;
 }
@@ -3439,6 +3439,8 @@ int h3d_mg_project_resident(h3d_mg* h, double dt, double alfapr, const h3d_solve
   set_projection_scalars(h, dt, alfapr);
   h->proj = true;
   h->per_block = false;
+  SolveScope scope(h);
+  TRY(scope.begin());
   h3d_solve_info I{};
   const int maxcy = opts->maxcy > 0 ? opts->maxcy : h->desc.maxcy;
   const int inner = h->mixed ? h->desc.inner_cycles : 1;
@@ -3549,6 +3551,7 @@ extern "C" {
 int h3d_mg_put_level(h3d_mg* h, int32_t g, int32_t field, int32_t ib, const double* a) {
   if (!level_ok(h, g) || !a || ib < 0 || ib >= (int)h->blocks.size() || field < 0 || field > 1) return H3D_ERR_ARG;
   CU(cudaSetDevice(h->device));
+  h->unclean = true;
   CU(cudaStreamSynchronize(h->st));
   Level& V = h->lev[g];
   const BlkLev& B = V.geom.bl[ib];
@@ -3558,8 +3561,6 @@ int h3d_mg_put_level(h3d_mg* h, int32_t g, int32_t field, int32_t ib, const doub
     std::memcpy(buf.data(), a, nb * 8);
   } else {
     for (int z = 1; z <= B.nz; ++z)
-  SolveScope scope(h);
-  TRY(scope.begin());
       for (int y = 1; y <= B.ny; ++y)
         for (int x = 1; x <= B.nx; ++x)
           buf[((size_t)z * (B.ny + 2) + y) * (B.nx + 2) + x] = a[((size_t)(z - 1) * B.ny + (y - 1)) * B.nx + (x - 1)];
@@ -3609,6 +3610,7 @@ int h3d_mg_get_level(h3d_mg* h, int32_t g, int32_t field, int32_t ib, double* a)
 int h3d_mg_mgrelax(h3d_mg* h, int32_t g, int32_t it) {
   if (!level_ok(h, g) || it < 0) return H3D_ERR_ARG;
   CU(cudaSetDevice(h->device));
+  h->unclean = true;
   TRY(ensure_coeffs(h));
   Exec ex{h};
   TRY(ex.relax(g, it));
@@ -3619,6 +3621,7 @@ int h3d_mg_mgrelax(h3d_mg* h, int32_t g, int32_t it) {
 int h3d_mg_mgrestr(h3d_mg* h, int32_t g) {
   if (!level_ok(h, g) || g < 2) return H3D_ERR_ARG;
   CU(cudaSetDevice(h->device));
+  h->unclean = true;
   TRY(ensure_coeffs(h));
   Exec ex{h};
   TRY(ex.restrict_to(g));
@@ -3633,6 +3636,7 @@ int h3d_mg_mgrestr(h3d_mg* h, int32_t g) {
 int h3d_mg_mgcorr(h3d_mg* h, int32_t g) {
   if (!level_ok(h, g) || g >= h->L) return H3D_ERR_ARG;
   CU(cudaSetDevice(h->device));
+  h->unclean = true;
   Exec ex{h};
   TRY(ex.correct(g));
   CU(cudaStreamSynchronize(h->st));
@@ -3642,6 +3646,7 @@ int h3d_mg_mgcorr(h3d_mg* h, int32_t g) {
 // Applies a halo table of `kind` out of place on the current iterate of level g.
 static int apply_table_hook(h3d_mg* h, int g, int kind) {
   CU(cudaSetDevice(h->device));
+  h->unclean = true;
   Level& V = h->lev[g];
   if (V.expr && kind == kHaloExchange) {  // exchangepp between blocks of different rdv
     if (!V.xe.built) TRY(upload_xfill(h, g, kHaloExchange, V.xe));
@@ -3670,7 +3675,6 @@ static int apply_table_hook(h3d_mg* h, int g, int kind) {
     std::vector<uint32_t> d, s;
     std::string err;
     int rc = build_halo_table(h->blocks, g, kind, true, d, s, &err);
-  h->unclean = true;
     if (rc != H3D_OK) return fail(h, rc, err);
     TRY(upload_halo(h, *H, d, s));
     H->built = true;
@@ -3709,6 +3713,7 @@ int h3d_mg_exchangepp(h3d_mg* h, int32_t g) {
 int h3d_mg_vcycle(h3d_mg* h) {
   if (!h) return H3D_ERR_ARG;
   CU(cudaSetDevice(h->device));
+  h->unclean = true;
   TRY(ensure_coeffs(h));
   Exec ex{h};
   TRY(ex.vcycle());
@@ -3719,6 +3724,7 @@ int h3d_mg_vcycle(h3d_mg* h) {
 int h3d_mg_mgkcyc(h3d_mg* h, double* const* pp, const double* const* su) {
   if (!h || !pp || !su) return H3D_ERR_ARG;
   CU(cudaSetDevice(h->device));
+  h->unclean = true;
   TRY(ensure_coeffs(h));
   Level& V = h->lev[1];
   // pp (incl. one ghost layer) -> level-1 iterate, su -> level-1 rhs (mgsolver.for:239-266)
@@ -3729,7 +3735,6 @@ int h3d_mg_mgkcyc(h3d_mg* h, double* const* pp, const double* const* su) {
     } else {
       TRY(stage_in(h, 0, ib, pp[ib], V.phi64[V.cur64], true));
       TRY(stage_in(h, 1, ib, su[ib], V.rhs64, false));
-  h->unclean = true;
     }
   }
   if (h->mixed) {
@@ -3740,7 +3745,6 @@ int h3d_mg_mgkcyc(h3d_mg* h, double* const* pp, const double* const* su) {
     V.zero64 = false;
   }
   Exec ex{h};
-  h->unclean = true;
   TRY(ex.vcycle());
   if (h->mixed) CU(launch_convert_f2d(V.phi32[V.cur32], h->p64[1 - h->pc], V.geom.n_elems, h->st));
   for (int ib = 0; ib < (int)h->blocks.size(); ++ib)
@@ -3755,7 +3759,6 @@ int h3d_mg_sync(h3d_mg* h) {
   CU(cudaStreamSynchronize(h->st));
   return H3D_OK;
 }
-  h->unclean = true;
 
 int h3d_mg_set_wait_limit(h3d_mg* h, int64_t clocks) {
   if (!h) return H3D_ERR_ARG;
@@ -3765,7 +3768,6 @@ int h3d_mg_set_wait_limit(h3d_mg* h, int64_t clocks) {
   return H3D_OK;
 }
 
-  h->unclean = true;
 int h3d_mg_wait_probe(h3d_mg* h) {
   if (!h) return H3D_ERR_ARG;
   CU(cudaSetDevice(h->device));
@@ -3832,6 +3834,4 @@ int h3d_mg_smoother_bytes(h3d_mg* h, double* bytes) {
   return H3D_OK;
 }
 
-  h->unclean = true;
 }  // extern "C"
-  h->unclean = true;
