@@ -144,12 +144,6 @@ __device__ __forceinline__ void relax_resident(const BlkLev& B, T* phi, T* diag,
   }
 }
 
-// Sweeps of a visit from which relax_resident pays in the fused coarse end: its
-// code and set-up, cold in every launch, cost about 10 us there (2 to 3 sweeps a level: 39.7
-// us with the tables, 52 us resident; 32 sweeps of 512 cells: a solve of
-// eight such launches 1.18 against 0.98 ms).
-constexpr int kResidentSweeps = 8;
-
 // Pairs a thread needs for a block (relax_resident), or 0: more than four.
 __device__ __forceinline__ int resident_pairs(const BlkLev& B) {
   const int np = (B.nx + 1) / 2 * B.ny * B.nz, k = (np + (int)blockDim.x - 1) / (int)blockDim.x;
@@ -548,16 +542,121 @@ __global__ void __launch_bounds__(1024) k_coarse_tail(const TailLevel* __restric
   }
 }
 
+// ---------------------------------------------------------------------------
 // The coarse end of a V-cycle as one thread-block cluster: CTA b holds block
 // b of every tail level in its shared memory (compact layout, every block of
 // a level the same size) and runs the same op program as k_coarse_tail on
 // it.  Restrictions, corrections and conversions only touch the CTA's own
 // block; after the colours of a sweep the cluster synchronises, every CTA
-// gathers its ghost cells from the other CTAs' shared memory (fdst: own
-// compact index; fsrc: source rank << 24 | its compact index), and the
-// cluster synchronises again before any interior changes.
+// gathers its ghost cells from the other CTAs' shared memory (fill pairs: own
+// compact index; source rank << 24 | its compact index), and the cluster
+// synchronises again before any interior changes.
+//
+// Latency bounds it: a program of short ops on a few thousand cells, every
+// instruction fetched cold.  So the code is kept small and a cell cheap: cells come
+// from 32-bit tables (x, y, z, and the block faces the cell lies on), red before
+// black, and right-hand sides are stored in the tables' order; the diagonal and its
+// reciprocal come from a table by wall faces, so that an update divides by
+// multiply-adds (div_known); all tables are staged by one flat copy while the predecessor
+// finishes; a sweep fills the ghosts that the next one reads, the last one all of
+// them.  With 64-bit tables decoded through the block records and 512 threads a
+// launch took 67 us for 16 blocks of 16^3 .. 2^3 cells and 46 us for one of 16^3 and 8^3
+// cells in FP64; 61 and 32 us here.
+// Sweeps of a visit from which its cells go to registers (the 32 of a converged
+// coarsest level; two or three sweeps do not repay the extra code).
+constexpr int kResidentSweeps = 8;
+struct Cell3 {
+  int x, y, z, w;  // w: block faces (bit f)
+};
+__device__ __forceinline__ Cell3 cell3(uint32_t e) {
+  return Cell3{(int)(e & 0xff), (int)(e >> 8 & 0xff), (int)(e >> 16 & 0xff), (int)(e >> 24)};
+}
+__device__ __forceinline__ int compact_at(const BlkLev& B, int x, int y, int z) {
+  return (z * (B.ny + 2) + y) * (B.nx + 2) + x;
+}
+// Place of a cell's right-hand side: the tables list cells in natural order,
+// red ones first, and every two neighbours in that order are one of each.
+__device__ __forceinline__ int rhs_at(const BlkLev& B, int nred, int x, int y, int z) {
+  return ((x + y + z) & 1 ? 0 : nred) + ((((z - 1) * B.ny + (y - 1)) * B.nx + (x - 1)) >> 1);
+}
+
+// One colour (0: red) of a sweep.  The ghosts of physical walls are zero, so
+// all cells use the interior coefficients.
+template <typename T>
+__device__ void cluster_colour(const BlkLev& B, const TailLevel& L, T* phi, const T* rhs, const T* diag, int colour) {
+  const int sx = B.nx + 2, sxy = sx * (B.ny + 2), k1 = colour ? L.nint : L.nred;
+  const T ax = (T)B.ax, ay = (T)B.ay, az = (T)B.az;
+  for (int k = (colour ? L.nred : 0) + threadIdx.x; k < k1; k += blockDim.x) {
+    const Cell3 c = cell3(L.cells32[k]);
+    T* q = phi + compact_at(B, c.x, c.y, c.z);
+    const int w = c.w & B.phys;
+    *q = cell_update(q, sx, sxy, ax, ay, az, rhs[k], diag[2 * w], diag[2 * w + 1], L.om);
+  }
+}
+
+// mgrestr into a tail level: the residual sum over the eight children in
+// k_restrict's order; one thread a coarse cell.
+template <typename T>
+__device__ void cluster_restrict(const BlkLev& F, const TailLevel& Fl, const TailLevel& Cl, const T* P, const T* rhs,
+                                 T* rhs_c, int zero_fine) {
+  const int sx = F.nx + 2, sxy = sx * (F.ny + 2);
+  for (int k = threadIdx.x; k < Cl.nint; k += blockDim.x) {
+    const Cell3 cc = cell3(Cl.cells32[k]);
+    T sum = T(0);
+#pragma unroll 1
+    for (int d = 0; d < 8; ++d) {
+      const int x = 2 * cc.x - 1 + (d & 1), y = 2 * cc.y - 1 + (d >> 1 & 1), z = 2 * cc.z - 1 + (d >> 2);
+      T r = rhs[rhs_at(F, Fl.nred, x, y, z)];
+      if (!zero_fine) {
+        const T* q = P + compact_at(F, x, y, z);
+        const Coef<T> cf = cell_coef<T, false>(F, x, y, z, 0, nullptr, nullptr, nullptr);
+        r = r - (cf.aw * q[-1] + cf.ae * q[1] + cf.as * q[-sx] + cf.an * q[sx] + cf.ab * q[-sxy] + cf.at * q[sxy] +
+                 coef_ap(cf) * q[0]);
+      }
+      sum = d ? sum + r : r;
+    }
+    rhs_c[k] = T(0.125) * sum;
+  }
+  __syncthreads();
+}
+
+// mgcorr + mgbound into a tail level in place (see tail_prolong).
+template <typename T>
+__device__ void cluster_prolong(const BlkLev& F, const BlkLev& C, const TailLevel& L, const T* phi_c, T* phi,
+                                T* scratch, int zero_old) {
+  for (int k = threadIdx.x; k < L.nghost; k += blockDim.x) {
+    const Cell3 c = cell3(L.cells32[L.nint + k]);
+    scratch[k] = tail_prolong_value(F, C, phi_c, phi, c.x, c.y, c.z, zero_old);
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < L.nint; k += blockDim.x) {
+    const Cell3 c = cell3(L.cells32[k]);
+    phi[compact_at(F, c.x, c.y, c.z)] = tail_prolong_value(F, C, phi_c, phi, c.x, c.y, c.z, zero_old);
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < L.nghost; k += blockDim.x) {
+    const Cell3 c = cell3(L.cells32[L.nint + k]);
+    phi[compact_at(F, c.x, c.y, c.z)] = scratch[k];
+  }
+  __syncthreads();
+}
+
+// A tail level back to global memory: iterate (interior and ghost cells) and rhs.
+template <typename T>
+__device__ void cluster_store(const BlkLev& G, const BlkLev& B, const TailLevel& L, const T* phi, const T* rhs,
+                              T* __restrict__ gphi, T* __restrict__ grhs) {
+  for (int k = threadIdx.x; k < L.nint + L.nghost; k += blockDim.x) {
+    const Cell3 c = cell3(L.cells32[k]);
+    const long long gi = global_index(G, c.x, c.y, c.z);
+    gphi[gi] = phi[compact_at(B, c.x, c.y, c.z)];
+    if (k < L.nint) grhs[gi] = rhs[k];
+  }
+  __syncthreads();
+}
+
 __global__ void __launch_bounds__(kClusterTailThreads) k_coarse_cluster(const TailLevel* __restrict__ lvg,
-                                                                        const TailOp* __restrict__ opsg, int nops,
+                                                                        const TailOp* __restrict__ opsg,
+                                                                        const uint4* __restrict__ tables, int nops,
                                                                         int nlev, unsigned curmask) {
   pdl_trigger();
   namespace cg = cooperative_groups;
@@ -566,115 +665,147 @@ __global__ void __launch_bounds__(kClusterTailThreads) k_coarse_cluster(const Ta
   __shared__ TailLevel lv[kTailMaxLevels];
   __shared__ BlkLev gtab[kTailMaxLevels], ctab[kTailMaxLevels];  // this block per level: global / compact layout
   __shared__ TailOp ops[kClusterTailMaxOps];
-  __shared__ double diag64[128];
+  __shared__ double diag64[128];  // diagonal and reciprocal by wall faces
   extern __shared__ unsigned char smem_raw[];
   unsigned char* arena = smem_base128(smem_raw);
-  // the program, the level records and this block's tables are setup data:
-  // stage them in shared memory (cell and ghost tables, this block's fill
-  // entries) while the predecessor finishes
-  for (int q = threadIdx.x; q < nops; q += blockDim.x) ops[q] = opsg[q];
-  if (threadIdx.x < nlev) lv[threadIdx.x] = lvg[threadIdx.x];
-  __syncthreads();
-  for (int l = 0; l < nlev; ++l) {
-    const TailLevel& G = lvg[l];
-    unsigned long long* cs = reinterpret_cast<unsigned long long*>(arena + lv[l].s_cells);
-    for (int k = threadIdx.x; k < G.nint + G.nghost; k += blockDim.x)
-      cs[k] = k < G.nint ? __ldg(G.cells + k) : __ldg(G.ghosts + (k - G.nint));
-    const int f0 = __ldg(G.fstart + b), f1 = __ldg(G.fstart + b + 1);
-    uint32_t* fd = reinterpret_cast<uint32_t*>(arena + lv[l].s_fill);
-    for (int k = threadIdx.x; k < f1 - f0; k += blockDim.x) {
-      fd[2 * k] = __ldg(G.fdst + f0 + k);
-      fd[2 * k + 1] = __ldg(G.fsrc + f0 + k);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      lv[l].cells = cs;
-      lv[l].ghosts = cs + G.nint;
-      lv[l].fdst = fd;
-      lv[l].nfill = f1 - f0;
-      lv[l].nlive = __ldg(G.flive + b);
+  // the program, the level records and this block's tables are setup data: staged
+  // while the predecessor finishes
+  {
+    const int tab0 = lvg[0].s_cells, words = lvg[0].tab_words;
+    uint4* dst = reinterpret_cast<uint4*>(arena + tab0);
+    for (int q = threadIdx.x; q < words; q += blockDim.x) dst[q] = __ldg(tables + (size_t)b * words + q);
+    for (int q = threadIdx.x; q < nops; q += blockDim.x) ops[q] = opsg[q];
+    if (threadIdx.x < nlev) {
+      TailLevel l = lvg[threadIdx.x];
+      l.nfill = __ldg(l.fstart + b + 1) - __ldg(l.fstart + b);
+      l.nlive = __ldg(l.flive + b);
+      l.cells32 = reinterpret_cast<const uint32_t*>(arena + l.s_cells);
+      l.fdst = reinterpret_cast<const uint32_t*>(arena + l.s_fill);
+      lv[threadIdx.x] = l;
+      const BlkLev G = l.gbl[b];
+      gtab[threadIdx.x] = G;
+      BlkLev c = G;
+      c.off = 0;
+      c.sx = G.nx + 2;
+      c.sxy = (long long)(G.nx + 2) * (G.ny + 2);
+      c.pad = 0;
+      ctab[threadIdx.x] = c;
     }
   }
   __syncthreads();
   pdl_wait();
-  auto compact = [](BlkLev B) {
-    B.off = 0;
-    B.sx = B.nx + 2;
-    B.sxy = (long long)(B.nx + 2) * (B.ny + 2);
-    B.pad = 0;
-    return B;
+  const bool alone = cl.num_blocks() == 1;
+  auto barrier = [&] {
+    if (alone) __syncthreads();
+    else cl.sync();
   };
-  if (threadIdx.x < nlev) {
-    const BlkLev G = lvg[threadIdx.x].gbl[b];
-    gtab[threadIdx.x] = G;
-    ctab[threadIdx.x] = compact(G);
-  }
-  __syncthreads();
+  // ghosts of the first n fill pairs from every block's interior
+  auto gather = [&](const TailLevel& F, auto* phi, int n) {
+    barrier();  // every block's cells are written
+    for (int q = threadIdx.x; q < n; q += blockDim.x) {  // (dst, src) pairs of this block
+      const uint32_t src = F.fdst[2 * q + 1];
+      phi[F.fdst[2 * q]] = cl.map_shared_rank(phi, (int)(src >> 24))[src & 0xffffffu];
+    }
+    barrier();  // every ghost gathered before any interior changes
+  };
   for (int o = 0; o < nops; ++o) {
     const TailOp op = ops[o];
     const TailLevel& F = lv[op.fine];
     const TailLevel& C = lv[op.coarse];
     // this block's tables at the op's levels (staged once; every op ends with
     // a barrier of the CTA or the cluster)
-    const BlkLev* gb = gtab + op.fine;
-    const BlkLev* fb = ctab + op.fine;
-    const BlkLev* cb = ctab + op.coarse;
+    const BlkLev& gb = gtab[op.fine];
+    const BlkLev& fb = ctab[op.fine];
+    const BlkLev& cb = ctab[op.coarse];
     auto at32 = [&](int off) { return reinterpret_cast<float*>(arena + off); };
     auto at64 = [&](int off) { return reinterpret_cast<double*>(arena + off); };
     switch (op.kind) {
-      case kTailLoadRhs:
-        if (op.f64) tail_load_rhs<double>(gb, fb, F, F.rhs64, at64(F.s_rhs64));
-        else tail_load_rhs<float>(gb, fb, F, F.rhs32, at32(F.s_rhs32));
+      case kTailLoadRhs: {
+        auto load = [&](const auto* __restrict__ g, auto* rhs) {
+#pragma unroll 4
+          for (int k = threadIdx.x; k < F.nint; k += blockDim.x) {
+            const Cell3 c = cell3(F.cells32[k]);
+            rhs[k] = g[global_index(gb, c.x, c.y, c.z)];
+          }
+        };
+        if (op.f64) load(F.rhs64, at64(F.s_rhs64));
+        else load(F.rhs32, at32(F.s_rhs32));
+        __syncthreads();
         break;
+      }
       case kTailRelax: {
         auto relax = [&](auto* phi, const auto* rhs) {
           using T = typename std::remove_pointer<decltype(phi)>::type;
+          T* diag = reinterpret_cast<T*>(diag64);
+          if (threadIdx.x < 64) {
+            Coef<T> c;
+            c.aw = threadIdx.x & 1 ? T(0) : (T)fb.ax;
+            c.ae = threadIdx.x & 2 ? T(0) : (T)fb.ax;
+            c.as = threadIdx.x & 4 ? T(0) : (T)fb.ay;
+            c.an = threadIdx.x & 8 ? T(0) : (T)fb.ay;
+            c.ab = threadIdx.x & 16 ? T(0) : (T)fb.az;
+            c.at = threadIdx.x & 32 ? T(0) : (T)fb.az;
+            diag[2 * threadIdx.x] = coef_ap(c);
+            diag[2 * threadIdx.x + 1] = T(1) / coef_ap(c);
+          }
           if (op.zero) {
             for (int q = threadIdx.x; q < F.npad; q += blockDim.x) phi[q] = T(0);
-            __syncthreads();
+          } else {
+            for (int q = threadIdx.x; q < F.nghost; q += blockDim.x) {
+              const Cell3 c = cell3(F.cells32[F.nint + q]);
+              if (c.w & fb.phys) phi[compact_at(fb, c.x, c.y, c.z)] = T(0);
+            }
           }
-          const int ncol = F.rb_global ? 2 : 1;  // 2: a fill after each colour (order across blocks)
-          const bool alone = F.nb == 1;
-          auto barrier = [&] {
-            if (alone) __syncthreads();
-            else cl.sync();
-          };
-          // ghosts from every block's interior: all of them after the last sweep, before
-          // that the ones that a sweep reads
-          auto fill = [&](bool last) {
-            if (!last && !F.any_live) {
-              __syncthreads();
-              return;
-            }
-            barrier();  // every block's sweep done
-            const int n = last ? F.nfill : F.nlive;
-            for (int q = threadIdx.x; q < n; q += blockDim.x) {  // (dst, src) pairs of this block
-              const uint32_t dsti = F.fdst[2 * q], src = F.fdst[2 * q + 1];
-              const T* remote = cl.map_shared_rank(phi, (int)(src >> 24));
-              phi[dsti] = remote[src & 0xffffffu];
-            }
-            barrier();  // every ghost gathered before any interior changes
-          };
+          __syncthreads();
           if constexpr (sizeof(T) == 8) {
-            // many sweeps (the converged coarsest level): cells resident in registers
-            const int k = op.sweeps >= kResidentSweeps ? resident_pairs(*fb) : 0;
-            if (k) {
-              if (!op.zero)
-                for (int q = threadIdx.x; q < F.nghost; q += blockDim.x) {
-                  const CellRef c = cell_ref(F.ghosts[q]);
-                  if (wall_ghost(*fb, c.x, c.y, c.z)) phi[c.i] = T(0);
+            // many sweeps (the converged coarsest level): one red and one black cell a
+            // thread, kept in registers; a block alone only has the warps with cells meet
+            if (op.sweeps >= kResidentSweeps && F.nred <= (int)blockDim.x) {
+              const int na = alone ? (F.nred + 31) / 32 * 32 : (int)blockDim.x;
+              if ((int)threadIdx.x < na) {
+                auto meet = [&] { asm volatile("bar.sync 1, %0;\n" ::"r"(na) : "memory"); };
+                const int sx = fb.nx + 2, sxy = sx * (fb.ny + 2);
+                int at[2];
+                T r[2], ap[2], inv[2];
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                  const int k = threadIdx.x + (c ? F.nred : 0);
+                  const bool in = (int)threadIdx.x < F.nred && k < F.nint;
+                  const Cell3 q = cell3(F.cells32[in ? k : 0]);
+                  at[c] = in ? compact_at(fb, q.x, q.y, q.z) : -1;
+                  r[c] = in ? rhs[k] : T(0);
+                  ap[c] = diag[2 * (q.w & fb.phys)];
+                  inv[c] = diag[2 * (q.w & fb.phys) + 1];
                 }
-              auto rhs_at = [&](int x, int y, int z) { return rhs[rhs_index(*fb, x, y, z)]; };
-              if (k == 1) relax_resident<T, 1>(*fb, phi, diag64, rhs_at, op.sweeps, F.om, ncol, fill);
-              else if (k == 2) relax_resident<T, 2>(*fb, phi, diag64, rhs_at, op.sweeps, F.om, ncol, fill);
-              else relax_resident<T, 4>(*fb, phi, diag64, rhs_at, op.sweeps, F.om, ncol, fill);
+                for (int it = 0; it < op.sweeps; ++it)
+#pragma unroll
+                  for (int c = 0; c < 2; ++c) {
+                    if (at[c] >= 0)
+                      phi[at[c]] = cell_update(phi + at[c], sx, sxy, fb.ax, fb.ay, fb.az, r[c], ap[c], inv[c], 1.f);
+                    const bool last = c && it + 1 == op.sweeps;
+                    const int n = last ? F.nfill : F.any_live && (c || F.rb_global) ? F.nlive : -1;
+                    if (!alone && n >= 0) {
+                      gather(F, phi, n);
+                    } else {
+                      meet();
+                      for (int q = threadIdx.x; q < n; q += na) phi[F.fdst[2 * q]] = phi[F.fdst[2 * q + 1] & 0xffffffu];
+                      if (n > 0) meet();
+                    }
+                  }
+              }
+              __syncthreads();
               return;
             }
           }
           for (int it = 0; it < op.sweeps; ++it)
-            for (int pass = 0; pass < ncol; ++pass) {
-              tail_colours<T>(fb, F, phi, rhs, ncol == 2 ? pass : -1);
-              fill(it + 1 == op.sweeps && pass + 1 == ncol);
+            for (int colour = 0; colour < 2; ++colour) {
+              cluster_colour<T>(fb, F, phi, rhs, diag, colour);
+              const bool last = colour && it + 1 == op.sweeps;
+              // a fill after each colour: the order across block faces; else after the black
+              // cells; all ghosts after the last, before that the ones a sweep reads
+              if (last) gather(F, phi, F.nfill);
+              else if (F.any_live && (colour || F.rb_global)) gather(F, phi, F.nlive);
+              else __syncthreads();
             }
         };
         if (op.f64) relax(at64(F.s_phi64), (const double*)at64(F.s_rhs64));
@@ -687,12 +818,13 @@ __global__ void __launch_bounds__(kClusterTailThreads) k_coarse_cluster(const Ta
         if (op.zero) {
           for (int q = threadIdx.x; q < F.npad; q += blockDim.x) phi[q] = 0.0;
         }
-        cl.sync();  // every block's rhs is complete
+        barrier();  // every block's rhs is complete
         const int nper = F.nint, n = F.dense_n;
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-        const BlkLev& B = fb[0];
         for (int i = warp; i < nper; i += nwarp) {  // a warp per row of this block; lanes split the columns
-          const double* Pr = F.dense + (long long)(b * nper + i) * n;
+          const Cell3 c = cell3(F.cells32[i]);
+          const int row = ((c.z - 1) * fb.ny + (c.y - 1)) * fb.nx + (c.x - 1);
+          const double* Pr = F.dense + (long long)(b * nper + row) * n;
           double s = 0.0;
           for (int j = lane; j < n; j += 32) {
             const double* r = cl.map_shared_rank(rhs, j / nper);
@@ -700,27 +832,18 @@ __global__ void __launch_bounds__(kClusterTailThreads) k_coarse_cluster(const Ta
           }
 #pragma unroll
           for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-          if (lane == 0) {
-            const int x = i % B.nx + 1, y = (i / B.nx) % B.ny + 1, z = i / (B.nx * B.ny) + 1;
-            phi[(long long)z * B.sxy + (long long)y * B.sx + x] = s;
-          }
+          if (lane == 0) phi[compact_at(fb, c.x, c.y, c.z)] = s;
         }
-        cl.sync();  // every block's interior is written
-        for (int q = threadIdx.x; q < F.nfill; q += blockDim.x) {
-          const uint32_t dsti = F.fdst[2 * q], src = F.fdst[2 * q + 1];
-          const double* remote = cl.map_shared_rank(phi, (int)(src >> 24));
-          phi[dsti] = remote[src & 0xffffffu];
-        }
-        cl.sync();  // every ghost gathered before any interior changes
+        gather(F, phi, F.nfill);
         break;
       }
       case kTailRestrict:
-        if (op.f64) tail_restrict<double>(fb, cb, C, at64(F.s_phi64), at64(F.s_rhs64), at64(C.s_rhs64), op.zero);
-        else tail_restrict<float>(fb, cb, C, at32(F.s_phi32), at32(F.s_rhs32), at32(C.s_rhs32), op.zero);
+        if (op.f64) cluster_restrict<double>(fb, F, C, at64(F.s_phi64), at64(F.s_rhs64), at64(C.s_rhs64), op.zero);
+        else cluster_restrict<float>(fb, F, C, at32(F.s_phi32), at32(F.s_rhs32), at32(C.s_rhs32), op.zero);
         break;
       case kTailProlong:
-        if (op.f64) tail_prolong<double>(fb, cb, F, at64(C.s_phi64), at64(F.s_phi64), at64(op.sweeps), op.zero);
-        else tail_prolong<float>(fb, cb, F, at32(C.s_phi32), at32(F.s_phi32), at32(op.sweeps), op.zero);
+        if (op.f64) cluster_prolong<double>(fb, cb, F, at64(C.s_phi64), at64(F.s_phi64), at64(op.sweeps), op.zero);
+        else cluster_prolong<float>(fb, cb, F, at32(C.s_phi32), at32(F.s_phi32), at32(op.sweeps), op.zero);
         break;
       case kTailRhsF2D: {
         const float* x = at32(F.s_rhs32);
@@ -738,15 +861,15 @@ __global__ void __launch_bounds__(kClusterTailThreads) k_coarse_cluster(const Ta
       }
       case kTailStore: {
         const int c32 = (curmask >> (2 * op.fine)) & 1, c64 = (curmask >> (2 * op.fine + 1)) & 1;
-        if (F.s_phi32 >= 0) tail_store<float>(gb, fb, F, at32(F.s_phi32), at32(F.s_rhs32), F.phi32[c32], F.rhs32);
-        if (F.s_phi64 >= 0) tail_store<double>(gb, fb, F, at64(F.s_phi64), at64(F.s_rhs64), F.phi64[c64], F.rhs64);
+        if (F.s_phi32 >= 0) cluster_store<float>(gb, fb, F, at32(F.s_phi32), at32(F.s_rhs32), F.phi32[c32], F.rhs32);
+        if (F.s_phi64 >= 0) cluster_store<double>(gb, fb, F, at64(F.s_phi64), at64(F.s_rhs64), F.phi64[c64], F.rhs64);
         break;
       }
       default:
         break;
     }
   }
-  cl.sync();  // no CTA leaves while another may still read its shared memory
+  if (!alone) cl.sync();  // no CTA leaves while another may still read its shared memory
 }
 
 cudaError_t coarse_tail_attributes() {
@@ -792,14 +915,14 @@ int coarse_cluster_fits(int nb, int smem_bytes) {
 }
 
 cudaError_t launch_coarse_cluster(int nb, const TailLevel* lv, int nlev, const TailOp* ops, int nops,
-                                  unsigned curmask, int smem_bytes, cudaStream_t st) {
+                                  const uint4* tables, unsigned curmask, int smem_bytes, cudaStream_t st) {
   if (nops <= 0 || nops > kClusterTailMaxOps || nlev > kTailMaxLevels) return cudaErrorInvalidValue;
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at[2];
   cluster_config(nb, smem_bytes, st, &cfg, at);
-  cfg.numAttrs = 2;  // (its tables are staged while the predecessor finishes)
+  cfg.numAttrs = pdl_mode() == 0 ? 1 : 2;  // (its tables are staged while the predecessor finishes)
   g_prev_grid = nb;
-  return cudaLaunchKernelEx(&cfg, k_coarse_cluster, lv, ops, nops, nlev, curmask);
+  return cudaLaunchKernelEx(&cfg, k_coarse_cluster, lv, ops, tables, nops, nlev, curmask);
 }
 
 cudaError_t launch_coarse_tail(const TailLevel* lv, const TailOp* ops, int nops, unsigned curmask, int smem_bytes,

@@ -115,6 +115,8 @@ struct TailLevel {
   double* rhs64;
   int s_phi32, s_rhs32, s_phi64, s_rhs64;
   int s_cells, s_fill;  // cluster tail: arena offsets of the staged cell tables and this block's fill pairs
+  const uint32_t* cells32;  // cluster tail: cells (red, black, ghosts) as x | y << 8 | z << 16 | block faces << 24
+  int tab_words;        // cluster tail: 16-byte words of a block's tables (first level)
   const double* dense;  // coarsest level solved directly: its pseudo-inverse, dense_n x dense_n, row-major
   int dense_n;
   float om;             // over-relaxation of the level's FP32 sweeps (1: Gauss-Seidel)
@@ -150,12 +152,13 @@ cudaError_t launch_coarse_tail(const TailLevel* lv, const TailOp* ops, int nops,
                                cudaStream_t st);
 // The same program as one cluster of nb CTAs (nb <= 16), CTA b holding block b
 // of every tail level (all blocks of a level the same size).
-constexpr int kClusterTailThreads = 512;
+constexpr int kClusterTailThreads = 1024;
 constexpr int kClusterTailMaxBlocks = 16;
 int coarse_cluster_fits(int nb, int smem_bytes);  // clusters that can be resident at once (0: none)
 constexpr int kClusterTailMaxOps = 160;
+// tables: every block's staged tables, back to back.
 cudaError_t launch_coarse_cluster(int nb, const TailLevel* lv, int nlev, const TailOp* ops, int nops,
-                                  unsigned curmask, int smem_bytes, cudaStream_t st);
+                                  const uint4* tables, unsigned curmask, int smem_bytes, cudaStream_t st);
 
 // First red-black sweep from a zero iterate of an FP32 constant-coefficient
 // level (every block's nx a multiple of 4, at most 1024): tiles (block, y0 =

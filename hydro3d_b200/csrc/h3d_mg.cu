@@ -186,7 +186,8 @@ struct h3d_mg {
   bool lmr = false;  // blocks of different refinement ratio or level count (LMR = 2)
   TailLevel* d_tail_lv = nullptr;
   TailOp* d_tail_ops = nullptr;
-  unsigned long long* d_tail_cells = nullptr;  // cell tables of all tail levels
+  unsigned long long* d_tail_cells = nullptr;  // cell tables of all tail levels (single-CTA tail)
+  uint4* d_tail_tables = nullptr;              // cluster tail: every block's tables
   BlkLev* d_tail_cbl = nullptr;                // compact block tables of the tail levels
   int* d_tail_starts = nullptr;                // cluster tail: per-block fill ranges
   int tail_cluster = 0;                        // cluster tail: CTAs of the cluster (0: single-CTA tail)
@@ -843,8 +844,8 @@ struct Exec {
       mask |= (unsigned)(V.cur64 & 1) << (2 * (g - g0) + 1);
     }
     if (h->tail_cluster)
-      CU(launch_coarse_cluster(h->tail_cluster, h->d_tail_lv, h->tail_nlev, h->d_tail_ops, h->tail_nops, mask,
-                               h->tail_smem, h->st));
+      CU(launch_coarse_cluster(h->tail_cluster, h->d_tail_lv, h->tail_nlev, h->d_tail_ops, h->tail_nops,
+                               h->d_tail_tables, mask, h->tail_smem, h->st));
     else
       CU(launch_coarse_tail(h->d_tail_lv, h->d_tail_ops, h->tail_nops, mask, h->tail_smem, h->st));
     TRY(chk("coarse tail", g0));
@@ -2210,6 +2211,18 @@ int build_dense_coarse(h3d_mg* h) {
     for (int j = 0; j < n; ++j) csum[root(j)] += Inv[(size_t)i * n + j];
     for (int j = 0; j < n; ++j) P[(size_t)i * n + j] = Inv[(size_t)i * n + j] - csum[root(j)] / csize[root(j)];
   }
+  // columns in the order the cluster keeps a block's right-hand sides (red cells first)
+  const BlkLev& B0 = h->lev[h->L].geom.bl[0];
+  const int nper = B0.nx * B0.ny * B0.nz, nred = (nper + 1) / 2;
+  std::vector<double> row(n);
+  for (int i = 0; i < n; ++i) {
+    double* Pi = P.data() + (size_t)i * n;
+    for (int j = 0; j < n; ++j) {
+      const int m = j % nper, x = m % B0.nx, y = m / B0.nx % B0.ny, z = m / (B0.nx * B0.ny);
+      row[j - m + ((x + y + z) & 1 ? nred : 0) + m / 2] = Pi[j];
+    }
+    std::copy(row.begin(), row.end(), Pi);
+  }
   TRY(dalloc(h, &h->d_dense, P.size()));
   CU(cudaMemcpy(h->d_dense, P.data(), P.size() * 8, cudaMemcpyHostToDevice));
   h->dense_n = n;
@@ -2247,7 +2260,7 @@ int build_cluster_tail(h3d_mg* h) {
   auto al = [](int v) { return (v + 15) & ~15; };
   struct Lay { int npad, nint, s_phi32, s_rhs32, s_phi64, s_rhs64, s_cells, s_fill; };
   std::vector<Lay> lay;
-  int g0 = Lv + 1, bytes = 0, scratch_at = 0;
+  int g0 = Lv + 1, bytes = 0, scratch_at = 0, tab_bytes = 0;
   for (int g = Lv; g >= 2; --g) {
     const Level& V = h->lev[g];
     const BlkLev& B0 = V.geom.bl[0];
@@ -2275,7 +2288,7 @@ int build_cluster_tail(h3d_mg* h) {
       const BlkLev& Bq = h->lev[q].geom.bl[0];
       const int npad = (Bq.nx + 2) * (Bq.ny + 2) * (Bq.nz + 2);
       L2[q - g].s_cells = tab;
-      tab = al(tab + npad * 8);
+      tab = al(tab + npad * 4);
       L2[q - g].s_fill = tab;
       tab = al(tab + (npad - Bq.nx * Bq.ny * Bq.nz) * 8);  // (dst, src) pairs: a ghost is filled once at most
     }
@@ -2283,6 +2296,7 @@ int build_cluster_tail(h3d_mg* h) {
     if (need > kTailSmemBytes) break;
     g0 = g;
     lay = L2;
+    tab_bytes = tab - L2[0].s_cells;
     bytes = need;
     scratch_at = at;
   }
@@ -2293,34 +2307,33 @@ int build_cluster_tail(h3d_mg* h) {
   TRY(build_dense_coarse(h));
   emit_tail_ops(h, g0, scratch_at, ops, z32, z64, h->d_dense != nullptr);
   // per level: cell tables (block field 0) and per-block fill tables
-  std::vector<unsigned long long> cells;
-  std::vector<uint32_t> fills;
   std::vector<int> starts;
-  struct At { size_t cells, ghosts, fdst, fsrc, fstart, flive; int nred, nint, nghost, any_live; };
+  std::vector<unsigned char> tables((size_t)tab_bytes * nb, 0);
+  struct At { size_t fstart, flive; int nred, nint, nghost, any_live; };
   std::vector<At> at;
   for (int q = g0; q <= Lv; ++q) {
     const Level& V = h->lev[q];
     const BlkLev& B = V.geom.bl[0];
     const int sx = B.nx + 2, sxy = (B.nx + 2) * (B.ny + 2);
     At a{};
-    std::vector<unsigned long long> red, black, ghost;
+    std::vector<uint32_t> red, black, ghost;
     for (int z = 0; z <= B.nz + 1; ++z)
       for (int y = 0; y <= B.ny + 1; ++y)
         for (int x = 0; x <= B.nx + 1; ++x) {
-          const unsigned long long e = tail_cell((long long)z * sxy + (long long)y * sx + x, x, y, z, 0);
           const bool gh = x == 0 || y == 0 || z == 0 || x == B.nx + 1 || y == B.ny + 1 || z == B.nz + 1;
-          if (gh) ghost.push_back(e);
-          else if ((x + y + z) & 1) red.push_back(e);
-          else black.push_back(e);
+          // block faces: those an interior cell lies on, those a ghost lies beyond
+          const uint32_t w = gh ? (x == 0) | (x == B.nx + 1) << 1 | (y == 0) << 2 | (y == B.ny + 1) << 3 |
+                                      (z == 0) << 4 | (z == B.nz + 1) << 5
+                                : (x == 1) | (x == B.nx) << 1 | (y == 1) << 2 | (y == B.ny) << 3 | (z == 1) << 4 |
+                                      (z == B.nz) << 5;
+          const uint32_t e = (uint32_t)x | (uint32_t)y << 8 | (uint32_t)z << 16 | w << 24;
+          (gh ? ghost : (x + y + z) & 1 ? red : black).push_back(e);
         }
-    a.cells = cells.size();
     a.nred = (int)red.size();
     a.nint = (int)(red.size() + black.size());
-    cells.insert(cells.end(), red.begin(), red.end());
-    cells.insert(cells.end(), black.begin(), black.end());
-    a.ghosts = cells.size();
     a.nghost = (int)ghost.size();
-    cells.insert(cells.end(), ghost.begin(), ghost.end());
+    red.insert(red.end(), black.begin(), black.end());
+    red.insert(red.end(), ghost.begin(), ghost.end());
     std::vector<uint32_t> d, sidx;
     std::string err;
     int rc = build_halo_table(h->blocks, q, kHaloSweep, true, d, sidx, &err);
@@ -2347,8 +2360,7 @@ int build_cluster_tail(h3d_mg* h) {
       per[bd].push_back({cd, ((uint32_t)bs << 24) | cs});
     }
     a.fstart = starts.size();
-    a.fdst = fills.size();
-    std::vector<uint32_t> fd, fs;
+    const Lay& l = lay[q - g0];
     int acc = 0;
     std::vector<int> live;  // entries that a sweep reads come first
     for (int b = 0; b < nb; ++b) {
@@ -2360,28 +2372,25 @@ int build_cluster_tail(h3d_mg* h) {
       live.push_back((int)(mid - per[b].begin()));
       a.any_live |= live.back() > 0;
       starts.push_back(acc);
-      for (auto& pr : per[b]) { fd.push_back(pr.first); fs.push_back(pr.second); }
       acc += (int)per[b].size();
+      if ((int)per[b].size() > l.npad - l.nint) return H3D_OK;  // every block's fill list must fit its staged region
+      unsigned char* t = tables.data() + (size_t)tab_bytes * b;
+      std::memcpy(t + (l.s_cells - lay[0].s_cells), red.data(), red.size() * 4);
+      std::memcpy(t + (l.s_fill - lay[0].s_cells), per[b].data(), per[b].size() * 8);
     }
     starts.push_back(acc);
     a.flive = starts.size();
     starts.insert(starts.end(), live.begin(), live.end());
-    fills.insert(fills.end(), fd.begin(), fd.end());
-    a.fsrc = fills.size();
-    fills.insert(fills.end(), fs.begin(), fs.end());
     at.push_back(a);
   }
+  static_assert(sizeof(std::pair<uint32_t, uint32_t>) == 8, "fill pairs are staged as they are");
   int rc;
-  uint32_t* d_fills = nullptr;
   int* d_starts = nullptr;
-  if ((rc = dalloc(h, &h->d_tail_cells, cells.size())) != H3D_OK ||
-      (rc = dalloc(h, &d_fills, std::max<size_t>(fills.size(), 1))) != H3D_OK ||
+  if ((rc = dalloc(h, &h->d_tail_tables, tables.size() / 16)) != H3D_OK ||
       (rc = dalloc(h, &d_starts, starts.size())) != H3D_OK)
     return rc;
-  h->d_tail_fills = d_fills;
   h->d_tail_starts = d_starts;
-  if (cudaMemcpy(h->d_tail_cells, cells.data(), cells.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
-      (!fills.empty() && cudaMemcpy(d_fills, fills.data(), fills.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess) ||
+  if (cudaMemcpy(h->d_tail_tables, tables.data(), tables.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(d_starts, starts.data(), starts.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
     return fail(h, H3D_ERR_CUDA, "cluster tail tables");
   std::vector<TailLevel> lv;
@@ -2392,10 +2401,7 @@ int build_cluster_tail(h3d_mg* h) {
     TailLevel t{};
     t.gbl = V.d_bl;
     t.cbl = nullptr;
-    t.cells = h->d_tail_cells + a.cells;
-    t.ghosts = h->d_tail_cells + a.ghosts;
-    t.fdst = d_fills + a.fdst;
-    t.fsrc = d_fills + a.fsrc;
+    t.tab_words = tab_bytes / 16;
     t.fstart = d_starts + a.fstart;
     t.flive = d_starts + a.flive;
     t.any_live = a.any_live;
@@ -2422,14 +2428,6 @@ int build_cluster_tail(h3d_mg* h) {
     t.om = f32_level(h, q) ? h->omega : 1.f;
     t.rb_global = f32_level(h, q) && h->rb_global ? 1 : 0;
     lv.push_back(t);
-  }
-  // every block's fill list must fit its staged region
-  for (int q = g0; q <= Lv; ++q) {
-    const Lay& l = lay[q - g0];
-    const int cap = l.npad - l.nint;
-    const size_t f0 = at[q - g0].fstart;
-    for (int b = 0; b < nb; ++b)
-      if (starts[f0 + b + 1] - starts[f0 + b] > cap) return H3D_OK;
   }
   if ((int)ops.size() > kClusterTailMaxOps) return H3D_OK;
   if ((rc = dalloc(h, &h->d_tail_lv, lv.size())) != H3D_OK) return rc;
@@ -2480,6 +2478,7 @@ int h3d_mg_destroy(h3d_mg* h) {
   dfree(h->d_tail_ops);
   dfree(h->d_dense);
   dfree(h->d_tail_cells);
+  dfree(h->d_tail_tables);
   dfree(h->d_tail_cbl);
   dfree(h->d_tail_fills);
   dfree(h->d_tail_starts);
