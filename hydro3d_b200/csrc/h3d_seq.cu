@@ -872,7 +872,7 @@ cudaError_t launch_sip_sweep_c(const SipPlan& P, const BlkLev* bl, const long lo
 
 // Which TDMA kernel a level takes: whole blocks in shared memory where they fit
 // (16x16x24 cells in FP64), else clusters with the diagonals around the current
-// one there (80^3 in FP64), else, and with variable coefficients, one thread a
+// one there (78^3 in FP64), else, and with variable coefficients, one thread a
 // line in global memory (k_tdma).
 TdmaPlan tdma_plan(const std::vector<BlkLev>& bl, bool var, int word) {
   TdmaPlan P;
