@@ -54,7 +54,8 @@ LevelGeom make_level_geom(const std::vector<h3d_block_desc>& blocks, int g, bool
     L.clamped.push_back(g > d.ngrid);
     L.same_next.push_back(g >= d.ngrid);
   }
-  L.n_elems = off;
+  // (passes over whole arrays move pairs of words)
+  L.n_elems = pad ? (off + kRowAlign - 1) / kRowAlign * kRowAlign : off;
   return L;
 }
 

@@ -45,7 +45,7 @@ struct LevelGeom {
   // restriction into this level is a copy), and block whose next coarser level
   // has this level's size (g >= ngrid, its correction from it is an add)
   std::vector<char> clamped, same_next;
-  int64_t n_elems = 0;      // total cells incl. ghosts
+  int64_t n_elems = 0;      // words of a level array: total cells incl. ghosts (padded: up to a multiple of kRowAlign)
   int64_t n_interior = 0;   // total interior cells
 };
 

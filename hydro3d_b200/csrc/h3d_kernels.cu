@@ -2867,6 +2867,7 @@ template cudaError_t launch_defect_vec<float, float>(const BlkLev*, const Tile*,
 
 template <typename TE>
 cudaError_t launch_apply(const double* p, const TE* e, double* p_next, int64_t n, cudaStream_t st) {
+  if (n & 1) return cudaErrorInvalidValue;  // the kernel moves pairs
   pdl_launch(k_apply<TE>, (int)std::min<int64_t>((n / 2 + 255) / 256, 148 * 16), 256, 0, st, p, e, p_next, n);
   return cudaGetLastError();
 }

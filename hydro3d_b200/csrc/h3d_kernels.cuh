@@ -235,7 +235,8 @@ cudaError_t launch_defect_march(int gp, const BlkLev* bl, const Tile* tiles, int
                                 double rscale, double* partials, cudaStream_t st);
 int defect_march_rows();
 
-// p_next = p + e on n words (level arrays: a multiple of two); p_next may be p.
+// p_next = p + e on n words, n even (padded level arrays are a multiple of
+// kRowAlign long; any other n is refused); p_next may be p.
 template <typename TE>
 cudaError_t launch_apply(const double* p, const TE* e, double* p_next, int64_t n, cudaStream_t st);
 // Level-1 FP64 defect: r = b - A p on the interior, rhs_out = r - mean_b (as
