@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(1024) k_relax_blocks(const BlkLev* __restrict_
   pdl_trigger();
   const BlkLev B = bls[blockIdx.x];
   const int f0 = fstart[blockIdx.x], f1 = fstart[blockIdx.x + 1];
-  pdl_wait();
+  pdl_wait(phi, rhs);
   if (zero) {
     const long long n = (long long)(B.nz + 2) * B.sxy;
     for (long long q = threadIdx.x; q < n; q += blockDim.x) phi[B.off + q] = T(0);
@@ -218,11 +218,13 @@ __global__ void __launch_bounds__(kResidentThreads) k_relax_resident(
   const int f0 = fstart[blockIdx.x], f1 = fstart[blockIdx.x + 1], fl = f0 + live[blockIdx.x];
   T* P = reinterpret_cast<T*>(block_smem);
   const int ex = B.nx + 2, ey = B.ny + 2, n = ex * ey * (B.nz + 2);
-  pdl_wait();
+  pdl_wait(phi, rhs);
   for (int q = threadIdx.x; q < n; q += blockDim.x) {
     const int x = q % ex, y = (q / ex) % ey, z = q / (ex * ey);
-    P[q] = zero || wall_ghost(B, x, y, z) ? T(0) : phi[B.off + (long long)z * B.sxy + (long long)y * B.sx + x];
+    if (zero || wall_ghost(B, x, y, z)) P[q] = T(0);
+    else cp_async_word(P + q, phi + B.off + (long long)z * B.sxy + (long long)y * B.sx + x);
   }
+  asm volatile("cp.async.wait_all;\n" ::: "memory");  // (relax_resident meets before the first sweep)
   auto rhs_at = [&](int x, int y, int z) { return rhs[B.off + (long long)z * B.sxy + (long long)y * B.sx + x]; };
   auto fill = [&](bool last) {
     __syncthreads();
@@ -256,7 +258,7 @@ __global__ void __launch_bounds__(1024) k_relax_small(const BlkLev* __restrict__
   // while the predecessor finishes
   for (int b = threadIdx.x; b < nb; b += blockDim.x) sb[b] = bls[b];
   for (int b = threadIdx.x; b <= nb; b += blockDim.x) ss[b] = start[b];
-  pdl_wait();
+  pdl_wait(phi, rhs);
   __syncthreads();
   small_relax<T, VAR>(sb, ss, nb, phi, rhs, fx, fy, fz, fdst, fsrc, nfill, sweeps, zero, nelems, om, rb);
 }

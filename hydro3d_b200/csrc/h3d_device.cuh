@@ -17,7 +17,26 @@ namespace h3d {
 // measured 60.1 ms against 56.1 ms without on the 33.5M-cell solve (the
 // early launched grids hold SM resources the running ones need).
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+//
+// A kernel that starts early runs while its predecessors still write, so what
+// they write is not constant for its lifetime, as `const __restrict__` data is for the
+// compiler: such loads (ld.global.nc) are not held back by the wait.  (The load of
+// the mean that remove_mean subtracts was moved above it: solves of up to 75,000 words
+// kept their mean in up to a third of the calls.)  The wait therefore takes the
+// pointers to data that predecessors write and makes them opaque; tables written
+// once at set-up are left out.  Plain loads are not moved ahead of stores and
+// barriers either, which costs the large streaming kernels (the variable-density solve
+// of 256^3: 20.6 ms, 25.6 ms), and large launches gain nothing from starting early:
+// those kernels are built in two forms, EARLY with opaque pointers and one without.
+template <typename Ptr>
+__device__ __forceinline__ void make_opaque(Ptr& p) {
+  asm volatile("" : "+l"(p));
+}
+template <bool EARLY = true, typename... Ptr>
+__device__ __forceinline__ void pdl_wait(Ptr&... written) {
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  if constexpr (EARLY) (make_opaque(written), ...);
+}
 
 // Launch policy (H3D_PDL): "1" every kernel, "0" none; by default only a
 // kernel of at most kPdlGrid CTAs that follows one of at most kPdlGrid CTAs
@@ -37,9 +56,22 @@ inline int pdl_mode() {
 }
 inline thread_local long long g_prev_grid = 1LL << 40;
 
+// Tile kernels of few CTAs may still run for 100 us (256^3 cells in one block): from
+// this many cells on they do not start early (the early forms of the
+// variable-density sweep and restriction: 21.5 ms a solve of 256^3, 20.6 ms without).
+constexpr long long kPdlCells = 1LL << 20;
+
+// The next launch of this host thread, of n CTAs: does it start early?
+inline bool pdl_early(long long n, long long cells = 0) {
+  const int mode = pdl_mode();
+  const bool early = mode == 1 || (mode == 2 && n <= kPdlGrid && g_prev_grid <= kPdlGrid && cells < kPdlCells);
+  g_prev_grid = n;
+  return early;
+}
+
 template <typename... KArgs, typename... Args>
-inline cudaError_t pdl_launch(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                              Args... args) {
+inline cudaError_t launch_kernel(void (*k)(KArgs...), bool early, dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                 Args... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -49,11 +81,44 @@ inline cudaError_t pdl_launch(void (*k)(KArgs...), dim3 grid, dim3 block, size_t
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  const long long n = (long long)grid.x * grid.y * grid.z;
-  const int mode = pdl_mode();
-  cfg.numAttrs = (mode == 1 || (mode == 2 && n <= kPdlGrid && g_prev_grid <= kPdlGrid)) ? 1 : 0;
-  g_prev_grid = n;
+  cfg.numAttrs = early ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, k, static_cast<KArgs>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+inline cudaError_t pdl_launch(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                              Args... args) {
+  return launch_kernel(k, pdl_early((long long)grid.x * grid.y * grid.z), grid, block, smem, st, args...);
+}
+
+// The two forms of a kernel (see pdl_wait); H3D_BOTH(k, a, b): those of k<a, b, EARLY>.
+template <typename... KArgs>
+struct KernelPair {
+  void (*plain)(KArgs...);
+  void (*early)(KArgs...);
+  long long cells = 0;  // of a tile kernel's launch
+};
+template <typename... KArgs>
+KernelPair(void (*)(KArgs...), void (*)(KArgs...)) -> KernelPair<KArgs...>;
+#define H3D_BOTH(k, ...) KernelPair{k<__VA_ARGS__, false>, k<__VA_ARGS__, true>}
+
+template <typename... KArgs, typename... Args>
+inline cudaError_t pdl_launch(KernelPair<KArgs...> k, dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                              Args... args) {
+  const bool early = pdl_early((long long)grid.x * grid.y * grid.z, k.cells);
+  return launch_kernel(early ? k.early : k.plain, early, grid, block, smem, st, args...);
+}
+
+template <typename... KArgs>
+inline KernelPair<KArgs...> sized(KernelPair<KArgs...> k, long long cells) {
+  k.cells = cells;
+  return k;
+}
+
+template <typename... KArgs>
+inline cudaError_t kernel_smem(KernelPair<KArgs...> k, int bytes) {
+  cudaError_t e = cudaFuncSetAttribute(k.plain, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  return e != cudaSuccess ? e : cudaFuncSetAttribute(k.early, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
 __device__ __forceinline__ int find_block(const int* __restrict__ start, int nb, int cta) {
@@ -113,6 +178,12 @@ __device__ __forceinline__ float sorf(float old, float gs, float om) { return fm
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+
+template <typename T>
+__device__ __forceinline__ void cp_async_word(T* s, const T* g) {
+  const unsigned a = smem_u32(s);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(a), "l"(g), "n"(sizeof(T)) : "memory");
 }
 
 // First 128-byte boundary of the dynamic shared memory, by pointer arithmetic

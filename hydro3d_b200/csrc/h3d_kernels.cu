@@ -51,13 +51,13 @@ __device__ __noinline__ bool h3d_oob(int kid, int b, long long idx, long long li
 // of plane z-1 from the new red values and stores plane z-1.  Ghost cells are
 // never updated inside a sweep, exactly like the reference, where they change
 // only in the mgbound/exchangepp call after the whole sweep.
-template <typename T, int TX, int TY, int NT, bool VAR, bool ZERO>
+template <typename T, int TX, int TY, int NT, bool VAR, bool ZERO, bool EARLY>
 __global__ void __launch_bounds__(NT) k_rbgs(const BlkLev* __restrict__ bls, const Tile* __restrict__ tiles,
                                              int zc, const T* __restrict__ src, T* __restrict__ dst,
                                              const T* __restrict__ rhs, const T* __restrict__ fx,
                                              const T* __restrict__ fy, const T* __restrict__ fz, float om) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait<EARLY>(src, rhs);
   constexpr int RX = TX + 4, RY = TY + 4, RN = RX * RY;
   constexpr int R1X = TX + 2, R1N = (TX + 2) * (TY + 2);
   __shared__ T ring[4][RN];
@@ -158,6 +158,7 @@ __global__ void __launch_bounds__(NT) k_rbgs(const BlkLev* __restrict__ bls, con
 // in registers; rows y+-1 and the two cells beside the group come from L1.
 // 1/ap of a cell depends only on which wall faces it touches: a 64-entry
 // table per CTA.  Ghost pushes as in the window sweep.
+template <bool EARLY>
 __global__ void __launch_bounds__(256, 3) k_rbgs_zero32(const BlkLev* __restrict__ bls, const Tile* __restrict__ tiles,
                                                      int zc, const float* __restrict__ rhs, float* __restrict__ dst,
                                                      const long long* __restrict__ push, float om) {
@@ -174,7 +175,7 @@ __global__ void __launch_bounds__(256, 3) k_rbgs_zero32(const BlkLev* __restrict
     ivtab[m] = 1.f / (-(aw + ae + as + an + ab + at));
   }
   __syncthreads();
-  pdl_wait();
+  pdl_wait<EARLY>(rhs);
   const int G = nx >> 2;           // groups per row
   const int rows = blockDim.x / G;  // rows of this tile
   const int r = threadIdx.x / G, g = threadIdx.x - r * G;
@@ -303,7 +304,7 @@ __global__ void __launch_bounds__(256, 3) k_rbgs_zero32(const BlkLev* __restrict
 cudaError_t launch_rbgs_zero32(const BlkLev* bl, const Tile* tiles, int ntiles, int zc, const float* rhs, float* dst,
                                const long long* push, float om, cudaStream_t st) {
   if (ntiles <= 0) return cudaSuccess;
-  pdl_launch(k_rbgs_zero32, ntiles, 256, 0, st, bl, tiles, zc, rhs, dst, push, om);
+  pdl_launch(KernelPair{k_rbgs_zero32<false>, k_rbgs_zero32<true>}, ntiles, 256, 0, st, bl, tiles, zc, rhs, dst, push, om);
   return cudaGetLastError();
 }
 
@@ -343,7 +344,7 @@ __global__ void __launch_bounds__(512) k_gslex(const BlkLev* __restrict__ bls, c
                                                const T* __restrict__ fx, const T* __restrict__ fy,
                                                const T* __restrict__ fz, bool zero) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(src, rhs);
   const BlkLev B = bls[blockIdx.x];
   T* __restrict__ D = dst + B.off;
   const T* __restrict__ R = rhs + B.off;
@@ -441,7 +442,7 @@ __global__ void __launch_bounds__(256) k_tdma(const BlkLev* __restrict__ bls, co
                                               const T* __restrict__ fx, const T* __restrict__ fy,
                                               const T* __restrict__ fz, bool zero) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(src, rhs);
   const BlkLev B = bls[blockIdx.x];
   T* __restrict__ D = dst + B.off;
   T* __restrict__ A = acoef + B.off;
@@ -560,7 +561,7 @@ struct RowGs {
 // exactly one cell is red and one black, so neither colour phase diverges.
 // Shared memory holds four staged planes of rows y0-2 .. y0+TY+1; column c
 // holds x = c-1.  Same out-of-place contract and arithmetic as k_rbgs.
-template <typename T, int TPR, int CP, int TY, bool VAR, bool ZERO>
+template <typename T, int TPR, int CP, int TY, bool VAR, bool ZERO, bool EARLY>
 __global__ void __launch_bounds__(TPR*(TY + 2)) k_rbgs_rows(const BlkLev* __restrict__ bls,
                                                            const Tile* __restrict__ tiles, int zc,
                                                            const T* __restrict__ src, T* __restrict__ dst,
@@ -568,7 +569,7 @@ __global__ void __launch_bounds__(TPR*(TY + 2)) k_rbgs_rows(const BlkLev* __rest
                                                            const T* __restrict__ fy, const T* __restrict__ fz,
                                                            float om) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait<EARLY>(src, rhs);
   constexpr int SP = 2 * CP * TPR + 4;
   constexpr int SR = TY + 4;
   constexpr int PL = SR * SP;
@@ -1085,7 +1086,7 @@ __global__ void __launch_bounds__(TPR*(TY + 2)) k_rbgs_vec(const BlkLev* __restr
 }
 
 // ---------------------------------------------------------------------------
-template <typename T, bool ZERO_OLD>
+template <typename T, bool ZERO_OLD, bool EARLY>
 __global__ void k_fill(const uint32_t* __restrict__ dsts, const uint32_t* __restrict__ srcs, int64_t n,
                        T* __restrict__ out, const T* __restrict__ cur, const T* __restrict__ old) {
   pdl_trigger();
@@ -1097,7 +1098,7 @@ __global__ void k_fill(const uint32_t* __restrict__ dsts, const uint32_t* __rest
     s = __ldg(srcs + e);
     d = __ldg(dsts + e);
   }
-  pdl_wait();
+  pdl_wait<EARLY>(cur, old);
   for (; e < n; e += (int64_t)gridDim.x * blockDim.x) {
     T v;
     if (s & kOldFlag) v = ZERO_OLD ? T(0) : old[s & kIdxMask];
@@ -1133,14 +1134,14 @@ __device__ __forceinline__ RowRef row_of(const BlkLev* __restrict__ bls, const i
 
 // mgrestr: resf = su - (A phi) on the fine interior (mgsolver.for:707-714),
 // coarse rhs = 0.125 * sum of the 2x2x2 children, i fastest (:748-752).
-template <typename T, bool VAR, bool ZERO>
+template <typename T, bool VAR, bool ZERO, bool EARLY>
 __global__ void __launch_bounds__(256) k_restrict(const BlkLev* __restrict__ fine, const BlkLev* __restrict__ coarse,
                                                   const int* __restrict__ row_start, int nb, int nrows,
                                                   const T* __restrict__ phi, const T* __restrict__ rhs,
                                                   T* __restrict__ rhs_c, const T* __restrict__ fx,
                                                   const T* __restrict__ fy, const T* __restrict__ fz) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait<EARLY>(phi, rhs);
   const int lane = threadIdx.x & 31;
   for (int rid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; rid < nrows; rid += (gridDim.x * blockDim.x) >> 5) {
     const RowRef rr = row_of(coarse, row_start, nb, rid, true);
@@ -1189,7 +1190,7 @@ __global__ void __launch_bounds__(256) k_prolong(const BlkLev* __restrict__ fine
                                                  const T* __restrict__ phi_c, const T* __restrict__ old,
                                                  T* __restrict__ out) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(phi_c, old);
   const int lane = threadIdx.x & 31;
   for (int rid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; rid < nrows; rid += (gridDim.x * blockDim.x) >> 5) {
     const RowRef rr = row_of(fine, row_start, nb, rid, false);
@@ -1234,11 +1235,11 @@ __global__ void __launch_bounds__(256) k_prolong(const BlkLev* __restrict__ fine
 
 // p_next = p + e over whole level arrays (ghosts included, newsolv_mg.for:39-48);
 // p_next may be p.
-template <typename TE>
+template <typename TE, bool EARLY>
 __global__ void __launch_bounds__(256) k_apply(const double* p, const TE* __restrict__ e, double* p_next,
                                                int64_t n) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait<EARLY>(p, e);
   using E2 = typename std::conditional<sizeof(TE) == 4, float2, double2>::type;
   for (int64_t i = 2 * (blockIdx.x * (int64_t)blockDim.x + threadIdx.x); i < n;
        i += 2 * (int64_t)gridDim.x * blockDim.x) {
@@ -1253,7 +1254,7 @@ __global__ void __launch_bounds__(256) k_apply(const double* p, const TE* __rest
 // p + e is a pass of its own before it: added at each of the seven points of
 // the stencil it took 505 us on 256^3 cells with variable coefficients, against
 // 206 us for this kernel and 50 us for the pass.)
-template <typename TR, bool VAR>
+template <typename TR, bool VAR, bool EARLY>
 __global__ void __launch_bounds__(256) k_defect(const BlkLev* __restrict__ bls, const int* __restrict__ row_start,
                                                 int nb, int nrows, const double* __restrict__ p,
                                                 const double* __restrict__ bvec, TR* __restrict__ rhs_out,
@@ -1261,7 +1262,7 @@ __global__ void __launch_bounds__(256) k_defect(const BlkLev* __restrict__ bls, 
                                                 const double* __restrict__ fy, const double* __restrict__ fz,
                                                 double* __restrict__ partials) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait<EARLY>(p, bvec);
   const int lane = threadIdx.x & 31;
   double rr = 0, bb = 0, rm = 0, rs = 0;
   for (int rid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; rid < nrows; rid += (gridDim.x * blockDim.x) >> 5) {
@@ -1295,7 +1296,7 @@ __global__ void __launch_bounds__(256) k_defect(const BlkLev* __restrict__ bls, 
 // range, staging fine iterate planes (rows 2Y0-2 .. 2Y0+2TYC-1) in a 3-plane
 // ring.  Each thread keeps the running sum of its coarse cells and adds the
 // eight child residuals in the reference order (i fastest, then j, then k).
-template <typename T, bool VAR, bool ZERO, int TPR, int CPX, int TYC>
+template <typename T, bool VAR, bool ZERO, int TPR, int CPX, int TYC, bool EARLY>
 __global__ void __launch_bounds__(TPR* TYC) k_restrict_tile(const BlkLev* __restrict__ fine,
                                                            const BlkLev* __restrict__ coarse,
                                                            const Tile* __restrict__ tiles, int zc,
@@ -1303,7 +1304,7 @@ __global__ void __launch_bounds__(TPR* TYC) k_restrict_tile(const BlkLev* __rest
                                                            T* __restrict__ rhs_c, const T* __restrict__ fx,
                                                            const T* __restrict__ fy, const T* __restrict__ fz) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait<EARLY>(phi, rhs);
   constexpr int SP = 2 * CPX * TPR + 4;
   constexpr int SR = 2 * TYC + 2;
   constexpr int PL = SR * SP;
@@ -1382,14 +1383,14 @@ __global__ void __launch_bounds__(TPR* TYC) k_restrict_tile(const BlkLev* __rest
 
 // mgcorr + mgbound with one thread per fine cell pair (2q, 2q+1) of a row:
 // both cells of a pair interpolate from the same eight coarse cells.
-template <typename T, bool ZERO_OLD>
+template <typename T, bool ZERO_OLD, bool EARLY>
 __global__ void __launch_bounds__(256) k_prolong_pairs(const BlkLev* __restrict__ fine,
                                                        const BlkLev* __restrict__ coarse,
                                                        const int* __restrict__ row_start, int nb, int nrows,
                                                        const T* __restrict__ phi_c, const T* __restrict__ old,
                                                        T* __restrict__ out) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait<EARLY>(phi_c, old);
   const int lane = threadIdx.x & 31;
   for (int rid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; rid < nrows; rid += (gridDim.x * blockDim.x) >> 5) {
     const RowRef rr = row_of(fine, row_start, nb, rid, false);
@@ -1445,7 +1446,7 @@ __global__ void __launch_bounds__(256) k_prolong_pairs(const BlkLev* __restrict_
 
 __global__ void __launch_bounds__(1024) k_reduce4(const double* __restrict__ partials, int n, double* __restrict__ out) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(partials);
   double a0 = 0, a1 = 0, a2 = 0, a3 = 0;
   for (int q = threadIdx.x; q < n; q += 1024) {
     a0 += partials[4 * (size_t)q];
@@ -1461,7 +1462,7 @@ __global__ void __launch_bounds__(1024) k_reduce4(const double* __restrict__ par
 __global__ void __launch_bounds__(256) k_reduce4_blocks(const double* __restrict__ partials,
                                                         const int* __restrict__ start, double* __restrict__ out) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(partials);
   const int b = blockIdx.x;
   double a0 = 0, a1 = 0, a2 = 0, a3 = 0;
   for (int q = start[b] + threadIdx.x; q < start[b + 1]; q += 256) {
@@ -1475,11 +1476,12 @@ __global__ void __launch_bounds__(256) k_reduce4_blocks(const double* __restrict
 
 // Sum of a field over the interior cells: a warp a row at a time (grid-stride
 // over the level's interior rows), one partial sum per CTA in a fixed order.
+template <bool EARLY>
 __global__ void __launch_bounds__(256) k_sum_interior(const BlkLev* __restrict__ bls, const int* __restrict__ row_start,
                                                       int nb, int nrows, const double* __restrict__ a,
                                                       double* __restrict__ partials) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait<EARLY>(a);
   const int lane = threadIdx.x & 31;
   double s = 0;
   for (int rid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; rid < nrows; rid += (gridDim.x * blockDim.x) >> 5) {
@@ -1491,23 +1493,26 @@ __global__ void __launch_bounds__(256) k_sum_interior(const BlkLev* __restrict__
   block_reduce4<256>(s, 0.0, 0.0, 0.0, partials + 4 * (size_t)blockIdx.x);
 }
 
+template <bool EARLY>
 __global__ void k_shift(double* __restrict__ a, int64_t n, const double* __restrict__ s, double scale) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait<EARLY>(a, s);
   const double v = s[0] * scale;
   for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x)
     a[q] = a[q] - v;
 }
 
+template <bool EARLY>
 __global__ void k_d2f(const double* __restrict__ a, float* __restrict__ b, int64_t n) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait<EARLY>(a);
   for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x)
     b[q] = (float)a[q];
 }
+template <bool EARLY>
 __global__ void k_f2d(const float* __restrict__ a, double* __restrict__ b, int64_t n) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait<EARLY>(a);
   for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x)
     b[q] = (double)a[q];
 }
@@ -1518,7 +1523,7 @@ __global__ void __launch_bounds__(256) k_dens_restrict(const BlkLev* __restrict_
                                                        const int* __restrict__ cta_start, int nb,
                                                        const double* __restrict__ df, double* __restrict__ dc) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(df);
   const int b = find_block(cta_start, nb, blockIdx.x);
   const BlkLev C = coarse[b], F = fine[b];
   const int local = (blockIdx.x - cta_start[b]) * blockDim.x + threadIdx.x;
@@ -1539,7 +1544,7 @@ __global__ void __launch_bounds__(256) k_face_coef(const BlkLev* __restrict__ bl
                                                    const double* __restrict__ h3, double* __restrict__ fx,
                                                    double* __restrict__ fy, double* __restrict__ fz) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(dens);
   const int b = find_block(cta_start, nb, blockIdx.x);
   const BlkLev B = bls[b];
   const int local = (blockIdx.x - cta_start[b]) * blockDim.x + threadIdx.x;
@@ -1648,11 +1653,11 @@ static cudaError_t rbgs_dispatch(bool var, bool zero, const BlkLev* bl, const Ti
   if (ntiles <= 0) return cudaSuccess;
   dim3 grid(ntiles), block(NT);
   if (var) {
-    if (zero) pdl_launch(k_rbgs<T, TX, TY, NT, true, true>, grid, block, 0, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
-    else pdl_launch(k_rbgs<T, TX, TY, NT, true, false>, grid, block, 0, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
+    if (zero) pdl_launch(H3D_BOTH(k_rbgs, T, TX, TY, NT, true, true), grid, block, 0, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
+    else pdl_launch(H3D_BOTH(k_rbgs, T, TX, TY, NT, true, false), grid, block, 0, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
   } else {
-    if (zero) pdl_launch(k_rbgs<T, TX, TY, NT, false, true>, grid, block, 0, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
-    else pdl_launch(k_rbgs<T, TX, TY, NT, false, false>, grid, block, 0, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
+    if (zero) pdl_launch(H3D_BOTH(k_rbgs, T, TX, TY, NT, false, true), grid, block, 0, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
+    else pdl_launch(H3D_BOTH(k_rbgs, T, TX, TY, NT, false, false), grid, block, 0, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
   }
   return cudaGetLastError();
 }
@@ -1666,10 +1671,10 @@ template <typename T, int TPR, int CP, int TY>
 static cudaError_t rows_attr() {
   const int sm = (int)rows_smem<T, TPR, CP, TY>();
   cudaError_t e;
-  if ((e = cudaFuncSetAttribute(k_rbgs_rows<T, TPR, CP, TY, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))) return e;
-  if ((e = cudaFuncSetAttribute(k_rbgs_rows<T, TPR, CP, TY, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))) return e;
-  if ((e = cudaFuncSetAttribute(k_rbgs_rows<T, TPR, CP, TY, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))) return e;
-  return cudaFuncSetAttribute(k_rbgs_rows<T, TPR, CP, TY, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+  if ((e = kernel_smem(H3D_BOTH(k_rbgs_rows, T, TPR, CP, TY, true, true), sm))) return e;
+  if ((e = kernel_smem(H3D_BOTH(k_rbgs_rows, T, TPR, CP, TY, true, false), sm))) return e;
+  if ((e = kernel_smem(H3D_BOTH(k_rbgs_rows, T, TPR, CP, TY, false, true), sm))) return e;
+  return kernel_smem(H3D_BOTH(k_rbgs_rows, T, TPR, CP, TY, false, false), sm);
 }
 
 template <typename T, int TPR, int CP, int TY>
@@ -1680,12 +1685,13 @@ static cudaError_t rows_dispatch(bool var, bool zero, const BlkLev* bl, const Ti
   constexpr int NT = TPR * (TY + 2);
   constexpr size_t SM = rows_smem<T, TPR, CP, TY>();
   dim3 grid(ntiles), block(NT);
+  const long long cells = (long long)ntiles * TY * zc * (2 * CP * TPR);  // at most
   if (var) {
-    if (zero) pdl_launch(k_rbgs_rows<T, TPR, CP, TY, true, true>, grid, block, SM, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
-    else pdl_launch(k_rbgs_rows<T, TPR, CP, TY, true, false>, grid, block, SM, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
+    if (zero) pdl_launch(sized(H3D_BOTH(k_rbgs_rows, T, TPR, CP, TY, true, true), cells), grid, block, SM, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
+    else pdl_launch(sized(H3D_BOTH(k_rbgs_rows, T, TPR, CP, TY, true, false), cells), grid, block, SM, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
   } else {
-    if (zero) pdl_launch(k_rbgs_rows<T, TPR, CP, TY, false, true>, grid, block, SM, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
-    else pdl_launch(k_rbgs_rows<T, TPR, CP, TY, false, false>, grid, block, SM, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
+    if (zero) pdl_launch(sized(H3D_BOTH(k_rbgs_rows, T, TPR, CP, TY, false, true), cells), grid, block, SM, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
+    else pdl_launch(sized(H3D_BOTH(k_rbgs_rows, T, TPR, CP, TY, false, false), cells), grid, block, SM, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
   }
   return cudaGetLastError();
 }
@@ -2249,8 +2255,8 @@ cudaError_t launch_fill(const uint32_t* dsts, const uint32_t* srcs, int64_t n, T
                         bool zero_old, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
   int g = grid_for(n, 256);
-  if (zero_old) pdl_launch(k_fill<T, true>, g, 256, 0, st, dsts, srcs, n, out, cur, old);
-  else pdl_launch(k_fill<T, false>, g, 256, 0, st, dsts, srcs, n, out, cur, old);
+  if (zero_old) pdl_launch(H3D_BOTH(k_fill, T, true), g, 256, 0, st, dsts, srcs, n, out, cur, old);
+  else pdl_launch(H3D_BOTH(k_fill, T, false), g, 256, 0, st, dsts, srcs, n, out, cur, old);
   return cudaGetLastError();
 }
 
@@ -2268,7 +2274,7 @@ cudaError_t launch_fill(const uint32_t* dsts, const uint32_t* srcs, int64_t n, T
 // block sizes a ghost cell of red colour is read by black cells only, so the
 // sweep's red cells still see their old black neighbours, and no entry reads a
 // cell another entry writes.
-template <bool VAR>
+template <bool VAR, bool EARLY>
 __global__ void __launch_bounds__(256) k_red_ahead(const uint32_t* __restrict__ dst, const uint32_t* __restrict__ src,
                                                    const int* __restrict__ info, int64_t n, int nb,
                                                    const BlkLev* __restrict__ bls, float* __restrict__ phi,
@@ -2281,7 +2287,7 @@ __global__ void __launch_bounds__(256) k_red_ahead(const uint32_t* __restrict__ 
   if (staged)
     for (int q = threadIdx.x; q < nb; q += blockDim.x) sb[q] = bls[q];
   __syncthreads();
-  pdl_wait();
+  pdl_wait<EARLY>(phi, rhs);
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
     // info: block (bits 0-15) and the cell's wall faces (bits 16-21, W E S N B T)
     const long long gi = src[e];
@@ -2308,8 +2314,8 @@ cudaError_t launch_red_ahead(bool var, const uint32_t* dst, const uint32_t* src,
                              const float* fz, float om, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
   const int g = grid_for(n, 256);
-  if (var) pdl_launch(k_red_ahead<true>, g, 256, 0, st, dst, src, info, n, nb, bl, phi, rhs, fx, fy, fz, om);
-  else pdl_launch(k_red_ahead<false>, g, 256, 0, st, dst, src, info, n, nb, bl, phi, rhs, fx, fy, fz, om);
+  if (var) pdl_launch(H3D_BOTH(k_red_ahead, true), g, 256, 0, st, dst, src, info, n, nb, bl, phi, rhs, fx, fy, fz, om);
+  else pdl_launch(H3D_BOTH(k_red_ahead, false), g, 256, 0, st, dst, src, info, n, nb, bl, phi, rhs, fx, fy, fz, om);
   return cudaGetLastError();
 }
 
@@ -2324,9 +2330,9 @@ cudaError_t launch_restrict(bool var, bool zero_phi, const BlkLev* fine, const B
                             cudaStream_t st) {
   if (rt.nrows <= 0) return cudaSuccess;
   const int g = row_grid(rt.nrows);
-  if (zero_phi) pdl_launch(k_restrict<T, false, true>, g, 256, 0, st, fine, coarse, rt.start, rt.nb, rt.nrows, phi, rhs, rhs_c, fx, fy, fz);
-  else if (var) pdl_launch(k_restrict<T, true, false>, g, 256, 0, st, fine, coarse, rt.start, rt.nb, rt.nrows, phi, rhs, rhs_c, fx, fy, fz);
-  else pdl_launch(k_restrict<T, false, false>, g, 256, 0, st, fine, coarse, rt.start, rt.nb, rt.nrows, phi, rhs, rhs_c, fx, fy, fz);
+  if (zero_phi) pdl_launch(H3D_BOTH(k_restrict, T, false, true), g, 256, 0, st, fine, coarse, rt.start, rt.nb, rt.nrows, phi, rhs, rhs_c, fx, fy, fz);
+  else if (var) pdl_launch(H3D_BOTH(k_restrict, T, true, false), g, 256, 0, st, fine, coarse, rt.start, rt.nb, rt.nrows, phi, rhs, rhs_c, fx, fy, fz);
+  else pdl_launch(H3D_BOTH(k_restrict, T, false, false), g, 256, 0, st, fine, coarse, rt.start, rt.nb, rt.nrows, phi, rhs, rhs_c, fx, fy, fz);
   return cudaGetLastError();
 }
 
@@ -2341,7 +2347,7 @@ cudaError_t launch_restrict(bool var, bool zero_phi, const BlkLev* fine, const B
 // one vector load of the old iterate and one vector store per row.  Lanes 0
 // and 1 take the ghost columns.  Same interpolation, term order and mgbound
 // source as k_prolong_pairs.  Needs nx a multiple of VEC and ny, nz even.
-template <typename T, bool ZERO_OLD>
+template <typename T, bool ZERO_OLD, bool EARLY>
 __global__ void __launch_bounds__(256, 3) k_prolong_vec(const BlkLev* __restrict__ fine, const BlkLev* __restrict__ coarse,
                                                      const Tile* __restrict__ tiles, const T* __restrict__ phi_c,
                                                      const T* __restrict__ old, T* __restrict__ out) {
@@ -2370,7 +2376,7 @@ __global__ void __launch_bounds__(256, 3) k_prolong_vec(const BlkLev* __restrict
   }
   const long long cy = C.sx, cz = C.sxy;
   const int ng = F.nx / VEC;
-  pdl_wait();  // everything above reads only setup data
+  pdl_wait<EARLY>(phi_c, old);  // everything above reads only setup data
 #pragma unroll 2
   for (int k = threadIdx.x >> 5; k <= F.ny / 2; k += 8) {  // two row pairs in flight a warp
     // rows 2k, 2k+1 and their sources
@@ -2404,6 +2410,14 @@ __global__ void __launch_bounds__(256, 3) k_prolong_vec(const BlkLev* __restrict
         cq[2][c] = R01[c0 + c];
         cq[3][c] = R11[c0 + c];
       }
+      V ov[2][2];  // all loads before the first store
+#pragma unroll
+      for (int iz = 0; iz < 2; ++iz)
+#pragma unroll
+        for (int iy = 0; iy < 2; ++iy)
+          ov[iz][iy] = ZERO_OLD ? V{}
+                                : *reinterpret_cast<const V*>(old + F.off + (long long)szq[iz] * F.sxy +
+                                                              (long long)syq[iy] * F.sx + x0);
 #pragma unroll
       for (int iz = 0; iz < 2; ++iz)
 #pragma unroll
@@ -2413,12 +2427,8 @@ __global__ void __launch_bounds__(256, 3) k_prolong_vec(const BlkLev* __restrict
           // the eight weights of odd (wo) and even (we) fine columns: products of small integers
           const T wo[8] = {w00, w10, w01, w11, T(3) * w00, T(3) * w10, T(3) * w01, T(3) * w11};
           const T we[8] = {T(3) * w00, T(3) * w10, T(3) * w01, T(3) * w11, w00, w10, w01, w11};
-          const long long ro = F.off + (long long)szq[iz] * F.sxy + (long long)syq[iy] * F.sx;
-          V ov;
-          if (ZERO_OLD) ov = V{};
-          else ov = *reinterpret_cast<const V*>(old + ro + x0);
           T o[VEC], r[VEC];
-          *reinterpret_cast<V*>(o) = ov;
+          *reinterpret_cast<V*>(o) = ov[iz][iy];
 #pragma unroll
           for (int m = 0; m < VEC; ++m) {
             const int kq = (m + 1) >> 1;  // (x >> 1) - (x0 >> 1) for x = x0 + m, x0 odd
@@ -2458,24 +2468,30 @@ __global__ void __launch_bounds__(256, 3) k_prolong_vec(const BlkLev* __restrict
       if (x == F.nx + 1 && (ph & 2)) sx = F.nx;
       const T wx0 = (sx & 1) ? T(1) : T(3), wx1 = (sx & 1) ? T(3) : T(1);
       const T* Q = Pc + (x >> 1);
+      const T q000 = Q[0], q010 = Q[cy], q001 = Q[cz], q011 = Q[cy + cz], q100 = Q[1], q110 = Q[1 + cy],
+              q101 = Q[1 + cz], q111 = Q[1 + cy + cz];
+      T o[2][2];
+#pragma unroll
+      for (int iz = 0; iz < 2; ++iz)
+#pragma unroll
+        for (int iy = 0; iy < 2; ++iy)
+          o[iz][iy] = ZERO_OLD ? T(0) : old[F.off + (long long)szq[iz] * F.sxy + (long long)syq[iy] * F.sx + sx];
 #pragma unroll
       for (int iz = 0; iz < 2; ++iz)
 #pragma unroll
         for (int iy = 0; iy < 2; ++iy) {
           const T w00 = wy0[iy] * wz0[iz], w10 = wy1[iy] * wz0[iz], w01 = wy0[iy] * wz1[iz],
                   w11 = wy1[iy] * wz1[iz];
-          const long long ro = F.off + (long long)szq[iz] * F.sxy + (long long)syq[iy] * F.sx;
-          const T o = ZERO_OLD ? T(0) : old[ro + sx];
           // term order (di,dj,dk): 000, 010, 001, 011, 100, 110, 101, 111 (mgsolver.for:838-892)
-          T sum = (wx0 * w00) * Q[0];
-          sum = sum + (wx0 * w10) * Q[cy];
-          sum = sum + (wx0 * w01) * Q[cz];
-          sum = sum + (wx0 * w11) * Q[cy + cz];
-          sum = sum + (wx1 * w00) * Q[1];
-          sum = sum + (wx1 * w10) * Q[1 + cy];
-          sum = sum + (wx1 * w01) * Q[1 + cz];
-          sum = sum + (wx1 * w11) * Q[1 + cy + cz];
-          out[F.off + (long long)zq[iz] * F.sxy + (long long)yq[iy] * F.sx + x] = o + sum / T(64);
+          T sum = (wx0 * w00) * q000;
+          sum = sum + (wx0 * w10) * q010;
+          sum = sum + (wx0 * w01) * q001;
+          sum = sum + (wx0 * w11) * q011;
+          sum = sum + (wx1 * w00) * q100;
+          sum = sum + (wx1 * w10) * q110;
+          sum = sum + (wx1 * w01) * q101;
+          sum = sum + (wx1 * w11) * q111;
+          out[F.off + (long long)zq[iz] * F.sxy + (long long)yq[iy] * F.sx + x] = o[iz][iy] + sum / T(64);
         }
     }
   }
@@ -2485,8 +2501,8 @@ template <typename T>
 cudaError_t launch_prolong_vec(bool zero_old, const BlkLev* fine, const BlkLev* coarse, const Tile* tiles, int ntiles,
                                const T* phi_c, const T* old, T* out, cudaStream_t st) {
   if (ntiles <= 0) return cudaSuccess;
-  if (zero_old) pdl_launch(k_prolong_vec<T, true>, ntiles, 256, 0, st, fine, coarse, tiles, phi_c, old, out);
-  else pdl_launch(k_prolong_vec<T, false>, ntiles, 256, 0, st, fine, coarse, tiles, phi_c, old, out);
+  if (zero_old) pdl_launch(H3D_BOTH(k_prolong_vec, T, true), ntiles, 256, 0, st, fine, coarse, tiles, phi_c, old, out);
+  else pdl_launch(H3D_BOTH(k_prolong_vec, T, false), ntiles, 256, 0, st, fine, coarse, tiles, phi_c, old, out);
   return cudaGetLastError();
 }
 template cudaError_t launch_prolong_vec<double>(bool, const BlkLev*, const BlkLev*, const Tile*, int, const double*,
@@ -2499,8 +2515,8 @@ cudaError_t launch_prolong(bool zero_old, const BlkLev* fine, const BlkLev* coar
                            const T* old, T* out, cudaStream_t st) {
   if (rt.nrows <= 0) return cudaSuccess;
   const int g = row_grid(rt.nrows);
-  if (zero_old) pdl_launch(k_prolong_pairs<T, true>, g, 256, 0, st, fine, coarse, rt.start, rt.nb, rt.nrows, phi_c, old, out);
-  else pdl_launch(k_prolong_pairs<T, false>, g, 256, 0, st, fine, coarse, rt.start, rt.nb, rt.nrows, phi_c, old, out);
+  if (zero_old) pdl_launch(H3D_BOTH(k_prolong_pairs, T, true), g, 256, 0, st, fine, coarse, rt.start, rt.nb, rt.nrows, phi_c, old, out);
+  else pdl_launch(H3D_BOTH(k_prolong_pairs, T, false), g, 256, 0, st, fine, coarse, rt.start, rt.nb, rt.nrows, phi_c, old, out);
   return cudaGetLastError();
 }
 
@@ -2516,14 +2532,14 @@ int defect_grid(int nrows) {
 // left and right of a pair are read singly, the ghost columns by lanes 0, 1.
 // Same residual arithmetic as k_defect; per-CTA partial sums in a fixed order.
 // Needs nx even and constant coefficients.
-template <typename TE, typename TR, bool HAS_E>
+template <typename TE, typename TR, bool HAS_E, bool EARLY>
 __global__ void __launch_bounds__(256) k_defect_vec(const BlkLev* __restrict__ bls, const Tile* __restrict__ tiles,
                                                     int ntiles, const double* __restrict__ p,
                                                     const TE* __restrict__ e, double* __restrict__ p_next,
                                                     const double* __restrict__ bvec, TR* __restrict__ rhs_out,
                                                     double mean_b, double rscale, double* __restrict__ partials) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait<EARLY>(p, e, bvec);
   using E2 = typename std::conditional<sizeof(TE) == 4, float2, double2>::type;
   using R2 = typename std::conditional<sizeof(TR) == 4, float2, double2>::type;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -2725,7 +2741,7 @@ __global__ void __launch_bounds__(32 * (kDefectRows + 2)) k_defect_march(
     if (gc) p_next[rz + gx] = g;
   };
 
-  pdl_wait();  // everything above reads only setup data
+  pdl_wait(p, e, bvec);  // everything above reads only setup data
 #pragma unroll
   for (int q = 0; q < NR; ++q) issue(zs - 1 + q);
   // face coefficients (mgsolver.for:186-205): walls zero the face term; a pair
@@ -2854,8 +2870,8 @@ cudaError_t launch_defect_vec(const BlkLev* bl, const Tile* tiles, int ntiles, c
                               double* partials, int grid, cudaStream_t st) {
   if (ntiles <= 0) return cudaSuccess;
   grid = ntiles;  // one tile per CTA (partials holds one quadruple per tile)
-  if (e) pdl_launch(k_defect_vec<TE, TR, true>, grid, 256, 0, st, bl, tiles, ntiles, p, e, p_next, b, rhs_out, mean_b, rscale, partials);
-  else pdl_launch(k_defect_vec<TE, TR, false>, grid, 256, 0, st, bl, tiles, ntiles, p, e, p_next, b, rhs_out, mean_b, rscale, partials);
+  if (e) pdl_launch(H3D_BOTH(k_defect_vec, TE, TR, true), grid, 256, 0, st, bl, tiles, ntiles, p, e, p_next, b, rhs_out, mean_b, rscale, partials);
+  else pdl_launch(H3D_BOTH(k_defect_vec, TE, TR, false), grid, 256, 0, st, bl, tiles, ntiles, p, e, p_next, b, rhs_out, mean_b, rscale, partials);
   return cudaGetLastError();
 }
 template cudaError_t launch_defect_vec<double, double>(const BlkLev*, const Tile*, int, const double*, const double*,
@@ -2868,7 +2884,7 @@ template cudaError_t launch_defect_vec<float, float>(const BlkLev*, const Tile*,
 template <typename TE>
 cudaError_t launch_apply(const double* p, const TE* e, double* p_next, int64_t n, cudaStream_t st) {
   if (n & 1) return cudaErrorInvalidValue;  // the kernel moves pairs
-  pdl_launch(k_apply<TE>, (int)std::min<int64_t>((n / 2 + 255) / 256, 148 * 16), 256, 0, st, p, e, p_next, n);
+  pdl_launch(H3D_BOTH(k_apply, TE), (int)std::min<int64_t>((n / 2 + 255) / 256, 148 * 16), 256, 0, st, p, e, p_next, n);
   return cudaGetLastError();
 }
 
@@ -2879,10 +2895,10 @@ cudaError_t launch_defect(bool var, const BlkLev* bl, RowTab rt, const double* p
   if (rt.nrows <= 0) return cudaSuccess;
   const int g = defect_grid(rt.nrows);
   if (var)
-    pdl_launch(k_defect<TR, true>, g, 256, 0, st, bl, rt.start, rt.nb, rt.nrows, p, b, rhs_out, mean_b, rscale, fx,
+    pdl_launch(H3D_BOTH(k_defect, TR, true), g, 256, 0, st, bl, rt.start, rt.nb, rt.nrows, p, b, rhs_out, mean_b, rscale, fx,
                fy, fz, partials);
   else
-    pdl_launch(k_defect<TR, false>, g, 256, 0, st, bl, rt.start, rt.nb, rt.nrows, p, b, rhs_out, mean_b, rscale, fx,
+    pdl_launch(H3D_BOTH(k_defect, TR, false), g, 256, 0, st, bl, rt.start, rt.nb, rt.nrows, p, b, rhs_out, mean_b, rscale, fx,
                fy, fz, partials);
   return cudaGetLastError();
 }
@@ -3060,9 +3076,9 @@ template <typename T, int TPR, int CPX, int TYC>
 static cudaError_t rtile_attr() {
   const int sm = (int)rtile_smem<T, TPR, CPX, TYC>();
   cudaError_t e;
-  if ((e = cudaFuncSetAttribute(k_restrict_tile<T, true, false, TPR, CPX, TYC>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))) return e;
-  if ((e = cudaFuncSetAttribute(k_restrict_tile<T, false, false, TPR, CPX, TYC>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))) return e;
-  return cudaFuncSetAttribute(k_restrict_tile<T, false, true, TPR, CPX, TYC>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+  if ((e = kernel_smem(H3D_BOTH(k_restrict_tile, T, true, false, TPR, CPX, TYC), sm))) return e;
+  if ((e = kernel_smem(H3D_BOTH(k_restrict_tile, T, false, false, TPR, CPX, TYC), sm))) return e;
+  return kernel_smem(H3D_BOTH(k_restrict_tile, T, false, true, TPR, CPX, TYC), sm);
 }
 
 template <typename T, int TPR, int CPX, int TYC>
@@ -3071,9 +3087,10 @@ static cudaError_t rtile_dispatch(bool var, bool zero, const BlkLev* fine, const
                                   const T* fz, cudaStream_t st) {
   if (ntiles <= 0) return cudaSuccess;
   constexpr size_t SM = rtile_smem<T, TPR, CPX, TYC>();
-  if (zero) pdl_launch(k_restrict_tile<T, false, true, TPR, CPX, TYC>, ntiles, TPR * TYC, SM, st, fine, coarse, tiles, zc, phi, rhs, rhs_c, fx, fy, fz);
-  else if (var) pdl_launch(k_restrict_tile<T, true, false, TPR, CPX, TYC>, ntiles, TPR * TYC, SM, st, fine, coarse, tiles, zc, phi, rhs, rhs_c, fx, fy, fz);
-  else pdl_launch(k_restrict_tile<T, false, false, TPR, CPX, TYC>, ntiles, TPR * TYC, SM, st, fine, coarse, tiles, zc, phi, rhs, rhs_c, fx, fy, fz);
+  const long long cells = 8LL * ntiles * TYC * zc * (TPR * CPX);  // at most
+  if (zero) pdl_launch(sized(H3D_BOTH(k_restrict_tile, T, false, true, TPR, CPX, TYC), cells), ntiles, TPR * TYC, SM, st, fine, coarse, tiles, zc, phi, rhs, rhs_c, fx, fy, fz);
+  else if (var) pdl_launch(sized(H3D_BOTH(k_restrict_tile, T, true, false, TPR, CPX, TYC), cells), ntiles, TPR * TYC, SM, st, fine, coarse, tiles, zc, phi, rhs, rhs_c, fx, fy, fz);
+  else pdl_launch(sized(H3D_BOTH(k_restrict_tile, T, false, false, TPR, CPX, TYC), cells), ntiles, TPR * TYC, SM, st, fine, coarse, tiles, zc, phi, rhs, rhs_c, fx, fy, fz);
   return cudaGetLastError();
 }
 
@@ -3169,10 +3186,11 @@ template cudaError_t launch_restrict_tile<float>(int, bool, bool, const BlkLev*,
 // a device staging buffer; these kernels move the region g0 .. (extent) of
 // the canonical block (ghost layer included when g0 = 0) between staging and
 // the padded device layout.
+template <bool EARLY>
 __global__ void k_stage_scatter(const double* __restrict__ stg, int tx, int ty, int pl, int g0, int ex, int ey,
                                 int ez, double* __restrict__ dev, int sx, long long sxy) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait<EARLY>(stg);
   const long long n = (long long)ex * ey * ez;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
     const int x = (int)(e % ex), y = (int)((e / ex) % ey), z = (int)(e / ((long long)ex * ey));
@@ -3181,10 +3199,11 @@ __global__ void k_stage_scatter(const double* __restrict__ stg, int tx, int ty, 
   }
 }
 
+template <bool EARLY>
 __global__ void k_stage_gather(double* __restrict__ stg, int tx, int ty, int pl, int g0, int ex, int ey, int ez,
                                const double* __restrict__ dev, int sx, long long sxy) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait<EARLY>(dev);
   const long long n = (long long)ex * ey * ez;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
     const int x = (int)(e % ex), y = (int)((e / ex) % ey), z = (int)(e / ((long long)ex * ey));
@@ -3198,8 +3217,8 @@ cudaError_t launch_stage(bool to_device, double* stg, int tx, int ty, int pl, in
   const long long n = (long long)ex * ey * ez;
   if (n <= 0) return cudaSuccess;
   const int grid = (int)std::min<long long>((n + 255) / 256, 148LL * 16);
-  if (to_device) pdl_launch(k_stage_scatter, grid, 256, 0, st, stg, tx, ty, pl, g0, ex, ey, ez, dev, sx, sxy);
-  else pdl_launch(k_stage_gather, grid, 256, 0, st, stg, tx, ty, pl, g0, ex, ey, ez, dev, sx, sxy);
+  if (to_device) pdl_launch(KernelPair{k_stage_scatter<false>, k_stage_scatter<true>}, grid, 256, 0, st, stg, tx, ty, pl, g0, ex, ey, ez, dev, sx, sxy);
+  else pdl_launch(KernelPair{k_stage_gather<false>, k_stage_gather<true>}, grid, 256, 0, st, stg, tx, ty, pl, g0, ex, ey, ez, dev, sx, sxy);
   return cudaGetLastError();
 }
 
@@ -3218,22 +3237,22 @@ cudaError_t launch_sum_interior(const BlkLev* bl, RowTab rt, const double* a, do
   *nparts = 0;
   if (rt.nrows <= 0) return cudaSuccess;
   const int g = defect_grid(rt.nrows);
-  pdl_launch(k_sum_interior, g, 256, 0, st, bl, rt.start, rt.nb, rt.nrows, a, partials);
+  pdl_launch(KernelPair{k_sum_interior<false>, k_sum_interior<true>}, g, 256, 0, st, bl, rt.start, rt.nb, rt.nrows, a, partials);
   *nparts = g;
   return cudaGetLastError();
 }
 
 cudaError_t launch_shift(double* a, int64_t n, const double* s, double scale, cudaStream_t st) {
-  pdl_launch(k_shift, grid_for(n, 256), 256, 0, st, a, n, s, scale);
+  pdl_launch(KernelPair{k_shift<false>, k_shift<true>}, grid_for(n, 256), 256, 0, st, a, n, s, scale);
   return cudaGetLastError();
 }
 
 cudaError_t launch_convert_d2f(const double* a, float* b, int64_t n, cudaStream_t st) {
-  pdl_launch(k_d2f, grid_for(n, 256), 256, 0, st, a, b, n);
+  pdl_launch(KernelPair{k_d2f<false>, k_d2f<true>}, grid_for(n, 256), 256, 0, st, a, b, n);
   return cudaGetLastError();
 }
 cudaError_t launch_convert_f2d(const float* a, double* b, int64_t n, cudaStream_t st) {
-  pdl_launch(k_f2d, grid_for(n, 256), 256, 0, st, a, b, n);
+  pdl_launch(KernelPair{k_f2d<false>, k_f2d<true>}, grid_for(n, 256), 256, 0, st, a, b, n);
   return cudaGetLastError();
 }
 
@@ -3257,7 +3276,7 @@ __global__ void __launch_bounds__(256) k_face_coef_sum(const BlkLev* __restrict_
                                                        const double* __restrict__ ffz, double* __restrict__ cfx,
                                                        double* __restrict__ cfy, double* __restrict__ cfz) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(ffx, ffy, ffz);
   const int b = find_block(cta_start, nb, blockIdx.x);
   const BlkLev C = coarse[b];
   const BlkLev F = fine[b];
@@ -3306,7 +3325,7 @@ __device__ __forceinline__ bool interior_cell(const BlkLev* __restrict__ bls, co
 // divided by the face density 0.5*(dens(i)+dens(i+1)) for L_LSM.  Operand
 // order as written there (dtal = dt*alfapr, then *(dp), /dx, /face density).
 // h3: spacings of every block, then their reciprocals.
-template <bool LSM>
+template <bool LSM, bool EARLY>
 __global__ void __launch_bounds__(256) k_calvel(const BlkLev* __restrict__ bls, const int* __restrict__ cta_start,
                                                 int nb, int ncta, const double* __restrict__ h3,
                                                 const double* __restrict__ p, const double* __restrict__ dens,
@@ -3314,7 +3333,7 @@ __global__ void __launch_bounds__(256) k_calvel(const BlkLev* __restrict__ bls, 
                                                 const double* __restrict__ ws, double* __restrict__ u,
                                                 double* __restrict__ v, double* __restrict__ w, double dtal) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait<EARLY>(p, dens, us, vs, ws);
   for (int c = blockIdx.x; c < ncta; c += gridDim.x) {
     int b, x, y, z;
     if (!interior_cell(bls, cta_start, nb, c, &b, &x, &y, &z)) continue;
@@ -3347,7 +3366,7 @@ __global__ void __launch_bounds__(256) k_gather3(const uint32_t* __restrict__ ds
                                                  int64_t n, double* __restrict__ a0, double* __restrict__ a1,
                                                  double* __restrict__ a2) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(a0, a1, a2);
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
     const uint32_t d = dst[e], s = src[e];
     a0[d] = a0[s];
@@ -3364,14 +3383,14 @@ __global__ void __launch_bounds__(256) k_gather3(const uint32_t* __restrict__ ds
 // One thread a cell, eight CTAs an SM: a warp a row kept too few loads in
 // flight (2.6M cells: 75 us, 46 us here), and the divisions by the spacings and
 // dt are exact multiply-adds (div_known).
-template <bool LSM, typename TR>
+template <bool LSM, typename TR, bool EARLY>
 __global__ void __launch_bounds__(256) k_calmas(const BlkLev* __restrict__ bls, const int* __restrict__ cta_start,
                                                 int nb, int ncta, const double* __restrict__ h3,
                                                 const double* __restrict__ u, const double* __restrict__ v,
                                                 const double* __restrict__ w, double dt, double* __restrict__ bout,
                                                 TR* __restrict__ rhs_out, double* __restrict__ partials) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait<EARLY>(u, v, w);
   double ss = 0, rm = 0, rs = 0;
   const double idt = 1.0 / dt;
   for (int c = blockIdx.x; c < ncta; c += gridDim.x) {
@@ -3461,7 +3480,7 @@ __global__ void __launch_bounds__(512) k_sip_factor(const BlkLev* __restrict__ b
 __global__ void __launch_bounds__(512) k_sip_sweep(const BlkLev* __restrict__ bls, SipLU lu, double* __restrict__ fi_all,
                                                    const double* __restrict__ su_all, double* __restrict__ partials) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(fi_all, su_all);
   __shared__ double red[16];
   const BlkLev B = bls[blockIdx.x];
   const double *lb = lu.lb + B.off, *lw = lu.lw + B.off, *ls = lu.ls + B.off, *lpr = lu.lpr + B.off;
@@ -3514,7 +3533,7 @@ __global__ void __launch_bounds__(512) k_sip_sweep(const BlkLev* __restrict__ bl
 __global__ void __launch_bounds__(256) k_gather1(const uint32_t* __restrict__ dst, const uint32_t* __restrict__ src,
                                                  int64_t n, double* __restrict__ a) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait(a);
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x)
     a[dst[e]] = a[src[e]];
 }
@@ -3583,10 +3602,10 @@ cudaError_t launch_calvel(bool lsm, const BlkLev* bl, CellTab ct, const double* 
   if (ct.ncta <= 0) return cudaSuccess;
   const int g = ct.ncta;
   if (lsm)
-    pdl_launch(k_calvel<true>, g, 256, 0, st, bl, ct.cta_start, ct.nb, ct.ncta, h3, p, dens, us, vs, ws, u, v, w,
+    pdl_launch(H3D_BOTH(k_calvel, true), g, 256, 0, st, bl, ct.cta_start, ct.nb, ct.ncta, h3, p, dens, us, vs, ws, u, v, w,
                dtal);
   else
-    pdl_launch(k_calvel<false>, g, 256, 0, st, bl, ct.cta_start, ct.nb, ct.ncta, h3, p, dens, us, vs, ws, u, v, w,
+    pdl_launch(H3D_BOTH(k_calvel, false), g, 256, 0, st, bl, ct.cta_start, ct.nb, ct.ncta, h3, p, dens, us, vs, ws, u, v, w,
                dtal);
   return cudaGetLastError();
 }
@@ -3606,10 +3625,10 @@ cudaError_t launch_calmas(bool lsm, const BlkLev* bl, CellTab ct, const double* 
   if (ct.ncta <= 0) return cudaSuccess;
   const int g = std::min(ct.ncta, kCellCtas);
   if (lsm)
-    pdl_launch(k_calmas<true, TR>, g, 256, 0, st, bl, ct.cta_start, ct.nb, ct.ncta, h3, u, v, w, dt, bout, rhs_out,
+    pdl_launch(H3D_BOTH(k_calmas, true, TR), g, 256, 0, st, bl, ct.cta_start, ct.nb, ct.ncta, h3, u, v, w, dt, bout, rhs_out,
                partials);
   else
-    pdl_launch(k_calmas<false, TR>, g, 256, 0, st, bl, ct.cta_start, ct.nb, ct.ncta, h3, u, v, w, dt, bout, rhs_out,
+    pdl_launch(H3D_BOTH(k_calmas, false, TR), g, 256, 0, st, bl, ct.cta_start, ct.nb, ct.ncta, h3, u, v, w, dt, bout, rhs_out,
                partials);
   *nparts = g;
   return cudaGetLastError();

@@ -61,12 +61,6 @@ struct SipSkew {
   }
 };
 
-template <typename T>
-__device__ __forceinline__ void cp_async_word(T* s, const T* g) {
-  const unsigned a = (unsigned)__cvta_generic_to_shared(s);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(a), "l"(g), "n"(sizeof(T)) : "memory");
-}
-
 // One CTA's share of a march over `steps` hyperplanes: step(d, k) for its
 // active ones, in ascending (FWD) or descending order, a CTA barrier after
 // each, a cluster barrier after every phase.  prefetch(d, k) starts a thread's
@@ -334,6 +328,7 @@ __device__ __forceinline__ bool sip_cell(const BlkLev* __restrict__ bls, const i
 
 // Residual of every block (sipsol.for:146-157) into the skewed res, and the
 // CTA's sum |res| in a fixed order into partials[4 * cta].
+template <bool EARLY>
 __global__ void __launch_bounds__(256) k_sip_residual(const BlkLev* __restrict__ bls,
                                                       const long long* __restrict__ offs,
                                                       const int* __restrict__ cta_start, int nb,
@@ -341,7 +336,7 @@ __global__ void __launch_bounds__(256) k_sip_residual(const BlkLev* __restrict__
                                                       const double* __restrict__ su_all, double* __restrict__ res,
                                                       double* __restrict__ partials) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait<EARLY>(fi_all, su_all);
   __shared__ double red[8];
   int b, x, y, z;
   double acc = 0.0;
@@ -371,11 +366,12 @@ __global__ void __launch_bounds__(256) k_sip_residual(const BlkLev* __restrict__
 }
 
 // fi = fi + res (sipsol.for:176).
+template <bool EARLY>
 __global__ void __launch_bounds__(256) k_sip_correct(const BlkLev* __restrict__ bls, const long long* __restrict__ offs,
                                                      const int* __restrict__ cta_start, int nb,
                                                      double* __restrict__ fi, const double* __restrict__ res) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait<EARLY>(fi, res);
   int b, x, y, z;
   if (!sip_cell(bls, cta_start, nb, &b, &x, &y, &z)) return;
   const BlkLev& B = bls[b];
@@ -655,15 +651,17 @@ __global__ void __launch_bounds__(kTdmaThreads) k_tdma_s(const BlkLev* __restric
   T* D = reinterpret_cast<T*>(tdma_smem);
   T* R = D + (size_t)sxy * (B.nz + 2);
   T* tab = R + (size_t)sxy * (B.nz + 2);
-  pdl_wait();
+  pdl_wait(src, rhs);
   const int ex = B.nx + 2, ey = B.ny + 2, ncell = ex * ey * (B.nz + 2);
   for (int q = threadIdx.x; q < ncell; q += blockDim.x) {
     const int x = q % ex, y = (q / ex) % ey, z = q / (ex * ey);
     const long long i = B.off + (long long)z * B.sxy + (long long)y * B.sx + x;
     const int o = z * sxy + y * sx + x;
-    D[o] = zero ? T(0) : src[i];
-    R[o] = rhs[i];
+    if (zero) D[o] = T(0);
+    else cp_async_word(D + o, src + i);
+    cp_async_word(R + o, rhs + i);
   }
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
   __syncthreads();
   tdma_s_pass<T, 1>(B, D, R, tab);
   tdma_s_pass<T, 0>(B, D, R, tab);
@@ -691,13 +689,13 @@ __device__ __forceinline__ long long tdma_at(const BlkLev& B, int x, int y, int 
 // Rearranges the iterate and the right-hand side of every block for the pass
 // along AXIS: from the level (FROM < 0; zero: the zero iterate) or from the rows of
 // the pass along FROM.  256 cells a CTA, ghosts included.
-template <typename T, int FROM, int AXIS>
+template <typename T, int FROM, int AXIS, bool EARLY>
 __global__ void __launch_bounds__(256) k_tdma_rows(const BlkLev* __restrict__ bls, const int* __restrict__ cta_start,
                                                    int nb, const T* __restrict__ src, const T* __restrict__ rhs,
                                                    const T* __restrict__ from, T* __restrict__ to,
                                                    T* __restrict__ rows, long long words, bool zero) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait<EARLY>(src, rhs, from);
   const int b = find_block(cta_start, nb, blockIdx.x);
   const BlkLev& B = bls[b];
   const int ex = B.nx + 2, ey = B.ny + 2, q = (blockIdx.x - cta_start[b]) * blockDim.x + threadIdx.x;
@@ -711,12 +709,12 @@ __global__ void __launch_bounds__(256) k_tdma_rows(const BlkLev* __restrict__ bl
 }
 
 // The rows of the last pass (along z) back into the level.
-template <typename T>
+template <typename T, bool EARLY>
 __global__ void __launch_bounds__(256) k_tdma_level(const BlkLev* __restrict__ bls, const int* __restrict__ cta_start,
                                                     int nb, const T* __restrict__ from, T* __restrict__ dst,
                                                     long long words) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait<EARLY>(from);
   const int b = find_block(cta_start, nb, blockIdx.x);
   const BlkLev& B = bls[b];
   const int ex = B.nx + 2, ey = B.ny + 2, q = (blockIdx.x - cta_start[b]) * blockDim.x + threadIdx.x;
@@ -860,13 +858,13 @@ cudaError_t launch_sip_sweep_c(const SipPlan& P, const BlkLev* bl, const long lo
                              double* fi, const double* su, double* partials, cudaStream_t st) {
   if (interior.nb <= 0) return cudaSuccess;
   SipLU lu{a.lb, a.lw, a.ls, a.lpr, a.un, a.ue, a.ut, a.res};
-  pdl_launch(k_sip_residual, interior.ncta, 256, 0, st, bl, offs, interior.cta_start, interior.nb, fi, su, a.res,
+  pdl_launch(KernelPair{k_sip_residual<false>, k_sip_residual<true>}, interior.ncta, 256, 0, st, bl, offs, interior.cta_start, interior.nb, fi, su, a.res,
              partials);
   const int nb = interior.nb;
   cudaError_t e = P.one ? cluster_launch(k_sip_subst<true>, nb, P.ctas, kSipThreads, P.smem_subst, st, bl, offs, lu)
                         : cluster_launch(k_sip_subst<false>, nb, P.ctas, kSipThreads, P.smem_subst, st, bl, offs, lu);
   if (e != cudaSuccess) return e;
-  pdl_launch(k_sip_correct, interior.ncta, 256, 0, st, bl, offs, interior.cta_start, interior.nb, fi, a.res);
+  pdl_launch(KernelPair{k_sip_correct<false>, k_sip_correct<true>}, interior.ncta, 256, 0, st, bl, offs, interior.cta_start, interior.nb, fi, a.res);
   return cudaGetLastError();
 }
 
@@ -914,13 +912,13 @@ cudaError_t launch_tdma(const TdmaPlan& P, bool zero, const BlkLev* bl, CellTab 
   const long long w = P.words;
   const size_t sm = (size_t)P.smem;
   T *a = scratch, *b = a + nb * w, *rows = b + nb * w;
-  pdl_launch(k_tdma_rows<T, -1, 1>, all.ncta, 256, 0, st, bl, all.cta_start, nb, src, rhs, b, a, rows, w, zero);
+  pdl_launch(H3D_BOTH(k_tdma_rows, T, -1, 1), all.ncta, 256, 0, st, bl, all.cta_start, nb, src, rhs, b, a, rows, w, zero);
   pdl_launch(k_tdma_g<T, 1>, nb, kTdmaThreads, sm, st, bl, a, rows, w, P.nbuf);
-  pdl_launch(k_tdma_rows<T, 1, 0>, all.ncta, 256, 0, st, bl, all.cta_start, nb, src, rhs, a, b, rows, w, zero);
+  pdl_launch(H3D_BOTH(k_tdma_rows, T, 1, 0), all.ncta, 256, 0, st, bl, all.cta_start, nb, src, rhs, a, b, rows, w, zero);
   pdl_launch(k_tdma_g<T, 0>, nb, kTdmaThreads, sm, st, bl, b, rows, w, P.nbuf);
-  pdl_launch(k_tdma_rows<T, 0, 2>, all.ncta, 256, 0, st, bl, all.cta_start, nb, src, rhs, b, a, rows, w, zero);
+  pdl_launch(H3D_BOTH(k_tdma_rows, T, 0, 2), all.ncta, 256, 0, st, bl, all.cta_start, nb, src, rhs, b, a, rows, w, zero);
   pdl_launch(k_tdma_g<T, 2>, nb, kTdmaThreads, sm, st, bl, a, rows, w, P.nbuf);
-  pdl_launch(k_tdma_level<T>, all.ncta, 256, 0, st, bl, all.cta_start, nb, a, dst, w);
+  pdl_launch(H3D_BOTH(k_tdma_level, T), all.ncta, 256, 0, st, bl, all.cta_start, nb, a, dst, w);
   return cudaGetLastError();
 }
 template cudaError_t launch_tdma<double>(const TdmaPlan&, bool, const BlkLev*, CellTab, const double*, double*,

@@ -20,7 +20,7 @@ namespace {
 constexpr int kDefectVarThreads = 256;
 __device__ __forceinline__ double2 ld2(const double* p) { return *reinterpret_cast<const double2*>(p); }
 
-template <typename TR>
+template <typename TR, bool EARLY>
 __global__ void __launch_bounds__(kDefectVarThreads) k_defect_var(
     const BlkLev* __restrict__ bls, const Tile* __restrict__ tiles, int zc, const double* __restrict__ p,
     const double* __restrict__ bvec, TR* __restrict__ rhs_out, double mean_b, double rscale,
@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(kDefectVarThreads) k_defect_var(
     double2 ps, pn, b, fx, fy, fs, fz;
     double pw, pe, fw;
   };
-  pdl_wait();
+  pdl_wait<EARLY>(p, bvec);
   if (in) {
     const long long r0 = B.off + (long long)y * sx + x0;
     auto load = [&](int z, Plane& q) {
@@ -105,7 +105,7 @@ cudaError_t launch_defect_var(const BlkLev* bl, const Tile* tiles, int ntiles, i
                               const double* b, TR* rhs_out, double mean_b, double rscale, const double* fx,
                               const double* fy, const double* fz, double* partials, cudaStream_t st) {
   if (ntiles <= 0) return cudaSuccess;
-  pdl_launch(k_defect_var<TR>, ntiles, kDefectVarThreads, 0, st, bl, tiles, zc, p, b, rhs_out, mean_b, rscale, fx,
+  pdl_launch(H3D_BOTH(k_defect_var, TR), ntiles, kDefectVarThreads, 0, st, bl, tiles, zc, p, b, rhs_out, mean_b, rscale, fx,
              fy, fz, partials);
   return cudaGetLastError();
 }
