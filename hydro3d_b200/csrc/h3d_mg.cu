@@ -680,7 +680,8 @@ struct Exec {
   }
 
   // live_next: the visit's next reader of level g is a restriction from it or
-  // another sweep of it (they read the live ghosts only)
+  // another sweep of it (they read the live ghosts only), and a sweep with the whole
+  // fill comes before its next correction or prolongation is read
   int relax(int g, int it, bool live_next = false) {
     Level& V = L(g);
     if (it > 0 && V.small && g > 1 && h->desc.mg_itrsch == 3) {  // all sweeps and fills of this visit in one launch
@@ -872,7 +873,10 @@ struct Exec {
       TRY(relax(1, irestr));
       return relax(1, iproln);
     }
-    TRY(relax(1, irestr, true));
+    // the sweeps after the correction fill every ghost; without any (iproln = 0) the
+    // correction, which reads edges and corners too, follows the pre-smoothing's fill
+    const bool later = iproln > 0;
+    TRY(relax(1, irestr, later));
     TRY(restrict_to(2));
     int kount[kMaxLevels + 2] = {0};
     int g = 2, nrel = irestr;
@@ -886,7 +890,7 @@ struct Exec {
         continue;
       }
       kount[g] += 1;
-      TRY(relax_at(g, nrel, true, kount[g] != 2 && g < Lv));
+      TRY(relax_at(g, nrel, true, later && kount[g] != 2 && g < Lv));
       if (kount[g] == 2) {
         TRY(correct(g - 1));
         kount[g] = 0;
