@@ -96,7 +96,7 @@ struct Level {
   int nqtiles = 0;
   Tile* d_dtiles = nullptr;       // level 1: z-march defect tiles (defect_march_rows() rows x dzc planes)
   int ndtiles = 0, dzc = 1, dgp = 0;  // dgp: pairs per lane of the z-march defect (0: not usable)
-  int* d_dstart = nullptr;        // level 1: first z-march defect tile of each block (nb + 1 entries)
+  int* d_dstart = nullptr;        // level 1, constant coefficients: first z-march defect tile of each block (nb + 1 entries)
   int* d_pstart = nullptr;        // level 1: first tiled-defect tile of each block (nb + 1 entries)
   bool pvec32 = false, pvec64 = false;  // every block's nx a multiple of 4 (FP32) / 2 (FP64) cells, ny and nz even
   int nrtiles = 0, rvariant = 0, rzc = 1;
@@ -967,8 +967,9 @@ struct Exec {
     h->kernels += 2;
     if (h->per_block && h->blocks.size() > 1) {
       // the march and tiled defects write one partial per tile, tiles grouped by block
+      // (independent blocks of variable density are not a case of the per-block rule)
       const int* start = march ? V.d_dstart : tiled ? V.d_pstart : nullptr;
-      if (!start) return fail(h, H3D_ERR_BAD_CONFIG, "per-block stop rule: the defect of this layout has no per-block partial sums");
+      if (!start) return fail(h, H3D_ERR_BAD_CONFIG, "per-block stop rule: needs constant coefficients and even nx in every block");
       const int nb = (int)h->blocks.size();
       CU(launch_reduce4_blocks(h->partials, start, nb, h->d_resb, h->st));
       TRY(chk("reduce per block", 1));
@@ -2845,7 +2846,7 @@ int h3d_mg_create(h3d_mg** out, const h3d_mg_desc* desc) {
         if (cudaMemcpy(V.d_dtiles, dt.data(), dt.size() * sizeof(Tile), cudaMemcpyHostToDevice) != cudaSuccess)
           return bail(fail(h, H3D_ERR_CUDA, "defect tiles"));
         V.ndtiles = (int)dt.size();
-        if ((rc = upload_tile_starts(h, dt, (int)V.geom.bl.size(), &V.d_dstart)) != H3D_OK) return bail(rc);
+        if (!h->var && (rc = upload_tile_starts(h, dt, (int)V.geom.bl.size(), &V.d_dstart)) != H3D_OK) return bail(rc);
       }
     }
     if ((rc = build_tensor_maps(h, g)) != H3D_OK) return bail(rc);

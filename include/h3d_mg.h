@@ -98,7 +98,8 @@ typedef struct h3d_solve_opts {
   int32_t stop_rule;      /* 0: ||b-Ap||2/||b||2 <= tol, checked before each cycle;
                              1: reference rule rmax < tol .and. iter > 1 (newsolv_mg.for:57);
                              2: every block's own ||b-Ap||2/||b||2 <= tol (independent
-                                blocks; needs even nx in every block) */
+                                blocks; needs constant coefficients and even nx in
+                                every block) */
   int32_t remove_mean;    /* 1: subtract the FP64 mean of p at the end (all-Neumann) */
   int32_t record_history; /* 1: keep ||r||/||b|| per cycle (read with h3d_mg_history) */
 } h3d_solve_opts;
