@@ -174,7 +174,8 @@ struct h3d_mg {
   std::map<std::vector<int>, CachedGraph> graphs;
   bool capturing = false;
   bool solving = false;     // inside a solve (its FP64 sweeps fill the live ghosts only)
-  bool unclean = true;      // some level array may hold a NaN or infinity, which a ghost left unfilled would keep
+  bool unclean = true;      // some level array may hold a NaN or infinity, which a ghost left unfilled would keep:
+                            // set but after a solve that came to a finite residual without an error
   bool debug_sync = false;  // H3D_DEBUG_SYNC=1: synchronize and check after every launch
   std::vector<double> history;
   // whole host block arrays staged on the device (0: pressure, 1: rhs) for
@@ -1158,15 +1159,21 @@ int run_iteration(h3d_mg* h, int inner, double* prof_ms, int64_t* prof_n, double
 }
 
 // A solve leaves the ghosts of physical walls unfilled between its sweeps (live
-// fills): they must be finite.  Clears the level iterates after calls that may
-// have put anything there; a solve that ends with a finite residual leaves them
-// finite.
+// fills): they must be finite.  begin, before the first cycle, clears the level
+// iterates after calls that may have put anything there; only a solve that ends
+// with a finite residual and without an error leaves them finite (end).  Every other
+// way out leaves the handle unclean.
 struct SolveScope {
   h3d_mg* h;
+  bool begun = false;
   explicit SolveScope(h3d_mg* h_) : h(h_) { h->solving = true; }
   ~SolveScope() { h->solving = false; }
   int begin() {
-    if (!h->unclean) return H3D_OK;
+    if (begun) return H3D_OK;
+    begun = true;
+    const bool clear = h->unclean;
+    h->unclean = true;
+    if (!clear) return H3D_OK;
     for (int g = 1; g <= h->L; ++g) {
       Level& V = h->lev[g];
       for (int q = 0; q < 2; ++q) {
@@ -1175,8 +1182,10 @@ struct SolveScope {
         if (V.phi32[q]) CU(cudaMemsetAsync(V.phi32[q], 0, n * sizeof(float), h->st));
       }
     }
-    h->unclean = false;
     return H3D_OK;
+  }
+  void end() {
+    if (begun) h->unclean = false;
   }
 };
 
@@ -3014,7 +3023,6 @@ int h3d_mg_solve_resident(h3d_mg* h, const h3d_solve_opts* opts, h3d_solve_info*
   } pb_guard{h};
   h->per_block = opts->stop_rule == 2 && nb > 1;
   SolveScope scope(h);
-  TRY(scope.begin());
   h3d_solve_info I{};
   const int maxcy = opts->maxcy > 0 ? opts->maxcy : h->desc.maxcy;
   const int inner = h->mixed ? h->desc.inner_cycles : 1;
@@ -3072,6 +3080,7 @@ int h3d_mg_solve_resident(h3d_mg* h, const h3d_solve_opts* opts, h3d_solve_info*
   double prof_ms = 0, prof_bytes = 0;
   int64_t prof_n = 0;
   while (status != 0 && iter < maxcy) {
+    TRY(scope.begin());
     TRY(run_iteration(h, inner, &prof_ms, &prof_n, &prof_bytes));
     iter += 1;
     I.cycles += inner;
@@ -3079,7 +3088,7 @@ int h3d_mg_solve_resident(h3d_mg* h, const h3d_solve_opts* opts, h3d_solve_info*
     rinf = h->h_res[2];
     relb = block_max();
     if (opts->record_history) h->history.push_back(opts->stop_rule == 2 ? relb : rel);
-    if (!std::isfinite(rel) || rel > 1e8 || !std::isfinite(relb)) { status = 2; h->unclean = true; break; }
+    if (!std::isfinite(rel) || rel > 1e8 || !std::isfinite(relb)) { status = 2; break; }
     if (opts->stop_rule == 0 && rel <= opts->tol) status = 0;
     if (opts->stop_rule == 1 && rinf < opts->tol && iter > 1) status = 0;  // newsolv_mg.for:57
     if (opts->stop_rule == 2 && relb <= opts->tol) status = 0;
@@ -3109,6 +3118,7 @@ int h3d_mg_solve_resident(h3d_mg* h, const h3d_solve_opts* opts, h3d_solve_info*
   I.kernel_launches = h->kernels - k0;
   if (info) *info = I;
   TRY(check_device_error(h));
+  if (status != 2) scope.end();
   if (status == 2) return fail(h, H3D_ERR_DIVERGED, "residual is not finite or grew beyond 1e8");
   if (status != 0) return fail(h, H3D_ERR_NOT_CONVERGED, "not converged within maxcy cycles");
   return H3D_OK;
@@ -3444,7 +3454,6 @@ int h3d_mg_project_resident(h3d_mg* h, double dt, double alfapr, const h3d_solve
   h->proj = true;
   h->per_block = false;
   SolveScope scope(h);
-  TRY(scope.begin());
   h3d_solve_info I{};
   const int maxcy = opts->maxcy > 0 ? opts->maxcy : h->desc.maxcy;
   const int inner = h->mixed ? h->desc.inner_cycles : 1;
@@ -3466,13 +3475,14 @@ int h3d_mg_project_resident(h3d_mg* h, double dt, double alfapr, const h3d_solve
   double prof_ms = 0, prof_bytes = 0;
   int64_t prof_n = 0;
   while (status != 0 && iter < maxcy) {
+    TRY(scope.begin());
     TRY(run_iteration(h, inner, &prof_ms, &prof_n, &prof_bytes));
     iter += 1;
     I.cycles += inner;
     rel = std::sqrt(h->h_res[0]) / bn;
     rmax = h->h_res[2];
     if (opts->record_history) h->history.push_back(opts->stop_rule == 1 ? rmax : rel);
-    if (!std::isfinite(rel) || !std::isfinite(rmax) || rel > 1e8) { status = 2; h->unclean = true; break; }
+    if (!std::isfinite(rel) || !std::isfinite(rmax) || rel > 1e8) { status = 2; break; }
     if (opts->stop_rule == 0 && rel <= opts->tol) status = 0;
     if (opts->stop_rule == 1 && rmax < opts->tol && iter > 1) status = 0;  // newsolv_mg.for:57
   }
@@ -3494,6 +3504,7 @@ int h3d_mg_project_resident(h3d_mg* h, double dt, double alfapr, const h3d_solve
   I.kernel_launches = h->kernels - k0;
   if (info) *info = I;
   TRY(check_device_error(h));
+  if (status != 2) scope.end();
   if (status == 2) return fail(h, H3D_ERR_DIVERGED, "divergence not finite or rmax above 10");
   if (status != 0) return fail(h, H3D_ERR_NOT_CONVERGED, "not converged within maxcy cycles");
   return H3D_OK;

@@ -74,3 +74,20 @@ def test_solve_after_divergence(oracle_mod, h3d):
         p, _ = _solve(h3d, s, blocks, b, 2)
         assert np.array_equal(h3d.interior(p[0], blocks[0]), ref["p"][0][1:-1, 1:-1, 1:-1]), how
     s.close()
+
+
+def test_solve_without_a_cycle_leaves_the_levels(oracle_mod, h3d):
+    """Level iterates are cleared for the live fills before the first cycle: a solve that
+    needs none changes nothing, and the cycle after it starts from what was put there."""
+    blocks, s, orc, b = _pair(oracle_mod, h3d, (1, 1, 1), (16, 24, 16), [W] * 6, 3)
+    nz, ny, nx = s.level_dims(1, 0)
+    phi = np.random.default_rng(5).standard_normal((nz + 2, ny + 2, nx + 2))
+    s.put_level(1, "phi", 0, phi)
+    s.zero_field("p")
+    s.zero_field("b")
+    assert s.solve_resident(tol=1e-8)["outer"] == 0
+    assert np.array_equal(s.get_level(1, "phi", 0), phi)
+    ref = orc.solve([np.zeros((nz + 2, ny + 2, nx + 2))], b, tol=0.0, maxcy=2)
+    p, _ = _solve(h3d, s, blocks, b, 2)
+    assert np.array_equal(h3d.interior(p[0], blocks[0]), ref["p"][0][1:-1, 1:-1, 1:-1])
+    s.close()
