@@ -886,11 +886,11 @@ cudaError_t coarse_tail_attributes() {
   return cudaFuncSetAttribute(k_coarse_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
 }
 
-static cudaError_t cluster_config(int nb, int smem_bytes, cudaStream_t st, cudaLaunchConfig_t* cfg,
+static cudaError_t cluster_config(int nb, int threads, int smem_bytes, cudaStream_t st, cudaLaunchConfig_t* cfg,
                                   cudaLaunchAttribute* at) {
   *cfg = cudaLaunchConfig_t{};
   cfg->gridDim = dim3(nb);
-  cfg->blockDim = dim3(kClusterTailThreads);
+  cfg->blockDim = dim3(threads);
   cfg->dynamicSmemBytes = (size_t)smem_bytes;
   cfg->stream = st;
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -904,10 +904,10 @@ static cudaError_t cluster_config(int nb, int smem_bytes, cudaStream_t st, cudaL
   return cudaSuccess;
 }
 
-int coarse_cluster_fits(int nb, int smem_bytes) {
+int coarse_cluster_fits(int nb, int threads, int smem_bytes) {
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at[2];
-  cluster_config(nb, smem_bytes, nullptr, &cfg, at);
+  cluster_config(nb, threads, smem_bytes, nullptr, &cfg, at);
   int n = 0;
   if (cudaOccupancyMaxActiveClusters(&n, k_coarse_cluster, &cfg) != cudaSuccess) {
     cudaGetLastError();
@@ -916,12 +916,12 @@ int coarse_cluster_fits(int nb, int smem_bytes) {
   return n;
 }
 
-cudaError_t launch_coarse_cluster(int nb, const TailLevel* lv, int nlev, const TailOp* ops, int nops,
+cudaError_t launch_coarse_cluster(int nb, int threads, const TailLevel* lv, int nlev, const TailOp* ops, int nops,
                                   const uint4* tables, unsigned curmask, int smem_bytes, cudaStream_t st) {
   if (nops <= 0 || nops > kClusterTailMaxOps || nlev > kTailMaxLevels) return cudaErrorInvalidValue;
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at[2];
-  cluster_config(nb, smem_bytes, st, &cfg, at);
+  cluster_config(nb, threads, smem_bytes, st, &cfg, at);
   cfg.numAttrs = pdl_mode() == 0 ? 1 : 2;  // (its tables are staged while the predecessor finishes)
   g_prev_grid = nb;
   return cudaLaunchKernelEx(&cfg, k_coarse_cluster, lv, ops, tables, nops, nlev, curmask);

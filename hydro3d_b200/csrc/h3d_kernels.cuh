@@ -152,12 +152,12 @@ cudaError_t launch_coarse_tail(const TailLevel* lv, const TailOp* ops, int nops,
                                cudaStream_t st);
 // The same program as one cluster of nb CTAs (nb <= 16), CTA b holding block b
 // of every tail level (all blocks of a level the same size).
-constexpr int kClusterTailThreads = 1024;
+constexpr int kClusterTailThreads = 1024;  // at most
 constexpr int kClusterTailMaxBlocks = 16;
-int coarse_cluster_fits(int nb, int smem_bytes);  // clusters that can be resident at once (0: none)
+int coarse_cluster_fits(int nb, int threads, int smem_bytes);  // clusters that can be resident at once (0: none)
 constexpr int kClusterTailMaxOps = 160;
 // tables: every block's staged tables, back to back.
-cudaError_t launch_coarse_cluster(int nb, const TailLevel* lv, int nlev, const TailOp* ops, int nops,
+cudaError_t launch_coarse_cluster(int nb, int threads, const TailLevel* lv, int nlev, const TailOp* ops, int nops,
                                   const uint4* tables, unsigned curmask, int smem_bytes, cudaStream_t st);
 
 // First red-black sweep from a zero iterate of an FP32 constant-coefficient

@@ -192,6 +192,7 @@ struct h3d_mg {
   BlkLev* d_tail_cbl = nullptr;                // compact block tables of the tail levels
   int* d_tail_starts = nullptr;                // cluster tail: per-block fill ranges
   int tail_cluster = 0;                        // cluster tail: CTAs of the cluster (0: single-CTA tail)
+  int tail_threads = 0;                        // ... and threads of a CTA
   int tail_nlev = 0;
   uint32_t* d_tail_fills = nullptr;            // compact sweep fill tables of the tail levels
   double* d_dense = nullptr;                   // pseudo-inverse of the coarsest level (coarse_direct)
@@ -846,7 +847,7 @@ struct Exec {
       mask |= (unsigned)(V.cur64 & 1) << (2 * (g - g0) + 1);
     }
     if (h->tail_cluster)
-      CU(launch_coarse_cluster(h->tail_cluster, h->d_tail_lv, h->tail_nlev, h->d_tail_ops, h->tail_nops,
+      CU(launch_coarse_cluster(h->tail_cluster, h->tail_threads, h->d_tail_lv, h->tail_nlev, h->d_tail_ops, h->tail_nops,
                                h->d_tail_tables, mask, h->tail_smem, h->st));
     else
       CU(launch_coarse_tail(h->d_tail_lv, h->d_tail_ops, h->tail_nops, mask, h->tail_smem, h->st));
@@ -2102,6 +2103,15 @@ int build_tail(h3d_mg* h) {
   return H3D_OK;
 }
 
+// The largest blocks of a level that joins a cluster tail of two levels or more.  A
+// block is one CTA's work there, and the whole chip's outside it.  us a cycle
+// with the level in and out: FP32 16^3, 4 blocks 89 and 91, 12 blocks 133 and
+// 139; 24 x 16 x 16, 4 blocks 130 and 130, 12 blocks 150 and 139; 20^3, 4 blocks 137 and
+// 130; FP64 20 x 16 x 16, 4 blocks 113 and 101.  One FP32 block alone: 24 x 16 x 16 80 and
+// 86, 20^3 88 and 93, 24 x 20 x 20 97 and 95.  (As the second level, without which nothing
+// is fused, any that fits: 24 x 20 x 18, 4 blocks: 150 and 224.)
+constexpr int kClusterJoin = 4096, kClusterJoinAlone = 8192;
+
 // The fused coarse tail as one cluster of CTAs, CTA b holding block b of
 // every tail level: the deepest run of levels g..L (g >= 2, at least two
 // levels) whose blocks are all the same size at each level and whose arrays,
@@ -2281,6 +2291,7 @@ int build_cluster_tail(h3d_mg* h) {
     bool same = true;
     for (const auto& B : V.geom.bl) same = same && B.nx == B0.nx && B.ny == B0.ny && B.nz == B0.nz;
     if (!same || B0.nx + 1 > 255 || B0.ny + 1 > 255 || B0.nz + 1 > 255) break;
+    if (g0 < Lv && B0.nx * B0.ny * B0.nz > (nb == 1 && f32_level(h, g) ? kClusterJoinAlone : kClusterJoin)) break;
     // arena with levels g..L (one block each) plus the ghost scratch of the fine levels
     std::vector<Lay> L2;
     int at = 0, scratch = 0;
@@ -2315,7 +2326,16 @@ int build_cluster_tail(h3d_mg* h) {
     scratch_at = at;
   }
   if (g0 > Lv - 1 || Lv - g0 + 1 > kTailMaxLevels) return H3D_OK;
-  if (coarse_cluster_fits(nb, bytes) < 1) return H3D_OK;
+  // threads of a CTA: every barrier costs more with more warps (12 blocks of 48^3, 32
+  // sweeps of the coarsest level: 70 us a launch with 512, 76 with 1024); 1024 where
+  // the coarsest level has more than 512 cells a colour (12 x 10 x 9, two blocks: 163 and
+  // 150 us a cycle) or a block is alone with such a level (64^3 FP64: 36.1 and 33.8 us)
+  auto colour = [&](int q) {
+    const BlkLev& B = h->lev[q].geom.bl[0];
+    return (B.nx * B.ny * B.nz + 1) / 2;
+  };
+  const int threads = colour(Lv) > 512 || (nb == 1 && colour(g0) > 512) ? kClusterTailThreads : 512;
+  if (coarse_cluster_fits(nb, threads, bytes) < 1) return H3D_OK;
   std::vector<TailOp> ops;
   std::vector<char> z32, z64;
   TRY(build_dense_coarse(h));
@@ -2456,6 +2476,7 @@ int build_cluster_tail(h3d_mg* h) {
   h->tail_zero64.assign(z64.begin() + g0, z64.begin() + Lv + 1);
   h->tail_g = g0;
   h->tail_cluster = nb;
+  h->tail_threads = threads;
   return H3D_OK;
 }
 

@@ -55,6 +55,8 @@ def test_periodic_block_visit_bitexact(oracle_mod, h3d, bc):
     ((1, 1, 1), (16, 32, 24), [W] * 6),
     ((2, 2, 1), (20, 24, 24), [P, P, W, W, W, W]),
     ((3, 1, 2), (24, 24, 56), [W] * 6),
+    ((2, 1, 1), (40, 32, 32), [P, P, W, W, W, W]),  # the second level is above the size that joins two
+    ((1, 1, 1), (40, 32, 32), [W] * 6),             # the same alone: 1024 threads
 ])
 def test_cluster_many_sweeps_bitexact(oracle_mod, h3d, nblk, n, bc):
     """A V-cycle whose coarsest level takes 12 sweeps: the cluster keeps its cells in
@@ -83,3 +85,36 @@ def test_cluster_many_sweeps_bitexact(oracle_mod, h3d, nblk, n, bc):
             a, b = s.get_level(1, "phi", ib), orc.get_phi(1, ib)
             assert np.array_equal(a, b), (sweeps, ib, float(np.abs(a - b).max()))
         s.close()
+
+
+@pytest.mark.parametrize("nblk", [(1, 1, 1), (2, 1, 1)])
+def test_mixed_cluster_large_coarsest_level(h3d, nblk):
+    """FP32 blocks of 24 x 20 x 18 over an FP64 coarsest level of 540 cells a colour (1024 threads, a
+    pass a colour), swept 12 times: the cycle through the level entry points, whose FP32
+    updates round in another order (2e-5: test_gpu_parity's bound for FP32 sweeps)."""
+    blocks = h3d.topology.block_grid(nblk, (48, 40, 36), [W] * 6, [1.0 / 32] * 3, 3)
+    rng = np.random.default_rng(10)
+    phi = [rng.standard_normal((d.n[2] + 2, d.n[1] + 2, d.n[0] + 2)) for d in blocks]
+    rhs = [rng.standard_normal((d.n[2], d.n[1], d.n[0])) for d in blocks]
+    out = []
+    for whole in (True, False):
+        s = h3d.MultigridSolver(blocks, 3, precision="mixed", coarse_sweeps=12)
+        for ib in range(len(blocks)):
+            s.put_level(1, "phi", ib, phi[ib])
+            s.put_level(1, "rhs", ib, rhs[ib])
+        if whole:
+            s.vcycle()
+        else:
+            s.mgrelax(1, 2)
+            s.mgrestr(2)
+            s.mgrelax(2, 2)
+            s.mgrestr(3)
+            s.mgrelax(3, 12)
+            s.mgcorr(2)
+            s.mgrelax(2, 1)
+            s.mgcorr(1)
+            s.mgrelax(1, 1)
+        out.append([s.get_level(1, "phi", ib) for ib in range(len(blocks))])
+        s.close()
+    for a, b in zip(*out):
+        np.testing.assert_allclose(a, b, rtol=2e-5, atol=2e-5 * np.abs(b).max())
