@@ -25,9 +25,10 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 // kept their mean in up to a third of the calls.)  The wait therefore takes the
 // pointers to data that predecessors write and makes them opaque; tables written
 // once at set-up are left out.  Plain loads are not moved ahead of stores and
-// barriers either, which costs the large streaming kernels (the variable-density solve
-// of 256^3: 20.6 ms, 25.6 ms), and large launches gain nothing from starting early:
-// those kernels are built in two forms, EARLY with opaque pointers and one without.
+// barriers either, which costs the large streaming kernels (every kernel in this form:
+// 192^3 in FP64 9.74 -> 9.99 ms, 256^3 of variable density 20.6 -> 25.6 ms), and
+// large launches do not start early: those kernels are built in two forms, EARLY
+// with opaque pointers and one without.
 template <typename Ptr>
 __device__ __forceinline__ void make_opaque(Ptr& p) {
   asm volatile("" : "+l"(p));
@@ -38,7 +39,7 @@ __device__ __forceinline__ void pdl_wait(Ptr&... written) {
   if constexpr (EARLY) (make_opaque(written), ...);
 }
 
-// Launch policy (H3D_PDL): "1" every kernel, "0" none; by default only a
+// Launch policy (H3D_PDL): "1" every pdl_launch, "0" none; by default only a
 // kernel of at most kPdlGrid CTAs that follows one of at most kPdlGrid CTAs
 // on the same host thread.  Such a predecessor runs in a single wave, so the
 // early-launched grid only takes SM slots that the predecessor leaves idle,
@@ -56,15 +57,10 @@ inline int pdl_mode() {
 }
 inline thread_local long long g_prev_grid = 1LL << 40;
 
-// Tile kernels of few CTAs may still run for 100 us (256^3 cells in one block): from
-// this many cells on they do not start early (the early forms of the
-// variable-density sweep and restriction: 21.5 ms a solve of 256^3, 20.6 ms without).
-constexpr long long kPdlCells = 1LL << 20;
-
 // The next launch of this host thread, of n CTAs: does it start early?
-inline bool pdl_early(long long n, long long cells = 0) {
+inline bool pdl_early(long long n) {
   const int mode = pdl_mode();
-  const bool early = mode == 1 || (mode == 2 && n <= kPdlGrid && g_prev_grid <= kPdlGrid && cells < kPdlCells);
+  const bool early = mode == 1 || (mode == 2 && n <= kPdlGrid && g_prev_grid <= kPdlGrid);
   g_prev_grid = n;
   return early;
 }
@@ -91,12 +87,21 @@ inline cudaError_t pdl_launch(void (*k)(KArgs...), dim3 grid, dim3 block, size_t
   return launch_kernel(k, pdl_early((long long)grid.x * grid.y * grid.z), grid, block, smem, st, args...);
 }
 
+// Never early, with pdl_wait<false>: the sweep and the restriction that stage planes by
+// plain loads between barriers (variable density, 88 x 88 x 104 cells: 291 us a cycle,
+// 345 early; 64^3 176, 199), and sequential kernels that run for long on few CTAs.
+template <typename... KArgs, typename... Args>
+inline cudaError_t plain_launch(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                Args... args) {
+  g_prev_grid = (long long)grid.x * grid.y * grid.z;
+  return launch_kernel(k, false, grid, block, smem, st, args...);
+}
+
 // The two forms of a kernel (see pdl_wait); H3D_BOTH(k, a, b): those of k<a, b, EARLY>.
 template <typename... KArgs>
 struct KernelPair {
   void (*plain)(KArgs...);
   void (*early)(KArgs...);
-  long long cells = 0;  // of a tile kernel's launch
 };
 template <typename... KArgs>
 KernelPair(void (*)(KArgs...), void (*)(KArgs...)) -> KernelPair<KArgs...>;
@@ -105,20 +110,8 @@ KernelPair(void (*)(KArgs...), void (*)(KArgs...)) -> KernelPair<KArgs...>;
 template <typename... KArgs, typename... Args>
 inline cudaError_t pdl_launch(KernelPair<KArgs...> k, dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                               Args... args) {
-  const bool early = pdl_early((long long)grid.x * grid.y * grid.z, k.cells);
+  const bool early = pdl_early((long long)grid.x * grid.y * grid.z);
   return launch_kernel(early ? k.early : k.plain, early, grid, block, smem, st, args...);
-}
-
-template <typename... KArgs>
-inline KernelPair<KArgs...> sized(KernelPair<KArgs...> k, long long cells) {
-  k.cells = cells;
-  return k;
-}
-
-template <typename... KArgs>
-inline cudaError_t kernel_smem(KernelPair<KArgs...> k, int bytes) {
-  cudaError_t e = cudaFuncSetAttribute(k.plain, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  return e != cudaSuccess ? e : cudaFuncSetAttribute(k.early, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
 __device__ __forceinline__ int find_block(const int* __restrict__ start, int nb, int cta) {

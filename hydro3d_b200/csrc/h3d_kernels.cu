@@ -331,10 +331,19 @@ template <typename T>
 __device__ __forceinline__ void copy_block(const BlkLev& B, const T* __restrict__ S, T* __restrict__ D, bool zero) {
   const int ex = B.nx + 2, ey = B.ny + 2, ez = B.nz + 2;
   const long long n = (long long)ex * ey * ez;
-  for (long long q = threadIdx.x; q < n; q += blockDim.x) {
-    const int x = (int)(q % ex), y = (int)((q / ex) % ey), z = (int)(q / ((long long)ex * ey));
-    const long long i = (long long)z * B.sxy + (long long)y * B.sx + x;
-    D[i] = zero ? T(0) : S[i];
+  constexpr int U = 8;  // cells in flight a thread
+  for (long long q0 = threadIdx.x; q0 < n; q0 += U * blockDim.x) {
+    long long i[U];
+    T v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long q = min(q0 + (long long)u * blockDim.x, n - 1);
+      const int x = (int)(q % ex), y = (int)((q / ex) % ey), z = (int)(q / ((long long)ex * ey));
+      i[u] = (long long)z * B.sxy + (long long)y * B.sx + x;
+      v[u] = zero ? T(0) : S[i[u]];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) D[i[u]] = v[u];
   }
 }
 
@@ -442,7 +451,7 @@ __global__ void __launch_bounds__(256) k_tdma(const BlkLev* __restrict__ bls, co
                                               const T* __restrict__ fx, const T* __restrict__ fy,
                                               const T* __restrict__ fz, bool zero) {
   pdl_trigger();
-  pdl_wait(src, rhs);
+  pdl_wait<false>();
   const BlkLev B = bls[blockIdx.x];
   T* __restrict__ D = dst + B.off;
   T* __restrict__ A = acoef + B.off;
@@ -467,8 +476,8 @@ cudaError_t launch_seq_smoother(int itrsch, bool var, bool zero, const BlkLev* b
     if (var) pdl_launch(k_gslex<T, true>, nb, 512, 0, st, bl, src, dst, rhs, fx, fy, fz, zero);
     else pdl_launch(k_gslex<T, false>, nb, 512, 0, st, bl, src, dst, rhs, fx, fy, fz, zero);
   } else {
-    if (var) pdl_launch(k_tdma<T, true>, nb, 256, 0, st, bl, src, dst, rhs, acoef, fx, fy, fz, zero);
-    else pdl_launch(k_tdma<T, false>, nb, 256, 0, st, bl, src, dst, rhs, acoef, fx, fy, fz, zero);
+    if (var) plain_launch(k_tdma<T, true>, nb, 256, 0, st, bl, src, dst, rhs, acoef, fx, fy, fz, zero);
+    else plain_launch(k_tdma<T, false>, nb, 256, 0, st, bl, src, dst, rhs, acoef, fx, fy, fz, zero);
   }
   return cudaGetLastError();
 }
@@ -561,7 +570,7 @@ struct RowGs {
 // exactly one cell is red and one black, so neither colour phase diverges.
 // Shared memory holds four staged planes of rows y0-2 .. y0+TY+1; column c
 // holds x = c-1.  Same out-of-place contract and arithmetic as k_rbgs.
-template <typename T, int TPR, int CP, int TY, bool VAR, bool ZERO, bool EARLY>
+template <typename T, int TPR, int CP, int TY, bool VAR, bool ZERO>
 __global__ void __launch_bounds__(TPR*(TY + 2)) k_rbgs_rows(const BlkLev* __restrict__ bls,
                                                            const Tile* __restrict__ tiles, int zc,
                                                            const T* __restrict__ src, T* __restrict__ dst,
@@ -569,7 +578,7 @@ __global__ void __launch_bounds__(TPR*(TY + 2)) k_rbgs_rows(const BlkLev* __rest
                                                            const T* __restrict__ fy, const T* __restrict__ fz,
                                                            float om) {
   pdl_trigger();
-  pdl_wait<EARLY>(src, rhs);
+  pdl_wait<false>();
   constexpr int SP = 2 * CP * TPR + 4;
   constexpr int SR = TY + 4;
   constexpr int PL = SR * SP;
@@ -1296,7 +1305,7 @@ __global__ void __launch_bounds__(256) k_defect(const BlkLev* __restrict__ bls, 
 // range, staging fine iterate planes (rows 2Y0-2 .. 2Y0+2TYC-1) in a 3-plane
 // ring.  Each thread keeps the running sum of its coarse cells and adds the
 // eight child residuals in the reference order (i fastest, then j, then k).
-template <typename T, bool VAR, bool ZERO, int TPR, int CPX, int TYC, bool EARLY>
+template <typename T, bool VAR, bool ZERO, int TPR, int CPX, int TYC>
 __global__ void __launch_bounds__(TPR* TYC) k_restrict_tile(const BlkLev* __restrict__ fine,
                                                            const BlkLev* __restrict__ coarse,
                                                            const Tile* __restrict__ tiles, int zc,
@@ -1304,7 +1313,7 @@ __global__ void __launch_bounds__(TPR* TYC) k_restrict_tile(const BlkLev* __rest
                                                            T* __restrict__ rhs_c, const T* __restrict__ fx,
                                                            const T* __restrict__ fy, const T* __restrict__ fz) {
   pdl_trigger();
-  pdl_wait<EARLY>(phi, rhs);
+  pdl_wait<false>();
   constexpr int SP = 2 * CPX * TPR + 4;
   constexpr int SR = 2 * TYC + 2;
   constexpr int PL = SR * SP;
@@ -1671,10 +1680,10 @@ template <typename T, int TPR, int CP, int TY>
 static cudaError_t rows_attr() {
   const int sm = (int)rows_smem<T, TPR, CP, TY>();
   cudaError_t e;
-  if ((e = kernel_smem(H3D_BOTH(k_rbgs_rows, T, TPR, CP, TY, true, true), sm))) return e;
-  if ((e = kernel_smem(H3D_BOTH(k_rbgs_rows, T, TPR, CP, TY, true, false), sm))) return e;
-  if ((e = kernel_smem(H3D_BOTH(k_rbgs_rows, T, TPR, CP, TY, false, true), sm))) return e;
-  return kernel_smem(H3D_BOTH(k_rbgs_rows, T, TPR, CP, TY, false, false), sm);
+  if ((e = cudaFuncSetAttribute(k_rbgs_rows<T, TPR, CP, TY, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))) return e;
+  if ((e = cudaFuncSetAttribute(k_rbgs_rows<T, TPR, CP, TY, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))) return e;
+  if ((e = cudaFuncSetAttribute(k_rbgs_rows<T, TPR, CP, TY, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))) return e;
+  return cudaFuncSetAttribute(k_rbgs_rows<T, TPR, CP, TY, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
 }
 
 template <typename T, int TPR, int CP, int TY>
@@ -1685,13 +1694,12 @@ static cudaError_t rows_dispatch(bool var, bool zero, const BlkLev* bl, const Ti
   constexpr int NT = TPR * (TY + 2);
   constexpr size_t SM = rows_smem<T, TPR, CP, TY>();
   dim3 grid(ntiles), block(NT);
-  const long long cells = (long long)ntiles * TY * zc * (2 * CP * TPR);  // at most
   if (var) {
-    if (zero) pdl_launch(sized(H3D_BOTH(k_rbgs_rows, T, TPR, CP, TY, true, true), cells), grid, block, SM, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
-    else pdl_launch(sized(H3D_BOTH(k_rbgs_rows, T, TPR, CP, TY, true, false), cells), grid, block, SM, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
+    if (zero) plain_launch(k_rbgs_rows<T, TPR, CP, TY, true, true>, grid, block, SM, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
+    else plain_launch(k_rbgs_rows<T, TPR, CP, TY, true, false>, grid, block, SM, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
   } else {
-    if (zero) pdl_launch(sized(H3D_BOTH(k_rbgs_rows, T, TPR, CP, TY, false, true), cells), grid, block, SM, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
-    else pdl_launch(sized(H3D_BOTH(k_rbgs_rows, T, TPR, CP, TY, false, false), cells), grid, block, SM, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
+    if (zero) plain_launch(k_rbgs_rows<T, TPR, CP, TY, false, true>, grid, block, SM, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
+    else plain_launch(k_rbgs_rows<T, TPR, CP, TY, false, false>, grid, block, SM, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
   }
   return cudaGetLastError();
 }
@@ -3076,9 +3084,9 @@ template <typename T, int TPR, int CPX, int TYC>
 static cudaError_t rtile_attr() {
   const int sm = (int)rtile_smem<T, TPR, CPX, TYC>();
   cudaError_t e;
-  if ((e = kernel_smem(H3D_BOTH(k_restrict_tile, T, true, false, TPR, CPX, TYC), sm))) return e;
-  if ((e = kernel_smem(H3D_BOTH(k_restrict_tile, T, false, false, TPR, CPX, TYC), sm))) return e;
-  return kernel_smem(H3D_BOTH(k_restrict_tile, T, false, true, TPR, CPX, TYC), sm);
+  if ((e = cudaFuncSetAttribute(k_restrict_tile<T, true, false, TPR, CPX, TYC>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))) return e;
+  if ((e = cudaFuncSetAttribute(k_restrict_tile<T, false, false, TPR, CPX, TYC>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))) return e;
+  return cudaFuncSetAttribute(k_restrict_tile<T, false, true, TPR, CPX, TYC>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
 }
 
 template <typename T, int TPR, int CPX, int TYC>
@@ -3087,10 +3095,9 @@ static cudaError_t rtile_dispatch(bool var, bool zero, const BlkLev* fine, const
                                   const T* fz, cudaStream_t st) {
   if (ntiles <= 0) return cudaSuccess;
   constexpr size_t SM = rtile_smem<T, TPR, CPX, TYC>();
-  const long long cells = 8LL * ntiles * TYC * zc * (TPR * CPX);  // at most
-  if (zero) pdl_launch(sized(H3D_BOTH(k_restrict_tile, T, false, true, TPR, CPX, TYC), cells), ntiles, TPR * TYC, SM, st, fine, coarse, tiles, zc, phi, rhs, rhs_c, fx, fy, fz);
-  else if (var) pdl_launch(sized(H3D_BOTH(k_restrict_tile, T, true, false, TPR, CPX, TYC), cells), ntiles, TPR * TYC, SM, st, fine, coarse, tiles, zc, phi, rhs, rhs_c, fx, fy, fz);
-  else pdl_launch(sized(H3D_BOTH(k_restrict_tile, T, false, false, TPR, CPX, TYC), cells), ntiles, TPR * TYC, SM, st, fine, coarse, tiles, zc, phi, rhs, rhs_c, fx, fy, fz);
+  if (zero) plain_launch(k_restrict_tile<T, false, true, TPR, CPX, TYC>, ntiles, TPR * TYC, SM, st, fine, coarse, tiles, zc, phi, rhs, rhs_c, fx, fy, fz);
+  else if (var) plain_launch(k_restrict_tile<T, true, false, TPR, CPX, TYC>, ntiles, TPR * TYC, SM, st, fine, coarse, tiles, zc, phi, rhs, rhs_c, fx, fy, fz);
+  else plain_launch(k_restrict_tile<T, false, false, TPR, CPX, TYC>, ntiles, TPR * TYC, SM, st, fine, coarse, tiles, zc, phi, rhs, rhs_c, fx, fy, fz);
   return cudaGetLastError();
 }
 
@@ -3449,7 +3456,7 @@ __device__ __forceinline__ void sip_plane(const BlkLev& B, int d, F&& f) {
 
 __global__ void __launch_bounds__(512) k_sip_factor(const BlkLev* __restrict__ bls, SipLU lu) {
   pdl_trigger();
-  pdl_wait();
+  pdl_wait<false>();
   const BlkLev B = bls[blockIdx.x];
   const double alfa = 0.92, small = 1e-20;  // sipsol.for:32-33
   double *lb = lu.lb + B.off, *lw = lu.lw + B.off, *ls = lu.ls + B.off, *lpr = lu.lpr + B.off;
@@ -3480,7 +3487,7 @@ __global__ void __launch_bounds__(512) k_sip_factor(const BlkLev* __restrict__ b
 __global__ void __launch_bounds__(512) k_sip_sweep(const BlkLev* __restrict__ bls, SipLU lu, double* __restrict__ fi_all,
                                                    const double* __restrict__ su_all, double* __restrict__ partials) {
   pdl_trigger();
-  pdl_wait(fi_all, su_all);
+  pdl_wait<false>();
   __shared__ double red[16];
   const BlkLev B = bls[blockIdx.x];
   const double *lb = lu.lb + B.off, *lw = lu.lw + B.off, *ls = lu.ls + B.off, *lpr = lu.lpr + B.off;
@@ -3543,7 +3550,7 @@ __global__ void __launch_bounds__(256) k_gather1(const uint32_t* __restrict__ ds
 cudaError_t launch_sip_factor(const BlkLev* bl, int nb, SipArrays a, cudaStream_t st) {
   if (nb <= 0) return cudaSuccess;
   SipLU lu{a.lb, a.lw, a.ls, a.lpr, a.un, a.ue, a.ut, a.res};
-  pdl_launch(k_sip_factor, nb, 512, 0, st, bl, lu);
+  plain_launch(k_sip_factor, nb, 512, 0, st, bl, lu);
   return cudaGetLastError();
 }
 
@@ -3551,7 +3558,7 @@ cudaError_t launch_sip_sweep(const BlkLev* bl, int nb, SipArrays a, double* fi, 
                              cudaStream_t st) {
   if (nb <= 0) return cudaSuccess;
   SipLU lu{a.lb, a.lw, a.ls, a.lpr, a.un, a.ue, a.ut, a.res};
-  pdl_launch(k_sip_sweep, nb, 512, 0, st, bl, lu, fi, su, partials);
+  plain_launch(k_sip_sweep, nb, 512, 0, st, bl, lu, fi, su, partials);
   return cudaGetLastError();
 }
 
