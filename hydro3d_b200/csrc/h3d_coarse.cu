@@ -23,7 +23,7 @@ namespace h3d {
 // start[b]: first flat interior index of block b (start[nb] = all cells).
 // sb / ss: the block table and those starts, in shared memory.
 template <typename T, bool VAR>
-__device__ void small_relax(const BlkLev* sb, const int* ss, int nb, T* __restrict__ phi, const T* __restrict__ rhs,
+__device__ void small_relax(const BlkLev* sb, const int* ss, int nb, T* __restrict__ phi, const T* rhs,
                             const T* __restrict__ fx, const T* __restrict__ fy, const T* __restrict__ fz,
                             const uint32_t* __restrict__ fdst, const uint32_t* __restrict__ fsrc, int nfill,
                             int sweeps, int zero, long long nelems, float om, int rb) {
@@ -423,7 +423,7 @@ __device__ void tail_prolong(const BlkLev* fb, const BlkLev* cb, const TailLevel
 // The rhs of a tail level from global memory (the restriction into the
 // first tail level ran outside); eight loads in flight a thread.
 template <typename T>
-__device__ void tail_load_rhs(const BlkLev* gb, const BlkLev* cb, const TailLevel& L, const T* __restrict__ g, T* rhs) {
+__device__ void tail_load_rhs(const BlkLev* gb, const BlkLev* cb, const TailLevel& L, const T* g, T* rhs) {
   constexpr int U = 8;
   for (int k0 = threadIdx.x; k0 < L.nint; k0 += U * blockDim.x) {
     T v[U];
@@ -723,7 +723,7 @@ __global__ void __launch_bounds__(kClusterTailThreads) k_coarse_cluster(const Ta
     auto at64 = [&](int off) { return reinterpret_cast<double*>(arena + off); };
     switch (op.kind) {
       case kTailLoadRhs: {
-        auto load = [&](const auto* __restrict__ g, auto* rhs) {
+        auto load = [&](const auto* g, auto* rhs) {
 #pragma unroll 4
           for (int k = threadIdx.x; k < F.nint; k += blockDim.x) {
             const Cell3 c = cell3(F.cells32[k]);

@@ -24,7 +24,8 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 // the mean that remove_mean subtracts was moved above it: solves of up to 75,000 words
 // kept their mean in up to a third of the calls.)  The wait therefore takes the
 // pointers to data that predecessors write and makes them opaque; tables written
-// once at set-up are left out.  Plain loads are not moved ahead of stores and
+// once at set-up are left out (and no const __restrict__ is put on them again
+// behind the wait).  Plain loads are not moved ahead of stores and
 // barriers either, which costs the large streaming kernels (every kernel in this form:
 // 192^3 in FP64 9.74 -> 9.99 ms, 256^3 of variable density 20.6 -> 25.6 ms), and
 // large launches do not start early: those kernels are built in two forms, EARLY

@@ -65,9 +65,9 @@ __global__ void __launch_bounds__(NT) k_rbgs(const BlkLev* __restrict__ bls, con
   const BlkLev B = bls[t.b];
   const int nx = B.nx, ny = B.ny, nz = B.nz;
   const long long sx = B.sx, sxy = B.sxy;
-  const T* __restrict__ S = src + B.off;
+  const T* S = src + B.off;
   T* __restrict__ D = dst + B.off;
-  const T* __restrict__ R = rhs + B.off;
+  const T* R = rhs + B.off;
   const T* FX = VAR ? fx + B.off : nullptr;
   const T* FY = VAR ? fy + B.off : nullptr;
   const T* FZ = VAR ? fz + B.off : nullptr;
@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(256, 3) k_rbgs_zero32(const BlkLev* __restrict
   if (r >= rows || y > ny) return;
   const int x0 = 1 + 4 * g;
   const long long sx = B.sx, sxy = B.sxy;
-  const float* __restrict__ R = rhs + B.off;
+  const float* R = rhs + B.off;
   float* __restrict__ D = dst + B.off;
   const int zs = t.z0, ze = min(t.z0 + zc - 1, nz);
   // wall mask of a cell (only faces that are physical walls count)
@@ -328,7 +328,7 @@ namespace {
 
 // The block's cells, ghosts included, from src (or zeros) into dst.
 template <typename T>
-__device__ __forceinline__ void copy_block(const BlkLev& B, const T* __restrict__ S, T* __restrict__ D, bool zero) {
+__device__ __forceinline__ void copy_block(const BlkLev& B, const T* S, T* D, bool zero) {
   const int ex = B.nx + 2, ey = B.ny + 2, ez = B.nz + 2;
   const long long n = (long long)ex * ey * ez;
   constexpr int U = 8;  // cells in flight a thread
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(512) k_gslex(const BlkLev* __restrict__ bls, c
   pdl_wait(src, rhs);
   const BlkLev B = bls[blockIdx.x];
   T* __restrict__ D = dst + B.off;
-  const T* __restrict__ R = rhs + B.off;
+  const T* R = rhs + B.off;
   const T* FX = VAR ? fx + B.off : nullptr;
   const T* FY = VAR ? fy + B.off : nullptr;
   const T* FZ = VAR ? fz + B.off : nullptr;
