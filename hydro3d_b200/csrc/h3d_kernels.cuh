@@ -172,15 +172,16 @@ template <typename T>
 cudaError_t launch_seq_smoother(int itrsch, bool var, bool zero, const BlkLev* bl, int nb, const T* src, T* dst,
                                 const T* rhs, T* acoef, const T* fx, const T* fy, const T* fz, cudaStream_t st);
 // The TDMA sweep with the chains' operands in shared memory (h3d_seq.cu).
-// scratch: 3 * words * nb words (kDiagonals only).
+// scratch: 3 * words words, blocks from offs (kDiagonals only).
 struct TdmaPlan {
   enum Mode { kGlobal = 0, kWhole = 1, kDiagonals = 2 };
   int mode = kGlobal, smem = 0, nbuf = 0;
   long long words = 0;
+  std::vector<long long> offs;
 };
 TdmaPlan tdma_plan(const std::vector<BlkLev>& bl, bool var, int word);
 template <typename T>
-cudaError_t launch_tdma(const TdmaPlan& P, bool zero, const BlkLev* bl, CellTab all, const T* src, T* dst,
+cudaError_t launch_tdma(const TdmaPlan& P, bool zero, const BlkLev* bl, const long long* offs, CellTab all, const T* src, T* dst,
                         const T* rhs, T* scratch, cudaStream_t st);
 template <typename T>
 cudaError_t launch_relax_small(bool var, const BlkLev* bl, const int* start, int nb, T* phi, const T* rhs,

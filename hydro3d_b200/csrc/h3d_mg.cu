@@ -117,6 +117,7 @@ struct Level {
   bool use_z32 = true;          // the zero-source kernel beat the tuned sweep's zero mode (autotuner)
   int nztiles = 0, zzc = 1;
   TdmaPlan tdma;                // the line-TDMA kernel of the level (mg_itrsch 2) and its scratch
+  long long* d_tdma_off = nullptr;  // first scratch word of each block
   double* seq64 = nullptr;
   float* seq32 = nullptr;
   // local mesh refinement
@@ -178,6 +179,7 @@ struct h3d_mg {
                             // set but after a solve that came to a finite residual without an error
   bool debug_sync = false;  // H3D_DEBUG_SYNC=1: synchronize and check after every launch
   std::vector<double> history;
+  bool stage_held = false;  // a call still reads its staged host arrays (give_back)
   // whole host block arrays staged on the device (0: pressure, 1: rhs) for
   // contiguous host transfers; allocated on first use
   double* stage[2] = {nullptr, nullptr};
@@ -211,7 +213,8 @@ struct h3d_mg {
   uint32_t* d_vsrc = nullptr;
   int64_t nvfill = 0;
   double* sip[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};  // SIP factors, res
-  SipPlan sip_plan;                  // sip: in the skewed layout of the cluster kernels where d_sip_off is set
+  SipPlan sip_plan;                  // sip: in the skewed layout of the cluster kernels where sip_plan.fits
+  bool sip_held = false;             // the factors are being allocated (give_back)
   long long* d_sip_off = nullptr;    // first word of each block there
   double* sip_pp = nullptr;  // the SIP pressure correction (level-1 layout)
   bool proj = false;        // outer iterations end with p += pp, calvel, calmas
@@ -241,11 +244,59 @@ int fail(h3d_mg* h, int code, const std::string& msg) {
     if (_r != H3D_OK) return _r;    \
   } while (0)
 
+// Device memory that a handle holds for speed alone, given back when an allocation
+// that a call cannot do without finds none: the staging copy of host fields and
+// the SIP factors (made again by the next call that wants them), then the scratch
+// of the line-TDMA kernels, whose levels keep the kernel that needs a word a cell.
+// Returns whether any was freed.
+bool give_back(h3d_mg* h) {
+  if (cudaStreamSynchronize(h->st) != cudaSuccess) return false;
+  bool any = false;
+  auto drop = [&](auto*& p) {
+    if (!p) return;
+    cudaFree(p);
+    p = nullptr;
+    any = true;
+  };
+  if (!h->stage_held)
+    for (double*& p : h->stage) drop(p);
+  if (!h->sip_held)
+    for (double*& p : h->sip) drop(p);
+  if (any) return true;
+  for (Level& V : h->lev) {
+    if (V.tdma.mode != TdmaPlan::kDiagonals || !(V.seq64 || V.seq32)) continue;
+    const size_t n = (size_t)V.geom.n_elems;
+    const bool f32 = V.seq32 != nullptr;
+    drop(V.seq64);
+    drop(V.seq32);
+    drop(V.d_tdma_off);
+    V.tdma.mode = TdmaPlan::kGlobal;
+    // (without a word a cell the next sweep of the level reports it)
+    if (f32 ? cudaMalloc((void**)&V.seq32, n * 4) : cudaMalloc((void**)&V.seq64, n * 8)) cudaGetLastError();
+  }
+  if (any) {  // captured graphs launch the other kernels
+    for (auto& kv : h->graphs)
+      if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
+    h->graphs.clear();
+  }
+  return any;
+}
+
+// optional: the caller has another way, so nothing is given back for it.
 template <typename T>
-int dalloc(h3d_mg* h, T** p, size_t n) {
+int dalloc(h3d_mg* h, T** p, size_t n, bool optional = false) {
   *p = nullptr;
   if (n == 0) return H3D_OK;
-  CU(cudaMalloc((void**)p, n * sizeof(T)));
+  cudaError_t e = cudaMalloc((void**)p, n * sizeof(T));
+  while (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    *p = nullptr;
+    if (optional || !give_back(h)) break;
+    e = cudaMalloc((void**)p, n * sizeof(T));
+  }
+  if (e != cudaSuccess)
+    return fail(h, e == cudaErrorMemoryAllocation ? H3D_ERR_OOM : H3D_ERR_CUDA,
+                std::string("cudaMalloc: ") + cudaGetErrorString(e));
   // The zero fill must be complete before the caller fills the array: uploads
   // with cudaMemcpy run on the legacy stream, which is not ordered after the
   // solver's non-blocking stream (a late zero fill once wiped freshly
@@ -601,11 +652,13 @@ struct Exec {
       const int nb = (int)V.geom.bl.size();
       const CellTab all{V.d_cta_all, nb, V.ncta_all};
       if (h->desc.mg_itrsch == 2 && V.tdma.mode == TdmaPlan::kDiagonals) h->kernels += 6;
+      if (h->desc.mg_itrsch == 2 && V.tdma.mode == TdmaPlan::kGlobal && !(mixed_level(g) ? (void*)V.seq32 : V.seq64))
+        return fail(h, H3D_ERR_OOM, "line-TDMA scratch");
       if (mixed_level(g)) {
         float* src = V.phi32[V.cur32];
         float* dst = V.phi32[1 - V.cur32];
         if (h->desc.mg_itrsch == 2 && V.tdma.mode != TdmaPlan::kGlobal)
-          CU(launch_tdma<float>(V.tdma, V.zero32, V.d_bl, all, src, dst, V.rhs32, V.seq32, st));
+          CU(launch_tdma<float>(V.tdma, V.zero32, V.d_bl, V.d_tdma_off, all, src, dst, V.rhs32, V.seq32, st));
         else
           CU(launch_seq_smoother<float>(h->desc.mg_itrsch, h->var, V.zero32, V.d_bl, nb, src, dst, V.rhs32, V.seq32,
                                         V.fx32, V.fy32, V.fz32, st));
@@ -619,7 +672,7 @@ struct Exec {
         double* src = V.phi64[V.cur64];
         double* dst = V.phi64[1 - V.cur64];
         if (h->desc.mg_itrsch == 2 && V.tdma.mode != TdmaPlan::kGlobal)
-          CU(launch_tdma<double>(V.tdma, V.zero64, V.d_bl, all, src, dst, V.rhs64, V.seq64, st));
+          CU(launch_tdma<double>(V.tdma, V.zero64, V.d_bl, V.d_tdma_off, all, src, dst, V.rhs64, V.seq64, st));
         else
           CU(launch_seq_smoother<double>(h->desc.mg_itrsch, h->var, V.zero64, V.d_bl, nb, src, dst, V.rhs64,
                                          V.seq64, V.fx64, V.fy64, V.fz64, st));
@@ -1229,7 +1282,7 @@ int check_block_host_dims(h3d_mg* h, const h3d_block_desc& d) {
 // staging and the padded layout.  stage_out writes back whole host planes, so
 // it is only used in calls that staged the same host array in (the planes'
 // other cells then round-trip unchanged).
-int ensure_stage(h3d_mg* h, int f) {
+int ensure_stage(h3d_mg* h, int f, bool optional = false) {
   if (h->stage[f]) return H3D_OK;
   size_t n = 0;
   h->stage_off.clear();
@@ -1237,7 +1290,7 @@ int ensure_stage(h3d_mg* h, int f) {
     h->stage_off.push_back(n);
     n += (size_t)d.ttc[0] * d.ttc[1] * d.ttc[2];
   }
-  return dalloc(h, &h->stage[f], n);
+  return dalloc(h, &h->stage[f], n, optional);
 }
 
 int stage_in(h3d_mg* h, int f, int ib, const double* host, double* dev_level, bool with_ghosts) {
@@ -1282,10 +1335,9 @@ int field_in(h3d_mg* h, const double* host, int ib, double* dev_level, bool with
   const size_t whole = (size_t)d.ttc[0] * d.ttc[1] * d.ttc[2];
   const size_t need = (size_t)(B.nx + 2) * (B.ny + 2) * (B.nz + 2);
   if (whole <= 2 * need) {
-    const int rc = ensure_stage(h, 0);
+    const int rc = ensure_stage(h, 0, true);
     if (rc == H3D_OK) return stage_in(h, 0, ib, host, dev_level, with_ghosts);
     if (rc != H3D_ERR_OOM) return rc;
-    cudaGetLastError();
   }
   return copy_field_3d(h, true, dev_level, B, const_cast<double*>(host), d, with_ghosts);
 }
@@ -2495,7 +2547,7 @@ int h3d_mg_destroy(h3d_mg* h) {
                   V.phi32[1], V.rhs32, V.fx64, V.fy64, V.fz64, V.fx32, V.fy32, V.fz32, V.dens,
                   V.sweep.d_dst, V.sweep.d_src, V.faces.d_dst, V.faces.d_src, V.exch.d_dst, V.exch.d_src,
                   V.bound.d_dst, V.bound.d_src, V.sweep_push.d_dst, V.sweep_push.d_src, V.live.d_dst, V.live.d_src, V.live_push.d_dst, V.live_push.d_src, V.red.d_dst, V.red.d_src, V.d_red_info, V.d_push, V.d_maps, V.d_rmaps, V.d_rtiles, V.d_ptiles, V.d_qtiles, V.d_dtiles, V.d_cstart, V.d_dstart, V.d_pstart, V.seq64, V.seq32, V.d_ztiles, V.lfill.d_dst, V.lfill.d_src, V.d_lfstart,
-                  V.cfill.d_dst, V.cfill.d_src, V.d_clive,
+                  V.cfill.d_dst, V.cfill.d_src, V.d_clive, V.d_tdma_off,
                   V.xs.d_nodes, V.xs.d_dst, V.xs.d_src, V.xe.d_nodes, V.xe.d_dst, V.xe.d_src, V.xscratch, V.d_rsame,
                   V.d_psame, V.d_prows};
     for (void* p : ps) dfree(p);
@@ -2664,11 +2716,17 @@ int h3d_mg_create(h3d_mg** out, const h3d_mg_desc* desc) {
       auto scratch = [&](size_t words) { return f32 ? dalloc(h, &V.seq32, words) : dalloc(h, &V.seq64, words); };
       rc = H3D_OK;
       if (V.tdma.mode == TdmaPlan::kDiagonals) {
-        rc = scratch(3 * (size_t)V.tdma.words * V.geom.bl.size());
-        if (rc == H3D_ERR_OOM) {
-          cudaGetLastError();
-          V.tdma.mode = TdmaPlan::kGlobal;
-        }
+        auto optional = [&](size_t words) {
+          return f32 ? dalloc(h, &V.seq32, words, true) : dalloc(h, &V.seq64, words, true);
+        };
+        rc = optional(3 * (size_t)V.tdma.words);
+        if (rc == H3D_ERR_OOM) V.tdma.mode = TdmaPlan::kGlobal;
+      }
+      if (V.tdma.mode == TdmaPlan::kDiagonals) {
+        if ((rc = dalloc(h, &V.d_tdma_off, V.tdma.offs.size())) != H3D_OK) return bail(rc);
+        if (cudaMemcpy(V.d_tdma_off, V.tdma.offs.data(), V.tdma.offs.size() * sizeof(long long),
+                       cudaMemcpyHostToDevice) != cudaSuccess)
+          return bail(fail(h, H3D_ERR_CUDA, "line-TDMA scratch offsets"));
       }
       if (V.tdma.mode == TdmaPlan::kGlobal) rc = scratch(n);
       if (rc != H3D_OK) return bail(rc);
@@ -3149,6 +3207,11 @@ int h3d_mg_newsolv(h3d_mg* h, double* const* p, const double* const* b, const h3
                    h3d_solve_info* info) {
   if (!h || !p || !b || !opts) return H3D_ERR_ARG;
   CU(cudaSetDevice(h->device));
+  struct Held {  // the staged pressure is written back from its staging array
+    h3d_mg* h;
+    ~Held() { h->stage_held = false; }
+  } held{h};
+  h->stage_held = true;
   for (int ib = 0; ib < (int)h->blocks.size(); ++ib) {
     TRY(stage_in(h, 0, ib, p[ib], h->p64[h->pc], true));
     TRY(stage_in(h, 1, ib, b[ib], h->b64, false));
@@ -3226,11 +3289,11 @@ static int ensure_face_table(h3d_mg* h) {
 static int ensure_velocity(h3d_mg* h) {
   if (h->lmr)
     return fail(h, H3D_ERR_BAD_CONFIG, "the projection loop with local mesh refinement is not supported");
-  if (h->vel[0]) return H3D_OK;
+  if (h->vstar[2]) return H3D_OK;  // (the last)
   const size_t n = (size_t)h->lev[1].geom.n_elems;
   for (int c = 0; c < 3; ++c) {
-    TRY(dalloc(h, &h->vel[c], n));
-    TRY(dalloc(h, &h->vstar[c], n));
+    if (!h->vel[c]) TRY(dalloc(h, &h->vel[c], n));
+    if (!h->vstar[c]) TRY(dalloc(h, &h->vstar[c], n));
   }
   return ensure_face_table(h);
 }
@@ -3247,17 +3310,27 @@ static int ensure_sip(h3d_mg* h) {
   if (h->var) return fail(h, H3D_ERR_BAD_CONFIG, "SIP: constant coefficients only (press.for:407-438)");
   if (h->lmr) return fail(h, H3D_ERR_BAD_CONFIG, "SIP with local mesh refinement is not supported");
   if ((int)h->blocks.size() > h->npartials) return fail(h, H3D_ERR_BAD_CONFIG, "SIP: too many blocks");
-  if (h->sip_pp) return H3D_OK;
+  if (h->sip_pp && h->sip[7]) return H3D_OK;  // (the last factor array: they are made and given back together)
   TRY(ensure_face_table(h));
   const LevelGeom& G = h->lev[1].geom;
   const size_t n = (size_t)G.n_elems;
-  auto alloc_factors = [&](size_t words) -> int {
-    for (int q = 0; q < 8; ++q) {
-      dfree(h->sip[q]);
-      h->sip[q] = nullptr;
+  struct Held {
+    h3d_mg* h;
+    ~Held() { h->sip_held = false; }
+  } held{h};
+  h->sip_held = true;
+  auto drop = [&] {
+    for (double*& p : h->sip) {
+      dfree(p);
+      p = nullptr;
     }
-    for (int q = 0; q < 8; ++q) TRY(dalloc(h, &h->sip[q], words));
-    return H3D_OK;
+  };
+  auto alloc = [&](size_t words, bool optional) -> int {
+    drop();
+    int rc = h->sip_pp ? H3D_OK : dalloc(h, &h->sip_pp, n, optional);
+    for (int q = 0; q < 8 && rc == H3D_OK; ++q) rc = dalloc(h, &h->sip[q], words, optional);
+    if (rc != H3D_OK) drop();
+    return rc;
   };
   // the skewed layout of the cluster kernels, up to twice a level, where the
   // blocks' cross-sections and the device's memory allow it
@@ -3270,20 +3343,17 @@ static int ensure_sip(h3d_mg* h) {
       off.push_back(words);
       words += ((long long)B.nz * (B.nx + B.ny - 1) * B.ny + 15) / 16 * 16;
     }
-    rc = alloc_factors((size_t)words);
-    if (rc == H3D_OK && !h->d_sip_off) {
+    if (!h->d_sip_off) {
       TRY(dalloc(h, &h->d_sip_off, off.size()));
       CU(cudaMemcpy(h->d_sip_off, off.data(), off.size() * sizeof(long long), cudaMemcpyHostToDevice));
     }
+    rc = alloc((size_t)words, true);
   }
   if (rc == H3D_ERR_OOM) {
-    cudaGetLastError();
     h->sip_plan.fits = false;
-    rc = alloc_factors(n);
+    rc = alloc(n, false);
   }
-  if (rc != H3D_OK) return rc;
-  TRY(dalloc(h, &h->sip_pp, n));
-  return H3D_OK;
+  return rc;
 }
 
 // sipsol(44) (sipsol.for:2-205) on the resident correction with the resident
@@ -3342,8 +3412,8 @@ int h3d_mg_pressure_1sweep(h3d_mg* h, double dt, double alfapr, double eps, int3
   if (!h || niter < 1 || nswp < 1) return H3D_ERR_ARG;
   if (!(dt > 0)) return fail(h, H3D_ERR_ARG, "dt must be positive");
   CU(cudaSetDevice(h->device));
-  TRY(ensure_sip(h));
   TRY(ensure_velocity(h));
+  TRY(ensure_sip(h));  // (last: an allocation after it could take its factors back)
   Level& V = h->lev[1];
   h3d_solve_info I{};
   h->history.clear();

@@ -693,7 +693,8 @@ template <typename T, int FROM, int AXIS, bool EARLY>
 __global__ void __launch_bounds__(256) k_tdma_rows(const BlkLev* __restrict__ bls, const int* __restrict__ cta_start,
                                                    int nb, const T* __restrict__ src, const T* __restrict__ rhs,
                                                    const T* __restrict__ from, T* __restrict__ to,
-                                                   T* __restrict__ rows, long long words, bool zero) {
+                                                   T* __restrict__ rows, const long long* __restrict__ offs,
+                                                   bool zero) {
   pdl_trigger();
   pdl_wait<EARLY>(src, rhs, from);
   const int b = find_block(cta_start, nb, blockIdx.x);
@@ -702,9 +703,9 @@ __global__ void __launch_bounds__(256) k_tdma_rows(const BlkLev* __restrict__ bl
   if (q >= ex * ey * (B.nz + 2)) return;
   const int x = q % ex, y = (q / ex) % ey, z = q / (ex * ey);
   const long long i = B.off + (long long)z * B.sxy + (long long)y * B.sx + x;
-  const long long o = b * words + tdma_at<AXIS>(B, x, y, z);
+  const long long o = offs[b] + tdma_at<AXIS>(B, x, y, z);
   if (FROM < 0) to[o] = zero ? T(0) : src[i];
-  else to[o] = from[b * words + tdma_at<FROM < 0 ? 0 : FROM>(B, x, y, z)];
+  else to[o] = from[offs[b] + tdma_at<FROM < 0 ? 0 : FROM>(B, x, y, z)];
   rows[o] = rhs[i];
 }
 
@@ -712,7 +713,7 @@ __global__ void __launch_bounds__(256) k_tdma_rows(const BlkLev* __restrict__ bl
 template <typename T, bool EARLY>
 __global__ void __launch_bounds__(256) k_tdma_level(const BlkLev* __restrict__ bls, const int* __restrict__ cta_start,
                                                     int nb, const T* __restrict__ from, T* __restrict__ dst,
-                                                    long long words) {
+                                                    const long long* __restrict__ offs) {
   pdl_trigger();
   pdl_wait<EARLY>(from);
   const int b = find_block(cta_start, nb, blockIdx.x);
@@ -720,19 +721,20 @@ __global__ void __launch_bounds__(256) k_tdma_level(const BlkLev* __restrict__ b
   const int ex = B.nx + 2, ey = B.ny + 2, q = (blockIdx.x - cta_start[b]) * blockDim.x + threadIdx.x;
   if (q >= ex * ey * (B.nz + 2)) return;
   const int x = q % ex, y = (q / ex) % ey, z = q / (ex * ey);
-  dst[B.off + (long long)z * B.sxy + (long long)y * B.sx + x] = from[b * words + tdma_at<2>(B, x, y, z)];
+  dst[B.off + (long long)z * B.sxy + (long long)y * B.sx + x] = from[offs[b] + tdma_at<2>(B, x, y, z)];
 }
 
 // One pass, a CTA per block, on the rearranged iterate (in place) and rhs.
 template <typename T, int AXIS>
 __global__ void __launch_bounds__(kTdmaThreads) k_tdma_g(const BlkLev* __restrict__ bls, T* __restrict__ iter,
-                                                         const T* __restrict__ rows, long long words, int nbuf) {
+                                                         const T* __restrict__ rows,
+                                                         const long long* __restrict__ offs, int nbuf) {
   extern __shared__ __align__(16) unsigned char tdma_smem[];
   using L = LineAxes<AXIS>;
   pdl_trigger();
   const BlkLev B = bls[blockIdx.x];
-  T* Dk = iter + blockIdx.x * words;
-  const T* Rk = rows + blockIdx.x * words;
+  T* Dk = iter + offs[blockIdx.x];
+  const T* Rk = rows + offs[blockIdx.x];
   const int ex[3] = {B.nx, B.ny, B.nz};
   const int nu = ex[L::US], nv = ex[L::VS], n = ex[L::SS], pitch = nu + 2, row = (n + 2) * pitch;
   T* P = reinterpret_cast<T*>(tdma_smem);  // [2][n + 2][pitch]: c and phi of the current and the previous diagonal
@@ -869,8 +871,8 @@ cudaError_t launch_sip_sweep_c(const SipPlan& P, const BlkLev* bl, const long lo
 }
 
 // Which TDMA kernel a level takes: whole blocks in shared memory where they fit
-// (16x16x24 cells in FP64), else clusters with the diagonals around the current
-// one there (78^3 in FP64), else, and with variable coefficients, one thread a
+// (16x16x24 cells in FP64), else the diagonals around the current one there
+// (78^3 in FP64), a CTA a block, else, and with variable coefficients, one thread a
 // line in global memory (k_tdma).
 TdmaPlan tdma_plan(const std::vector<BlkLev>& bl, bool var, int word) {
   TdmaPlan P;
@@ -878,14 +880,17 @@ TdmaPlan tdma_plan(const std::vector<BlkLev>& bl, bool var, int word) {
   long long whole = 0, diag[2] = {0, 0}, lines = 0;  // words; diag: one and two operand buffers
   for (const auto& B : bl) {
     const long long ex[3] = {B.nx, B.ny, B.nz}, mx = std::max(B.nx, std::max(B.ny, B.nz)) + 2;
+    long long own = 0;
     whole = std::max(whole, 2LL * tdma_s_sxy(B.nx, B.ny) * (B.nz + 2) + mx * 32);
     for (int axis = 0; axis < 3; ++axis) {
       const long long nu = axis == 0 ? ex[1] : ex[0], nv = axis == 2 ? ex[1] : ex[2], n = ex[axis];
       for (int k = 0; k < 2; ++k)
         diag[k] = std::max(diag[k], 2 * (n + 2) * (nu + 2) + (k + 1) * (2 * (n + 2) + 2) * (nu + 2) + (n + 1) * 32);
       lines = std::max(lines, std::min(nu, nv));
-      P.words = std::max(P.words, (tdma_rows((int)nu, (int)nv, (int)n) + 15) / 16 * 16);
+      own = std::max(own, (tdma_rows((int)nu, (int)nv, (int)n) + 15) / 16 * 16);
     }
+    P.offs.push_back(P.words);
+    P.words += own;
   }
   if (lines > kTdmaThreads) return P;
   if (whole * word <= kTdmaMaxSmem) {
@@ -900,8 +905,8 @@ TdmaPlan tdma_plan(const std::vector<BlkLev>& bl, bool var, int word) {
 }
 
 template <typename T>
-cudaError_t launch_tdma(const TdmaPlan& P, bool zero, const BlkLev* bl, CellTab all, const T* src, T* dst,
-                        const T* rhs, T* scratch, cudaStream_t st) {
+cudaError_t launch_tdma(const TdmaPlan& P, bool zero, const BlkLev* bl, const long long* offs, CellTab all,
+                        const T* src, T* dst, const T* rhs, T* scratch, cudaStream_t st) {
   const int nb = all.nb;
   if (nb <= 0) return cudaSuccess;
   if (P.mode == TdmaPlan::kWhole) {
@@ -909,21 +914,20 @@ cudaError_t launch_tdma(const TdmaPlan& P, bool zero, const BlkLev* bl, CellTab 
     return cudaGetLastError();
   }
   if (P.mode != TdmaPlan::kDiagonals) return cudaErrorInvalidValue;
-  const long long w = P.words;
   const size_t sm = (size_t)P.smem;
-  T *a = scratch, *b = a + nb * w, *rows = b + nb * w;
-  pdl_launch(H3D_BOTH(k_tdma_rows, T, -1, 1), all.ncta, 256, 0, st, bl, all.cta_start, nb, src, rhs, b, a, rows, w, zero);
-  pdl_launch(k_tdma_g<T, 1>, nb, kTdmaThreads, sm, st, bl, a, rows, w, P.nbuf);
-  pdl_launch(H3D_BOTH(k_tdma_rows, T, 1, 0), all.ncta, 256, 0, st, bl, all.cta_start, nb, src, rhs, a, b, rows, w, zero);
-  pdl_launch(k_tdma_g<T, 0>, nb, kTdmaThreads, sm, st, bl, b, rows, w, P.nbuf);
-  pdl_launch(H3D_BOTH(k_tdma_rows, T, 0, 2), all.ncta, 256, 0, st, bl, all.cta_start, nb, src, rhs, b, a, rows, w, zero);
-  pdl_launch(k_tdma_g<T, 2>, nb, kTdmaThreads, sm, st, bl, a, rows, w, P.nbuf);
-  pdl_launch(H3D_BOTH(k_tdma_level, T), all.ncta, 256, 0, st, bl, all.cta_start, nb, a, dst, w);
+  T *a = scratch, *b = a + P.words, *rows = b + P.words;
+  pdl_launch(H3D_BOTH(k_tdma_rows, T, -1, 1), all.ncta, 256, 0, st, bl, all.cta_start, nb, src, rhs, b, a, rows, offs, zero);
+  pdl_launch(k_tdma_g<T, 1>, nb, kTdmaThreads, sm, st, bl, a, rows, offs, P.nbuf);
+  pdl_launch(H3D_BOTH(k_tdma_rows, T, 1, 0), all.ncta, 256, 0, st, bl, all.cta_start, nb, src, rhs, a, b, rows, offs, zero);
+  pdl_launch(k_tdma_g<T, 0>, nb, kTdmaThreads, sm, st, bl, b, rows, offs, P.nbuf);
+  pdl_launch(H3D_BOTH(k_tdma_rows, T, 0, 2), all.ncta, 256, 0, st, bl, all.cta_start, nb, src, rhs, b, a, rows, offs, zero);
+  pdl_launch(k_tdma_g<T, 2>, nb, kTdmaThreads, sm, st, bl, a, rows, offs, P.nbuf);
+  pdl_launch(H3D_BOTH(k_tdma_level, T), all.ncta, 256, 0, st, bl, all.cta_start, nb, a, dst, offs);
   return cudaGetLastError();
 }
-template cudaError_t launch_tdma<double>(const TdmaPlan&, bool, const BlkLev*, CellTab, const double*, double*,
-                                         const double*, double*, cudaStream_t);
-template cudaError_t launch_tdma<float>(const TdmaPlan&, bool, const BlkLev*, CellTab, const float*, float*, const float*,
-                                        float*, cudaStream_t);
+template cudaError_t launch_tdma<double>(const TdmaPlan&, bool, const BlkLev*, const long long*, CellTab, const double*,
+                                         double*, const double*, double*, cudaStream_t);
+template cudaError_t launch_tdma<float>(const TdmaPlan&, bool, const BlkLev*, const long long*, CellTab, const float*,
+                                        float*, const float*, float*, cudaStream_t);
 
 }  // namespace h3d

@@ -22,7 +22,16 @@ W, P = 4, 5
     ((1, 1, 1), (96, 96, 4), [W] * 6),                # global: a diagonal's operands exceed shared memory
 ])
 def test_tdma_sweeps_bitexact(oracle_mod, h3d, nblk, n, bc):
-    blocks = h3d.topology.block_grid(nblk, n, bc, [1.0 / 32, 1.0 / 40, 1.0 / 24], 2)
+    _sweeps_bitexact(oracle_mod, h3d, h3d.topology.block_grid(nblk, n, bc, [1.0 / 32, 1.0 / 40, 1.0 / 24], 2))
+
+
+def test_tdma_sweeps_uneven_blocks_bitexact(oracle_mod, h3d):
+    """Blocks of different sizes in one launch: their scratch starts where the last one's ends."""
+    sizes = [(40, 8, 34), (32, 26, 18), (2, 2, 2), (6, 30, 44)]
+    _sweeps_bitexact(oracle_mod, h3d, h3d.topology.independent_blocks(sizes, (1.0 / 32, 1.0 / 40, 1.0 / 24), 2))
+
+
+def _sweeps_bitexact(oracle_mod, h3d, blocks):
     s = h3d.MultigridSolver(blocks, 2, mg_itrsch=2)
     orc = oracle_mod.Oracle(to_oracle_descs(oracle_mod, blocks), 2, 2, 2, 1)
     orc.coeff()
