@@ -561,9 +561,10 @@ __global__ void __launch_bounds__(1024) k_coarse_tail(const TailLevel* __restric
 // reciprocal come from a table by wall faces, so that an update divides by
 // multiply-adds (div_known); all tables are staged by one flat copy while the predecessor
 // finishes; a sweep fills the ghosts that the next one reads, the last one all of
-// them.  With 64-bit tables decoded through the block records and 512 threads a
-// launch took 67 us for 16 blocks of 16^3 .. 2^3 cells and 46 us for one of 16^3 and 8^3
-// cells in FP64; 61 and 32 us here.
+// them.  With 64-bit tables decoded through the block records a launch took 67 us for
+// 16 blocks of 16^3 .. 2^3 cells and 46 us for one of 16^3 and 8^3 cells in FP64; 58
+// (512 threads a CTA) and 34 us (1024) here.
+//
 // Sweeps of a visit from which its cells go to registers (the 32 of a converged
 // coarsest level; two or three sweeps do not repay the extra code).
 constexpr int kResidentSweeps = 8;

@@ -3435,10 +3435,6 @@ namespace {
 // one the reference's k, i, j loops compute, in its operand order.  Factor
 // and residual arrays are zero outside the interior (never written there),
 // as the reference's are.
-struct SipLU {
-  double *lb, *lw, *ls, *lpr, *un, *ue, *ut, *res;
-};
-
 // Calls f(x, y, z, i) for every interior cell of hyperplane x+y+z = d + 3,
 // spread over the CTA's threads.
 template <typename F>
@@ -3454,7 +3450,7 @@ __device__ __forceinline__ void sip_plane(const BlkLev& B, int d, F&& f) {
   }
 }
 
-__global__ void __launch_bounds__(512) k_sip_factor(const BlkLev* __restrict__ bls, SipLU lu) {
+__global__ void __launch_bounds__(512) k_sip_factor(const BlkLev* __restrict__ bls, SipArrays lu) {
   pdl_trigger();
   pdl_wait<false>();
   const BlkLev B = bls[blockIdx.x];
@@ -3484,7 +3480,7 @@ __global__ void __launch_bounds__(512) k_sip_factor(const BlkLev* __restrict__ b
 // One SIP sweep of every block (sipsol.for:144-179): residual, forward and
 // backward substitution, fi += correction; the block's sum |res| into
 // partials[4 * block] (the other three entries zero).
-__global__ void __launch_bounds__(512) k_sip_sweep(const BlkLev* __restrict__ bls, SipLU lu, double* __restrict__ fi_all,
+__global__ void __launch_bounds__(512) k_sip_sweep(const BlkLev* __restrict__ bls, SipArrays lu, double* __restrict__ fi_all,
                                                    const double* __restrict__ su_all, double* __restrict__ partials) {
   pdl_trigger();
   pdl_wait<false>();
@@ -3549,16 +3545,14 @@ __global__ void __launch_bounds__(256) k_gather1(const uint32_t* __restrict__ ds
 
 cudaError_t launch_sip_factor(const BlkLev* bl, int nb, SipArrays a, cudaStream_t st) {
   if (nb <= 0) return cudaSuccess;
-  SipLU lu{a.lb, a.lw, a.ls, a.lpr, a.un, a.ue, a.ut, a.res};
-  plain_launch(k_sip_factor, nb, 512, 0, st, bl, lu);
+  plain_launch(k_sip_factor, nb, 512, 0, st, bl, a);
   return cudaGetLastError();
 }
 
 cudaError_t launch_sip_sweep(const BlkLev* bl, int nb, SipArrays a, double* fi, const double* su, double* partials,
                              cudaStream_t st) {
   if (nb <= 0) return cudaSuccess;
-  SipLU lu{a.lb, a.lw, a.ls, a.lpr, a.un, a.ue, a.ut, a.res};
-  plain_launch(k_sip_sweep, nb, 512, 0, st, bl, lu, fi, su, partials);
+  plain_launch(k_sip_sweep, nb, 512, 0, st, bl, a, fi, su, partials);
   return cudaGetLastError();
 }
 

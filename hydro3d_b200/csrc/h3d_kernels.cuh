@@ -103,8 +103,9 @@ struct TailLevel {
   const BlkLev* cbl;
   const unsigned long long* cells;   // interior cells, red (x+y+z odd) first
   const unsigned long long* ghosts;  // ghost cells of the padded blocks
-  const uint32_t* fdst;              // sweep fill table, compact indices (cluster tail: own block)
-  const uint32_t* fsrc;              // (cluster tail: source rank << 24 | compact index in its block)
+  const uint32_t* fdst;              // sweep fill table, compact indices; cluster tail: the block's staged pairs of
+                                     // compact index and source (rank << 24 | compact index in its block)
+  const uint32_t* fsrc;              // its sources (single-CTA tail)
   const int* fstart;                 // cluster tail: fill entries of block b are fstart[b] .. fstart[b+1]-1,
   const int* flive;                  // the flive[b] first of them are ghosts that a sweep reads
   int nlive, any_live;               // cluster tail: this block's flive; some block has one

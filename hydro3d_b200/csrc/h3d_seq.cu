@@ -47,10 +47,6 @@ namespace {
 constexpr int kPhase = 8, kRing = 4 * kPhase, kAhead = 4;
 constexpr int kSipThreads = 512, kSipMaxCtas = 8, kSipMaxSmem = 200 * 1024;
 
-struct SipLU {
-  double *lb, *lw, *ls, *lpr, *un, *ue, *ut, *res;
-};
-
 // Position of interior cell (x, y, z) in the skewed arrays.
 struct SipSkew {
   long long off;
@@ -120,7 +116,7 @@ __device__ __forceinline__ void sip_clear(double* base, long long n) {
 
 // LU factors (sipsol.for:77-105).
 __global__ void __launch_bounds__(kSipThreads) k_sip_factor_c(const BlkLev* __restrict__ bls,
-                                                            const long long* __restrict__ offs, SipLU lu) {
+                                                            const long long* __restrict__ offs, SipArrays lu) {
   extern __shared__ double sm[];
   cg::cluster_group cl = cg::this_cluster();
   const int nr = (int)cl.num_blocks(), rank = (int)cl.block_rank();
@@ -196,7 +192,7 @@ __global__ void __launch_bounds__(kSipThreads) k_sip_factor_c(const BlkLev* __re
 // looped over and loaded at the point of use.
 template <bool ONE>
 __global__ void __launch_bounds__(kSipThreads) k_sip_subst(const BlkLev* __restrict__ bls,
-                                                           const long long* __restrict__ offs, SipLU lu) {
+                                                           const long long* __restrict__ offs, SipArrays lu) {
   extern __shared__ double sm[];
   cg::cluster_group cl = cg::this_cluster();
   const int nr = (int)cl.num_blocks(), rank = (int)cl.block_rank();
@@ -852,19 +848,17 @@ cudaError_t init_seq_attributes() {
 cudaError_t launch_sip_factor_c(const SipPlan& P, const BlkLev* bl, const long long* offs, int nb, SipArrays a,
                               cudaStream_t st) {
   if (nb <= 0) return cudaSuccess;
-  SipLU lu{a.lb, a.lw, a.ls, a.lpr, a.un, a.ue, a.ut, a.res};
-  return cluster_launch(k_sip_factor_c, nb, P.ctas, kSipThreads, P.smem_factor, st, bl, offs, lu);
+  return cluster_launch(k_sip_factor_c, nb, P.ctas, kSipThreads, P.smem_factor, st, bl, offs, a);
 }
 
 cudaError_t launch_sip_sweep_c(const SipPlan& P, const BlkLev* bl, const long long* offs, CellTab interior, SipArrays a,
                              double* fi, const double* su, double* partials, cudaStream_t st) {
   if (interior.nb <= 0) return cudaSuccess;
-  SipLU lu{a.lb, a.lw, a.ls, a.lpr, a.un, a.ue, a.ut, a.res};
   pdl_launch(KernelPair{k_sip_residual<false>, k_sip_residual<true>}, interior.ncta, 256, 0, st, bl, offs, interior.cta_start, interior.nb, fi, su, a.res,
              partials);
   const int nb = interior.nb;
-  cudaError_t e = P.one ? cluster_launch(k_sip_subst<true>, nb, P.ctas, kSipThreads, P.smem_subst, st, bl, offs, lu)
-                        : cluster_launch(k_sip_subst<false>, nb, P.ctas, kSipThreads, P.smem_subst, st, bl, offs, lu);
+  cudaError_t e = P.one ? cluster_launch(k_sip_subst<true>, nb, P.ctas, kSipThreads, P.smem_subst, st, bl, offs, a)
+                        : cluster_launch(k_sip_subst<false>, nb, P.ctas, kSipThreads, P.smem_subst, st, bl, offs, a);
   if (e != cudaSuccess) return e;
   pdl_launch(KernelPair{k_sip_correct<false>, k_sip_correct<true>}, interior.ncta, 256, 0, st, bl, offs, interior.cta_start, interior.nb, fi, a.res);
   return cudaGetLastError();

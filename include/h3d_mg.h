@@ -209,7 +209,7 @@ int h3d_mg_project(h3d_mg* h, double* const* p, double* const* u, double* const*
  * partners), stopping when sum |res| falls to 0.001 of the first sweep's or
  * changes by at most 0.00001 of it.  *nsweep receives the reference's
  * nsweep, *resab the last sum |res|.  The recurrences run as wavefronts
- * (hyperplanes x+y+z = const), one CTA per block.  Constant coefficients
+ * (hyperplanes x+y+z = const), a block by up to eight CTAs.  Constant coefficients
  * only (H3D_ERR_BAD_CONFIG for L_LSM handles). */
 int h3d_mg_sipsol(h3d_mg* h, int32_t nswp, int32_t* nsweep, double* resab);
 /* pressure_1sweep (press.for:382-519) on the resident fields, without the
