@@ -2157,12 +2157,12 @@ int build_tail(h3d_mg* h) {
 
 // The largest blocks of a level that joins a cluster tail of two levels or more.  A
 // block is one CTA's work there, and the whole chip's outside it.  us a cycle
-// with the level in and out: FP32 16^3, 4 blocks 89 and 91, 12 blocks 133 and
-// 139; 24 x 16 x 16, 4 blocks 130 and 130, 12 blocks 150 and 139; 20^3, 4 blocks 137 and
-// 130; FP64 20 x 16 x 16, 4 blocks 113 and 101.  One FP32 block alone: 24 x 16 x 16 80 and
-// 86, 20^3 88 and 93, 24 x 20 x 20 97 and 95.  (As the second level, without which nothing
-// is fused, any that fits: 24 x 20 x 18, 4 blocks: 150 and 224.)
-constexpr int kClusterJoin = 4096, kClusterJoinAlone = 8192;
+// with the level in and out: FP32 24 x 16 x 16, one block 80 and 86, 4 blocks 130 and
+// 130, 12 blocks 150 and 139; 20^3, one 88 and 93, 4 blocks 137 and 130; 24 x 20 x 20, one
+// 97 and 95, 4 blocks 147 and 134.  FP64 16^3, one 88 and 100, 12 blocks 113 and 113;
+// 20 x 16 x 16, 4 blocks 113 and 101.  (As the second level, without which nothing is
+// fused, any that fits: 24 x 20 x 18, 4 blocks: 150 and 224.)
+constexpr int kClusterJoin32 = 8000, kClusterJoin64 = 4096;
 
 // The fused coarse tail as one cluster of CTAs, CTA b holding block b of
 // every tail level: the deepest run of levels g..L (g >= 2, at least two
@@ -2343,7 +2343,7 @@ int build_cluster_tail(h3d_mg* h) {
     bool same = true;
     for (const auto& B : V.geom.bl) same = same && B.nx == B0.nx && B.ny == B0.ny && B.nz == B0.nz;
     if (!same || B0.nx + 1 > 255 || B0.ny + 1 > 255 || B0.nz + 1 > 255) break;
-    if (g0 < Lv && B0.nx * B0.ny * B0.nz > (nb == 1 && f32_level(h, g) ? kClusterJoinAlone : kClusterJoin)) break;
+    if (g0 < Lv && B0.nx * B0.ny * B0.nz > (f32_level(h, g) ? kClusterJoin32 : kClusterJoin64)) break;
     // arena with levels g..L (one block each) plus the ghost scratch of the fine levels
     std::vector<Lay> L2;
     int at = 0, scratch = 0;
