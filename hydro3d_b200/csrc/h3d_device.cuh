@@ -88,9 +88,10 @@ inline cudaError_t pdl_launch(void (*k)(KArgs...), dim3 grid, dim3 block, size_t
   return launch_kernel(k, pdl_early((long long)grid.x * grid.y * grid.z), grid, block, smem, st, args...);
 }
 
-// Never early, with pdl_wait<false>: the sweep and the restriction that stage planes by
-// plain loads between barriers (variable density, 88 x 88 x 104 cells: 291 us a cycle,
-// 345 early; 64^3 176, 199), and sequential kernels that run for long on few CTAs.
+// Never early, in the form without opaque pointers: the sweep and the restriction that
+// stage planes by plain loads between barriers, with variable density (88 x 88 x 104
+// cells: 291 us a cycle, 345 early; 64^3 176, 199) and on large levels, and sequential
+// kernels that run for long on few CTAs.
 template <typename... KArgs, typename... Args>
 inline cudaError_t plain_launch(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                                 Args... args) {
@@ -113,6 +114,12 @@ inline cudaError_t pdl_launch(KernelPair<KArgs...> k, dim3 grid, dim3 block, siz
                               Args... args) {
   const bool early = pdl_early((long long)grid.x * grid.y * grid.z);
   return launch_kernel(early ? k.early : k.plain, early, grid, block, smem, st, args...);
+}
+
+template <typename... KArgs>
+inline cudaError_t kernel_smem(KernelPair<KArgs...> k, int bytes) {
+  cudaError_t e = cudaFuncSetAttribute(k.plain, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  return e != cudaSuccess ? e : cudaFuncSetAttribute(k.early, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
 __device__ __forceinline__ int find_block(const int* __restrict__ start, int nb, int cta) {

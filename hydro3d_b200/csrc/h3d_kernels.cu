@@ -570,7 +570,7 @@ struct RowGs {
 // exactly one cell is red and one black, so neither colour phase diverges.
 // Shared memory holds four staged planes of rows y0-2 .. y0+TY+1; column c
 // holds x = c-1.  Same out-of-place contract and arithmetic as k_rbgs.
-template <typename T, int TPR, int CP, int TY, bool VAR, bool ZERO>
+template <typename T, int TPR, int CP, int TY, bool VAR, bool ZERO, bool EARLY>
 __global__ void __launch_bounds__(TPR*(TY + 2)) k_rbgs_rows(const BlkLev* __restrict__ bls,
                                                            const Tile* __restrict__ tiles, int zc,
                                                            const T* __restrict__ src, T* __restrict__ dst,
@@ -578,7 +578,7 @@ __global__ void __launch_bounds__(TPR*(TY + 2)) k_rbgs_rows(const BlkLev* __rest
                                                            const T* __restrict__ fy, const T* __restrict__ fz,
                                                            float om) {
   pdl_trigger();
-  pdl_wait<false>();
+  pdl_wait<EARLY>(src, rhs);
   constexpr int SP = 2 * CP * TPR + 4;
   constexpr int SR = TY + 4;
   constexpr int PL = SR * SP;
@@ -1680,10 +1680,10 @@ template <typename T, int TPR, int CP, int TY>
 static cudaError_t rows_attr() {
   const int sm = (int)rows_smem<T, TPR, CP, TY>();
   cudaError_t e;
-  if ((e = cudaFuncSetAttribute(k_rbgs_rows<T, TPR, CP, TY, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))) return e;
-  if ((e = cudaFuncSetAttribute(k_rbgs_rows<T, TPR, CP, TY, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))) return e;
-  if ((e = cudaFuncSetAttribute(k_rbgs_rows<T, TPR, CP, TY, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))) return e;
-  return cudaFuncSetAttribute(k_rbgs_rows<T, TPR, CP, TY, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+  if ((e = cudaFuncSetAttribute(k_rbgs_rows<T, TPR, CP, TY, true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))) return e;
+  if ((e = cudaFuncSetAttribute(k_rbgs_rows<T, TPR, CP, TY, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))) return e;
+  if ((e = kernel_smem(H3D_BOTH(k_rbgs_rows, T, TPR, CP, TY, false, true), sm))) return e;
+  return kernel_smem(H3D_BOTH(k_rbgs_rows, T, TPR, CP, TY, false, false), sm);
 }
 
 template <typename T, int TPR, int CP, int TY>
@@ -1694,13 +1694,17 @@ static cudaError_t rows_dispatch(bool var, bool zero, const BlkLev* bl, const Ti
   constexpr int NT = TPR * (TY + 2);
   constexpr size_t SM = rows_smem<T, TPR, CP, TY>();
   dim3 grid(ntiles), block(NT);
-  if (var) {
-    if (zero) plain_launch(k_rbgs_rows<T, TPR, CP, TY, true, true>, grid, block, SM, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
-    else plain_launch(k_rbgs_rows<T, TPR, CP, TY, true, false>, grid, block, SM, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
-  } else {
-    if (zero) plain_launch(k_rbgs_rows<T, TPR, CP, TY, false, true>, grid, block, SM, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
-    else plain_launch(k_rbgs_rows<T, TPR, CP, TY, false, false>, grid, block, SM, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
-  }
+  // small levels with constant coefficients start early (launched plain, the sweeps from
+  // a zero iterate cost 2-3 us more of a 160 us cycle on 12 blocks of 32 x 80 x 32)
+  const bool small = (long long)ntiles * TY * zc * (2 * CP * TPR) < 1 << 18;  // cells, at most
+  auto go = [&](auto both) {
+    if (small) pdl_launch(both, grid, block, SM, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
+    else plain_launch(both.plain, grid, block, SM, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
+  };
+  if (var && zero) plain_launch(k_rbgs_rows<T, TPR, CP, TY, true, true, false>, grid, block, SM, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
+  else if (var) plain_launch(k_rbgs_rows<T, TPR, CP, TY, true, false, false>, grid, block, SM, st, bl, tiles, zc, src, dst, rhs, fx, fy, fz, om);
+  else if (zero) go(H3D_BOTH(k_rbgs_rows, T, TPR, CP, TY, false, true));
+  else go(H3D_BOTH(k_rbgs_rows, T, TPR, CP, TY, false, false));
   return cudaGetLastError();
 }
 
